@@ -239,12 +239,6 @@ void mark(swr_context* c, int i, cudaStream_t s) {
   c->ev_used = k + 1;
 }
 
-int bits_for(uint32_t n) {
-  int b = 0;
-  while (b < 32 && (1ull << b) < (uint64_t)n) ++b;
-  return b;
-}
-
 bool grow_u32(uint32_t& cap, uint64_t need) {
   if (need <= cap) return true;
   uint64_t c = need + need / 4 + 1024;
@@ -312,7 +306,7 @@ int ensure_capacity(swr_context* c, uint32_t nverts_ptv, int S, uint32_t nsub, u
       d = c->dslice_done.ensure(slots * 4 + 16) && cudaMemset(c->dslice_done.p, 0, c->dslice_done.bytes) == cudaSuccess;
     c->dslice_ok = d;
   }
-  const size_t sw = sort_scratch_words(c->cap_pairs) + scan_scratch_words(c->cap_prims) + 64 + 2 * scan_scratch_words(ntiles * SWR_SEGS);
+  const size_t sw = scan_scratch_words(c->cap_prims) + 64 + 2 * scan_scratch_words(ntiles * SWR_SEGS);
   ok &= c->scratch.ensure(sw * 4);
   ok &= c->draws.ensure(sizeof(SwrDrawDesc));
   ok &= c->targets.ensure(sizeof(SwrTargetDesc));
@@ -366,6 +360,32 @@ bool geometry_front(swr_context* c, const VsOps* vs, const SwrDrawDesc* draws, i
   return true;
 }
 
+// Launches k_sort_big over the listed cells (ids in `in`, ordered into `out`), one warp per
+// cell with a bitmap of the segment's id range in shared memory, where that range fits in
+// kBigSortSmem (big_list); its last block also closes the draw.  The list buffer is [list
+// length, blocks done, cell ids...]; both words are zeroed when it is allocated and reset by
+// that last block.
+uint32_t* big_list(swr_context* c, uint32_t ncells, int seg_shift) {
+  const bool fits = ((size_t)1 << seg_shift) / 8 <= kBigSortSmem && c->big_cells.bytes >= (size_t)(ncells + 2) * 4;
+  return fits ? c->big_cells.as<uint32_t>() : nullptr;
+}
+
+void sort_big(swr_context* c, const uint32_t* cstart, uint32_t ncells, int seg_shift, const uint32_t* in,
+              uint32_t* out, uint32_t* big, cudaStream_t s) {
+  const size_t bm_bytes = ((size_t)1 << seg_shift) / 8;  // one warp's bitmap
+  const int warps = (int)std::min<size_t>(8, std::max<size_t>(1, kBigSortSmem / std::max<size_t>(bm_bytes, 1)));
+  swr::launch(k_sort_big, kBigSortWarps / warps, 32 * warps, bm_bytes * warps, s, c->status.as<uint32_t>(), cstart,
+              ncells, c->cap_pairs, seg_shift, in, out, big + 2, big);
+  c->launches += 1;
+}
+
+// Smallest shift that puts ids below `cap` into at most SWR_SEGS segments.
+int segment_shift(uint32_t cap) {
+  int shift = 0;
+  while (((uint64_t)(cap > 0 ? cap - 1 : 0) >> shift) >= SWR_SEGS) ++shift;
+  return shift;
+}
+
 // Setup, binning and tile raster for the primitives in c->tris (count on the device).
 // Binning: setup counts (tile, primitive segment) cells, a scan turns the counts into
 // offsets, k_fill_bins scatters primitive ids into their cells, k_sort_cells restores the
@@ -374,8 +394,7 @@ int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, i
                  uint32_t ntiles, cudaStream_t s, int ntargets, bool has_span) {
   uint32_t* st = c->status.as<uint32_t>();
   const uint32_t ncells = ntiles * SWR_SEGS;
-  int seg_shift = 0;
-  while (((uint64_t)(c->cap_prims > 0 ? c->cap_prims - 1 : 0) >> seg_shift) >= SWR_SEGS) ++seg_shift;
+  const int seg_shift = segment_shift(c->cap_prims);
   SetupArgs sa;
   memset(&sa, 0, sizeof(sa));
   sa.tris = c->tris.as<uint4>();
@@ -403,15 +422,6 @@ int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, i
   ps->fill_bins(st, c->cap_prims, c->recs.as<float>(), c->cell_count.as<uint32_t>(),
                 cstart, ncells, seg_shift, c->cap_pairs, c->draws.as<SwrDrawDesc>(), c->targets.as<SwrTargetDesc>(),
                 c->tile, c->keys0.as<uint32_t>(), st, s);
-  const uint32_t warps_per_block = 8;
-  // cells above 64 entries are sorted by k_sort_big, one warp per cell, with a bitmap of
-  // the segment's id range in shared memory, while that range fits in kBigSortSmem
-  const size_t bm_bytes = ((size_t)1 << seg_shift) / 8;  // one warp's bitmap
-  const int big_warps = (int)std::min<size_t>(8, std::max<size_t>(1, kBigSortSmem / std::max<size_t>(bm_bytes, 1)));
-  // (buffer: [list length, blocks done, cell ids...]; both words are zeroed when the buffer
-  // is allocated and reset by k_sort_big's last block, which also closes the draw)
-  const bool use_big = bm_bytes <= kBigSortSmem && c->big_cells.bytes >= (size_t)(ncells + 2) * 4;
-  uint32_t* big = use_big ? c->big_cells.as<uint32_t>() : nullptr;
   // heavy tiles listed by k_sort_cells: rasterized in runs of chunks (depth-min shaders,
   // tiles of more than slice_chunks raster chunks), or else as quadrant CTAs (16-px tiles,
   // shaders other than the overwrite ones; 8-px raster tiles split every tile)
@@ -422,14 +432,13 @@ int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, i
   const bool listed = dsl || quad_list;
   const uint32_t qcap = dsl ? slice_cap(ntiles) : quad_cap(ntiles);
   // (quad_count was zeroed by the draw's k_stage_copy)
-  swr::launch(k_sort_cells, (ntiles + warps_per_block - 1) / warps_per_block, 256, 0, s, st, cstart, ntiles, c->cap_pairs, c->keys0.as<uint32_t>(), c->vals0.as<uint32_t>(), use_big ? big + 2 : nullptr,
-      big, (uint32_t)SWR_RASTER_SORT,
-      listed ? c->quad_flag.as<uint8_t>() : nullptr, c->quad_tiles.as<uint32_t>(), c->quad_count.as<uint32_t>(), qcap,
-      dsl ? (uint32_t)(slice_chunks * ps->chunk) : kQuadMin);
-  if (use_big) {
-    swr::launch(k_sort_big, kBigSortWarps / big_warps, 32 * big_warps, bm_bytes * big_warps, s, st, cstart, ncells, c->cap_pairs, seg_shift, c->keys0.as<uint32_t>(), c->vals0.as<uint32_t>(), big + 2, big);
-    c->launches += 1;
-  }
+  uint32_t* big = big_list(c, ncells, seg_shift);
+  swr::launch(k_sort_cells, (ntiles + 7) / 8, 256, 0, s, st, cstart, ntiles, c->cap_pairs, c->keys0.as<uint32_t>(),
+              c->vals0.as<uint32_t>(), big ? big + 2 : nullptr, big, (uint32_t)SWR_RASTER_SORT,
+              listed ? c->quad_flag.as<uint8_t>() : nullptr, c->quad_tiles.as<uint32_t>(),
+              c->quad_count.as<uint32_t>(), qcap, dsl ? (uint32_t)(slice_chunks * ps->chunk) : kQuadMin);
+  if (big)
+    sort_big(c, cstart, ncells, seg_shift, c->keys0.as<uint32_t>(), c->vals0.as<uint32_t>(), big, s);
   mark(c, 4, s);
   RasterArgs ra;
   ra.status = st;
@@ -459,7 +468,7 @@ int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, i
   ps->raster(ra, ntiles, c->tile, s);
   if (ra.slices > 1) c->launches += 1;  // k_merge_slices
   mark(c, 5, s);
-  if (!use_big) {
+  if (!big) {
     swr::launch(k_close_draw, 1, 1, 0, s, st);
     c->launches += 1;
   }
@@ -467,10 +476,11 @@ int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, i
   return cuda_err(cudaGetLastError());
 }
 
-// Points and lines: per-primitive DDA setup, one fragment per step, stable sort by pixel,
-// per-pixel ordered shading.  Fragment buffers reuse the bin-pair queues.
-int lp_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, int vs_a, int vs_p,
-             const SwrTargetDesc& T, cudaStream_t s) {
+// Points and lines: per-primitive DDA setup, one fragment per step numbered in primitive
+// order, fragments binned by 16-px tile in the triangles' cells, one CTA per tile.  Fragment
+// buffers reuse the bin-pair queues.
+int lp_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, int vs_a, int vs_p, uint32_t ntiles,
+             int mode, uint32_t nsub, cudaStream_t s) {
   uint32_t* st = c->status.as<uint32_t>();
   SetupArgs sa;
   memset(&sa, 0, sizeof(sa));
@@ -488,51 +498,67 @@ int lp_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, int v
   sa.targets = c->targets.as<SwrTargetDesc>();
   sa.recs = c->recs.as<float>();
   sa.tile_count = c->tile_count.as<uint32_t>();
-  sa.tile = c->tile;
+  sa.tile = SWR_LP_TILE;
   ps->lp_setup(sa, s);
   mark(c, 3, s);
   uint32_t* scr = c->scratch.as<uint32_t>();
-  uint32_t* sort_scr = scr + scan_scratch_words(c->cap_prims) + 32;
   scan_exclusive(c->tile_count.as<uint32_t>(), c->pair_off.as<uint32_t>(), st + SWR_ST_PRIMS, c->cap_prims,
                  st + SWR_ST_PAIRS, scr, s);
-  const uint32_t invalid = (uint32_t)T.width * (uint32_t)T.height;
+  // segments over the fragments there can be: a point has one (its cells would be several times
+  // larger than needed over the whole queue), a line any number
+  const int seg_shift = segment_shift(mode == SWR_DRAW_POINT ? std::min(nsub, c->cap_pairs) : c->cap_pairs);
+  const uint32_t ncells = ntiles * SWR_SEGS;
   LpFragArgs fa;
   fa.status = st;
   fa.cap_prims = c->cap_prims;
   fa.recs = c->recs.as<float>();
+  fa.steps = c->tile_count.as<uint32_t>();
   fa.frag_off = c->pair_off.as<uint32_t>();
   fa.nfrags = st + SWR_ST_PAIRS;
   fa.cap_frags = c->cap_pairs;
   fa.draws = c->draws.as<SwrDrawDesc>();
   fa.targets = c->targets.as<SwrTargetDesc>();
   fa.keys = c->keys0.as<uint32_t>();
-  fa.vals = c->vals0.as<uint32_t>();
+  fa.prims = c->vals0.as<uint32_t>();
+  fa.cell_count = c->cell_count.as<uint32_t>();
+  fa.seg_shift = seg_shift;
   fa.status_w = st;
-  fa.invalid = invalid;
   ps->lp_frags(fa, s);
-  const int bits = bits_for(invalid + 1);
-  const int which = radix_sort_pairs(c->keys0.as<uint32_t>(), c->vals0.as<uint32_t>(), c->keys1.as<uint32_t>(),
-                                     c->vals1.as<uint32_t>(), st + SWR_ST_PAIRS, c->cap_pairs, bits, sort_scr, s);
+  uint32_t* cstart = c->cell_start.as<uint32_t>();
+  scan_exclusive(c->cell_count.as<uint32_t>(), cstart, nullptr, ncells, cstart + ncells, scr, s);
+  uint32_t* big = big_list(c, ncells, seg_shift);
+  const uint32_t want = (c->cap_pairs + 255) / 256;
+  swr::launch(k_lp_fill, want < 1216u ? (want ? want : 1u) : 1216u, 256, 0, s, st, st + SWR_ST_PAIRS, c->cap_pairs,
+              c->keys0.as<uint32_t>(), c->cell_count.as<uint32_t>(), cstart, ncells, seg_shift, c->keys1.as<uint32_t>(),
+              big ? big + 2 : nullptr, big);
+  if (big) {
+    sort_big(c, cstart, ncells, seg_shift, c->keys1.as<uint32_t>(), c->vals1.as<uint32_t>(), big, s);
+  } else {  // a segment beyond the bitmaps: every cell ordered by its tile's warp
+    swr::launch(k_sort_cells, (ntiles + 7) / 8, 256, 0, s, st, cstart, ntiles, c->cap_pairs, c->keys1.as<uint32_t>(),
+                c->vals1.as<uint32_t>(), nullptr, nullptr, 0u, nullptr, nullptr, nullptr, 0u, 0u);
+    c->launches += 1;
+  }
   mark(c, 4, s);
-  LpShadeArgs sh;
-  sh.status = st;
-  sh.cap_prims = c->cap_prims;
-  sh.recs = c->recs.as<float>();
-  sh.frag_off = c->pair_off.as<uint32_t>();
-  sh.nfrags = st + SWR_ST_PAIRS;
-  sh.cap_frags = c->cap_pairs;
-  sh.keys = which ? c->keys1.as<uint32_t>() : c->keys0.as<uint32_t>();
-  sh.vals = which ? c->vals1.as<uint32_t>() : c->vals0.as<uint32_t>();
-  sh.draws = c->draws.as<SwrDrawDesc>();
-  sh.targets = c->targets.as<SwrTargetDesc>();
-  sh.target_pixel_base = c->target_tile_base.as<uint32_t>();
-  sh.ntargets = 1;
-  sh.invalid = invalid;
-  sh.status_w = st;
-  ps->lp_shade(sh, s);
+  LpRasterArgs ra;
+  ra.status = st;
+  ra.recs = c->recs.as<float>();
+  ra.frag_off = c->pair_off.as<uint32_t>();
+  ra.keys = c->keys0.as<uint32_t>();
+  ra.prims = c->vals0.as<uint32_t>();
+  ra.cell_start = cstart;
+  ra.bin_raw = c->keys1.as<uint32_t>();
+  ra.bin = c->vals1.as<uint32_t>();
+  ra.draws = c->draws.as<SwrDrawDesc>();
+  ra.targets = c->targets.as<SwrTargetDesc>();
+  ra.ntiles = ntiles;
+  ra.status_w = st;
+  ps->lp_raster(ra, s);
   mark(c, 5, s);
-  swr::launch(k_close_draw, 1, 1, 0, s, st);
-  c->launches += 1 + 2 + 1 + 3 * ((bits + 7) / 8) + 1 + 1;
+  if (!big) {
+    swr::launch(k_close_draw, 1, 1, 0, s, st);
+    c->launches += 1;
+  }
+  c->launches += 1 + 2 + 1 + 2 + 1 + (ntiles ? 1 : 0);
   return cuda_err(cudaGetLastError());
 }
 
@@ -590,13 +616,14 @@ int end_single(swr_context* c, cudaStream_t s, int rc) {
   return rc;
 }
 
-SwrTargetDesc make_target(const swr_context* c) {
+SwrTargetDesc make_target(const swr_context* c, int mode) {
+  const int tile = mode == SWR_DRAW_TRIANGLE ? c->tile : SWR_LP_TILE;
   SwrTargetDesc T;
   memset(&T, 0, sizeof(T));
   T.width = c->u.width;
   T.height = c->u.height;
-  T.tiles_x = (T.width + c->tile - 1) / c->tile;
-  T.tiles_y = (T.height + c->tile - 1) / c->tile;
+  T.tiles_x = (T.width + tile - 1) / tile;
+  T.tiles_y = (T.height + tile - 1) / tile;
   T.tile_base = 0;
   T.first_draw = 0;
   return T;
@@ -844,7 +871,7 @@ int swr_draw_elements(swr_context* c, int mode, uint64_t count, const uint32_t* 
   if (nverts >= 0x7fffffffull) return SWR_EINVAL;
   const uint32_t nsub = (uint32_t)(count / per);
   const uint32_t nbatches = (nsub + SWR_BATCH_PRIMS - 1) / SWR_BATCH_PRIMS;
-  const SwrTargetDesc T = make_target(c);
+  const SwrTargetDesc T = make_target(c, mode);
   const uint32_t ntiles = (uint32_t)T.tiles_x * (uint32_t)T.tiles_y;
   int rc = ensure_capacity(c, (uint32_t)nverts, vs->S, nsub, nbatches, ntiles, ps->R > ps->lp_R ? ps->R : ps->lp_R, ps);
   if (rc) return rc;
@@ -897,7 +924,7 @@ int swr_draw_elements(swr_context* c, int mode, uint64_t count, const uint32_t* 
   }
   mark(c, 2, s);
   c->last_ntiles = ntiles;
-  if (mode != SWR_DRAW_TRIANGLE) return end_single(c, s, lp_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, T, s));
+  if (mode != SWR_DRAW_TRIANGLE) return end_single(c, s, lp_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, ntiles, mode, nsub, s));
   return end_single(c, s, raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, ntiles, s, 1,
                                        c->raster_mode != SWR_RASTER_BLOCK));
 }
@@ -914,7 +941,7 @@ int swr_draw_list(swr_context* c, int mode, const float* vertices, uint64_t nver
   if ((count && !indices) || (nverts && !vertices)) return SWR_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
   const uint32_t nsub = (uint32_t)(count / per);
-  const SwrTargetDesc T = make_target(c);
+  const SwrTargetDesc T = make_target(c, mode);
   const uint32_t ntiles = (uint32_t)T.tiles_x * (uint32_t)T.tiles_y;
   int rc = ensure_capacity(c, (uint32_t)nverts, ps->S, nsub, 1, ntiles, ps->R > ps->lp_R ? ps->R : ps->lp_R, ps);
   if (rc) return rc;
@@ -941,7 +968,7 @@ int swr_draw_list(swr_context* c, int mode, const float* vertices, uint64_t nver
   }
   mark(c, 2, s);
   c->last_ntiles = ntiles;
-  if (mode != SWR_DRAW_TRIANGLE) return end_single(c, s, lp_stage(c, ps, ps->S, 8, 8 + ps->A, ps->A, ps->P, T, s));
+  if (mode != SWR_DRAW_TRIANGLE) return end_single(c, s, lp_stage(c, ps, ps->S, 8, 8 + ps->A, ps->A, ps->P, ntiles, mode, nsub, s));
   return end_single(c, s, raster_stage(c, ps, ps->S, 8, 8 + ps->A, ps->A, ps->P, ntiles, s, 1,
                                        c->raster_mode != SWR_RASTER_BLOCK));
 }
@@ -996,7 +1023,6 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
       td.tiles_x = (u.width + c->tile - 1) / c->tile;
       td.tiles_y = (u.height + c->tile - 1) / c->tile;
       td.tile_base = (uint32_t)NT;
-      td.pixel_base = (uint32_t)PIX;
       td.first_draw = i;
       NT += (uint64_t)td.tiles_x * (uint64_t)td.tiles_y;
       PIX += (uint64_t)u.width * (uint64_t)u.height;

@@ -6,11 +6,19 @@
 //                                (endpoints replaced by lerps at t0 / t1), point rejection;
 //                                survivors keep submission order
 //   k_lp_setup                   per primitive: DDA step count and per-step increments
-//   k_lp_frags                   one thread per DDA step: the stepped vertex by exact fold,
-//                                the per-step scissor test, the pixel key
-//   (stable radix sort of fragments by pixel keeps primitive order, then step order,
-//    including a pixel hit twice by one line)
-//   k_lp_shade                   one thread per covered pixel applies its fragments in order
+//   k_lp_frags                   one fragment per DDA step, numbered in primitive order, then
+//                                step order: the stepped position by exact fold, the
+//                                per-step scissor test, the pixel; counts (tile, segment) cells
+//   k_lp_fill                    fragment numbers into their tile's bin (the triangles' cells:
+//                                a tile's fragments in SWR_SEGS runs of fragment numbers) and
+//                                a list of the cells above SWR_LP_CHUNK entries, which
+//                                k_sort_big orders; the tile's CTA orders the others
+//   k_lp_raster                  one CTA per 16 x 16 tile: each thread owns a pixel and applies
+//                                its fragments in order (a line may hit a pixel twice)
+//
+// Binning by tile took the place of a stable radix sort of all fragments by pixel (three
+// 8-bit passes of three kernels, then one thread per covered pixel searching each fragment's
+// primitive).  Sizes below: 1M points and 122,880 lines (0.5M fragments) at 1920x1080.
 #pragma once
 #include "swr_stages.cuh"
 
@@ -112,8 +120,8 @@ __global__ void __launch_bounds__(256) k_assemble_lp_count(AssembleArgs g) {
   const uint32_t p0 = (b - D.bbase) * SWR_BATCH_PRIMS;
   uint32_t sum = 0;
   for (int j = 0; j < 4; ++j) {
-    const uint32_t p = p0 + threadIdx.x * 4 + j;
-    if (p < D.nprims && p < p0 + SWR_BATCH_PRIMS) sum += assemble_lp_one<A, P>(g, D, p);
+    const uint32_t p = p0 + j * 256 + threadIdx.x;  // consecutive threads, consecutive primitives
+    if (p < D.nprims) sum += assemble_lp_one<A, P>(g, D, p);
   }
   uint32_t tot;
   swr_block_exscan(sum, tmp, &tot);
@@ -145,47 +153,68 @@ static __global__ void __launch_bounds__(256) k_assemble_lp_emit(AssembleArgs g)
   }
 }
 
-// Per primitive: start vertex and per-step increment (computeVertexStep, Rasterizer.h:210-222).
+// Words between the records of consecutive primitives: points have no step, so their records
+// end after the start vertex.
 template <class PS>
-__global__ void __launch_bounds__(256) k_lp_setup(SetupArgs g) {
+__device__ __forceinline__ int lp_stride(int draw_mode) {
+  return draw_mode == 0 ? 2 + LpRec<PS>::NV : LpRec<PS>::R;
+}
+
+constexpr int kLpSetupThreads = 128;
+
+// Per primitive: start vertex and per-step increment (computeVertexStep, Rasterizer.h:210-222).
+// Bound by memory: one or two gathered vertex records in, one record out.  Records are staged
+// in shared memory (odd stride: no bank conflicts) and written as contiguous words; one
+// thread storing its own 64-byte record word by word took 74 us for 1M points.
+template <class PS>
+__global__ void __launch_bounds__(kLpSetupThreads) k_lp_setup(SetupArgs g) {
   swr_pdl_entry();
   typedef LpRec<PS> RL;
+  constexpr int RS = RL::R | 1;
+  __shared__ float stage[kLpSetupThreads * RS];
   if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
   uint32_t np = g.status[SWR_ST_PRIMS];
   if (np > g.cap_prims) np = g.cap_prims;
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
-    const uint4 t = g.tris[p];
-    const SwrDrawDesc& D = g.draws[t.w];
-    const float* vp[2];
-    const uint32_t rr[2] = {t.x, t.y};
-    for (int k = 0; k < 2; ++k)
-      vp[k] = (rr[k] & SWR_CLIP_REF) ? g.clipv + (size_t)(rr[k] & ~SWR_CLIP_REF) * g.S : g.ptv + (size_t)rr[k] * g.S;
-    float a[RL::NV], s[RL::NV];
-    float b[RL::NV];
-    for (int k = 0; k < 2; ++k) {
-      float* o = k ? b : a;
-      o[0] = vp[k][4]; o[1] = vp[k][5]; o[2] = vp[k][6]; o[3] = vp[k][3];
-      for (int i = 0; i < RL::NA; ++i) o[4 + i] = i < g.vs_a ? vp[k][g.off_a + i] : 0.0f;
-      for (int i = 0; i < RL::NP; ++i) o[4 + RL::NA + i] = i < g.vs_p ? vp[k][g.off_p + i] : 0.0f;
+  const int mode = g.draws[0].draw_mode;  // points and lines are drawn one draw at a time
+  const uint32_t W = (uint32_t)lp_stride<PS>(mode);
+  // 16-byte aligned vertex records: words 0-3 clip position, 4-6 screen x, y, z, then avars and pvars
+  auto vertex = [&](uint32_t ref, float* o) {
+    const float* vp = (ref & SWR_CLIP_REF) ? g.clipv + (size_t)(ref & ~SWR_CLIP_REF) * g.S : g.ptv + (size_t)ref * g.S;
+    const float4 q = __ldg((const float4*)vp + 1);
+    o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = __ldg(vp + 3);
+    for (int i = 0; i < RL::NA; ++i) o[4 + i] = i < g.vs_a ? __ldg(vp + g.off_a + i) : 0.0f;
+    for (int i = 0; i < RL::NP; ++i) o[4 + RL::NA + i] = i < g.vs_p ? __ldg(vp + g.off_p + i) : 0.0f;
+  };
+  for (uint32_t p0 = blockIdx.x * kLpSetupThreads; p0 < np; p0 += gridDim.x * kLpSetupThreads) {
+    const uint32_t p = p0 + threadIdx.x;
+    if (p < np) {
+      const uint4 t = g.tris[p];
+      float a[RL::NV];
+      vertex(t.x, a);
+      float* rec = stage + threadIdx.x * RS;
+      int steps = 1;
+      if (mode == 1) {
+        float b[RL::NV];
+        vertex(t.y, b);
+        const int adx = abs(swr_trunc_int(b[0]) - swr_trunc_int(a[0]));
+        const int ady = abs(swr_trunc_int(b[1]) - swr_trunc_int(a[1]));
+        steps = adx > ady ? adx : ady;
+        const float fs = (float)steps;
+        for (int i = 0; i < RL::NV; ++i) rec[2 + RL::NV + i] = swr_div(swr_sub(b[i], a[i]), fs);
+      }
+      rec[0] = __int_as_float(steps);
+      rec[1] = __int_as_float((int)t.w);
+      for (int i = 0; i < RL::NV; ++i) rec[2 + i] = a[i];
+      g.tile_count[p] = (uint32_t)(steps > 0 ? steps : 0);
     }
-    int steps = 1;
-    if (D.draw_mode == 1) {
-      const int adx = abs(swr_trunc_int(b[0]) - swr_trunc_int(a[0]));
-      const int ady = abs(swr_trunc_int(b[1]) - swr_trunc_int(a[1]));
-      steps = adx > ady ? adx : ady;
-      const float fs = (float)steps;
-      for (int i = 0; i < RL::NV; ++i) s[i] = swr_div(swr_sub(b[i], a[i]), fs);
-    } else {
-      for (int i = 0; i < RL::NV; ++i) s[i] = 0.0f;
+    __syncthreads();
+    const uint32_t words = min((uint32_t)kLpSetupThreads, np - p0) * W;
+    float* dst = g.recs + (size_t)p0 * W;
+    for (uint32_t i = threadIdx.x; i < words; i += kLpSetupThreads) {
+      const uint32_t k = i / W;
+      dst[i] = stage[k * RS + (i - k * W)];
     }
-    float* rec = g.recs + (size_t)p * RL::R;
-    rec[0] = __int_as_float(steps);
-    rec[1] = __int_as_float((int)t.w);
-    for (int i = 0; i < RL::NV; ++i) {
-      rec[2 + i] = a[i];
-      rec[2 + RL::NV + i] = s[i];
-    }
-    g.tile_count[p] = (uint32_t)(steps > 0 ? steps : 0);
+    __syncthreads();
   }
 }
 
@@ -194,25 +223,34 @@ __global__ void __launch_bounds__(256) k_lp_setup(SetupArgs g) {
 template <class PS>
 __device__ __forceinline__ float lp_value(const float* rec, int i, int j) {
   typedef LpRec<PS> RL;
-  if ((i == 2 && !PS::InterpolateZ) || (i == 3 && !PS::InterpolateW)) return rec[2 + i];
+  if (j == 0 || (i == 2 && !PS::InterpolateZ) || (i == 3 && !PS::InterpolateW)) return rec[2 + i];
   return swr_fold(rec[2 + i], rec[2 + RL::NV + i], j);
 }
+
+#define SWR_LP_TILE 16                // tile edge of the point / line bins (one pixel per thread)
+#define SWR_LP_CHUNK 256              // fragments per raster chunk (one per thread)
+#define SWR_LP_INVALID 0xffffffffu    // key of a fragment that reaches no target pixel
 
 struct LpFragArgs {
   const uint32_t* status;
   uint32_t cap_prims;
   const float* recs;
-  const uint32_t* frag_off;   // exclusive scan of steps per primitive
+  const uint32_t* steps;      // per primitive: its fragments
+  const uint32_t* frag_off;   // their exclusive scan
   const uint32_t* nfrags;     // device total
   uint32_t cap_frags;
   const SwrDrawDesc* draws;
   const SwrTargetDesc* targets;
-  uint32_t* keys;
-  uint32_t* vals;
+  uint32_t* keys;             // per fragment: tile * 256 + pixel in the tile, or SWR_LP_INVALID
+  uint32_t* prims;            // per fragment: its primitive
+  uint32_t* cell_count;       // per (tile, segment): fragments
+  int seg_shift;              // segment = fragment number >> seg_shift
   uint32_t* status_w;
-  uint32_t invalid;           // key of fragments that reach no target pixel (sorts last)
 };
 
+// Fragments of the primitives, one warp per 32 consecutive primitives whose fragments are
+// spread over its lanes 32 at a time, so a long line does not hold up the warp and no
+// fragment has to search for its primitive.
 template <class PS>
 __global__ void __launch_bounds__(256) k_lp_frags(LpFragArgs g) {
   swr_pdl_entry();
@@ -228,100 +266,257 @@ __global__ void __launch_bounds__(256) k_lp_frags(LpFragArgs g) {
   }
   uint32_t np = g.status[SWR_ST_PRIMS];
   if (np > g.cap_prims) np = g.cap_prims;
-  for (uint32_t f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x) {
-    // primitive owning fragment f: last p with frag_off[p] <= f (primitives with zero
-    // steps share an offset with their successor, so take the last)
-    uint32_t lo = 0, hi = np - 1;
-    while (lo < hi) {
-      const uint32_t mid = (lo + hi + 1) >> 1;
-      if (g.frag_off[mid] <= f) lo = mid; else hi = mid - 1;
+  const SwrDrawDesc& D = g.draws[0];
+  const SwrTargetDesc& T = g.targets[D.target];
+  const uint32_t W = (uint32_t)lp_stride<PS>(D.draw_mode);
+  const float sx0 = (float)D.sc_minx, sx1 = (float)D.sc_maxx, sy0 = (float)D.sc_miny, sy1 = (float)D.sc_maxy;
+  const int width = T.width, height = T.height, tiles_x = T.tiles_x;
+  const int lane = threadIdx.x & 31;
+  // one fragment per lane (every lane of the warp calls it)
+  auto put = [&](bool on, uint32_t f, uint32_t prim, float x, float y) {
+    uint32_t key = SWR_LP_INVALID;
+    if (on) {
+      // Rasterizer::scissorTest on the stepped float position (Rasterizer.h:144-147)
+      if (x >= sx0 && x < sx1 && y >= sy0 && y < sy1) {
+        const int ix = swr_trunc_int(x), iy = swr_trunc_int(y);
+        if (ix >= 0 && iy >= 0 && ix < width && iy < height)
+          key = ((uint32_t)((iy / SWR_LP_TILE) * tiles_x + ix / SWR_LP_TILE) << 8) |
+                (uint32_t)((iy % SWR_LP_TILE) * SWR_LP_TILE + ix % SWR_LP_TILE);
+      }
+      g.keys[f] = key;
+      g.prims[f] = prim;
     }
-    const uint32_t p = lo;
-    const int j = (int)(f - g.frag_off[p]);
-    const float* rec = g.recs + (size_t)p * RL::R;
-    const SwrDrawDesc& D = g.draws[__float_as_int(rec[1])];
-    const SwrTargetDesc& T = g.targets[D.target];
-    const float x = lp_value<PS>(rec, 0, j), y = lp_value<PS>(rec, 1, j);
-    uint32_t key = g.invalid;
-    // Rasterizer::scissorTest on the stepped float position (Rasterizer.h:144-147)
-    if (x >= (float)D.sc_minx && x < (float)D.sc_maxx && y >= (float)D.sc_miny && y < (float)D.sc_maxy) {
-      const int ix = swr_trunc_int(x), iy = swr_trunc_int(y);
-      if (ix >= 0 && iy >= 0 && ix < T.width && iy < T.height)
-        key = T.pixel_base + (uint32_t)iy * (uint32_t)T.width + (uint32_t)ix;
+    const uint32_t cell = key != SWR_LP_INVALID ? (key >> 8) * SWR_SEGS + (f >> g.seg_shift) : SWR_LP_INVALID;
+    const uint32_t peers = __match_any_sync(0xffffffffu, cell);  // neighbours share cells
+    if (cell != SWR_LP_INVALID && lane == __ffs(peers) - 1) atomicAdd(&g.cell_count[cell], (uint32_t)__popc(peers));
+  };
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t p0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; p0 < np; p0 += stride) {
+    const uint32_t p = p0 + (uint32_t)lane;
+    uint32_t cnt = 0, off = 0;
+    float x = 0.0f, y = 0.0f, dx = 0.0f, dy = 0.0f;
+    if (p < np) {
+      cnt = g.steps[p];
+      off = g.frag_off[p];
+      const float* rec = g.recs + (size_t)p * W;
+      x = rec[2];
+      y = rec[3];
+      if (cnt > 1) {
+        dx = rec[2 + RL::NV];
+        dy = rec[3 + RL::NV];
+      }
     }
-    g.keys[f] = key;
-    g.vals[f] = f;
+    if (__reduce_max_sync(0xffffffffu, cnt) <= 1u) {  // points, lines of one step
+      put(cnt != 0, off, p, x, y);
+      continue;
+    }
+    uint32_t inc = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
+    for (uint32_t base = 0; base < total; base += 32) {
+      const uint32_t j = base + (uint32_t)lane;
+      int src = 0;  // owner: the number of lanes whose inclusive count is <= j
+#pragma unroll
+      for (int step = 16; step; step >>= 1) {
+        const uint32_t v = __shfl_sync(0xffffffffu, inc, src + step - 1);
+        if (v <= j) src += step;
+      }
+      src = src < 31 ? src : 31;
+      const uint32_t first = __shfl_sync(0xffffffffu, inc - cnt, src);
+      const uint32_t ooff = __shfl_sync(0xffffffffu, off, src);
+      const float ox = __shfl_sync(0xffffffffu, x, src), oy = __shfl_sync(0xffffffffu, y, src);
+      const float odx = __shfl_sync(0xffffffffu, dx, src), ody = __shfl_sync(0xffffffffu, dy, src);
+      const bool on = j < total;
+      const int k = on ? (int)(j - first) : 0;
+      put(on, ooff + (uint32_t)k, p0 + (uint32_t)src, swr_fold(ox, odx, k), swr_fold(oy, ody, k));
+    }
   }
 }
 
-struct LpShadeArgs {
+// Fragment numbers into their cells (arbitrary order inside a cell); takes every count of
+// k_lp_frags back, so the counters are zero again after the draw.  Lists the cells that do
+// not fit a raster chunk for k_sort_big (big_list holds every cell; null: none are listed).
+static __global__ void __launch_bounds__(256) k_lp_fill(const uint32_t* status, const uint32_t* nfrags,
+                                                        uint32_t cap_frags, const uint32_t* keys,
+                                                        uint32_t* cell_count, const uint32_t* cell_start,
+                                                        uint32_t ncells, int seg_shift, uint32_t* bin,
+                                                        uint32_t* big_list, uint32_t* big_count) {
+  swr_pdl_entry();
+  if (status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;  // (k_lp_frags counted nothing then)
+  const uint32_t nf = min(*nfrags, cap_frags);
+  const int lane = threadIdx.x & 31;
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t f0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; f0 < nf; f0 += stride) {
+    const uint32_t f = f0 + (uint32_t)lane;
+    const uint32_t key = f < nf ? keys[f] : SWR_LP_INVALID;
+    const uint32_t cell = key != SWR_LP_INVALID ? (key >> 8) * SWR_SEGS + (f >> seg_shift) : SWR_LP_INVALID;
+    const uint32_t peers = __match_any_sync(0xffffffffu, cell);
+    const int leader = __ffs(peers) - 1;
+    uint32_t pos = 0;
+    if (cell != SWR_LP_INVALID && lane == leader) {
+      const uint32_t n = (uint32_t)__popc(peers);
+      pos = cell_start[cell] + atomicSub(&cell_count[cell], n) - n;
+    }
+    pos = __shfl_sync(0xffffffffu, pos, leader);
+    if (cell != SWR_LP_INVALID) bin[pos + (uint32_t)__popc(peers & ((1u << lane) - 1u))] = f;
+  }
+  if (!big_list) return;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ncells; i += stride)
+    if (cell_start[i + 1] - cell_start[i] > SWR_LP_CHUNK) big_list[atomicAdd(big_count, 1u)] = i;
+}
+
+struct LpRasterArgs {
   const uint32_t* status;
-  uint32_t cap_prims;
   const float* recs;
   const uint32_t* frag_off;
-  const uint32_t* nfrags;
-  uint32_t cap_frags;
-  const uint32_t* keys;  // sorted
-  const uint32_t* vals;  // fragment ids in sorted order
+  const uint32_t* keys;        // per fragment (LpFragArgs)
+  const uint32_t* prims;
+  const uint32_t* cell_start;  // per (tile, segment) cell, plus the end
+  const uint32_t* bin_raw;     // fragment numbers, unordered inside a cell
+  const uint32_t* bin;         // ordered by k_sort_big, for cells of more than SWR_LP_CHUNK entries
   const SwrDrawDesc* draws;
   const SwrTargetDesc* targets;
-  const uint32_t* target_pixel_base;
-  int ntargets;
-  uint32_t invalid;
+  uint32_t ntiles;
   uint32_t* status_w;
 };
 
+// One CTA per 16 x 16 tile, one pixel per thread.  A chunk is as many whole cells of the
+// tile's bin as hold at most 256 fragments (a larger cell, ordered by k_sort_big, is a run of
+// chunks by itself): one fragment per thread is ranked inside its cell, interpolated, shaded
+// and marked under its rank in its pixel's set; then each thread applies its pixel's
+// fragments in increasing order (shaders with side effects of their own are evaluated there
+// instead, one drawPixel at a time).  Bound by the latency of the dependent gathers bin ->
+// primitive -> record.  Ordering the cells here instead of ahead (a warp ranking each cell of
+// 17 to 64 entries, a bitmap above) took the two sorts from 184 to 4 us on the points and
+// from 64 to 4 us on the lines.
 template <class PS>
-__global__ void __launch_bounds__(256) k_lp_shade(LpShadeArgs g) {
+__global__ void __launch_bounds__(256) k_lp_raster(LpRasterArgs g) {
   swr_pdl_entry();
   typedef LpRec<PS> RL;
+  typedef typename PS::Color Color;
+  constexpr bool kCompact = !SwrNoCompact<PS>::value;
+  constexpr int CH = SWR_LP_CHUNK, CW = CH / 32;
+  static_assert(CH == 256 && SWR_SEGS == 32, "one fragment per thread, one cell per lane");
+  __shared__ uint32_t sraw[CH];
+  __shared__ uint32_t scs[SWR_SEGS + 1];
+  __shared__ uint32_t smask[CW][256];  // per pixel: the chunk's fragments that hit it
+  __shared__ uint32_t sprim[CH];
+  __shared__ int sstep[kCompact ? 1 : CH];
+  __shared__ float sz[kCompact ? CH : 1];
+  __shared__ Color sc[kCompact ? CH : 1];
   __shared__ uint32_t sfr[32];
-  uint32_t frags = 0, passes = 0;
-  const bool ok = !(g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW);
-  const uint32_t nf = ok ? min(*g.nfrags, g.cap_frags) : 0u;
-  uint32_t np = g.status[SWR_ST_PRIMS];
-  if (np > g.cap_prims) np = g.cap_prims;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nf; i += gridDim.x * blockDim.x) {
-    const uint32_t key = g.keys[i];
-    if (key == g.invalid || (i > 0 && g.keys[i - 1] == key)) continue;
-    const int ti = g.ntargets > 1 ? swr_find_le(g.target_pixel_base, g.ntargets, key) : 0;
-    const SwrTargetDesc& T = g.targets[ti];
-    const SwrUniforms& U = g.draws[T.first_draw].u;
-    const uint32_t local = key - T.pixel_base;
-    const int x = (int)(local % (uint32_t)T.width), y = (int)(local / (uint32_t)T.width);
-    typename PS::State st;
-    PS::load(st, x, y, U);
-    for (uint32_t k = i; k < nf && g.keys[k] == key; ++k) {
-      const uint32_t f = g.vals[k];
-      uint32_t lo = 0, hi = np - 1;
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (g.frag_off[mid] <= f) lo = mid; else hi = mid - 1;
-      }
-      const float* rec = g.recs + (size_t)lo * RL::R;
-      const int j = (int)(f - g.frag_off[lo]);
-      // Rasterizer::pixelDataFromVertex (Rasterizer.h:161-173)
-      GpuPixel<PS> pd;
-      pd.x = x;
-      pd.y = y;
-      pd.eq = nullptr;  // points and lines carry no triangle equations
-      if (PS::InterpolateZ) pd.z = lp_value<PS>(rec, 2, j);
-      if (PS::InterpolateW) {
-        pd.w = lp_value<PS>(rec, 3, j);
-        pd.invw = swr_div(1.0f, pd.w);
-      }
-      for (int a = 0; a < RL::NA; ++a) pd.avar[a] = lp_value<PS>(rec, 4 + a, j);
-      for (int a = 0; a < RL::NP; ++a) pd.pvar[a] = lp_value<PS>(rec, 4 + RL::NA + a, j);
-      PS::drawPixel(pd, (int)lo, st, g.draws[__float_as_int(rec[1])].u);
-      frags++;
+  if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
+  const uint32_t tile = blockIdx.x;
+  if (tile >= g.ntiles) return;
+  const uint32_t* cells = g.cell_start + (size_t)tile * SWR_SEGS;
+  const uint32_t b = cells[0], e = cells[SWR_SEGS];
+  if (b == e) return;  // uniform per CTA
+  const SwrDrawDesc& D = g.draws[0];
+  const SwrTargetDesc& T = g.targets[D.target];
+  const SwrUniforms& U = D.u;
+  const int mode = D.draw_mode;
+  const uint32_t W = (uint32_t)lp_stride<PS>(mode);
+  const int tid = (int)threadIdx.x, lane = tid & 31;
+  const int x = (int)(tile % (uint32_t)T.tiles_x) * SWR_LP_TILE + tid % SWR_LP_TILE;
+  const int y = (int)(tile / (uint32_t)T.tiles_x) * SWR_LP_TILE + tid / SWR_LP_TILE;
+  const bool in = x < T.width && y < T.height;
+  typename PS::State st;
+  if (in) PS::load(st, x, y, U);
+  if (tid <= SWR_SEGS) scs[tid] = cells[tid] - b;
+  // Rasterizer::pixelDataFromVertex (Rasterizer.h:161-173) of step j of primitive `prim`
+  auto pixel = [&](uint32_t prim, int j, int fx, int fy, GpuPixel<PS>& pd) {
+    const float* rec = g.recs + (size_t)prim * W;
+    pd.x = fx;
+    pd.y = fy;
+    pd.eq = nullptr;  // points and lines carry no triangle equations
+    pd.z = 0.0f;
+    if (PS::InterpolateZ) pd.z = lp_value<PS>(rec, 2, j);
+    if (PS::InterpolateW) {
+      pd.w = lp_value<PS>(rec, 3, j);
+      pd.invw = swr_div(1.0f, pd.w);
     }
+    for (int a = 0; a < RL::NA; ++a) pd.avar[a] = lp_value<PS>(rec, 4 + a, j);
+    for (int a = 0; a < RL::NP; ++a) pd.pvar[a] = lp_value<PS>(rec, 4 + RL::NA + a, j);
+  };
+  uint32_t frags = 0, passes = 0;
+  __syncthreads();
+  const uint32_t total = e - b;
+  uint32_t c0 = 0;  // first entry of the chunk, relative to b
+  int cell = 0;     // the cell it lies in
+  while (c0 < total) {
+    // the chunk: cells [cell, last), or a run of an ordered cell that is larger than a chunk
+    const int last = __popc(__ballot_sync(0xffffffffu, scs[lane + 1] <= c0 + CH));
+    const bool whole = last > cell && scs[cell] == c0;
+    const uint32_t c1 = whole ? scs[last] : min(c0 + CH, scs[cell + 1]);
+    const int n = (int)(c1 - c0);
+    const int words = (n + 31) / 32;
+    __syncthreads();  // the previous chunk's shared state is no longer read
+    uint32_t f = 0;
+    if (tid < n) {
+      f = whole ? g.bin_raw[b + c0 + tid] : g.bin[b + c0 + tid];
+      sraw[tid] = f;
+    }
+    for (int w = 0; w < words; ++w) smask[w][tid] = 0u;
+    __syncthreads();
+    if (tid < n) {
+      const uint32_t prim = g.prims[f];
+      const int pix = (int)(g.keys[f] & 255u);
+      const int j = mode == 0 ? 0 : (int)(f - g.frag_off[prim]);
+      int k = tid;  // the fragment's place in the chunk
+      if (whole) {
+        const uint32_t at = c0 + (uint32_t)tid;
+        int lo = cell, hi = last - 1;  // its cell: the last one starting at or before it
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (scs[mid] <= at) lo = mid; else hi = mid - 1;
+        }
+        const int r0 = (int)(scs[lo] - c0), r1 = (int)(scs[lo + 1] - c0);
+        k = r0;
+        for (int i = r0; i < r1; ++i) k += sraw[i] < f;  // numbers are unique
+      }
+      sprim[k] = prim;
+      if constexpr (kCompact) {
+        GpuPixel<PS> pd;
+        pixel(prim, j, x - tid % SWR_LP_TILE + pix % SWR_LP_TILE, y - tid / SWR_LP_TILE + pix / SWR_LP_TILE, pd);
+        sz[k] = pd.z;
+        sc[k] = PS::shade(pd, U);
+      } else {
+        sstep[k] = j;
+      }
+      atomicOr(&smask[k >> 5][pix], 1u << (k & 31));
+    }
+    __syncthreads();
+    c0 = c1;
+    while (cell < SWR_SEGS && scs[cell + 1] <= c0) ++cell;
+    if (!in) continue;
+    for (int w = 0; w < words; ++w) {
+      uint32_t m = smask[w][tid];
+      while (m) {
+        const int k = w * 32 + __ffs(m) - 1;
+        m &= m - 1u;
+        frags++;
+        if constexpr (kCompact) {
+          PS::apply(st, sz[k], sc[k], (int)sprim[k]);
+        } else {
+          GpuPixel<PS> pd;
+          pixel(sprim[k], sstep[k], x, y, pd);
+          PS::drawPixel(pd, (int)sprim[k], st, U);
+        }
+      }
+    }
+  }
+  if (in && frags) {
     PS::store(st, x, y, U);
-    passes += st.writes;
+    passes = st.writes;
   }
   uint32_t tot, ptot;
   swr_block_exscan(frags, sfr, &tot);
   swr_block_exscan(passes, sfr, &ptot);
-  if (threadIdx.x == 0 && tot) {
+  if (tid == 0 && tot) {
     atomicAdd((unsigned long long*)&g.status_w[SWR_ST_SHADED_LO], (unsigned long long)tot);
     atomicAdd((unsigned long long*)&g.status_w[SWR_ST_PASSES_LO], (unsigned long long)ptot);
   }

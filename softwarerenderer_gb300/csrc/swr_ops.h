@@ -38,7 +38,7 @@ struct PsOps {
   int lp_R;  // point / line record words
   void (*lp_setup)(const SetupArgs& a, cudaStream_t s);
   void (*lp_frags)(const LpFragArgs& a, cudaStream_t s);
-  void (*lp_shade)(const LpShadeArgs& a, cudaStream_t s);
+  void (*lp_raster)(const LpRasterArgs& a, cudaStream_t s);
   int needs_eq;  // shade() reads the triangle equations: triangles only
   int overwrite;    // SwrOverwrite: large tiles may be rasterized in slices (RasterArgs.slices)
   int state_bytes;  // sizeof(PS::State), per pixel and slice of RasterArgs.slice_state
@@ -58,7 +58,7 @@ const PsOps* ps_ops(int id);
 // these headers in the caller's unit, so the library checks that both sides agree on the
 // layout of every structure that crosses between them.
 #define SWR_PROGRAM_MAGIC 0x50525753u  // "SWRP"
-#define SWR_PROGRAM_ABI 3u             // bumped with any change to VsOps, PsOps or their argument structs
+#define SWR_PROGRAM_ABI 4u             // bumped with any change to VsOps, PsOps or their argument structs
 #define SWR_PROGRAM_VERTEX 1u
 #define SWR_PROGRAM_PIXEL 2u
 
@@ -81,6 +81,6 @@ inline void swr_program_layout(uint32_t* s) {
   s[5] = (uint32_t)sizeof(swr::SetupArgs);
   s[6] = (uint32_t)sizeof(swr::RasterArgs);
   s[7] = (uint32_t)sizeof(swr::LpFragArgs);
-  s[8] = (uint32_t)sizeof(swr::LpShadeArgs);
+  s[8] = (uint32_t)sizeof(swr::LpRasterArgs);
   s[9] = (uint32_t)sizeof(SwrUniforms);
 }

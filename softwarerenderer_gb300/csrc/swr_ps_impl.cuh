@@ -69,7 +69,7 @@ void run_raster(const RasterArgs& a, uint32_t ntiles, int tile, cudaStream_t s) 
 
 template <class PS>
 void run_lp_setup(const SetupArgs& a, cudaStream_t s) {
-  swr::launch(k_lp_setup<PS>, kGrid, 256, 0, s, a);
+  swr::launch(k_lp_setup<PS>, kGrid, kLpSetupThreads, 0, s, a);
 }
 
 template <class PS>
@@ -78,8 +78,8 @@ void run_lp_frags(const LpFragArgs& a, cudaStream_t s) {
 }
 
 template <class PS>
-void run_lp_shade(const LpShadeArgs& a, cudaStream_t s) {
-  swr::launch(k_lp_shade<PS>, kGrid, 256, 0, s, a);
+void run_lp_raster(const LpRasterArgs& a, cudaStream_t s) {
+  if (a.ntiles) swr::launch(k_lp_raster<PS>, a.ntiles, 256, 0, s, a);
 }
 
 template <class PS>
@@ -97,7 +97,7 @@ PsOps make_ps() {
   o.lp_R = LpRec<PS>::R;
   o.lp_setup = &run_lp_setup<PS>;
   o.lp_frags = &run_lp_frags<PS>;
-  o.lp_shade = &run_lp_shade<PS>;
+  o.lp_raster = &run_lp_raster<PS>;
   o.needs_eq = SwrNeedsEquations<PS>::value;
   o.overwrite = SwrOverwrite<PS>::value;
   o.state_bytes = (int)sizeof(typename PS::State);
