@@ -89,6 +89,18 @@ __global__ void k_close_draw(uint32_t* st) {
   swr_close_status(st);
 }
 
+// swr_finish: the status words to pinned host memory, and zero again for the next draws, in
+// one launch and one wait (a copy, a wait, a memset and another wait before it: a synchronous
+// 12-triangle draw went 99.6 -> 86.7 us).
+__global__ void k_report_status(uint32_t* st, uint32_t* host) {
+  swr_pdl_entry();
+  const int i = (int)threadIdx.x;
+  if (i < kStatusWords) {
+    host[i] = st[i];
+    st[i] = 0u;
+  }
+}
+
 // Device bytes a context holds, and the cap swr_set_memory_limit puts on them (0: none).
 struct MemBudget {
   size_t used = 0;
@@ -1220,7 +1232,8 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
 int swr_finish(swr_context* c, void* stream, swr_stats* stats) {
   if (!c) return SWR_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
-  int rc = cuda_err(cudaMemcpyAsync(c->status_host, c->status.p, kStatusWords * 4, cudaMemcpyDeviceToHost, s));
+  swr::launch(k_report_status, 1, 32, 0, s, c->status.as<uint32_t>(), c->status_host);
+  int rc = cuda_err(cudaGetLastError());
   if (rc) return rc;
   if ((rc = cuda_err(cudaStreamSynchronize(s)))) return rc;
   const uint32_t* h = c->status_host;
@@ -1241,8 +1254,6 @@ int swr_finish(swr_context* c, void* stream, swr_stats* stats) {
     grow_u32(c->cap_prims, h[kStickyBase + SWR_ST_PRIMS]);
     grow_u32(c->cap_pairs, h[kStickyBase + SWR_ST_PAIRS]);
   }
-  cudaMemsetAsync(c->status.p, 0, kStatusWords * 4, s);
-  if ((rc = cuda_err(cudaStreamSynchronize(s)))) return rc;
   if (flags & SWR_F_ANY_OVERFLOW) return SWR_EOVERFLOW;
   if (flags & SWR_F_BARRIER_TIMEOUT) return SWR_ECUDA;
   if (flags & (SWR_F_BAD_INDEX | SWR_F_BAD_GRAD_INPUT)) return SWR_EINDEX;
