@@ -180,7 +180,8 @@ SWR_API int swr_set_tile_split(swr_context* ctx, int on);
  * the runs are merged in primitive order: colour, depth, winner and fragment counts are
  * those of the sequential draw.  Only the `passes` statistic differs: each run counts its
  * depth-test passes against the depth its run started from.  chunks = 0 turns it off, -1
- * (the default) takes the shader's own setting (the Lambert shader: 1; the others: off). */
+ * (the default) takes the shader's own setting (the Lambert shader: 1; the others: off; draws
+ * of at most 1,024 triangles are then never cut into runs). */
 SWR_API int swr_set_tile_slicing(swr_context* ctx, int chunks);
 /* Persistent geometry front end (no reference counterpart): triangle draws and batches run
  * vertex shading and triangle assembly as one cooperative launch whose CTAs stay resident

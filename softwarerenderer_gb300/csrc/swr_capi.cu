@@ -354,6 +354,29 @@ void fill_draw(const swr_context* c, SwrDrawDesc& D, int mode) {
   D.u = c->u;
 }
 
+AssembleArgs assemble_args(swr_context* c, int ndraws, uint32_t* draw_prim_base) {
+  AssembleArgs aa;
+  memset(&aa, 0, sizeof(aa));
+  aa.draws = c->draws.as<SwrDrawDesc>();
+  aa.ndraws = ndraws;
+  aa.draw_bbase = c->draw_bbase.as<uint32_t>();
+  aa.ptv = c->ptv.as<float>();
+  aa.clipv = c->clipv.as<float>();
+  aa.clip_table = c->clip_table.as<SwrClipEntry>();
+  aa.clip_slot = c->clip_slot.as<uint32_t>();
+  aa.tri_flags = c->tri_flags.as<uint8_t>();
+  aa.batch_counts = c->batch_counts.as<uint2>();
+  aa.batch_base = c->batch_base.as<uint32_t>();
+  aa.tris = c->tris.as<uint4>();
+  aa.lp_refs = c->lp_refs.as<uint2>();
+  aa.draw_prim_base = draw_prim_base;
+  aa.status = c->status.as<uint32_t>();
+  aa.cap_clip_slots = c->cap_clip_slots;
+  aa.cap_clip_verts = c->cap_clip_verts;
+  aa.cap_prims = c->cap_prims;
+  return aa;
+}
+
 // The persistent geometry front end (swr_set_persistent_geometry): vertex shading, assembly
 // count and emit as one cooperative launch.  False when it could not be launched; the
 // caller then launches the three kernels.
@@ -453,6 +476,7 @@ int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, i
     sort_big(c, cstart, ncells, seg_shift, c->keys0.as<uint32_t>(), c->vals0.as<uint32_t>(), big, s);
   mark(c, 4, s);
   RasterArgs ra;
+  memset(&ra, 0, sizeof(ra));
   ra.status = st;
   ra.tile_start = cstart;
   ra.tile_stride = SWR_SEGS;
@@ -485,6 +509,69 @@ int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, i
     c->launches += 1;
   }
   c->launches += 1 + 2 + 1 + 1 + (ntiles ? 1 : 0);
+  return cuda_err(cudaGetLastError());
+}
+
+// Draws of few triangles skip the bins: setup leaves each primitive's tile box in one word and
+// every tile's CTA picks its own primitives from all of them.  The general path's scan, fill
+// and sort kernels (5 launches of about 4 us each) and, for large triangles, the setup's and
+// the fill's walks over every tile of a primitive (14 us each for the textured cube) cost more
+// than reading 1,024 boxes per tile does.  Options that act on bins keep the general path.
+constexpr uint32_t kSmallTris = 1024;   // submitted triangles (one batch)
+constexpr uint32_t kSmallVerts = 4096;  // vertices one CTA shades (k_front)
+
+bool small_draw(const swr_context* c, uint64_t nsub, const SwrTargetDesc& T) {
+  return nsub > 0 && nsub <= kSmallTris && c->tile == 16 && c->quad_mode == 0 && c->dslice_chunks < 0 &&
+         !c->fixed_pairs && T.tiles_x <= 255 && T.tiles_y <= 255;
+}
+
+// ... and their vertex shading and assembly run as one CTA (k_front) in one launch.
+bool small_front(const swr_context* c, uint64_t nsub, uint64_t nverts, const SwrTargetDesc& T) {
+  return small_draw(c, nsub, T) && nverts <= kSmallVerts && !c->persistent_geometry;
+}
+
+int small_raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, int vs_a, int vs_p, uint32_t nsub,
+                       uint32_t ntiles, cudaStream_t s, bool has_span) {
+  uint32_t* st = c->status.as<uint32_t>();
+  SetupArgs sa;
+  memset(&sa, 0, sizeof(sa));
+  sa.tris = c->tris.as<uint4>();
+  sa.status = st;
+  sa.cap_prims = c->cap_prims;
+  sa.ptv = c->ptv.as<float>();
+  sa.clipv = c->clipv.as<float>();
+  sa.S = S;
+  sa.off_a = off_a;
+  sa.off_p = off_p;
+  sa.vs_a = vs_a;
+  sa.vs_p = vs_p;
+  sa.draws = c->draws.as<SwrDrawDesc>();
+  sa.targets = c->targets.as<SwrTargetDesc>();
+  sa.recs = c->recs.as<float>();
+  sa.tile = 16;
+  sa.boxes = c->tile_count.as<uint32_t>();
+  sa.status_w = st;
+  sa.grid = (nsub + kSetupThreads - 1) / kSetupThreads;
+  ps->setup(sa, s);
+  mark(c, 3, s);
+  mark(c, 4, s);
+  RasterArgs ra;
+  memset(&ra, 0, sizeof(ra));
+  ra.status = st;
+  ra.recs = c->recs.as<float>();
+  ra.draws = c->draws.as<SwrDrawDesc>();
+  ra.targets = c->targets.as<SwrTargetDesc>();
+  ra.ntargets = 1;
+  ra.draw_prim_base = c->use_draw_pbase ? c->draw_pbase.as<uint32_t>() : nullptr;
+  ra.status_w = st;
+  ra.ntiles = ntiles;
+  ra.has_span = has_span ? 1 : 0;
+  ra.slices = 1;
+  ra.boxes = c->tile_count.as<uint32_t>();
+  ra.cap_prims = c->cap_prims;
+  ps->raster(ra, ntiles, 16, s);
+  mark(c, 5, s);
+  c->launches += 1 + (ntiles ? 1 : 0);
   return cuda_err(cudaGetLastError());
 }
 
@@ -893,32 +980,36 @@ int swr_draw_elements(swr_context* c, int mode, uint64_t count, const uint32_t* 
   D.nidx = (uint32_t)count;
   D.nverts = (uint32_t)nverts;
   D.nprims = nsub;
-  if ((rc = upload_single(c, D, T, s))) return rc;
   uint32_t* st = c->status.as<uint32_t>();
+  if (mode == SWR_DRAW_TRIANGLE && small_front(c, nsub, nverts, T)) {
+    FrontArgs fa;
+    memset(&fa, 0, sizeof(fa));
+    fa.draw = D;
+    fa.target = T;
+    fa.draws = c->draws.as<SwrDrawDesc>();
+    fa.targets = c->targets.as<SwrTargetDesc>();
+    fa.nverts = (uint32_t)nverts;
+    fa.nhb = 2 * nbatches;
+    fa.ptv = c->ptv.as<float>();
+    fa.aa = assemble_args(c, 1, nullptr);
+    mark(c, 0, s);
+    vs->front(fa, s);
+    c->launches += 1;
+    mark(c, 1, s);
+    mark(c, 2, s);
+    c->use_draw_pbase = false;
+    c->last_ntiles = ntiles;
+    return small_raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, nsub, ntiles, s,
+                              c->raster_mode != SWR_RASTER_BLOCK);
+  }
+  if ((rc = upload_single(c, D, T, s))) return rc;
   mark(c, 0, s);
   // triangles with the persistent geometry front end: vertex shading and assembly in one launch
   const bool geo = mode == SWR_DRAW_TRIANGLE && c->persistent_geometry && nbatches;
   if (!geo) vs->vertex(c->draws.as<SwrDrawDesc>(), 1, c->draw_vbase.as<uint32_t>(), (uint32_t)nverts, c->ptv.as<float>(), s);
   mark(c, 1, s);
   c->launches += (nverts ? 1 : 0) + (nbatches ? 2 : 0) + (mode == SWR_DRAW_TRIANGLE ? 0 : 1);
-  AssembleArgs aa;
-  aa.draws = c->draws.as<SwrDrawDesc>();
-  aa.ndraws = 1;
-  aa.draw_bbase = c->draw_bbase.as<uint32_t>();
-  aa.ptv = c->ptv.as<float>();
-  aa.clipv = c->clipv.as<float>();
-  aa.clip_table = c->clip_table.as<SwrClipEntry>();
-  aa.clip_slot = c->clip_slot.as<uint32_t>();
-  aa.tri_flags = c->tri_flags.as<uint8_t>();
-  aa.batch_counts = c->batch_counts.as<uint2>();
-  aa.batch_base = c->batch_base.as<uint32_t>();
-  aa.tris = c->tris.as<uint4>();
-  aa.lp_refs = c->lp_refs.as<uint2>();
-  aa.draw_prim_base = nullptr;  // a single draw numbers its primitives from 0
-  aa.status = st;
-  aa.cap_clip_slots = c->cap_clip_slots;
-  aa.cap_clip_verts = c->cap_clip_verts;
-  aa.cap_prims = c->cap_prims;
+  const AssembleArgs aa = assemble_args(c, 1, nullptr);  // a single draw numbers its primitives from 0
   c->use_draw_pbase = false;
   if (mode == SWR_DRAW_TRIANGLE) {
     if (!(geo && geometry_front(c, vs, c->draws.as<SwrDrawDesc>(), 1, c->draw_vbase.as<uint32_t>(),
@@ -980,6 +1071,11 @@ int swr_draw_list(swr_context* c, int mode, const float* vertices, uint64_t nver
   }
   mark(c, 2, s);
   c->last_ntiles = ntiles;
+  if (mode == SWR_DRAW_TRIANGLE && small_draw(c, nsub, T)) {
+    c->use_draw_pbase = false;
+    return end_single(c, s, small_raster_stage(c, ps, ps->S, 8, 8 + ps->A, ps->A, ps->P, nsub, ntiles, s,
+                                               c->raster_mode != SWR_RASTER_BLOCK));
+  }
   if (mode != SWR_DRAW_TRIANGLE) return end_single(c, s, lp_stage(c, ps, ps->S, 8, 8 + ps->A, ps->A, ps->P, ntiles, mode, nsub, s));
   return end_single(c, s, raster_stage(c, ps, ps->S, 8, 8 + ps->A, ps->A, ps->P, ntiles, s, 1,
                                        c->raster_mode != SWR_RASTER_BLOCK));
@@ -1130,6 +1226,8 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
   mix((uint64_t)(uintptr_t)vs); mix((uint64_t)(uintptr_t)ps);  // the programs (their kernels)
   mix((uint64_t)c->quad_mode);
   mix((uint64_t)c->persistent_geometry);
+  const bool small = n == 1 && small_front(c, P, V, T[0]);
+  mix((uint64_t)small);
   mix((uint64_t)vs->S); mix((uint64_t)ps->R); mix((uint64_t)c->tile); mix((uint64_t)n);
   mix(c->cap_prims); mix(c->cap_pairs); mix(c->cap_clip_slots); mix(c->cap_clip_verts);
   const void* bufs[] = {c->ptv.p, c->clipv.p, c->clip_table.p, c->clip_slot.p, c->tri_flags.p, c->batch_counts.p,
@@ -1175,39 +1273,36 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
   q = q ? q : cuda_err(cudaGetLastError());
   uint32_t* st = c->status.as<uint32_t>();
   mark(c, 0, s);
-  const bool geo = c->persistent_geometry && B;
-  if (!geo) vs->vertex(c->draws.as<SwrDrawDesc>(), n, c->draw_vbase.as<uint32_t>(), (uint32_t)V, c->ptv.as<float>(), s);
-  mark(c, 1, s);
-  AssembleArgs aa;
-  memset(&aa, 0, sizeof(aa));
-  aa.draws = c->draws.as<SwrDrawDesc>();
-  aa.ndraws = n;
-  aa.draw_bbase = c->draw_bbase.as<uint32_t>();
-  aa.ptv = c->ptv.as<float>();
-  aa.clipv = c->clipv.as<float>();
-  aa.clip_table = c->clip_table.as<SwrClipEntry>();
-  aa.clip_slot = c->clip_slot.as<uint32_t>();
-  aa.tri_flags = c->tri_flags.as<uint8_t>();
-  aa.batch_counts = c->batch_counts.as<uint2>();
-  aa.batch_base = c->batch_base.as<uint32_t>();
-  aa.tris = c->tris.as<uint4>();
-  aa.lp_refs = c->lp_refs.as<uint2>();
-  aa.draw_prim_base = c->draw_pbase.as<uint32_t>();
-  aa.status = st;
-  aa.cap_clip_slots = c->cap_clip_slots;
-  aa.cap_clip_verts = c->cap_clip_verts;
-  aa.cap_prims = c->cap_prims;
+  const AssembleArgs aa = assemble_args(c, n, c->draw_pbase.as<uint32_t>());
   c->use_draw_pbase = true;
-  if (!(geo && geometry_front(c, vs, c->draws.as<SwrDrawDesc>(), n, c->draw_vbase.as<uint32_t>(), (uint32_t)V, aa,
-                              (uint32_t)B, s))) {
-    if (geo) vs->vertex(c->draws.as<SwrDrawDesc>(), n, c->draw_vbase.as<uint32_t>(), (uint32_t)V, c->ptv.as<float>(), s);
-    vs->assemble_count(aa, (uint32_t)B, s);
-    vs->assemble_emit(aa, (uint32_t)B, s);
+  if (small) {
+    FrontArgs fa;
+    memset(&fa, 0, sizeof(fa));
+    fa.staged = 1;
+    fa.nverts = (uint32_t)V;
+    fa.nhb = 2 * (uint32_t)B;
+    fa.ptv = c->ptv.as<float>();
+    fa.aa = aa;
+    vs->front(fa, s);
+    c->launches += 1;
+    mark(c, 1, s);
+    mark(c, 2, s);
+    rc = small_raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, (uint32_t)P, (uint32_t)NT, s, any_span);
+  } else {
+    const bool geo = c->persistent_geometry && B;
+    if (!geo) vs->vertex(c->draws.as<SwrDrawDesc>(), n, c->draw_vbase.as<uint32_t>(), (uint32_t)V, c->ptv.as<float>(), s);
+    mark(c, 1, s);
+    if (!(geo && geometry_front(c, vs, c->draws.as<SwrDrawDesc>(), n, c->draw_vbase.as<uint32_t>(), (uint32_t)V, aa,
+                                (uint32_t)B, s))) {
+      if (geo) vs->vertex(c->draws.as<SwrDrawDesc>(), n, c->draw_vbase.as<uint32_t>(), (uint32_t)V, c->ptv.as<float>(), s);
+      vs->assemble_count(aa, (uint32_t)B, s);
+      vs->assemble_emit(aa, (uint32_t)B, s);
+    }
+    mark(c, 2, s);
+    c->launches += (V ? 1 : 0) + (B ? 2 : 0);
+    if (!q) q = cuda_err(cudaGetLastError());
+    rc = raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, (uint32_t)NT, s, ntg, any_span);
   }
-  mark(c, 2, s);
-  c->launches += (V ? 1 : 0) + (B ? 2 : 0);
-  if (!q) q = cuda_err(cudaGetLastError());
-  rc = raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, (uint32_t)NT, s, ntg, any_span);
   if (q) rc = q;
   c->use_draw_pbase = false;
   if (c->graph_mode) {

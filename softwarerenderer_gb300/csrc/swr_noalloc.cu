@@ -283,6 +283,8 @@ extern "C" int swr_draw_triangle_list_noalloc(const struct SwrUniforms* u, int p
   ra.dslice = 0;  // no heavy-tile runs: they need the runs' State buffer
   ra.dslice_state = nullptr;
   ra.dslice_done = nullptr;
+  ra.boxes = nullptr;
+  ra.cap_prims = kMaxTris;
   ps->raster(ra, ntiles, kTile, s);
   if (cudaGetLastError() != cudaSuccess) return SWR_ECUDA;  // a launch failed: the status words are stale
   uint32_t h[16];

@@ -20,6 +20,7 @@ struct VsOps {
   // bar: two zeroed words of device memory.  Returns a CUDA error (nothing queued on failure).
   cudaError_t (*geometry)(const SwrDrawDesc* draws, int ndraws, const uint32_t* draw_vbase, uint32_t nverts,
                           float* ptv, const AssembleArgs& a, uint32_t nbatches, uint32_t* bar, cudaStream_t s);
+  void (*front)(const FrontArgs& a, cudaStream_t s);  // small draws: all of the above in one CTA
 };
 
 struct PsOps {
@@ -82,5 +83,5 @@ inline void swr_program_layout(uint32_t* s) {
   s[6] = (uint32_t)sizeof(swr::RasterArgs);
   s[7] = (uint32_t)sizeof(swr::LpFragArgs);
   s[8] = (uint32_t)sizeof(swr::LpRasterArgs);
-  s[9] = (uint32_t)sizeof(SwrUniforms);
+  s[9] = (uint32_t)sizeof(SwrUniforms) + ((uint32_t)sizeof(swr::FrontArgs) << 16);
 }

@@ -19,7 +19,7 @@ void run_direct(const float* rv, uint32_t n, float* ptv, cudaStream_t s) {
 
 template <class PS>
 void run_setup(const SetupArgs& a, cudaStream_t s) {
-  swr::launch(k_setup<PS>, kGrid, kSetupThreads, 0, s, a);
+  swr::launch(k_setup<PS>, a.grid ? a.grid : (uint32_t)kGrid, kSetupThreads, 0, s, a);
 }
 
 template <class PS>
@@ -44,6 +44,11 @@ template <class PS>
 void run_raster(const RasterArgs& a, uint32_t ntiles, int tile, cudaStream_t s) {
   constexpr int kChunk = SwrRasterChunk<PS>::value;  // primitives staged in shared memory per bin chunk
   if (!ntiles) return;
+  if (a.boxes) {  // a small draw: 16-px tiles, one CTA each
+    if (a.has_span) swr::launch(k_raster<PS, 16, kChunk, true, true>, ntiles, 256, 0, s, a);
+    else swr::launch(k_raster<PS, 16, kChunk, false, true>, ntiles, 256, 0, s, a);
+    return;
+  }
   // one CTA per tile, or per (tile, slice) for sliced overwrite shaders; Block-only
   // submissions run the instantiation without the Span-mode passes
   const bool sliced = SwrOverwrite<PS>::value && a.slices > 1;

@@ -205,7 +205,9 @@ struct AssembleArgs {
   uint32_t cap_clip_slots, cap_clip_verts, cap_prims;
 };
 
-template <int A, int P>
+// SAME: the vertex records were written by this launch (k_geometry, k_front), so they are read
+// with plain loads; k_assemble_count reads them through the read-only path.
+template <int A, int P, bool SAME>
 __device__ void assemble_one(const AssembleArgs& g, const SwrDrawDesc& D, uint32_t p, uint32_t i0,
                              uint32_t i1, uint32_t i2, uint32_t& in_kept, uint32_t& ex_kept) {
   typedef VLayout<A, P> L;
@@ -221,7 +223,7 @@ __device__ void assemble_one(const AssembleArgs& g, const SwrDrawDesc& D, uint32
   // words 4-7 of a record (16-byte aligned: S is a multiple of 4): screen x, y, z, outcode
   float4 q[3];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) q[k] = __ldg((const float4*)(v[k] + 4));
+  for (int k = 0; k < 3; ++k) q[k] = SAME ? *(const float4*)(v[k] + 4) : __ldg((const float4*)(v[k] + 4));
   const int m = __float_as_int(q[0].w) | __float_as_int(q[1].w) | __float_as_int(q[2].w);
   if (m == 0) {
     const int c = cull_decision(D.cull, q[0].x, q[0].y, q[1].x, q[1].y, q[2].x, q[2].y);
@@ -313,7 +315,7 @@ __device__ __forceinline__ uint32_t batch_count(const SwrDrawDesc& D, uint32_t p
 
 // One CTA per half batch (512 triangles, one per thread): clip / cull and count the
 // survivors: batch_counts[h] = (kept input slots, kept extra fan triangles).
-template <int A, int P>
+template <int A, int P, bool SAME>
 __device__ __forceinline__ void assemble_count_block(const AssembleArgs& g, uint32_t hb) {
   __shared__ uint32_t tmp[64];
   const uint32_t b = hb >> 1;
@@ -325,7 +327,7 @@ __device__ __forceinline__ void assemble_count_block(const AssembleArgs& g, uint
   const uint32_t q = threadIdx.x;
   if (q < n) {
     const uint32_t* ix = D.indices + (size_t)3 * (p0 + q);
-    assemble_one<A, P>(g, D, p0 + q, __ldg(ix), __ldg(ix + 1), __ldg(ix + 2), ik, ek);
+    assemble_one<A, P, SAME>(g, D, p0 + q, __ldg(ix), __ldg(ix + 1), __ldg(ix + 2), ik, ek);
   }
   uint32_t tin, tex;
   swr_block_sum2(ik, ek, tmp, tin, tex);
@@ -335,7 +337,7 @@ __device__ __forceinline__ void assemble_count_block(const AssembleArgs& g, uint
 template <int A, int P>
 __global__ void __launch_bounds__(SWR_HALF) k_assemble_count(AssembleArgs g) {
   swr_pdl_entry();
-  assemble_count_block<A, P>(g, blockIdx.x);
+  assemble_count_block<A, P, false>(g, blockIdx.x);
 }
 
 // Exclusive scan of per-batch totals -> batch bases; primitive total into the status word.
@@ -365,7 +367,10 @@ template <int A, int P>
 __device__ __forceinline__ void assemble_emit_block(const AssembleArgs& g, uint32_t hb, uint32_t nhb) {
   __shared__ uint32_t tmp[64];
   __shared__ uint32_t tmps[32];
-  if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
+  // An overflow of the count stage (flags set by atomics, of this launch in k_geometry and
+  // k_front).  One that another block of this stage found does not count: the last block
+  // still has to publish the primitive count the queue must grow to.
+  if (__ldcg(&g.status[SWR_ST_FLAGS]) & (SWR_F_ANY_OVERFLOW & ~SWR_F_PRIM_OVERFLOW)) return;
   const uint32_t b = hb >> 1, half = hb & 1;
   const int d = g.ndraws > 1 ? swr_find_le(g.draw_bbase, g.ndraws, b) : 0;
   const SwrDrawDesc& D = g.draws[d];
@@ -498,12 +503,53 @@ __global__ void __launch_bounds__(SWR_HALF) k_geometry(const SwrDrawDesc* draws,
   vertex_stage<VS>(draws, ndraws, draw_vbase, nverts, ptv);
   if (!swr_grid_sync(bar, g.status)) return;
   for (uint32_t hb = blockIdx.x; hb < nhb; hb += gridDim.x) {
-    assemble_count_block<VS::AVarCount, VS::PVarCount>(g, hb);
+    assemble_count_block<VS::AVarCount, VS::PVarCount, true>(g, hb);
     __syncthreads();  // the block's shared scratch is reused by its next half batch
   }
   if (!swr_grid_sync(bar, g.status)) return;
   for (uint32_t hb = blockIdx.x; hb < nhb; hb += gridDim.x) {
     assemble_emit_block<VS::AVarCount, VS::PVarCount>(g, hb, nhb);
+    __syncthreads();
+  }
+}
+
+// The geometry front end of a small draw: descriptor upload, vertex shading and assembly in
+// one CTA.  Such a draw is bound by its chain of dependent launches (4 us each, whatever they
+// do); see small_draw in swr_capi.cu for the sizes.
+struct FrontArgs {
+  SwrDrawDesc draw;      // the draw's descriptors, by value; with `staged` they are in place already
+  SwrTargetDesc target;
+  int staged;
+  SwrDrawDesc* draws;
+  SwrTargetDesc* targets;
+  uint32_t nverts, nhb;  // vertices, half batches
+  float* ptv;
+  AssembleArgs aa;
+};
+
+template <class VS>
+__global__ void __launch_bounds__(SWR_HALF) k_front(const __grid_constant__ FrontArgs a) {
+  swr_pdl_entry();
+  AssembleArgs g = a.aa;
+  if (!a.staged) {
+    g.draws = &a.draw;
+    const uint32_t* s = (const uint32_t*)&a.draw;
+    uint32_t* d = (uint32_t*)a.draws;
+    for (uint32_t i = threadIdx.x; i < sizeof(SwrDrawDesc) / 4; i += SWR_HALF) d[i] = s[i];
+    s = (const uint32_t*)&a.target;
+    d = (uint32_t*)a.targets;
+    for (uint32_t i = threadIdx.x; i < sizeof(SwrTargetDesc) / 4; i += SWR_HALF) d[i] = s[i];
+    if (threadIdx.x < 5) g.status[SWR_ST_CLIP_SLOTS + threadIdx.x] = 0u;  // the draw's working counters
+    __threadfence();  // the counters are zero before this CTA's atomics reach them
+  }
+  vertex_stage<VS>(g.draws, 1, nullptr, a.nverts, a.ptv);
+  __syncthreads();
+  for (uint32_t hb = 0; hb < a.nhb; ++hb) {
+    assemble_count_block<VS::AVarCount, VS::PVarCount, true>(g, hb);
+    __syncthreads();  // the block's shared scratch is reused by its next half batch
+  }
+  for (uint32_t hb = 0; hb < a.nhb; ++hb) {
+    assemble_emit_block<VS::AVarCount, VS::PVarCount>(g, hb, a.nhb);
     __syncthreads();
   }
 }
@@ -607,7 +653,17 @@ struct SetupArgs {
   int tile;  // tile edge in pixels
   uint32_t* cell_count;  // per (tile, primitive segment): bin entries (counted with atomics)
   int seg_shift;         // primitive segment = primitive index >> seg_shift (< SWR_SEGS)
+  uint32_t* boxes;       // small draws (null otherwise): per primitive its packed tile box instead of
+                         // cell counts (SWR_NO_BOX: no tile); bin entries are summed in the status
+  uint32_t* status_w;    // small draws: the status words
+  uint32_t grid;         // CTAs to launch (0: the default)
 };
+
+// A tile box packed in a word, 8 bits each: x0 | y0 << 8 | x1 << 16 | y1 << 24 (inclusive).
+#define SWR_NO_BOX 0x000000ffu  // x0 = 255 > x1 = 0: hits no tile
+__device__ __forceinline__ bool swr_box_hit(uint32_t box, uint32_t tx, uint32_t ty) {
+  return tx >= (box & 255u) && tx <= ((box >> 16) & 255u) && ty >= ((box >> 8) & 255u) && ty <= (box >> 24);
+}
 
 struct SpanHalf {
   float ox, oy, is1, is2;
@@ -635,6 +691,8 @@ __global__ void __launch_bounds__(kSetupThreads) k_setup(SetupArgs g) {
   // 32 different banks (a stride of R = 40 words put 32 threads in 4 banks)
   constexpr int RS = RL::R + 1;
   __shared__ float stage[kSetupThreads * RS];
+  // a small draw's queue requests are final here (bin entries are no queue of it)
+  if (g.boxes && blockIdx.x == 0 && threadIdx.x == 0) swr_close_status(g.status_w);
   if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
   uint32_t np = g.status[SWR_ST_PRIMS];
   if (np > g.cap_prims) np = g.cap_prims;
@@ -673,7 +731,7 @@ __global__ void __launch_bounds__(kSetupThreads) k_setup(SetupArgs g) {
       }
     }
     float* rec = stage + threadIdx.x * RS;
-    uint32_t tiles = 0;
+    uint32_t tiles = 0, box = SWR_NO_BOX;
     // TriangleEquations: e0 = (v1, v2), e1 = (v2, v0), e2 = (v0, v1)
     const Edge e0 = make_edge(x[1], y[1], x[2], y[2]);
     const Edge e1 = make_edge(x[2], y[2], x[0], y[0]);
@@ -811,6 +869,7 @@ __global__ void __launch_bounds__(kSetupThreads) k_setup(SetupArgs g) {
       if (bx0 <= bx1 && by0 <= by1) {
         const int tx0 = bx0 / g.tile, tx1 = bx1 / g.tile, ty0 = by0 / g.tile, ty1 = by1 / g.tile;
         tiles = (uint32_t)((tx1 - tx0 + 1) * (ty1 - ty0 + 1));
+        box = (uint32_t)tx0 | (uint32_t)ty0 << 8 | (uint32_t)tx1 << 16 | (uint32_t)ty1 << 24;
         if (g.cell_count) {
           const uint32_t seg = p >> g.seg_shift;
           for (int ty = ty0; ty <= ty1; ++ty)
@@ -825,7 +884,12 @@ __global__ void __launch_bounds__(kSetupThreads) k_setup(SetupArgs g) {
     rec[1] = __int_as_float((int)t.w);
     rec[2] = __int_as_float(bx0); rec[3] = __int_as_float(by0);
     rec[4] = __int_as_float(bx1); rec[5] = __int_as_float(by1);
-    g.tile_count[p] = flags ? tiles : 0u;
+    if (g.boxes) {
+      g.boxes[p] = box;
+      if (tiles) atomicAdd(&g.status_w[SWR_ST_PAIRS], tiles);
+    } else {
+      g.tile_count[p] = flags ? tiles : 0u;
+    }
   }
   __syncthreads();
   const uint32_t cnt = min((uint32_t)kSetupThreads, np - p0);
@@ -1197,6 +1261,10 @@ struct RasterArgs {
   // (swr_depth_merge) and stores.  CTAs [0, SWR_DSLICES quad_cap) take the listed tiles'
   // slices; CTA SWR_DSLICES quad_cap + t takes tile t unless it is listed.
   int dslice;
+  // Small draws (k_raster<..., true>): no bins; every CTA picks its tile's primitives, in order,
+  // from the packed tile boxes of all `status[SWR_ST_PRIMS]` primitives.
+  const uint32_t* boxes;
+  uint32_t cap_prims;
   void* dslice_state;      // [slot][slice][TILE * TILE] PS::State
   uint32_t* dslice_done;   // per slot: the slices finished (zero between draws)
 };
@@ -1364,10 +1432,11 @@ __device__ __forceinline__ float build_z(const float* eq, bool blockmode, float 
 //      every covering fragment to the pixel's register-resident State: compacted fragments
 //      through apply(), others by rebuilding the interpolants in place (z first: a failing
 //      depth test needs nothing else) and drawPixel().
+// DIRECT: the raster of a small draw, which has no bins (RasterArgs.boxes).
 // A heavy tile of a depth-min shader (RasterArgs.dslice) is run by up to SWR_DSLICES CTAs,
 // each over its own run of whole chunks from the draw's starting State; the last run to
 // finish merges the runs' States in bin order (swr_depth_merge) and stores.
-template <class PS, int TILE, int CH, bool SPAN>
+template <class PS, int TILE, int CH, bool SPAN, bool DIRECT = false>
 __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRasterOccupancy<PS>::value)
     k_raster(RasterArgs g) {
   swr_pdl_entry();
@@ -1428,13 +1497,13 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
   // rasterized from an empty State into slice_state and merged in order by k_merge_slices;
   // smaller tiles are rasterized whole by slice 0.
   uint32_t tile = blockIdx.x, slice = 0;
-  if (SwrOverwrite<PS>::value && g.slices > 1) {
+  if (SwrOverwrite<PS>::value && !DIRECT && g.slices > 1) {
     tile = blockIdx.x / (uint32_t)g.slices;
     slice = blockIdx.x - tile * (uint32_t)g.slices;
   }
   int quad = -1;  // the 8 x 8 quadrant (block) this CTA rasterizes alone, -1: the whole tile
   int dslot = -1;  // sliced heavy tile: its list slot (slice = its run)
-  if constexpr (SwrDepthMin<PS>::value) {
+  if constexpr (SwrDepthMin<PS>::value && !DIRECT) {
     if (g.dslice) {
       const uint32_t nq = SWR_DSLICES * g.quad_cap;
       if (blockIdx.x < nq) {
@@ -1449,7 +1518,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
       }
     }
   }
-  if constexpr (TILE == 16 && !SwrOverwrite<PS>::value) {
+  if constexpr (TILE == 16 && !SwrOverwrite<PS>::value && !DIRECT) {
     if (g.dslice) {
     } else if (g.quad_all) {
       tile = blockIdx.x >> 2;
@@ -1468,9 +1537,13 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
     }
   }
   if (tile >= g.ntiles) return;
-  uint32_t b = g.tile_start[(size_t)tile * g.tile_stride], e = g.tile_start[(size_t)(tile + 1) * g.tile_stride];
+  uint32_t b = 0, e = 0;
+  if constexpr (!DIRECT) {
+    b = g.tile_start[(size_t)tile * g.tile_stride];
+    e = g.tile_start[(size_t)(tile + 1) * g.tile_stride];
+  }
   bool sliced = false;
-  if constexpr (SwrOverwrite<PS>::value) {
+  if constexpr (SwrOverwrite<PS>::value && !DIRECT) {
     if (g.slices > 1) {
       if (e - b <= (uint32_t)SWR_RASTER_SORT) {
         if (slice) return;
@@ -1484,6 +1557,35 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
       }
     }
   }
+  // Small draws: the tile's primitives out of the next windows of 256 boxes, in order, until
+  // more than 256 are found (e = their count; ssorted holds SWR_RASTER_SORT) or none is left.
+  uint32_t scan_pos = 0, scan_np = 0;
+  auto gather = [&]() {
+    const uint32_t tx = tile % (uint32_t)g.targets[0].tiles_x, ty = tile / (uint32_t)g.targets[0].tiles_x;
+    e = 0;
+    while (scan_pos < scan_np && e <= SWR_RASTER_SORT - 256) {
+      const uint32_t i = scan_pos + threadIdx.x;
+      const bool hit = i < scan_np && swr_box_hit(g.boxes[i], tx, ty);
+      const uint32_t bal = __ballot_sync(0xffffffffu, hit);
+      __syncthreads();  // the previous window's counts (or the last chunk's ids) are no longer read
+      if (lane == 0) scs[warp] = (uint32_t)__popc(bal);
+      __syncthreads();
+      uint32_t at = e, all = 0;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        const uint32_t c = scs[w];
+        if (w < warp) at += c;
+        all += c;
+      }
+      if (hit) ssorted[at + (uint32_t)__popc(bal & ((1u << lane) - 1u))] = i;
+      e += all;
+      scan_pos += 256;
+    }
+  };
+  if constexpr (DIRECT) {
+    scan_np = min(g.status[SWR_ST_PRIMS], g.cap_prims);
+    gather();
+  }
   if (b == e && !sliced) return;  // uniform per CTA
   // the chunks this CTA rasterizes: the whole bin, or a sliced heavy tile's run
   uint32_t cb = b, ce = e;
@@ -1495,7 +1597,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
     cb = b + (uint32_t)((uint64_t)nch * slice / (uint32_t)nsl) * CH;
     ce = min(e, b + (uint32_t)((uint64_t)nch * (slice + 1) / (uint32_t)nsl) * CH);
   }
-  const int ti = g.ntargets > 1 ? swr_find_le(g.target_tile_base, g.ntargets, tile) : 0;
+  const int ti = !DIRECT && g.ntargets > 1 ? swr_find_le(g.target_tile_base, g.ntargets, tile) : 0;
   const SwrTargetDesc& T = g.targets[ti];
   const SwrUniforms& U = g.draws[T.first_draw].u;
   const uint32_t lt = tile - T.tile_base;
@@ -1519,8 +1621,8 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
   // A tile of at most SWR_RASTER_SORT entries orders its own bin: the cells (increasing id
   // segments) are contiguous, so an id's position is its cell's start plus the number of
   // smaller ids in that cell.  The raw ids are staged in the record area (used only later).
-  const bool self_sort = g.bin_raw && !sliced && e - b <= (uint32_t)SWR_RASTER_SORT;
-  if (self_sort) {
+  const bool self_sort = DIRECT || (g.bin_raw && !sliced && e - b <= (uint32_t)SWR_RASTER_SORT);
+  if (!DIRECT && self_sort) {
     uint32_t* sraw = (uint32_t*)srec4;
     const uint32_t ntot = e - b;
     if (threadIdx.x <= SWR_SEGS) scs[threadIdx.x] = g.tile_start[(size_t)tile * SWR_SEGS + threadIdx.x] - b;
@@ -1538,6 +1640,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
       ssorted[pos < ntot ? pos : 0] = v;
     }
   }
+  while (true) {  // once; small draws: per gathered run of the tile's primitives
   for (uint32_t c0 = cb; c0 < ce; c0 += CH) {
     const int n = (int)min((uint32_t)CH, ce - c0);
     __syncthreads();  // the previous chunk's shared state is no longer read; ssorted is complete
@@ -2036,7 +2139,12 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
       }
     }
   }
-  if constexpr (SwrDepthMin<PS>::value) {
+  if constexpr (!DIRECT) break;
+  gather();
+  if (e == 0) break;
+  ce = e;
+  }
+  if constexpr (SwrDepthMin<PS>::value && !DIRECT) {
     if (dslot >= 0) {
       // this run's States, then the last run to finish merges the tile's runs in bin order
       // (each thread owns the same pixels in every run's CTA)

@@ -66,6 +66,11 @@ cudaError_t run_geometry(const SwrDrawDesc* draws, int ndraws, const uint32_t* d
 }
 
 template <class VS>
+void run_front(const FrontArgs& a, cudaStream_t s) {
+  swr::launch(k_front<VS>, 1, SWR_HALF, 0, s, a);
+}
+
+template <class VS>
 VsOps make_vs() {
   VsOps o;
   o.attribs = VS::AttribCount;
@@ -80,6 +85,7 @@ VsOps make_vs() {
   o.assemble_lp_count = &run_lp_count<VS>;
   o.assemble_lp_emit = &run_lp_emit;
   o.geometry = &run_geometry<VS>;
+  o.front = &run_front<VS>;
   return o;
 }
 
