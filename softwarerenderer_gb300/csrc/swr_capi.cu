@@ -174,8 +174,8 @@ struct swr_context {
   bool persistent_geometry = false;  // swr_set_persistent_geometry
   bool geo_stall = false;             // swr_test_stall_geometry_barrier
   swr::Buffer geo_bar;                // its grid barrier's two words
-  swr::Buffer slice_state;  // overwrite shaders: per (tile, slice, pixel) State of sliced tiles
-  int slices = 1;           // slices the buffer holds for the current tile count
+  swr::Buffer over_best, over_done;  // overwrite shaders: sliced tiles' winners, slices finished
+  int slices = 1;                    // CTAs per sliced tile (1: the buffers could not be had)
   // depth-min shaders: heavy tiles rasterized in SWR_DSLICES runs (swr_set_tile_slicing)
   swr::Buffer dslice_state, dslice_done;
   int dslice_chunks = -1;  // tiles of more than this many raster chunks (-1: the shader's default)
@@ -221,7 +221,7 @@ struct swr_context {
                           &clip_table, &clip_slot, &tri_flags, &batch_counts, &batch_base, &tris, &recs,
                           &tile_count, &pair_off, &keys0, &vals0, &keys1, &vals1, &tile_start, &scratch,
                           &status, &direct_keep, &direct_pos, &lp_refs, &cell_count, &cell_start, &draw_pbase,
-                          &big_cells, &slice_state, &quad_flag, &quad_tiles, &quad_count, &geo_bar,
+                          &big_cells, &over_best, &over_done, &quad_flag, &quad_tiles, &quad_count, &geo_bar,
                           &dslice_state, &dslice_done};
     for (swr::Buffer* b : all) b->budget = &budget;
   }
@@ -259,9 +259,15 @@ bool grow_u32(uint32_t& cap, uint64_t need) {
   return true;
 }
 
+// Grows a buffer that must hold zeros between draws: zeroed on the draw's stream, ahead of it.
+bool zeroed(Buffer& b, size_t bytes, cudaStream_t s) {
+  if (bytes <= b.bytes) return true;
+  return b.ensure(bytes) && cudaMemsetAsync(b.p, 0, b.bytes, s) == cudaSuccess;
+}
+
 // Allocates every queue a draw with the given host-known sizes needs.
 int ensure_capacity(swr_context* c, uint32_t nverts_ptv, int S, uint32_t nsub, uint32_t nbatches,
-                    uint32_t ntiles, int R, const PsOps* ps) {
+                    uint32_t ntiles, int R, const PsOps* ps, cudaStream_t s) {
   if (!c->fixed_prims) grow_u32(c->cap_prims, (uint64_t)nsub + 1024);
   grow_u32(c->cap_clip_slots, (uint64_t)nsub / 16 + 1024);
   grow_u32(c->cap_clip_verts, (uint64_t)c->cap_clip_slots * 4);
@@ -284,39 +290,29 @@ int ensure_capacity(swr_context* c, uint32_t nverts_ptv, int S, uint32_t nsub, u
   ok &= c->keys1.ensure((size_t)c->cap_pairs * 4 + 16);
   ok &= c->vals1.ensure((size_t)c->cap_pairs * 4 + 16);
   ok &= c->tile_start.ensure((size_t)(ntiles + 1) * 4 + 16);
-  if (c->cell_count.bytes < (size_t)ntiles * SWR_SEGS * 4 + 16) {
-    // the per-cell counters start at zero and every draw leaves them at zero (k_fill_bins)
-    ok &= c->cell_count.ensure((size_t)ntiles * SWR_SEGS * 4 + 16);
-    ok &= c->cell_count.p && cudaMemset(c->cell_count.p, 0, c->cell_count.bytes) == cudaSuccess;
-  }
+  // the per-cell counters start at zero and every draw leaves them at zero (k_fill_bins)
+  ok &= zeroed(c->cell_count, (size_t)ntiles * SWR_SEGS * 4 + 16, s);
   ok &= c->cell_start.ensure(((size_t)ntiles * SWR_SEGS + 1) * 4 + 16);
   ok &= c->quad_flag.ensure((size_t)ntiles + 16);
   ok &= c->quad_tiles.ensure((size_t)quad_cap(ntiles) * 4 + 16);
   ok &= c->quad_count.ensure(16);
   ok &= c->geo_bar.ensure(16);
-  if (c->big_cells.bytes < ((size_t)ntiles * SWR_SEGS + 2) * 4) {
-    ok &= c->big_cells.ensure(((size_t)ntiles * SWR_SEGS + 2) * 4 + 16);
-    // the list length and completion counter start at zero (k_sort_big resets them)
-    ok &= c->big_cells.p && cudaMemset(c->big_cells.p, 0, 8) == cudaSuccess;
-  }
-  // Overwrite shaders: tiles of many layers are rasterized in up to SWR_SLICES_MAX slices
-  // (the buffer is kept under 512 MiB by using fewer slices on large targets).
+  // (the list length and completion counter start at zero; k_sort_big resets them)
+  ok &= zeroed(c->big_cells, ((size_t)ntiles * SWR_SEGS + 2) * 4 + 16, s);
+  // Overwrite shaders: a sliced tile's winners and finished slices (optional; both start at
+  // zero, and the last slice of a tile leaves them at zero)
   c->slices = 1;
   if (ps && ps->overwrite) {
-    const size_t per_slice = (size_t)ntiles * c->tile * c->tile * (size_t)ps->state_bytes;
-    int k = SWR_SLICES_MAX;
-    while (k > 1 && per_slice * (size_t)k > ((size_t)512 << 20)) --k;
-    if (k > 1 && c->slice_state.ensure(per_slice * (size_t)k)) c->slices = k;
+    const size_t px = (size_t)ntiles * c->tile * c->tile * 4;
+    if (zeroed(c->over_best, px, s) && zeroed(c->over_done, (size_t)ntiles * 4 + 16, s)) c->slices = SWR_SLICES_MAX;
   }
   // Depth-min shaders: the listed heavy tiles' runs (optional, like the slices above; the
   // per-slot completion counters start at zero and every merge leaves its own at zero)
   c->dslice_ok = false;
   if (ps && ps->depth_min && (c->dslice_chunks < 0 ? ps->slice_chunks : c->dslice_chunks) > 0) {
     const size_t slots = slice_cap(ntiles);
-    bool d = c->dslice_state.ensure(slots * SWR_DSLICES * c->tile * c->tile * (size_t)ps->state_bytes + 16);
-    if (d && c->dslice_done.bytes < slots * 4 + 16)
-      d = c->dslice_done.ensure(slots * 4 + 16) && cudaMemset(c->dslice_done.p, 0, c->dslice_done.bytes) == cudaSuccess;
-    c->dslice_ok = d;
+    c->dslice_ok = c->dslice_state.ensure(slots * SWR_DSLICES * c->tile * c->tile * (size_t)ps->state_bytes + 16) &&
+                   zeroed(c->dslice_done, slots * 4 + 16, s);
   }
   const size_t sw = scan_scratch_words(c->cap_prims) + 64 + 2 * scan_scratch_words(ntiles * SWR_SEGS);
   ok &= c->scratch.ensure(sw * 4);
@@ -467,13 +463,19 @@ int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, i
   const bool listed = dsl || quad_list;
   const uint32_t qcap = dsl ? slice_cap(ntiles) : quad_cap(ntiles);
   // (quad_count was zeroed by the draw's k_stage_copy)
-  uint32_t* big = big_list(c, ncells, seg_shift);
-  swr::launch(k_sort_cells, (ntiles + 7) / 8, 256, 0, s, st, cstart, ntiles, c->cap_pairs, c->keys0.as<uint32_t>(),
-              c->vals0.as<uint32_t>(), big ? big + 2 : nullptr, big, (uint32_t)SWR_RASTER_SORT,
-              listed ? c->quad_flag.as<uint8_t>() : nullptr, c->quad_tiles.as<uint32_t>(),
-              c->quad_count.as<uint32_t>(), qcap, dsl ? (uint32_t)(slice_chunks * ps->chunk) : kQuadMin);
-  if (big)
-    sort_big(c, cstart, ncells, seg_shift, c->keys0.as<uint32_t>(), c->vals0.as<uint32_t>(), big, s);
+  bool closed = ps->overwrite != 0;  // (k_overwrite takes the bins as they are, and closes the draw)
+  if (!ps->overwrite) {
+    uint32_t* big = big_list(c, ncells, seg_shift);
+    swr::launch(k_sort_cells, (ntiles + 7) / 8, 256, 0, s, st, cstart, ntiles, c->cap_pairs, c->keys0.as<uint32_t>(),
+                c->vals0.as<uint32_t>(), big ? big + 2 : nullptr, big, (uint32_t)SWR_RASTER_SORT,
+                listed ? c->quad_flag.as<uint8_t>() : nullptr, c->quad_tiles.as<uint32_t>(),
+                c->quad_count.as<uint32_t>(), qcap, dsl ? (uint32_t)(slice_chunks * ps->chunk) : kQuadMin);
+    c->launches += 1;
+    if (big) {
+      sort_big(c, cstart, ncells, seg_shift, c->keys0.as<uint32_t>(), c->vals0.as<uint32_t>(), big, s);
+      closed = true;
+    }
+  }
   mark(c, 4, s);
   RasterArgs ra;
   memset(&ra, 0, sizeof(ra));
@@ -492,7 +494,8 @@ int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, i
   ra.ntiles = ntiles;
   ra.has_span = has_span ? 1 : 0;
   ra.slices = ps->overwrite ? c->slices : 1;
-  ra.slice_state = c->slice_state.p;
+  ra.best = c->over_best.as<uint32_t>();
+  ra.best_done = c->over_done.as<uint32_t>();
   ra.quad_flag = listed ? c->quad_flag.as<uint8_t>() : nullptr;
   ra.quad_tiles = c->quad_tiles.as<uint32_t>();
   ra.quad_count = c->quad_count.as<uint32_t>();
@@ -502,13 +505,12 @@ int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, i
   ra.dslice_state = c->dslice_state.p;
   ra.dslice_done = c->dslice_done.as<uint32_t>();
   ps->raster(ra, ntiles, c->tile, s);
-  if (ra.slices > 1) c->launches += 1;  // k_merge_slices
   mark(c, 5, s);
-  if (!big) {
+  if (!closed) {
     swr::launch(k_close_draw, 1, 1, 0, s, st);
     c->launches += 1;
   }
-  c->launches += 1 + 2 + 1 + 1 + (ntiles ? 1 : 0);
+  c->launches += 1 + 2 + 1 + (ntiles ? 1 : 0);
   return cuda_err(cudaGetLastError());
 }
 
@@ -972,7 +974,7 @@ int swr_draw_elements(swr_context* c, int mode, uint64_t count, const uint32_t* 
   const uint32_t nbatches = (nsub + SWR_BATCH_PRIMS - 1) / SWR_BATCH_PRIMS;
   const SwrTargetDesc T = make_target(c, mode);
   const uint32_t ntiles = (uint32_t)T.tiles_x * (uint32_t)T.tiles_y;
-  int rc = ensure_capacity(c, (uint32_t)nverts, vs->S, nsub, nbatches, ntiles, ps->R > ps->lp_R ? ps->R : ps->lp_R, ps);
+  int rc = ensure_capacity(c, (uint32_t)nverts, vs->S, nsub, nbatches, ntiles, ps->R > ps->lp_R ? ps->R : ps->lp_R, ps, s);
   if (rc) return rc;
   SwrDrawDesc D;
   fill_draw(c, D, mode);
@@ -1046,7 +1048,7 @@ int swr_draw_list(swr_context* c, int mode, const float* vertices, uint64_t nver
   const uint32_t nsub = (uint32_t)(count / per);
   const SwrTargetDesc T = make_target(c, mode);
   const uint32_t ntiles = (uint32_t)T.tiles_x * (uint32_t)T.tiles_y;
-  int rc = ensure_capacity(c, (uint32_t)nverts, ps->S, nsub, 1, ntiles, ps->R > ps->lp_R ? ps->R : ps->lp_R, ps);
+  int rc = ensure_capacity(c, (uint32_t)nverts, ps->S, nsub, 1, ntiles, ps->R > ps->lp_R ? ps->R : ps->lp_R, ps, s);
   if (rc) return rc;
   if (!c->direct_keep.ensure((size_t)nsub * 4 + 16) || !c->direct_pos.ensure((size_t)nsub * 4 + 16))
     return SWR_ENOMEM;
@@ -1185,7 +1187,7 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
     return SWR_EINVAL;
   const int ntg = (int)T.size();
   int rc = ensure_capacity(c, (uint32_t)V, vs->S, (uint32_t)P, (uint32_t)B, (uint32_t)NT,
-                           ps->R > ps->lp_R ? ps->R : ps->lp_R, ps);
+                           ps->R > ps->lp_R ? ps->R : ps->lp_R, ps, s);
   if (rc) return rc;
   bool ok = c->draws.ensure(sizeof(SwrDrawDesc) * n) && c->targets.ensure(sizeof(SwrTargetDesc) * ntg) &&
             c->draw_vbase.ensure(4 * n + 16) && c->draw_bbase.ensure(4 * n + 16) && c->draw_pbase.ensure(4 * n + 16) &&
@@ -1234,7 +1236,7 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
                         c->tris.p, c->recs.p, c->tile_count.p, c->keys0.p, c->vals0.p, c->cell_count.p,
                         c->cell_start.p, c->scratch.p, c->draws.p, c->targets.p, c->draw_vbase.p,
                         c->draw_bbase.p, c->target_tile_base.p, c->draw_pbase.p, c->big_cells.p, h,
-                        c->slice_state.p, (const void*)(uintptr_t)c->slices, c->quad_flag.p, c->quad_tiles.p,
+                        c->over_best.p, c->over_done.p, (const void*)(uintptr_t)c->slices, c->quad_flag.p, c->quad_tiles.p,
                         c->quad_count.p, c->geo_bar.p, c->dslice_state.p, c->dslice_done.p,
                         (const void*)(uintptr_t)c->dslice_ok, (const void*)(intptr_t)c->dslice_chunks};
   for (const void* b : bufs) mix((uint64_t)(uintptr_t)b);

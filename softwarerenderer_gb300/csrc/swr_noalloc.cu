@@ -273,8 +273,9 @@ extern "C" int swr_draw_triangle_list_noalloc(const struct SwrUniforms* u, int p
   ra.status_w = st;
   ra.ntiles = ntiles;
   ra.has_span = raster_mode != SWR_RASTER_BLOCK;
-  ra.slices = 1;  // no slice buffer without allocation
-  ra.slice_state = nullptr;
+  ra.slices = 1;  // no buffer for sliced tiles' winners without allocation
+  ra.best = nullptr;
+  ra.best_done = nullptr;
   ra.quad_flag = nullptr;  // no heavy-tile quadrant CTAs: every tile is one CTA
   ra.quad_tiles = nullptr;
   ra.quad_count = nullptr;

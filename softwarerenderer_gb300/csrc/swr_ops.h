@@ -41,8 +41,8 @@ struct PsOps {
   void (*lp_frags)(const LpFragArgs& a, cudaStream_t s);
   void (*lp_raster)(const LpRasterArgs& a, cudaStream_t s);
   int needs_eq;  // shade() reads the triangle equations: triangles only
-  int overwrite;    // SwrOverwrite: large tiles may be rasterized in slices (RasterArgs.slices)
-  int state_bytes;  // sizeof(PS::State), per pixel and slice of RasterArgs.slice_state
+  int overwrite;    // SwrOverwrite: rasterized by k_overwrite, which needs no ordered bins
+  int state_bytes;  // sizeof(PS::State), per pixel and run of RasterArgs.dslice_state
   int depth_min;    // SwrDepthMin: heavy tiles may be rasterized in runs (RasterArgs.dslice)
   int slice_chunks; // SwrRasterSlices: by default tiles of more than this many chunks are (0: none)
   int chunk;        // SwrRasterChunk: primitives per raster chunk

@@ -687,18 +687,6 @@ struct SwrDepthCull<PS, decltype((void)PS::DepthCull)> {
   enum { value = PS::DepthCull && PS::HasDepth && PS::InterpolateZ && !SwrOverwrite<PS>::value };
 };
 
-// Overwrite shaders' State after two consecutive runs of fragments: the later run's last
-// writer (colour, winner) if it wrote at all, and the summed counters.  Lets a rasterizer
-// split one pixel's fragments into ordered slices and merge their states.
-SWR_HD void swr_overwrite_merge(SwrStateRGBA8& acc, const SwrStateRGBA8& later) {
-  if (later.writes) {
-    acc.color = later.color;
-    acc.winner = later.winner;
-  }
-  acc.frags += later.frags;
-  acc.writes += later.writes;
-}
-
 // Depth-tested RGBA8 shaders whose drawPixel is exactly `s.frags++; if (z < s.depth)
 // swr_write(s, z, shade(p, u), prim)` with a shade() that reads nothing but the fragment
 // (DepthMin = 1 in the shader).  In primitive order such a pixel ends with the depth

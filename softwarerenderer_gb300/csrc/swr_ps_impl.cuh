@@ -44,31 +44,35 @@ template <class PS>
 void run_raster(const RasterArgs& a, uint32_t ntiles, int tile, cudaStream_t s) {
   constexpr int kChunk = SwrRasterChunk<PS>::value;  // primitives staged in shared memory per bin chunk
   if (!ntiles) return;
-  if (a.boxes) {  // a small draw: 16-px tiles, one CTA each
-    if (a.has_span) swr::launch(k_raster<PS, 16, kChunk, true, true>, ntiles, 256, 0, s, a);
-    else swr::launch(k_raster<PS, 16, kChunk, false, true>, ntiles, 256, 0, s, a);
-    return;
-  }
-  // one CTA per tile, or per (tile, slice) for sliced overwrite shaders; Block-only
-  // submissions run the instantiation without the Span-mode passes
-  const bool sliced = SwrOverwrite<PS>::value && a.slices > 1;
-  uint32_t grid = sliced ? ntiles * (uint32_t)a.slices : ntiles;
-  if (SwrDepthMin<PS>::value && a.dslice) {  // the listed tiles' runs, then the other tiles
-    grid = SWR_DSLICES * a.quad_cap + ntiles;
-  } else if (tile == 16 && !SwrOverwrite<PS>::value) {  // quadrant CTAs (RasterArgs)
-    if (a.quad_all) grid = 4 * ntiles;
-    else if (a.quad_flag) grid = 4 * a.quad_cap + ntiles;
-  }
-  if (tile == 32) {
-    if (a.has_span) swr::launch(k_raster<PS, 32, kChunk, true>, grid, 256, 0, s, a);
-    else swr::launch(k_raster<PS, 32, kChunk, false>, grid, 256, 0, s, a);
-    if constexpr (SwrOverwrite<PS>::value)
-      if (sliced) swr::launch(k_merge_slices<PS, 32>, ntiles, 256, 0, s, a);
+  if constexpr (SwrOverwrite<PS>::value) {
+    if (a.boxes) {
+      swr::launch(k_overwrite<PS, 16, true>, ntiles, 256, 0, s, a);
+    } else {
+      const uint32_t grid = a.slices > 1 ? ntiles * (uint32_t)a.slices : ntiles;
+      if (tile == 32) swr::launch(k_overwrite<PS, 32, false>, grid, 256, 0, s, a);
+      else swr::launch(k_overwrite<PS, 16, false>, grid, 256, 0, s, a);
+    }
   } else {
-    if (a.has_span) swr::launch(k_raster<PS, 16, kChunk, true>, grid, 256, 0, s, a);
-    else swr::launch(k_raster<PS, 16, kChunk, false>, grid, 256, 0, s, a);
-    if constexpr (SwrOverwrite<PS>::value)
-      if (sliced) swr::launch(k_merge_slices<PS, 16>, ntiles, 256, 0, s, a);
+    if (a.boxes) {  // a small draw: 16-px tiles, one CTA each
+      if (a.has_span) swr::launch(k_raster<PS, 16, kChunk, true, true>, ntiles, 256, 0, s, a);
+      else swr::launch(k_raster<PS, 16, kChunk, false, true>, ntiles, 256, 0, s, a);
+      return;
+    }
+    // one CTA per tile; Block-only submissions run the instantiation without the Span-mode passes
+    uint32_t grid = ntiles;
+    if (SwrDepthMin<PS>::value && a.dslice) {  // the listed tiles' runs, then the other tiles
+      grid = SWR_DSLICES * a.quad_cap + ntiles;
+    } else if (tile == 16) {  // quadrant CTAs (RasterArgs)
+      if (a.quad_all) grid = 4 * ntiles;
+      else if (a.quad_flag) grid = 4 * a.quad_cap + ntiles;
+    }
+    if (tile == 32) {
+      if (a.has_span) swr::launch(k_raster<PS, 32, kChunk, true>, grid, 256, 0, s, a);
+      else swr::launch(k_raster<PS, 32, kChunk, false>, grid, 256, 0, s, a);
+    } else {
+      if (a.has_span) swr::launch(k_raster<PS, 16, kChunk, true>, grid, 256, 0, s, a);
+      else swr::launch(k_raster<PS, 16, kChunk, false>, grid, 256, 0, s, a);
+    }
   }
 }
 

@@ -1238,11 +1238,12 @@ struct RasterArgs {
   const uint32_t* draw_prim_base;    // per draw first primitive (null: a single draw from 0)
   uint32_t* status_w;
   uint32_t ntiles;
-  int slices;                        // overwrite shaders: CTAs per tile of more than SWR_RASTER_SORT
-                                     // entries (1: no slicing), each over an ordered slice of its bin
-  void* slice_state;                 // their per-pixel PS::State, [tile][slice][TILE * TILE]
+  int slices;                        // k_overwrite: CTAs per tile of more than SWR_RASTER_SORT entries
+                                     // (1: no slicing), each over a slice of its bin
+  uint32_t* best;                    // their pixels' winners, primitive id + 1, [tile][TILE * TILE]
+  uint32_t* best_done;               // per tile: the slices finished (both zero between draws)
   int has_span;                      // some draw rasterizes in Span or Adaptive mode (selects k_raster<..., true>)
-  // Quadrant CTAs (16-px tiles, shaders other than the overwrite ones): a heavy tile -- more
+  // Quadrant CTAs (16-px tiles): a heavy tile -- more
   // than quad_min bin entries; k_sort_cells lists up to quad_cap of them -- is rasterized by
   // four CTAs, one per 8 x 8 quadrant, each walking the whole bin for its own pixels, so the
   // slowest tiles no longer set the kernel's length.  CTAs [0, 4 quad_cap) take the listed
@@ -1474,13 +1475,13 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
   static_assert(CH % 32 == 0 && CH <= 128, "chunks of 32, 64, 96 or 128 primitives");
   __shared__ uint32_t sculr[kCull ? NREG * NW : 1];  // per region: primitives only counted there
   __shared__ int sminx[kCull && SPAN ? CH : 1];  // Span mode: leftmost start of a span reaching the tile
-  // Per-pixel walk (shaders without the depth cull or overwrite shortcut): each pixel keeps
+  // Per-pixel walk (shaders without the depth cull): each pixel keeps
   // the set of compacted primitives covering it (set in C1), so in C2 every lane visits only
   // its own pixel's primitives instead of all primitives touching its warp's half block.
   constexpr int HW = (CH + 63) / 64;  // 64-primitive words of a chunk
   // (Not for the depth-culling shaders: measured on the 4K soup, whose chunks mix compacted
   // small primitives with large ones, the per-lane loops cost 30 % more raster time.)
-  constexpr bool kPixWalk = SWR_PIX_WALK && kCompact && !kCull && !SwrOverwrite<PS>::value;
+  constexpr bool kPixWalk = SWR_PIX_WALK && kCompact && !kCull;
   __shared__ uint64_t spm[kPixWalk ? TILE * TILE * HW : 1];
   // per (primitive, block): the primitive's covered pixels in the tile's earlier blocks, so a
   // compacted fragment's slot is sex + spre + its rank in the block's mask (a compacted
@@ -1492,15 +1493,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
   uint32_t frags = 0, passes = 0;
   // One CTA per tile (a persistent grid pulling tiles from a counter measured no faster on
   // the dense mesh and slower where few tiles carry the work: they gather on fewer SMs).
-  // Overwrite shaders with g.slices > 1: CTA (tile, slice); a tile of more than
-  // SWR_RASTER_SORT entries (an ordered bin) is cut into g.slices runs of whole chunks, each
-  // rasterized from an empty State into slice_state and merged in order by k_merge_slices;
-  // smaller tiles are rasterized whole by slice 0.
   uint32_t tile = blockIdx.x, slice = 0;
-  if (SwrOverwrite<PS>::value && !DIRECT && g.slices > 1) {
-    tile = blockIdx.x / (uint32_t)g.slices;
-    slice = blockIdx.x - tile * (uint32_t)g.slices;
-  }
   int quad = -1;  // the 8 x 8 quadrant (block) this CTA rasterizes alone, -1: the whole tile
   int dslot = -1;  // sliced heavy tile: its list slot (slice = its run)
   if constexpr (SwrDepthMin<PS>::value && !DIRECT) {
@@ -1518,7 +1511,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
       }
     }
   }
-  if constexpr (TILE == 16 && !SwrOverwrite<PS>::value && !DIRECT) {
+  if constexpr (TILE == 16 && !DIRECT) {
     if (g.dslice) {
     } else if (g.quad_all) {
       tile = blockIdx.x >> 2;
@@ -1541,21 +1534,6 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
   if constexpr (!DIRECT) {
     b = g.tile_start[(size_t)tile * g.tile_stride];
     e = g.tile_start[(size_t)(tile + 1) * g.tile_stride];
-  }
-  bool sliced = false;
-  if constexpr (SwrOverwrite<PS>::value && !DIRECT) {
-    if (g.slices > 1) {
-      if (e - b <= (uint32_t)SWR_RASTER_SORT) {
-        if (slice) return;
-      } else {
-        sliced = true;
-        const uint32_t nch = (e - b + CH - 1) / CH, ns = (uint32_t)g.slices;
-        const uint32_t lo = b + (uint32_t)((uint64_t)nch * slice / ns) * CH;
-        const uint32_t hi = min(e, b + (uint32_t)((uint64_t)nch * (slice + 1) / ns) * CH);
-        b = lo;
-        e = hi > lo ? hi : lo;  // an empty slice still writes its (empty) states
-      }
-    }
   }
   // Small draws: the tile's primitives out of the next windows of 256 boxes, in order, until
   // more than 256 are found (e = their count; ssorted holds SWR_RASTER_SORT) or none is left.
@@ -1586,7 +1564,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
     scan_np = min(g.status[SWR_ST_PRIMS], g.cap_prims);
     gather();
   }
-  if (b == e && !sliced) return;  // uniform per CTA
+  if (b == e) return;  // uniform per CTA
   // the chunks this CTA rasterizes: the whole bin, or a sliced heavy tile's run
   uint32_t cb = b, ce = e;
   int nsl = 1;
@@ -1621,7 +1599,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
   // A tile of at most SWR_RASTER_SORT entries orders its own bin: the cells (increasing id
   // segments) are contiguous, so an id's position is its cell's start plus the number of
   // smaller ids in that cell.  The raw ids are staged in the record area (used only later).
-  const bool self_sort = DIRECT || (g.bin_raw && !sliced && e - b <= (uint32_t)SWR_RASTER_SORT);
+  const bool self_sort = DIRECT || (g.bin_raw && e - b <= (uint32_t)SWR_RASTER_SORT);
   if (!DIRECT && self_sort) {
     uint32_t* sraw = (uint32_t*)srec4;
     const uint32_t ntot = e - b;
@@ -2063,32 +2041,6 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
           }
         }
       }
-      uint32_t extra = 0;  // overwrite shaders: covering fragments before the last one
-      if (SwrOverwrite<PS>::value) {
-        // only the chunk's last covering primitive shades; the others only count
-        int last = -1;
-        uint32_t cnt = 0;
-#pragma unroll
-        for (int w = 0; w < HW; ++w) {
-          uint64_t h = hw[w];
-          while (h) {
-            const int k = w * 64 + __ffsll((long long)h) - 1;
-            h &= h - 1ull;
-            if (in[q] && ((smask[k * NB + blk[q]] >> bit) & 1ull)) {
-              ++cnt;
-              last = k;
-            }
-          }
-        }
-        if (cnt) {
-#pragma unroll
-          for (int w = 0; w < HW; ++w) hw[w] = (last >> 6) == w ? 1ull << (last & 63) : 0ull;
-          extra = cnt - 1;
-          frags += extra;
-          st[q].frags += extra;
-          st[q].writes += extra;
-        }
-      }
       // primitive-order walk over the words (one copy of the loop body)
       uint64_t hits = hw[0];
       uint64_t later = HW > 1 ? hw[HW - 1] : 0ull;
@@ -2189,13 +2141,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
 #pragma unroll
   for (int q = 0; q < PPT; ++q)
     if (in[q]) {
-      if (sliced) {
-        typename PS::State* ss = (typename PS::State*)g.slice_state +
-                                 ((size_t)tile * g.slices + slice) * (TILE * TILE);
-        ss[(py[q] - oy) * TILE + (px[q] - ox)] = st[q];
-      } else {
-        PS::store(st[q], px[q], py[q], U);
-      }
+      PS::store(st[q], px[q], py[q], U);
       passes += st[q].writes;
     }
   // fragment statistics: drawPixel calls and colour writes
@@ -2208,32 +2154,265 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
   }
 }
 
-// Merges the slices of the tiles k_raster sliced (more than SWR_RASTER_SORT entries):
-// per pixel the slices' States in bin order (swr_overwrite_merge), then the shader's store.
-template <class PS, int TILE>
-__global__ void __launch_bounds__(256) k_merge_slices(RasterArgs g) {
+// ---------------------------------------------------------------------------------
+// Overwrite shaders (SwrOverwrite): a pixel ends with the colour of its last covering
+// primitive -- the one with the largest id -- and with the number of primitives covering it.
+// Neither needs the bin in order, and only one fragment per pixel needs shading.
+//
+// One CTA per tile, or g.slices CTAs over parts of a tile's bin of more than SWR_RASTER_SORT
+// entries.  A work item is an entry and a group of its rows: the whole tile's rows, one
+// thread per entry, where entries are many (the record is read once, straight from global
+// memory; no staging, no barriers), single rows where they are few (a small draw's large
+// triangles would leave one thread walking 256 pixels).  An item adds up the lengths of its
+// rows' runs, and writes its id over smaller ones in the tile's winners; entries are taken
+// from the bin's end (the largest ids up to the order inside a cell), and once every pixel
+// has a winner, entries below all of them only count.  The last CTA of a tile shades its
+// winners.  Bound by the issue of the row loop.  Against ordering every bin and walking
+// 64-primitive chunks pixel by pixel (sorts 91 us, raster 1463 us), the 40,960 large
+// triangles of the reference's Benchmark program (640x480, 240M fragments) went
+// from 1888 to 585 us a draw.
+template <class PS, int TILE, bool DIRECT>
+__global__ void __launch_bounds__(256) k_overwrite(RasterArgs g) {
   swr_pdl_entry();
+  typedef Rec<PS> RL;
   constexpr int PPT = TILE * TILE / 256;
+  static_assert(RL::R >= 20, "words 0-19 of a record are read as five float4s");
+  __shared__ uint32_t sbest[TILE * TILE];      // per pixel: winner's id + 1
+  __shared__ int scnt[TILE * (TILE + 1)];      // per row: +1 at a run's first pixel, -1 past its last
+  __shared__ uint32_t sred[8];
+  __shared__ uint32_t sfr[32];
+  __shared__ uint32_t slast;
+  // the draw's queue requests are final (nothing after this stage counts)
+  if (blockIdx.x == 0 && threadIdx.x == 0 && !DIRECT) swr_close_status(g.status_w);
   if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
-  const uint32_t tile = blockIdx.x;
-  if (tile >= g.ntiles) return;
-  const uint32_t b = g.tile_start[(size_t)tile * g.tile_stride], e = g.tile_start[(size_t)(tile + 1) * g.tile_stride];
-  if (e - b <= (uint32_t)SWR_RASTER_SORT) return;
-  const int ti = g.ntargets > 1 ? swr_find_le(g.target_tile_base, g.ntargets, tile) : 0;
+  const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t tile = blockIdx.x, slice = 0, n = 0, hi = 0;
+  int nsl = 1;
+  if constexpr (DIRECT) {
+    n = min(g.status[SWR_ST_PRIMS], g.cap_prims);
+  } else {
+    if (g.slices > 1) {
+      tile = blockIdx.x / (uint32_t)g.slices;
+      slice = blockIdx.x - tile * (uint32_t)g.slices;
+    }
+    if (tile >= g.ntiles) return;
+    const uint32_t b = g.tile_start[(size_t)tile * g.tile_stride], e = g.tile_start[(size_t)(tile + 1) * g.tile_stride];
+    hi = e;
+    n = e - b;
+    if (n > (uint32_t)SWR_RASTER_SORT && g.slices > 1) {
+      nsl = g.slices;
+      const uint32_t lo = b + (uint32_t)((uint64_t)n * slice / (uint32_t)nsl);
+      hi = b + (uint32_t)((uint64_t)n * (slice + 1) / (uint32_t)nsl);
+      n = hi - lo;
+    } else if (slice) {
+      return;
+    }
+  }
+  if (tile >= g.ntiles || n == 0) return;  // (a slice of more than SWR_RASTER_SORT entries is never empty)
+  const int ti = !DIRECT && g.ntargets > 1 ? swr_find_le(g.target_tile_base, g.ntargets, tile) : 0;
   const SwrTargetDesc& T = g.targets[ti];
   const SwrUniforms& U = g.draws[T.first_draw].u;
   const uint32_t lt = tile - T.tile_base;
-  const int ox = (int)(lt % (uint32_t)T.tiles_x) * TILE, oy = (int)(lt / (uint32_t)T.tiles_x) * TILE;
-  const typename PS::State* ss = (const typename PS::State*)g.slice_state + (size_t)tile * g.slices * (TILE * TILE);
+  const uint32_t tx = lt % (uint32_t)T.tiles_x, ty = lt / (uint32_t)T.tiles_x;
+  const int ox = (int)tx * TILE, oy = (int)ty * TILE;
+  const int xend = min(ox + TILE, T.width), yend = min(oy + TILE, T.height);
+  const bool counts = U.frag_count != nullptr;
+#pragma unroll
+  for (int q = 0; q < PPT; ++q) sbest[q * 256 + tid] = 0u;
+  for (int i = tid; i < TILE * (TILE + 1); i += 256) scnt[i] = 0;
+  __syncthreads();
+  uint32_t smin = 0;  // no pixel's winner is below it
+  uint32_t frags = 0;
+  // pixels [x0, x1) of tile row `row` are covered by the primitive with id key - 1
+  auto run = [&](int row, int x0, int x1, uint32_t key) {
+    if (x1 <= x0) return;
+    frags += (uint32_t)(x1 - x0);
+    if (key > smin)
+      for (int x = x0; x < x1; ++x)
+        if (*(volatile uint32_t*)&sbest[row * TILE + x] < key) atomicMax(&sbest[row * TILE + x], key);
+    if (counts) {
+      atomicAdd(&scnt[row * (TILE + 1) + x0], 1);
+      atomicAdd(&scnt[row * (TILE + 1) + x1], -1);
+    }
+  };
+  // rows [r0, r1) of the tile, primitive p
+  auto cover = [&](uint32_t p, int r0, int r1) {
+    const float4* rc = (const float4*)(g.recs + (size_t)p * RL::R);
+    const float4 q0 = __ldg(rc), q1 = __ldg(rc + 1), q2 = __ldg(rc + 2), q3 = __ldg(rc + 3);
+    const int flags = __float_as_int(q0.x);
+    if (!(flags & 1)) return;
+    const int bx0 = __float_as_int(q0.z), by0 = __float_as_int(q0.w);
+    const int bx1 = __float_as_int(q1.x), by1 = __float_as_int(q1.y);
+    const int ylo = max(by0, oy + r0), yhi = min(min(by1 + 1, oy + r1), yend);
+    const uint32_t key = p + 1u;
+    if (!(flags & 2)) {  // Span: a run per row of either half, inside the box's 8-px blocks
+      const float4 q4 = __ldg(rc + 4);
+      const SwrDrawDesc& D = g.draws[__float_as_int(q0.y)];
+      const int minx = D.sc_minx, maxx = D.sc_maxx;
+      const int cx0 = max(bx0 & ~(SWR_BLOCK - 1), ox), cx1 = min((bx1 | (SWR_BLOCK - 1)) + 1, xend);
+      SpanHalf bot, top;
+      bot.y0 = __float_as_int(q1.z); bot.y1 = __float_as_int(q1.w);
+      bot.ox = q2.x; bot.oy = q2.y; bot.is1 = q2.z; bot.is2 = q2.w;
+      top.y0 = __float_as_int(q3.x); top.y1 = __float_as_int(q3.y);
+      top.ox = q3.z; top.oy = q3.w; top.is1 = q4.x; top.is2 = q4.y;
+      for (int y = ylo; y < yhi; ++y) {
+        const bool inb = (flags & 32) && y >= bot.y0 && y < bot.y1;
+        const bool int_ = (flags & 64) && y > top.y1 && y <= top.y0;
+        if (!inb && !int_) continue;
+        int xl, xr;
+        span_row(inb ? bot : top, y, minx, maxx, xl, xr);
+        run(y - oy, max(xl, cx0) - ox, min(xr, cx1) - ox, key);
+      }
+      return;
+    }
+    // Block: whole blocks, or the rows of the reference's stepped edge tests
+    const float r[15] = {0, 0, 0, 0, 0, 0, q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, q3.x, q3.y, q3.z};
+    const float t0 = (flags & 4) ? 0.0f : 0x1p-149f, t1 = (flags & 8) ? 0.0f : 0x1p-149f;
+    const float t2 = (flags & 16) ? 0.0f : 0x1p-149f;  // thresholds of edge_test
+    for (int by = ylo & ~(SWR_BLOCK - 1); by < yhi; by += SWR_BLOCK)
+      for (int bx = max(bx0 & ~(SWR_BLOCK - 1), ox); bx <= bx1 && bx < xend; bx += SWR_BLOCK) {
+        const int cls = block_class(r, flags, bx, by);
+        if (cls == 0) continue;
+        const int wx = min(SWR_BLOCK, xend - bx);
+        const float fx = swr_add((float)bx, 0.5f), fy = swr_add((float)by, 0.5f);
+        float i0 = swr_eval(r[6], r[7], r[8], fx, fy), i1 = swr_eval(r[9], r[10], r[11], fx, fy);
+        float i2 = swr_eval(r[12], r[13], r[14], fx, fy);
+        for (int y = by; y < min(by + SWR_BLOCK, yhi); ++y) {
+          uint32_t m = (1u << wx) - 1u;
+          if (cls == 2) {  // block_row_bits, the row starts stepped from row to row
+            float c0 = i0, c1 = i1, c2 = i2;
+#pragma unroll
+            for (int col = 0; col < SWR_BLOCK; ++col) {
+              if (!(c0 >= t0 && c1 >= t1 && c2 >= t2)) m &= ~(1u << col);
+              c0 = swr_add(c0, r[6]);
+              c1 = swr_add(c1, r[9]);
+              c2 = swr_add(c2, r[12]);
+            }
+            i0 = swr_add(i0, r[7]);
+            i1 = swr_add(i1, r[10]);
+            i2 = swr_add(i2, r[13]);
+          }
+          if (y < ylo) continue;
+          while (m) {  // the row's runs of covered pixels (one, up to rounding)
+            const int x0 = __ffs(m) - 1, x1 = x0 + __ffs(~(m >> x0)) - 1;
+            m &= ~0u << x1;
+            run(y - oy, bx - ox + x0, bx - ox + x1, key);
+          }
+        }
+      }
+  };
+  // rows per item: see above (n * groups items in all)
+  const int shift = n >= 128u ? 0 : (n >= 32u ? 2 : (TILE == 16 ? 4 : 5));
+  const int rows = TILE >> shift;
+  const uint32_t* bin = g.bin_raw ? g.bin_raw : g.bin;
+  const uint64_t items = (uint64_t)n << shift;
+  int round = 0;
+  for (uint64_t base = 0; base < items; base += 256, ++round) {
+    const uint64_t it = base + (uint64_t)tid;
+    if (it < items) {
+      const uint32_t k = (uint32_t)(it >> shift);
+      const int r0 = (int)((uint32_t)it & ((1u << shift) - 1u)) * rows;
+      if constexpr (DIRECT) {
+        const uint32_t p = n - 1u - k;
+        if (swr_box_hit(g.boxes[p], tx, ty)) cover(p, r0, r0 + rows);
+      } else {
+        cover(bin[hi - 1u - k], r0, r0 + rows);
+      }
+    }
+    if (round < 3 && base + 256 < items) {  // (uniform) a later, larger bound would save little
+      __syncthreads();
+      uint32_t m = 0xffffffffu;
+#pragma unroll
+      for (int q = 0; q < PPT; ++q) {
+        const int i = q * 256 + tid;
+        if (ox + i % TILE < xend && oy + i / TILE < yend) m = min(m, sbest[i]);
+      }
+      m = __reduce_min_sync(0xffffffffu, m);
+      if (lane == 0) sred[warp] = m;
+      __syncthreads();
+      smin = sred[0];
+#pragma unroll
+      for (int w = 1; w < 8; ++w) smin = min(smin, sred[w]);
+    }
+  }
+  __syncthreads();
+  uint32_t tot;
+  swr_block_exscan(frags, sfr, &tot);
+  if (tid == 0 && tot) {  // every fragment writes
+    atomicAdd((unsigned long long*)&g.status_w[SWR_ST_SHADED_LO], (unsigned long long)tot);
+    atomicAdd((unsigned long long*)&g.status_w[SWR_ST_PASSES_LO], (unsigned long long)tot);
+  }
+  uint32_t best[PPT];
 #pragma unroll
   for (int q = 0; q < PPT; ++q) {
-    const int i = q * 256 + threadIdx.x;
+    const int i = q * 256 + tid;
     const int x = ox + i % TILE, y = oy + i / TILE;
-    if (x >= T.width || y >= T.height) continue;
-    typename PS::State m;
-    PS::load(m, x, y, U);
-    for (int sl = 0; sl < g.slices; ++sl) swr_overwrite_merge(m, ss[(size_t)sl * (TILE * TILE) + i]);
-    PS::store(m, x, y, U);
+    best[q] = sbest[i];
+    if (!counts || x >= xend || y >= yend) continue;
+    int c = 0;
+    for (int k = 0; k <= i % TILE; ++k) c += scnt[(i / TILE) * (TILE + 1) + k];
+    if (!c) continue;
+    uint32_t* fc = U.frag_count + (size_t)y * (size_t)U.width + (size_t)x;
+    if (nsl > 1) atomicAdd(fc, (uint32_t)c); else *fc += (uint32_t)c;
+  }
+  if (nsl > 1) {
+    uint32_t* gb = g.best + (size_t)tile * (TILE * TILE);
+#pragma unroll
+    for (int q = 0; q < PPT; ++q)
+      if (best[q]) atomicMax(&gb[q * 256 + tid], best[q]);
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) slast = atomicAdd(&g.best_done[tile], 1u) == (uint32_t)(nsl - 1);
+    __syncthreads();
+    if (!slast) return;
+    __threadfence();
+#pragma unroll
+    for (int q = 0; q < PPT; ++q) {
+      best[q] = __ldcg(&gb[q * 256 + tid]);
+      if (best[q]) gb[q * 256 + tid] = 0u;  // ready for the next draw
+    }
+    if (tid == 0) g.best_done[tile] = 0u;
+  }
+#pragma unroll
+  for (int q = 0; q < PPT; ++q) {
+    const int i = q * 256 + tid;
+    const int x = ox + i % TILE, y = oy + i / TILE;
+    if (!best[q] || x >= xend || y >= yend) continue;
+    const uint32_t p = best[q] - 1u;
+    const float* r = g.recs + (size_t)p * RL::R;
+    const int flags = __float_as_int(r[0]);
+    const SwrDrawDesc& D = g.draws[__float_as_int(r[1])];
+    float fx, fy;
+    int ka, kb;
+    if (flags & 2) {
+      fx = swr_add((float)(x & ~7), 0.5f);
+      fy = swr_add((float)(y & ~7), 0.5f);
+      ka = x & 7;
+      kb = y & 7;
+    } else {  // from its row's span start
+      const bool inb = (flags & 32) && y >= __float_as_int(r[6]) && y < __float_as_int(r[7]);
+      SpanHalf h;
+      h.ox = inb ? r[8] : r[14]; h.oy = inb ? r[9] : r[15];
+      h.is1 = inb ? r[10] : r[16]; h.is2 = inb ? r[11] : r[17];
+      int xl, xr;
+      span_row(h, y, D.sc_minx, D.sc_maxx, xl, xr);
+      fx = swr_add((float)xl, 0.5f);
+      fy = swr_add((float)y, 0.5f);
+      ka = x - xl;
+      kb = 0;
+    }
+    const float* eq = r + RL::EQ0;
+    GpuPixel<PS> pd;
+    pd.x = x;
+    pd.y = y;
+    pd.eq = eq;
+    pd.z = build_z<PS>(eq, flags & 2, fx, fy, ka, kb);
+    build_pixel<PS>(eq, flags & 2, fx, fy, ka, kb, pd);
+    typename PS::State st;
+    PS::load(st, x, y, U);
+    PS::apply(st, pd.z, PS::shade(pd, D.u), prim_id(g, r, p));
+    st.frags = 0;  // counted above
+    PS::store(st, x, y, U);
   }
 }
 

@@ -1,0 +1,70 @@
+"""Overwrite shaders (no depth test): bins in any order, largest covering id per pixel, one
+shaded fragment per pixel.  Against the oracle at the edges of the work split (32 and 128
+entries per tile), of the slicing (512), in every raster mode and tile size, with and without
+the per-pixel counts, on the general path and on the small draws' one."""
+import numpy as np
+import pytest
+
+from softwarerenderer_gb300 import scenes
+from softwarerenderer_gb300.abi import PS, RasterMode, VS
+
+from .parity import describe, diff, oracle_render
+
+pytestmark = pytest.mark.gpu
+
+
+def _scene(n, raster, width=48, height=40, seed=0):
+    sc = scenes.stack_scene(seed, n, raster=raster, width=width, height=height)
+    sc.vs, sc.ps = VS.POS_RGB_AFFINE, PS.VCOLOR_AFFINE
+    return sc
+
+
+def _draw(sc, tile=16, aux=True, general=False, draws=1):
+    from softwarerenderer_gb300.device import DeviceScene, DeviceTarget
+    ds = DeviceScene(sc, tile=tile)
+    if general:
+        ds.rast.ctx.set_queue_capacity(0, 1 << 22)
+    for _ in range(draws):
+        tg = DeviceTarget(sc, aux=aux)
+        st = ds.draw(tg)
+    return tg.to_host(), st
+
+
+@pytest.mark.parametrize("raster", [RasterMode.Span, RasterMode.Block, RasterMode.Adaptive])
+@pytest.mark.parametrize("n", [1, 31, 32, 127, 128, 300, 512, 513, 1025, 5000])
+@pytest.mark.parametrize("tile", [16, 32])
+def test_piles(gpu_lib, port, n, raster, tile):
+    sc = _scene(n, raster, seed=n)
+    ref, rst = oracle_render(port, sc)
+    for aux in (True, False):
+        for general in (True, False):
+            got, st = _draw(sc, tile, aux, general)
+            want = ref if aux else {k: ref[k] for k in got}
+            assert not diff(want, got), (aux, general, [describe(want, got, k) for k in diff(want, got)])
+            assert st["fragments"] == st["passes"] == rst["fragments"]
+
+
+def test_wide_tall_target_and_repeated_draws(gpu_lib, port):
+    """Odd sizes; the winners and counters of sliced tiles are ready again for the next draw."""
+    sc = scenes.benchmark_scene(4096)
+    sc.width, sc.height = 333, 217
+    sc.viewport = sc.scissor = (0, 0, 333, 217)
+    ref, _ = oracle_render(port, sc)
+    for draws in (1, 3):
+        got, _ = _draw(sc, draws=draws)
+        assert not diff(ref, got), [describe(ref, got, k) for k in diff(ref, got)]
+
+
+def test_two_draws_into_one_target(gpu_lib, port):
+    """A batch whose items share a target: the later item's primitives win."""
+    from softwarerenderer_gb300.batch import BatchRenderer
+    from softwarerenderer_gb300.device import DeviceTarget
+    scs = [_scene(700, RasterMode.Adaptive, seed=s) for s in (1, 2)]
+    tg = DeviceTarget(scs[0])
+    br = BatchRenderer(scs, graph=False, targets=[tg, tg])
+    br.draw()
+    t = scenes.Target(scs[0])
+    for sc in scs:
+        port.draw(sc, t)
+    want, got = t.arrays(), tg.to_host()
+    assert not diff(want, got), [describe(want, got, k) for k in diff(want, got)]
