@@ -167,7 +167,7 @@ struct swr_context {
   swr::Buffer draws, targets, draw_vbase, draw_bbase, target_tile_base;
   swr::Buffer ptv, clipv, clip_table, clip_slot, tri_flags, batch_counts, batch_base;
   swr::Buffer tris, recs, tile_count, pair_off, keys0, vals0, keys1, vals1, tile_start;
-  swr::Buffer scratch, status, direct_keep, direct_pos, lp_refs, cell_count, cell_start, draw_pbase;
+  swr::Buffer scratch, status, direct_keep, direct_pos, lp_refs, cell_count, cell_start, cell_fill, draw_pbase;
   swr::Buffer big_cells;  // k_sort_cells -> k_sort_big: [count, cell ids...]
   swr::Buffer quad_flag, quad_tiles, quad_count;  // heavy 16-px tiles rasterized as four quadrant CTAs
   int quad_mode = 0;  // 0: off, 1: heavy tiles (more than kQuadMin entries), 2: every tile (8-px raster tiles)
@@ -220,7 +220,7 @@ struct swr_context {
     swr::Buffer* all[] = {&draws, &targets, &draw_vbase, &draw_bbase, &target_tile_base, &ptv, &clipv,
                           &clip_table, &clip_slot, &tri_flags, &batch_counts, &batch_base, &tris, &recs,
                           &tile_count, &pair_off, &keys0, &vals0, &keys1, &vals1, &tile_start, &scratch,
-                          &status, &direct_keep, &direct_pos, &lp_refs, &cell_count, &cell_start, &draw_pbase,
+                          &status, &direct_keep, &direct_pos, &lp_refs, &cell_count, &cell_start, &cell_fill, &draw_pbase,
                           &big_cells, &over_best, &over_done, &quad_flag, &quad_tiles, &quad_count, &geo_bar,
                           &dslice_state, &dslice_done};
     for (swr::Buffer* b : all) b->budget = &budget;
@@ -267,7 +267,7 @@ bool zeroed(Buffer& b, size_t bytes, cudaStream_t s) {
 
 // Allocates every queue a draw with the given host-known sizes needs.
 int ensure_capacity(swr_context* c, uint32_t nverts_ptv, int S, uint32_t nsub, uint32_t nbatches,
-                    uint32_t ntiles, int R, const PsOps* ps, cudaStream_t s) {
+                    uint32_t ntiles, int R, const PsOps* ps, int ndraws, cudaStream_t s) {
   if (!c->fixed_prims) grow_u32(c->cap_prims, (uint64_t)nsub + 1024);
   grow_u32(c->cap_clip_slots, (uint64_t)nsub / 16 + 1024);
   grow_u32(c->cap_clip_verts, (uint64_t)c->cap_clip_slots * 4);
@@ -293,6 +293,7 @@ int ensure_capacity(swr_context* c, uint32_t nverts_ptv, int S, uint32_t nsub, u
   // the per-cell counters start at zero and every draw leaves them at zero (k_fill_bins)
   ok &= zeroed(c->cell_count, (size_t)ntiles * SWR_SEGS * 4 + 16, s);
   ok &= c->cell_start.ensure(((size_t)ntiles * SWR_SEGS + 1) * 4 + 16);
+  if (ndraws == 1) ok &= c->cell_fill.ensure((size_t)ntiles * SWR_SEGS * 4 + 16);
   ok &= c->quad_flag.ensure((size_t)ntiles + 16);
   ok &= c->quad_tiles.ensure((size_t)quad_cap(ntiles) * 4 + 16);
   ok &= c->quad_count.ensure(16);
@@ -422,10 +423,11 @@ int segment_shift(uint32_t cap) {
 // offsets, k_fill_bins scatters primitive ids into their cells, k_sort_cells restores the
 // primitive order inside each cell; a tile's bin is then its cells' contiguous range.
 int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, int vs_a, int vs_p,
-                 uint32_t ntiles, cudaStream_t s, int ntargets, bool has_span) {
+                 uint32_t ntiles, cudaStream_t s, int ndraws, int ntargets, bool has_span) {
   uint32_t* st = c->status.as<uint32_t>();
   const uint32_t ncells = ntiles * SWR_SEGS;
   const int seg_shift = segment_shift(c->cap_prims);
+  const SwrCells cells = ndraws == 1 ? SwrCells{1u, ntiles} : SwrCells{SWR_SEGS, 1u};
   SetupArgs sa;
   memset(&sa, 0, sizeof(sa));
   sa.tris = c->tris.as<uint4>();
@@ -444,14 +446,22 @@ int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, i
   sa.tile_count = c->tile_count.as<uint32_t>();
   sa.tile = c->tile;
   sa.cell_count = c->cell_count.as<uint32_t>();
+  sa.cells = cells;
   sa.seg_shift = seg_shift;
   ps->setup(sa, s);
   mark(c, 3, s);
   uint32_t* scr = c->scratch.as<uint32_t>();
   uint32_t* cstart = c->cell_start.as<uint32_t>();
-  scan_exclusive(c->cell_count.as<uint32_t>(), cstart, nullptr, ncells, cstart + ncells, scr, s);
+  const uint32_t* fill = cstart;
+  if (cells.tile_stride == 1) {
+    fill = c->cell_fill.as<uint32_t>();
+    scan_cells(c->cell_count.as<uint32_t>(), ntiles, cstart, c->cell_fill.as<uint32_t>(), scr, s);
+  } else {
+    scan_exclusive(c->cell_count.as<uint32_t>(), cstart, nullptr, ncells, cstart + ncells, scr, s);
+  }
   ps->fill_bins(st, c->cap_prims, c->recs.as<float>(), c->cell_count.as<uint32_t>(),
-                cstart, ncells, seg_shift, c->cap_pairs, c->draws.as<SwrDrawDesc>(), c->targets.as<SwrTargetDesc>(),
+                fill, cstart + ncells, ncells, cells, seg_shift, c->cap_pairs,
+                c->draws.as<SwrDrawDesc>(), c->targets.as<SwrTargetDesc>(),
                 c->tile, c->keys0.as<uint32_t>(), st, s);
   // heavy tiles listed by k_sort_cells: rasterized in runs of chunks (depth-min shaders,
   // tiles of more than slice_chunks raster chunks), or else as quadrant CTAs (16-px tiles,
@@ -609,6 +619,7 @@ int lp_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, int v
   // larger than needed over the whole queue), a line any number
   const int seg_shift = segment_shift(mode == SWR_DRAW_POINT ? std::min(nsub, c->cap_pairs) : c->cap_pairs);
   const uint32_t ncells = ntiles * SWR_SEGS;
+  const SwrCells cells = {1u, ntiles};
   LpFragArgs fa;
   fa.status = st;
   fa.cap_prims = c->cap_prims;
@@ -622,15 +633,17 @@ int lp_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, int v
   fa.keys = c->keys0.as<uint32_t>();
   fa.prims = c->vals0.as<uint32_t>();
   fa.cell_count = c->cell_count.as<uint32_t>();
+  fa.cells = cells;
   fa.seg_shift = seg_shift;
   fa.status_w = st;
   ps->lp_frags(fa, s);
   uint32_t* cstart = c->cell_start.as<uint32_t>();
-  scan_exclusive(c->cell_count.as<uint32_t>(), cstart, nullptr, ncells, cstart + ncells, scr, s);
+  scan_cells(c->cell_count.as<uint32_t>(), ntiles, cstart, c->cell_fill.as<uint32_t>(), scr, s);
   uint32_t* big = big_list(c, ncells, seg_shift);
   const uint32_t want = (c->cap_pairs + 255) / 256;
   swr::launch(k_lp_fill, want < 1216u ? (want ? want : 1u) : 1216u, 256, 0, s, st, st + SWR_ST_PAIRS, c->cap_pairs,
-              c->keys0.as<uint32_t>(), c->cell_count.as<uint32_t>(), cstart, ncells, seg_shift, c->keys1.as<uint32_t>(),
+              c->keys0.as<uint32_t>(), c->cell_count.as<uint32_t>(), c->cell_fill.as<uint32_t>(), cstart, ncells, cells, seg_shift,
+              c->keys1.as<uint32_t>(),
               big ? big + 2 : nullptr, big);
   if (big) {
     sort_big(c, cstart, ncells, seg_shift, c->keys1.as<uint32_t>(), c->vals1.as<uint32_t>(), big, s);
@@ -974,7 +987,7 @@ int swr_draw_elements(swr_context* c, int mode, uint64_t count, const uint32_t* 
   const uint32_t nbatches = (nsub + SWR_BATCH_PRIMS - 1) / SWR_BATCH_PRIMS;
   const SwrTargetDesc T = make_target(c, mode);
   const uint32_t ntiles = (uint32_t)T.tiles_x * (uint32_t)T.tiles_y;
-  int rc = ensure_capacity(c, (uint32_t)nverts, vs->S, nsub, nbatches, ntiles, ps->R > ps->lp_R ? ps->R : ps->lp_R, ps, s);
+  int rc = ensure_capacity(c, (uint32_t)nverts, vs->S, nsub, nbatches, ntiles, ps->R > ps->lp_R ? ps->R : ps->lp_R, ps, 1, s);
   if (rc) return rc;
   SwrDrawDesc D;
   fill_draw(c, D, mode);
@@ -1030,7 +1043,7 @@ int swr_draw_elements(swr_context* c, int mode, uint64_t count, const uint32_t* 
   mark(c, 2, s);
   c->last_ntiles = ntiles;
   if (mode != SWR_DRAW_TRIANGLE) return end_single(c, s, lp_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, ntiles, mode, nsub, s));
-  return end_single(c, s, raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, ntiles, s, 1,
+  return end_single(c, s, raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, ntiles, s, 1, 1,
                                        c->raster_mode != SWR_RASTER_BLOCK));
 }
 
@@ -1048,7 +1061,7 @@ int swr_draw_list(swr_context* c, int mode, const float* vertices, uint64_t nver
   const uint32_t nsub = (uint32_t)(count / per);
   const SwrTargetDesc T = make_target(c, mode);
   const uint32_t ntiles = (uint32_t)T.tiles_x * (uint32_t)T.tiles_y;
-  int rc = ensure_capacity(c, (uint32_t)nverts, ps->S, nsub, 1, ntiles, ps->R > ps->lp_R ? ps->R : ps->lp_R, ps, s);
+  int rc = ensure_capacity(c, (uint32_t)nverts, ps->S, nsub, 1, ntiles, ps->R > ps->lp_R ? ps->R : ps->lp_R, ps, 1, s);
   if (rc) return rc;
   if (!c->direct_keep.ensure((size_t)nsub * 4 + 16) || !c->direct_pos.ensure((size_t)nsub * 4 + 16))
     return SWR_ENOMEM;
@@ -1079,7 +1092,7 @@ int swr_draw_list(swr_context* c, int mode, const float* vertices, uint64_t nver
                                                c->raster_mode != SWR_RASTER_BLOCK));
   }
   if (mode != SWR_DRAW_TRIANGLE) return end_single(c, s, lp_stage(c, ps, ps->S, 8, 8 + ps->A, ps->A, ps->P, ntiles, mode, nsub, s));
-  return end_single(c, s, raster_stage(c, ps, ps->S, 8, 8 + ps->A, ps->A, ps->P, ntiles, s, 1,
+  return end_single(c, s, raster_stage(c, ps, ps->S, 8, 8 + ps->A, ps->A, ps->P, ntiles, s, 1, 1,
                                        c->raster_mode != SWR_RASTER_BLOCK));
 }
 
@@ -1187,7 +1200,7 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
     return SWR_EINVAL;
   const int ntg = (int)T.size();
   int rc = ensure_capacity(c, (uint32_t)V, vs->S, (uint32_t)P, (uint32_t)B, (uint32_t)NT,
-                           ps->R > ps->lp_R ? ps->R : ps->lp_R, ps, s);
+                           ps->R > ps->lp_R ? ps->R : ps->lp_R, ps, n, s);
   if (rc) return rc;
   bool ok = c->draws.ensure(sizeof(SwrDrawDesc) * n) && c->targets.ensure(sizeof(SwrTargetDesc) * ntg) &&
             c->draw_vbase.ensure(4 * n + 16) && c->draw_bbase.ensure(4 * n + 16) && c->draw_pbase.ensure(4 * n + 16) &&
@@ -1234,7 +1247,7 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
   mix(c->cap_prims); mix(c->cap_pairs); mix(c->cap_clip_slots); mix(c->cap_clip_verts);
   const void* bufs[] = {c->ptv.p, c->clipv.p, c->clip_table.p, c->clip_slot.p, c->tri_flags.p, c->batch_counts.p,
                         c->tris.p, c->recs.p, c->tile_count.p, c->keys0.p, c->vals0.p, c->cell_count.p,
-                        c->cell_start.p, c->scratch.p, c->draws.p, c->targets.p, c->draw_vbase.p,
+                        c->cell_start.p, c->cell_fill.p, c->scratch.p, c->draws.p, c->targets.p, c->draw_vbase.p,
                         c->draw_bbase.p, c->target_tile_base.p, c->draw_pbase.p, c->big_cells.p, h,
                         c->over_best.p, c->over_done.p, (const void*)(uintptr_t)c->slices, c->quad_flag.p, c->quad_tiles.p,
                         c->quad_count.p, c->geo_bar.p, c->dslice_state.p, c->dslice_done.p,
@@ -1303,7 +1316,7 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
     mark(c, 2, s);
     c->launches += (V ? 1 : 0) + (B ? 2 : 0);
     if (!q) q = cuda_err(cudaGetLastError());
-    rc = raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, (uint32_t)NT, s, ntg, any_span);
+    rc = raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, (uint32_t)NT, s, n, ntg, any_span);
   }
   if (q) rc = q;
   c->use_draw_pbase = false;

@@ -87,6 +87,90 @@ __global__ void __launch_bounds__(kThreads) k_scan_down(const uint32_t* in, uint
   }
 }
 
+// --- (tile, segment) cells ------------------------------------------------------------
+// Blocks own contiguous ranges of whole 32-tile groups; a group's 32 x 32 counts are read a
+// segment row at a time and turned in shared memory.
+constexpr int kGroup = 32;
+static_assert(SWR_SEGS == 32, "a group of 32 tiles is a 32 x 32 square of cells");
+
+__global__ void __launch_bounds__(kThreads) k_cells_reduce(const uint32_t* count, uint32_t ntiles, uint32_t chunk,
+                                                           uint32_t* partials) {
+  swr_pdl_entry();
+  __shared__ uint32_t tmp[32];
+  uint32_t b, e;
+  chunk_range(ntiles, chunk, b, e);
+  uint32_t s = 0;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (uint32_t seg = warp; seg < SWR_SEGS; seg += kThreads / 32) {
+    const uint32_t* row = count + (size_t)seg * ntiles;
+#pragma unroll 4
+    for (uint32_t t = b + lane; t < e; t += 32) s += row[t];
+  }
+  uint32_t tot;
+  swr_block_exscan(s, tmp, &tot);
+  if (threadIdx.x == 0) partials[blockIdx.x] = tot;
+}
+
+__global__ void __launch_bounds__(kThreads) k_cells_down(const uint32_t* count, uint32_t ntiles, uint32_t chunk,
+                                                         const uint32_t* partials, uint32_t* start,
+                                                         uint32_t* fill_start) {
+  swr_pdl_entry();
+  __shared__ uint32_t tmp[32];
+  __shared__ uint32_t sq[kGroup][SWR_SEGS + 1];
+  __shared__ uint32_t pref[2];
+  uint32_t b, e;
+  chunk_range(ntiles, chunk, b, e);
+  {
+    uint32_t mine = 0, all = 0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += kThreads) {
+      const uint32_t v = partials[i];
+      all += v;
+      if (i < (int)blockIdx.x) mine += v;
+    }
+    uint32_t t0, t1;
+    swr_block_exscan(mine, tmp, &t0);
+    swr_block_exscan(all, tmp, &t1);
+    if (threadIdx.x == 0) { pref[0] = t0; pref[1] = t1; }
+    __syncthreads();
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) start[(size_t)ntiles * SWR_SEGS] = pref[1];
+  uint32_t run = pref[0];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t tl = threadIdx.x >> 3, sg = (threadIdx.x & 7) * 4;  // this thread's four cells of a group
+  for (uint32_t t0 = b; t0 < e; t0 += kGroup) {
+    const bool on = t0 + lane < e;
+#pragma unroll
+    for (int k = 0; k < SWR_SEGS / (kThreads / 32); ++k) {
+      const uint32_t seg = warp + k * (kThreads / 32);
+      sq[lane][seg] = on ? count[(size_t)seg * ntiles + t0 + lane] : 0u;
+    }
+    __syncthreads();
+    uint32_t v[4], s = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      v[j] = sq[tl][sg + j];
+      s += v[j];
+    }
+    uint32_t tot;
+    uint32_t ex = swr_block_exscan(s, tmp, &tot) + run;  // (its barriers order the reads above)
+    uint4 o;
+    o.x = ex;
+    o.y = o.x + v[0];
+    o.z = o.y + v[1];
+    o.w = o.z + v[2];
+    if (t0 + tl < e) *(uint4*)(start + (size_t)(t0 + tl) * SWR_SEGS + sg) = o;
+    sq[tl][sg] = o.x; sq[tl][sg + 1] = o.y; sq[tl][sg + 2] = o.z; sq[tl][sg + 3] = o.w;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < SWR_SEGS / (kThreads / 32); ++k) {
+      const uint32_t seg = warp + k * (kThreads / 32);
+      if (on) fill_start[(size_t)seg * ntiles + t0 + lane] = sq[lane][seg];
+    }
+    __syncthreads();
+    run += tot;
+  }
+}
+
 uint32_t chunk_for(uint32_t n_max, int blocks) {
   uint32_t c = (n_max + blocks - 1) / blocks;
   c = (c + kTile - 1) / kTile * kTile;
@@ -223,6 +307,14 @@ void scan_exclusive(const uint32_t* in, uint32_t* out, const uint32_t* n_dev, ui
   const uint32_t chunk = chunk_for(n_max, kScanBlocks);
   swr::launch(k_scan_reduce, kScanBlocks, kThreads, 0, s, in, n_dev, n_max, chunk, scratch);
   swr::launch(k_scan_down, kScanBlocks, kThreads, 0, s, in, out, n_dev, n_max, chunk, scratch, total);
+}
+
+void scan_cells(const uint32_t* count, uint32_t ntiles, uint32_t* start, uint32_t* fill_start, uint32_t* scratch,
+                cudaStream_t s) {
+  const uint32_t groups = (ntiles + kGroup - 1) / kGroup;
+  const uint32_t chunk = (groups + kScanBlocks - 1) / kScanBlocks * kGroup;
+  swr::launch(k_cells_reduce, kScanBlocks, kThreads, 0, s, count, ntiles, chunk, scratch);
+  swr::launch(k_cells_down, kScanBlocks, kThreads, 0, s, count, ntiles, chunk, scratch, start, fill_start);
 }
 
 size_t sort_scratch_words(uint32_t) { return 2 * 256 * kSortBlocks + 256; }

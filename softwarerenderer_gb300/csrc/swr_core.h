@@ -18,6 +18,12 @@ size_t scan_scratch_words(uint32_t n_max);
 void scan_exclusive(const uint32_t* in, uint32_t* out, const uint32_t* n_dev, uint32_t n_max,
                     uint32_t* total, uint32_t* scratch, cudaStream_t s);
 
+// Exclusive scan of the binning's (tile, segment) counts, in tile-major order (a tile's cells
+// are consecutive).  `count` and `fill_start` are segment-major (SwrCells), `start` is
+// tile-major with the total at start[ntiles * SWR_SEGS].  scratch: kScanBlocks words.
+void scan_cells(const uint32_t* count, uint32_t ntiles, uint32_t* start, uint32_t* fill_start, uint32_t* scratch,
+                cudaStream_t s);
+
 // Stable LSD radix sort of (key, value) pairs by the low `bits` bits of key; three kernels
 // per 8-bit pass (block histograms, per-digit offsets, stable scatter).
 // n = min(*n_dev, n_max).  Ping-pongs between (k0,v0) and (k1,v1); returns 0 when the

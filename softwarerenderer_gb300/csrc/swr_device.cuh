@@ -147,6 +147,20 @@ struct SwrClipEntry {
   uint16_t _pad;
 };
 
+// Place of a (tile, segment) counter and fill position, in one of two layouts.
+//   segment-major (1, ntiles), single draws: primitives close in submission order share a
+//     segment and a primitive's tiles are runs of neighbours, so a warp's atomics fall into few
+//     128-byte lines.  Against tile-major, the Benchmark program's 3.8M entries: k_setup 85 ->
+//     37 us, k_fill_bins 132 -> 85; the 1M-triangle soup's: 98 -> 82 and 210 -> 139.
+//   tile-major (SWR_SEGS, 1), batches of several items: the items being processed at one time
+//     lie in one or two segments, whose counters would share few 32-byte sectors: on 256
+//     meshes k_setup took 265 us segment-major, 194 us tile-major.
+// The raster's starts are always tile-major: a tile's bin is one range.
+struct SwrCells {
+  uint32_t tile_stride, seg_stride;
+  __device__ __forceinline__ uint32_t at(uint32_t tile, uint32_t seg) const { return tile * tile_stride + seg * seg_stride; }
+};
+
 // Index of the last element of sorted `base[0..n)` that is <= key.
 __device__ __forceinline__ int swr_find_le(const uint32_t* base, int n, uint32_t key) {
   int lo = 0, hi = n - 1;

@@ -244,6 +244,7 @@ struct LpFragArgs {
   uint32_t* keys;             // per fragment: tile * 256 + pixel in the tile, or SWR_LP_INVALID
   uint32_t* prims;            // per fragment: its primitive
   uint32_t* cell_count;       // per (tile, segment): fragments
+  SwrCells cells;
   int seg_shift;              // segment = fragment number >> seg_shift
   uint32_t* status_w;
 };
@@ -286,7 +287,7 @@ __global__ void __launch_bounds__(256) k_lp_frags(LpFragArgs g) {
       g.keys[f] = key;
       g.prims[f] = prim;
     }
-    const uint32_t cell = key != SWR_LP_INVALID ? (key >> 8) * SWR_SEGS + (f >> g.seg_shift) : SWR_LP_INVALID;
+    const uint32_t cell = key != SWR_LP_INVALID ? g.cells.at(key >> 8, f >> g.seg_shift) : SWR_LP_INVALID;
     const uint32_t peers = __match_any_sync(0xffffffffu, cell);  // neighbours share cells
     if (cell != SWR_LP_INVALID && lane == __ffs(peers) - 1) atomicAdd(&g.cell_count[cell], (uint32_t)__popc(peers));
   };
@@ -342,8 +343,9 @@ __global__ void __launch_bounds__(256) k_lp_frags(LpFragArgs g) {
 // not fit a raster chunk for k_sort_big (big_list holds every cell; null: none are listed).
 static __global__ void __launch_bounds__(256) k_lp_fill(const uint32_t* status, const uint32_t* nfrags,
                                                         uint32_t cap_frags, const uint32_t* keys,
-                                                        uint32_t* cell_count, const uint32_t* cell_start,
-                                                        uint32_t ncells, int seg_shift, uint32_t* bin,
+                                                        uint32_t* cell_count, const uint32_t* fill_start,
+                                                        const uint32_t* cell_start, uint32_t ncells,
+                                                        SwrCells cells, int seg_shift, uint32_t* bin,
                                                         uint32_t* big_list, uint32_t* big_count) {
   swr_pdl_entry();
   if (status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;  // (k_lp_frags counted nothing then)
@@ -353,13 +355,13 @@ static __global__ void __launch_bounds__(256) k_lp_fill(const uint32_t* status, 
   for (uint32_t f0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; f0 < nf; f0 += stride) {
     const uint32_t f = f0 + (uint32_t)lane;
     const uint32_t key = f < nf ? keys[f] : SWR_LP_INVALID;
-    const uint32_t cell = key != SWR_LP_INVALID ? (key >> 8) * SWR_SEGS + (f >> seg_shift) : SWR_LP_INVALID;
+    const uint32_t cell = key != SWR_LP_INVALID ? cells.at(key >> 8, f >> seg_shift) : SWR_LP_INVALID;
     const uint32_t peers = __match_any_sync(0xffffffffu, cell);
     const int leader = __ffs(peers) - 1;
     uint32_t pos = 0;
     if (cell != SWR_LP_INVALID && lane == leader) {
       const uint32_t n = (uint32_t)__popc(peers);
-      pos = cell_start[cell] + atomicSub(&cell_count[cell], n) - n;
+      pos = fill_start[cell] + atomicSub(&cell_count[cell], n) - n;
     }
     pos = __shfl_sync(0xffffffffu, pos, leader);
     if (cell != SWR_LP_INVALID) bin[pos + (uint32_t)__popc(peers & ((1u << lane) - 1u))] = f;

@@ -33,10 +33,11 @@ void run_pairs(const uint32_t* status, uint32_t cap_prims, const float* recs, co
 
 template <class PS>
 void run_fill(const uint32_t* status, uint32_t cap_prims, const float* recs,
-              uint32_t* cell_count, const uint32_t* cell_start, uint32_t ncells, int seg_shift, uint32_t cap_pairs,
+              uint32_t* cell_count, const uint32_t* fill_start, const uint32_t* pairs, uint32_t ncells, SwrCells cells, int seg_shift,
+              uint32_t cap_pairs,
               const SwrDrawDesc* draws, const SwrTargetDesc* targets, int tile, uint32_t* bin, uint32_t* status_w,
               cudaStream_t s) {
-  swr::launch(k_fill_bins<PS>, kGrid, 256, 0, s, status, cap_prims, recs, cell_count, cell_start, ncells,
+  swr::launch(k_fill_bins<PS>, kGrid, 256, 0, s, status, cap_prims, recs, cell_count, fill_start, pairs, ncells, cells,
                                         seg_shift, cap_pairs, draws, targets, tile, bin, status_w);
 }
 

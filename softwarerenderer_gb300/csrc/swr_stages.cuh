@@ -652,6 +652,7 @@ struct SetupArgs {
   uint32_t* tile_count;
   int tile;  // tile edge in pixels
   uint32_t* cell_count;  // per (tile, primitive segment): bin entries (counted with atomics)
+  SwrCells cells;
   int seg_shift;         // primitive segment = primitive index >> seg_shift (< SWR_SEGS)
   uint32_t* boxes;       // small draws (null otherwise): per primitive its packed tile box instead of
                          // cell counts (SWR_NO_BOX: no tile); bin entries are summed in the status
@@ -950,14 +951,14 @@ __global__ void __launch_bounds__(kSetupThreads) k_setup(SetupArgs g) {
       const uint32_t seg = p >> g.seg_shift;
       for (int i = 0; i < cnt; ++i) {
         const int tx = tx0 + (i < tnx ? i : i - tnx), ty = ty0 + (i < tnx ? 0 : 1);
-        atomicAdd(&g.cell_count[(tbase + (uint32_t)(ty * tiles_x + tx)) * SWR_SEGS + seg], 1u);
+        atomicAdd(&g.cell_count[g.cells.at(tbase + (uint32_t)(ty * tiles_x + tx), seg)], 1u);
       }
     } else {
       const uint32_t pw = p0 + (threadIdx.x & ~31u);
       warp_tiles(cnt, tnx, tx0, ty0, tbase, tiles_x, [&](const int (&owner)[4], const uint32_t (&tile)[4], const bool (&on)[4]) {
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-          if (on[u]) atomicAdd(&g.cell_count[tile[u] * SWR_SEGS + ((pw + (uint32_t)owner[u]) >> g.seg_shift)], 1u);
+          if (on[u]) atomicAdd(&g.cell_count[g.cells.at(tile[u], (pw + (uint32_t)owner[u]) >> g.seg_shift)], 1u);
       });
     }
   }
@@ -1016,8 +1017,8 @@ __global__ void __launch_bounds__(256) k_emit_pairs(const uint32_t* status, uint
 // the fill order is arbitrary and k_sort_cells restores increasing primitive order.
 template <class PS>
 __global__ void __launch_bounds__(256) k_fill_bins(const uint32_t* status, uint32_t cap_prims, const float* recs,
-                                                   uint32_t* cell_count,
-                                                   const uint32_t* cell_start, uint32_t ncells, int seg_shift,
+                                                   uint32_t* cell_count, const uint32_t* fill_start,
+                                                   const uint32_t* pairs, uint32_t ncells, SwrCells cells, int seg_shift,
                                                    uint32_t cap_pairs, const SwrDrawDesc* draws,
                                                    const SwrTargetDesc* targets, int tile, uint32_t* bin,
                                                    uint32_t* status_w) {
@@ -1025,7 +1026,7 @@ __global__ void __launch_bounds__(256) k_fill_bins(const uint32_t* status, uint3
   typedef Rec<PS> RL;
   // cell_count is all zero between draws: every entry counted by k_setup is taken back
   // here, and a draw that stops early zeroes the counts instead
-  const uint32_t total = cell_start[ncells];
+  const uint32_t total = *pairs;
   const bool overflow = status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW;
   if (overflow || total > cap_pairs) {
     if (!overflow && blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1071,9 +1072,9 @@ __global__ void __launch_bounds__(256) k_fill_bins(const uint32_t* status, uint3
     }
     const uint32_t seg = p >> seg_shift;
     auto put = [&](uint32_t prim, uint32_t pseg, uint32_t tb, int tw, int tx, int ty) {
-      const uint32_t cell = (tb + (uint32_t)(ty * tw + tx)) * SWR_SEGS + pseg;
+      const uint32_t cell = cells.at(tb + (uint32_t)(ty * tw + tx), pseg);
       const uint32_t pos = atomicSub(&cell_count[cell], 1u) - 1u;
-      bin[cell_start[cell] + pos] = prim;
+      bin[fill_start[cell] + pos] = prim;
     };
     if (__reduce_max_sync(0xffffffffu, (uint32_t)cnt) <= 2u) {
       // small primitives (the common case): every lane its own tiles
@@ -1084,8 +1085,8 @@ __global__ void __launch_bounds__(256) k_fill_bins(const uint32_t* status, uint3
       uint32_t at[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const uint32_t cell = tile[u] * SWR_SEGS + ((p0 + (uint32_t)owner[u]) >> seg_shift);
-        if (on[u]) at[u] = cell_start[cell] + atomicSub(&cell_count[cell], 1u) - 1u;
+        const uint32_t cell = cells.at(tile[u], (p0 + (uint32_t)owner[u]) >> seg_shift);
+        if (on[u]) at[u] = fill_start[cell] + atomicSub(&cell_count[cell], 1u) - 1u;
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u)
