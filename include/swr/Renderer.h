@@ -244,7 +244,6 @@ struct UserPS {
     s.winner = -1;
   }
   __device__ static void store(const State&, int, int, const SwrUniforms&) {}
-  __device__ static bool earlyReject(float, State&) { return false; }
   template <class PD>
   __device__ static Color shade(const PD&, const SwrUniforms&) {
     return 0u;  // never used: nothing is shaded ahead of drawPixel (NoCompact)

@@ -14,12 +14,9 @@
 // Pixel shader contract: static AVarCount, PVarCount, InterpolateZ, InterpolateW
 // (PixelShaderBase.h:44-53), a per-pixel State that the reference keeps in the
 // shader's own static buffers (with `frags` and `writes` counters), and
-// load / drawPixel / store / earlyReject / shade / apply.  earlyReject(z, s) returns true
-// when drawPixel with depth z would do nothing but count the fragment (a failing depth
-// test); it then counts it itself, so the rasterizer may skip building the other
-// interpolants.  Every built-in drawPixel is apply(s, z, shade(p, u), prim) with shade a
+// load / drawPixel / store / shade / apply.  Every built-in drawPixel is apply(s, z, shade(p, u), prim) with shade a
 // pure function of the fragment and the uniforms (evaluated only when it is used), so the
-// rasterizer may compute shade() for a fragment early and apply() it in primitive order.  drawPixel is the
+// rasterizer may compute shade() for a fragment at another time and apply() it in primitive order.  drawPixel is the
 // reference's drawPixel(const PixelData&) (PixelShaderBase.h:116); load/store move
 // the pixel's framebuffer values between memory and State.  Calling
 // load + drawPixel + store per fragment is exactly the reference's side effect; the
@@ -166,15 +163,6 @@ struct SwrStateRGBA32F {
   int32_t winner;
 };
 
-// Early depth rejection shared by the depth-tested shaders: their drawPixel does only
-// `s.frags++` when !(z < s.depth).
-template <class State>
-SWR_HD bool swr_depth_reject(float z, State& s) {
-  if (z < s.depth) return false;
-  s.frags++;
-  return true;
-}
-
 // Colour write of the RGBA8 depth-tested shaders, and their drawPixel in apply() form.
 SWR_HD void swr_write(SwrStateRGBA8& s, float z, uint32_t c, int prim) {
   s.depth = z;
@@ -220,11 +208,10 @@ SWR_HD uint32_t swr_tex_nearest(const SwrUniforms& u, float tu, float tv) {
 
 // Textured, depth-tested (config: textured cube).  PVar = uv.
 struct PsTexNearest {
-  enum { AVarCount = 0, PVarCount = 2, InterpolateZ = 1, InterpolateW = 1, HasDepth = 1, DepthMin = 1 };
+  enum { AVarCount = 0, PVarCount = 2, InterpolateZ = 1, InterpolateW = 1, HasDepth = 1, RasterOccupancy = 5, DepthMin = 1 };
   typedef SwrStateRGBA8 State;
   SWR_HD static void load(State& s, int x, int y, const SwrUniforms& u) { swr_load_rgba8<true>(s, x, y, u); }
   SWR_HD static void store(const State& s, int x, int y, const SwrUniforms& u) { swr_store_rgba8(s, x, y, u, true); }
-  SWR_HD static bool earlyReject(float z, State& s) { return swr_depth_reject(z, s); }
   typedef uint32_t Color;
   template <class PD>
   SWR_HD static Color shade(const PD& p, const SwrUniforms& u) {
@@ -241,14 +228,13 @@ struct PsTexNearest {
 // Lambert-lit procedural checker, depth-tested (config: dense icosphere).
 // AVar = normal, PVar = uv.
 struct PsLambert {
-  // 128-primitive chunks: on the dense 1080p mesh 2 % faster than 64 (fewer chunk passes in
-  // the silhouette tiles that set the raster's length); 64 suits the other workloads
-  enum { AVarCount = 3, PVarCount = 2, InterpolateZ = 1, InterpolateW = 1, HasDepth = 1, RasterOccupancy = 5,
+  // 128-primitive chunks: the dense 1080p mesh takes 112 us a frame, 127 with 96 and 135 with
+  // 64 (its heavy tiles, more than a chunk, then outnumber the run slots); 64 suits the others
+  enum { AVarCount = 3, PVarCount = 2, InterpolateZ = 1, InterpolateW = 1, HasDepth = 1, RasterOccupancy = 6,
          DepthCull = 0, RasterChunk = 128, DepthMin = 1, RasterSlices = 1 };
   typedef SwrStateRGBA8 State;
   SWR_HD static void load(State& s, int x, int y, const SwrUniforms& u) { swr_load_rgba8<true>(s, x, y, u); }
   SWR_HD static void store(const State& s, int x, int y, const SwrUniforms& u) { swr_store_rgba8(s, x, y, u, true); }
-  SWR_HD static bool earlyReject(float z, State& s) { return swr_depth_reject(z, s); }
   SWR_HD static float intensity(float n0, float n1, float n2, const SwrUniforms& u) {
     const float len2 = swr_add(swr_add(swr_mul(n0, n0), swr_mul(n1, n1)), swr_mul(n2, n2));
     float d = 0.0f;
@@ -283,11 +269,10 @@ struct PsLambert {
 // Lambert-lit and textured (nearest RGBA8), depth-tested (config: batched meshes).
 struct PsLambertTex {
   enum { AVarCount = 3, PVarCount = 2, InterpolateZ = 1, InterpolateW = 1, HasDepth = 1, RasterOccupancy = 6,
-         DepthCull = 0, DepthMin = 1 };
+         RasterOccupancyBlock = 7, DepthCull = 0, DepthMin = 1 };
   typedef SwrStateRGBA8 State;
   SWR_HD static void load(State& s, int x, int y, const SwrUniforms& u) { swr_load_rgba8<true>(s, x, y, u); }
   SWR_HD static void store(const State& s, int x, int y, const SwrUniforms& u) { swr_store_rgba8(s, x, y, u, true); }
-  SWR_HD static bool earlyReject(float z, State& s) { return swr_depth_reject(z, s); }
   typedef uint32_t Color;
   template <class PD>
   SWR_HD static Color shade(const PD& p, const SwrUniforms& u) {
@@ -307,11 +292,10 @@ struct PsLambertTex {
 
 // Perspective-correct vertex colour, depth-tested (config: triangle soup).  PVar = rgb.
 struct PsVColor {
-  enum { AVarCount = 0, PVarCount = 3, InterpolateZ = 1, InterpolateW = 1, HasDepth = 1, DepthMin = 1 };
+  enum { AVarCount = 0, PVarCount = 3, InterpolateZ = 1, InterpolateW = 1, HasDepth = 1, RasterOccupancy = 5, DepthMin = 1 };
   typedef SwrStateRGBA8 State;
   SWR_HD static void load(State& s, int x, int y, const SwrUniforms& u) { swr_load_rgba8<true>(s, x, y, u); }
   SWR_HD static void store(const State& s, int x, int y, const SwrUniforms& u) { swr_store_rgba8(s, x, y, u, true); }
-  SWR_HD static bool earlyReject(float z, State& s) { return swr_depth_reject(z, s); }
   typedef uint32_t Color;
   template <class PD>
   SWR_HD static Color shade(const PD& p, const SwrUniforms&) {
@@ -333,7 +317,6 @@ struct PsVColorAffine {
   typedef SwrStateRGBA8 State;
   SWR_HD static void load(State& s, int x, int y, const SwrUniforms& u) { swr_load_rgba8<false>(s, x, y, u); }
   SWR_HD static void store(const State& s, int x, int y, const SwrUniforms& u) { swr_store_rgba8(s, x, y, u, false); }
-  SWR_HD static bool earlyReject(float, State&) { return false; }
   typedef uint32_t Color;
   template <class PD>
   SWR_HD static Color shade(const PD& p, const SwrUniforms&) {
@@ -379,7 +362,7 @@ SWR_HD void swr_tex_bilinear_f32(const SwrUniforms& u, float tu, float tv, float
 // Differentiable-rendering shader: colour = vertex rgb * bilinear(texture, uv), RGBA32F
 // target, depth-tested.  PVar = {r, g, b, u, v}.
 struct PsDiff {
-  enum { AVarCount = 0, PVarCount = 5, InterpolateZ = 1, InterpolateW = 1, HasDepth = 1, RasterOccupancy = 5,
+  enum { AVarCount = 0, PVarCount = 5, InterpolateZ = 1, InterpolateW = 1, HasDepth = 1, RasterOccupancy = 6,
          DepthCull = 0 };
   typedef SwrStateRGBA32F State;
   SWR_HD static void load(State& s, int x, int y, const SwrUniforms& u) {
@@ -390,7 +373,6 @@ struct PsDiff {
     s.writes = 0u;
     s.winner = -1;
   }
-  SWR_HD static bool earlyReject(float z, State& s) { return swr_depth_reject(z, s); }
   SWR_HD static void store(const State& s, int x, int y, const SwrUniforms& u) {
     const size_t i = (size_t)y * (size_t)u.width + (size_t)x;
     if (s.writes) {
@@ -594,7 +576,6 @@ struct PsTexMip {
   typedef SwrStateRGBA8 State;
   SWR_HD static void load(State& s, int x, int y, const SwrUniforms& u) { swr_load_rgba8<false>(s, x, y, u); }
   SWR_HD static void store(const State& s, int x, int y, const SwrUniforms& u) { swr_store_rgba8(s, x, y, u, false); }
-  SWR_HD static bool earlyReject(float, State&) { return false; }
   typedef uint32_t Color;
   template <class PD>
   SWR_HD static Color shade(const PD& p, const SwrUniforms& u) {
@@ -621,7 +602,6 @@ struct PsPerspDeriv {
   enum { AVarCount = 0, PVarCount = 2, InterpolateZ = 1, InterpolateW = 1, HasDepth = 1, NeedsEquations = 1 };
   typedef SwrStateRGBA32F State;
   SWR_HD static void load(State& s, int x, int y, const SwrUniforms& u) { PsDiff::load(s, x, y, u); }
-  SWR_HD static bool earlyReject(float z, State& s) { return swr_depth_reject(z, s); }
   SWR_HD static void store(const State& s, int x, int y, const SwrUniforms& u) { PsDiff::store(s, x, y, u); }
   typedef PsDiff::Color Color;
   template <class PD>
@@ -670,14 +650,13 @@ struct SwrOverwrite<PS, decltype((void)PS::Overwrite)> {
   enum { value = PS::Overwrite };
 };
 
-// Depth-tested shaders (HasDepth, InterpolateZ, earlyReject = swr_depth_reject): a fragment
+// Depth-tested shaders (HasDepth, InterpolateZ): a fragment
 // with !(z < State::depth) only counts, and a write only lowers State::depth.  A rasterizer
 // may therefore count, without interpolating, every fragment of a primitive whose z is
 // provably not below the largest depth held by the pixels it covers.  A shader may opt out
-// with DepthCull = 0.  The Lambert and differentiable shaders do: their tile rasters run at
-// 5-6 CTAs per SM in 40-48 registers, where the cull's code made the Lambert rasters 3-5 %
-// slower on their single-mesh workloads (which have nothing to cull) and the differentiable
-// one spill.
+// with DepthCull = 0.  The Lambert and differentiable shaders do: their single-mesh workloads
+// have nothing to cull, and the cull's code takes registers from rasters that run at 6-7 CTAs
+// per SM.
 template <class PS, class = void>
 struct SwrDepthCull {
   enum { value = PS::HasDepth && PS::InterpolateZ && !SwrOverwrite<PS>::value };
@@ -733,14 +712,27 @@ SWR_HD void swr_depth_merge(SwrStateRGBA8& acc, const SwrStateRGBA8& later) {
 }
 
 // Resident tile-raster CTAs per SM the register allocation of a shader's k_raster must
-// allow (RasterOccupancy in the shader; measured per workload, default 4).
+// allow: RasterOccupancy in the shader (default 4), and RasterOccupancyBlock for submissions
+// of Block-mode draws alone where that differs.  Measured per workload, whole draws at 4 / 5 /
+// 6 / 7 CTAs per SM: vertex colour (4K soup) 4401 / 4217 / 4339 / 4569 us; Lambert (dense
+// 1080p mesh) 119.7 / 115.6 / 112.7 / 120.2; Lambert-textured in Block mode (256 meshes) 3914 /
+// 3524 / 3292 / 3172, in Span mode (20k triangles) 81 / 80 / 79 / 88; differentiable (16
+// views) 619 / 592 / 577 / 602.
 template <class PS, class = void>
-struct SwrRasterOccupancy {
+struct SwrRasterOccupancySpan {
   enum { value = 4 };
 };
 template <class PS>
-struct SwrRasterOccupancy<PS, decltype((void)PS::RasterOccupancy)> {
+struct SwrRasterOccupancySpan<PS, decltype((void)PS::RasterOccupancy)> {
   enum { value = PS::RasterOccupancy };
+};
+template <class PS, class = void>
+struct SwrRasterOccupancy {
+  enum { value = SwrRasterOccupancySpan<PS>::value, block = value };
+};
+template <class PS>
+struct SwrRasterOccupancy<PS, decltype((void)PS::RasterOccupancyBlock)> {
+  enum { value = SwrRasterOccupancySpan<PS>::value, block = PS::RasterOccupancyBlock };
 };
 
 // Pixel shaders whose drawPixel has side effects beyond its State (user shaders that write

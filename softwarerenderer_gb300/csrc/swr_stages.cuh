@@ -1359,24 +1359,102 @@ __device__ __forceinline__ int block_class(const float* r, int flags, int bx, in
   return 2;
 }
 
-// Row `row` of drawBlock<true> (PixelShaderBase.h:64-93): the row start is the block
-// corner's edge value stepped `row` times by b (eo.stepY), pixels step by a (ei.stepX).
-// Returns the row's 8 coverage bits.
-__device__ __forceinline__ uint32_t block_row_bits(const float* r, int flags, int bx, int by, int row) {
+// Four rows, 4 * half to 4 * half + 3, of drawBlock<true> (PixelShaderBase.h:64-93): the row
+// start is the block corner's edge value stepped row by row by b (eo.stepY), pixels step by a
+// (ei.stepX).  Returns the rows' coverage bits, 8 per row.  Four rows a lane: their starts
+// follow from each other (a row of its own costs a lane 21 predicated steps to reach it),
+// and a chunk's partial blocks still fill the CTA.
+__device__ __forceinline__ uint32_t block_rows_bits(const float* r, int flags, int bx, int by, int half) {
   const float fx = swr_add((float)bx, 0.5f), fy = swr_add((float)by, 0.5f);
-  const bool tie0 = (flags >> 2) & 1, tie1 = (flags >> 3) & 1, tie2 = (flags >> 4) & 1;
-  float i0 = fold7(swr_eval(r[6], r[7], r[8], fx, fy), r[7], row);
-  float i1 = fold7(swr_eval(r[9], r[10], r[11], fx, fy), r[10], row);
-  float i2 = fold7(swr_eval(r[12], r[13], r[14], fx, fy), r[13], row);
+  const float t0 = (flags & 4) ? 0.0f : 0x1p-149f, t1 = (flags & 8) ? 0.0f : 0x1p-149f;
+  const float t2 = (flags & 16) ? 0.0f : 0x1p-149f;  // thresholds of edge_test
+  const float a0 = r[6], b0 = r[7], a1 = r[9], b1 = r[10], a2 = r[12], b2 = r[13];
+  float i0 = swr_eval(a0, b0, r[8], fx, fy), i1 = swr_eval(a1, b1, r[11], fx, fy), i2 = swr_eval(a2, b2, r[14], fx, fy);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    i0 = half ? swr_add(i0, b0) : i0;
+    i1 = half ? swr_add(i1, b1) : i1;
+    i2 = half ? swr_add(i2, b2) : i2;
+  }
   uint32_t m = 0;
 #pragma unroll
-  for (int col = 0; col < SWR_BLOCK; ++col) {
-    if (edge_test(i0, tie0) && edge_test(i1, tie1) && edge_test(i2, tie2)) m |= 1u << col;
-    i0 = swr_add(i0, r[6]);
-    i1 = swr_add(i1, r[9]);
-    i2 = swr_add(i2, r[12]);
+  for (int row = 0; row < 4; ++row) {
+    float c0 = i0, c1 = i1, c2 = i2;
+#pragma unroll
+    for (int col = 0; col < SWR_BLOCK; ++col) {
+      if (c0 >= t0 && c1 >= t1 && c2 >= t2) m |= 1u << (row * 8 + col);
+      c0 = swr_add(c0, a0);
+      c1 = swr_add(c1, a1);
+      c2 = swr_add(c2, a2);
+    }
+    i0 = swr_add(i0, b0);
+    i1 = swr_add(i1, b1);
+    i2 = swr_add(i2, b2);
   }
   return m;
+}
+
+// Runs of pixels a Span-mode primitive covers inside the pixel rectangle [x0, x1) x [y0, y1)
+// (x0 a multiple of 8, the rectangle inside the target), by one thread straight from words 0-19
+// of its setup record: run(y, xa, xb, xs) for pixels [xa, xb) of row y, xs the row's span
+// start.  The coverage of k_raster's masks: each row's span inside the box's 8-px blocks.
+template <class Run>
+__device__ __forceinline__ void span_runs(const float4& q0, const float4& q1, const float4& q2, const float4& q3,
+                                          const float4& q4, int sc_minx, int sc_maxx, int x0, int x1, int y0, int y1,
+                                          Run run) {
+  const int flags = __float_as_int(q0.x);
+  const int ylo = max(__float_as_int(q0.w), y0), yhi = min(__float_as_int(q1.y) + 1, y1);
+  const int cx0 = max(__float_as_int(q0.z) & ~(SWR_BLOCK - 1), x0);
+  const int cx1 = min((__float_as_int(q1.x) | (SWR_BLOCK - 1)) + 1, x1);
+  SpanHalf bot, top;
+  bot.y0 = __float_as_int(q1.z); bot.y1 = __float_as_int(q1.w);
+  bot.ox = q2.x; bot.oy = q2.y; bot.is1 = q2.z; bot.is2 = q2.w;
+  top.y0 = __float_as_int(q3.x); top.y1 = __float_as_int(q3.y);
+  top.ox = q3.z; top.oy = q3.w; top.is1 = q4.x; top.is2 = q4.y;
+  for (int y = ylo; y < yhi; ++y) {
+    const bool in_bot = (flags & 32) && y >= bot.y0 && y < bot.y1;
+    const bool in_top = (flags & 64) && y > top.y1 && y <= top.y0;
+    if (!in_bot && !in_top) continue;
+    int xl, xr;
+    span_row(in_bot ? bot : top, y, sc_minx, sc_maxx, xl, xr);
+    const int xa = max(xl, cx0), xb = min(xr, cx1);
+    if (xb > xa) run(y, xa, xb, xl);
+  }
+}
+
+// The same of rows [ylo, yhi) of one Block-mode block at (bx, by), wx pixels of it wide, of
+// class cls (block_class; 1 whole, 2 by the stepped edge tests, as block_rows_bits):
+// run(y, xa, xb).
+template <class Run>
+__device__ __forceinline__ void block_runs(const float* r, int flags, int cls, int bx, int by, int wx, int ylo,
+                                           int yhi, Run run) {
+  const float t0 = (flags & 4) ? 0.0f : 0x1p-149f, t1 = (flags & 8) ? 0.0f : 0x1p-149f;
+  const float t2 = (flags & 16) ? 0.0f : 0x1p-149f;  // thresholds of edge_test
+  const float fx = swr_add((float)bx, 0.5f), fy = swr_add((float)by, 0.5f);
+  float i0 = swr_eval(r[6], r[7], r[8], fx, fy), i1 = swr_eval(r[9], r[10], r[11], fx, fy);
+  float i2 = swr_eval(r[12], r[13], r[14], fx, fy);
+  for (int y = by; y < yhi; ++y) {
+    uint32_t m = (1u << wx) - 1u;
+    if (cls == 2) {
+      float c0 = i0, c1 = i1, c2 = i2;
+#pragma unroll
+      for (int col = 0; col < SWR_BLOCK; ++col) {
+        if (!(c0 >= t0 && c1 >= t1 && c2 >= t2)) m &= ~(1u << col);
+        c0 = swr_add(c0, r[6]);
+        c1 = swr_add(c1, r[9]);
+        c2 = swr_add(c2, r[12]);
+      }
+      i0 = swr_add(i0, r[7]);
+      i1 = swr_add(i1, r[10]);
+      i2 = swr_add(i2, r[13]);
+    }
+    if (y < ylo) continue;
+    while (m) {  // the row's runs (one, up to rounding)
+      const int a = __ffs(m) - 1, b = a + __ffs(~(m >> a)) - 1;
+      m &= ~0u << b;
+      run(y, bx + a, bx + b);
+    }
+  }
 }
 
 // Primitive id handed to the pixel shader: the index within its own draw.
@@ -1384,18 +1462,16 @@ __device__ __forceinline__ int prim_id(const RasterArgs& g, const float* rec, ui
   return (int)(p - (g.draw_prim_base ? g.draw_prim_base[__float_as_int(rec[1])] : 0u));
 }
 
-// Position (0-63) of the j-th set bit of m (j < popcount(m)).
-__device__ __forceinline__ int nth_bit64(uint64_t m, int j) {
-  int off = 0;
-  uint32_t w = (uint32_t)m;
-  int c = __popc(w);
-  if (j >= c) { j -= c; w = (uint32_t)(m >> 32); off = 32; }
-  c = __popc(w & 0xffffu); if (j >= c) { j -= c; w >>= 16; off += 16; }
-  c = __popc(w & 0xffu);   if (j >= c) { j -= c; w >>= 8; off += 8; }
-  c = __popc(w & 0xfu);    if (j >= c) { j -= c; w >>= 4; off += 4; }
-  c = __popc(w & 0x3u);    if (j >= c) { j -= c; w >>= 2; off += 2; }
-  if (j >= (int)(w & 1u)) off += 1;
-  return off;
+// 32 x 32 bits turned across a warp: lane l brings row l, lane p leaves with column p (bit l =
+// bit p of lane l's row).
+__device__ __forceinline__ uint32_t warp_transpose(uint32_t x, int lane) {
+  uint32_t m = 0x0000ffffu;
+#pragma unroll
+  for (int j = 16; j; j >>= 1, m ^= m << j) {
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+    x = (lane & j) ? ((x & ~m) | ((y & ~m) >> j)) : ((x & m) | ((y & m) << j));
+  }
+  return x;
 }
 
 // Rebuilds the reference's incrementally stepped PixelData for pixel (x, y): the value
@@ -1468,77 +1544,113 @@ __device__ __forceinline__ float build_z(const float* eq, bool blockmode, float 
   return blockmode ? fold7(fold7(e, q3[1], kb), q3[0], ka) : swr_fold(e, q3[0], ka);
 }
 
+// PixelData of pixel (x, y) of the primitive with setup record r (in global memory); pd.z is
+// the caller's.
+template <class PS, bool SPAN>
+__device__ __forceinline__ void pixel_of_record(const float* r, const SwrDrawDesc* draws, int x, int y, GpuPixel<PS>& pd) {
+  typedef Rec<PS> RL;
+  const int flags = __float_as_int(r[0]);
+  const bool blockmode = !SPAN || (flags & 2);
+  float fx, fy;
+  int ka, kb;
+  if (blockmode) {
+    fx = swr_add((float)(x & ~7), 0.5f);
+    fy = swr_add((float)(y & ~7), 0.5f);
+    ka = x & 7;
+    kb = y & 7;
+  } else {  // from its row's span start
+    const SwrDrawDesc& D = draws[__float_as_int(r[1])];
+    const bool in_bot = (flags & 32) && y >= __float_as_int(r[6]) && y < __float_as_int(r[7]);
+    SpanHalf h;
+    h.ox = in_bot ? r[8] : r[14]; h.oy = in_bot ? r[9] : r[15];
+    h.is1 = in_bot ? r[10] : r[16]; h.is2 = in_bot ? r[11] : r[17];
+    int xl, xr;
+    span_row(h, y, D.sc_minx, D.sc_maxx, xl, xr);
+    fx = swr_add((float)xl, 0.5f);
+    fy = swr_add((float)y, 0.5f);
+    ka = x - xl;
+    kb = 0;
+  }
+  pd.x = x;
+  pd.y = y;
+  pd.eq = r + RL::EQ0;
+  build_pixel<PS>(pd.eq, blockmode, fx, fy, ka, kb, pd);
+}
+
 // One CTA per screen tile, 256 threads.  Per chunk of CH primitives of the tile's bin:
-//   A. stage the setup records in shared memory;
-//   B. exact coverage masks per (primitive, 8x8 block): one thread per pair classifies
-//      Block-mode blocks (the reference's corner test) and builds Span-mode rows from
-//      [xl, xr) (kept as each row's interpolation start); partially covered blocks are then
-//      finished by 8 lanes each, one row per lane, with the reference's stepped edge tests;
-//   C0. depth-tested shaders: per 8 x 4 pixel region, primitives whose z cannot pass any
-//      depth test of the chunk there (z_not_below against the region's largest depth) are
-//      only counted;
-//   C1. small primitives (<= 64 covered pixels in the tile, up to FB fragments per chunk)
-//      are compacted: one thread per covered fragment rebuilds the stepped interpolants and
-//      evaluates the pixel shader's pure shade() at full SIMT width;
-//   C2. each thread walks the chunk in primitive order for the pixels it owns and applies
-//      every covering fragment to the pixel's register-resident State: compacted fragments
-//      through apply(), others by rebuilding the interpolants in place (z first: a failing
-//      depth test needs nothing else) and drawPixel().
+//   A. stage in shared memory what coverage and depth need of the setup records.  Shaders with
+//      the depth cull, behind depths already written: only of primitives that may show; a
+//      thread per bin entry decides (verdict), and the others are only counted;
+//   B. exact coverage masks per (primitive, 8 x 8 block): one thread per pair classifies
+//      Block-mode blocks (the reference's corner test); one thread per four rows builds
+//      Span-mode rows from [xl, xr) (kept as each row's interpolation start) and finishes
+//      partially covered blocks with the reference's stepped edge tests;
+//   C0. depth cull: per 8 x 4 pixel region, primitives whose z cannot pass any depth test of
+//      the chunk there (z_not_below against the region's largest depth) are only counted;
+//   C2. each thread visits, in primitive order, the primitives covering the pixels it owns:
+//      the stepped z and the depth test against the pixel's register-resident State.  Shaders
+//      with side effects of their own run drawPixel() there instead.
+// At the end of the tile every pixel is shaded once, from the record of the last primitive
+// that passed its depth test.  Bound by SM issue and by the latency of the short stages
+// between barriers.
+//   Against shading fragments ahead of their depth tests, small primitives' compacted one
+// fragment per thread (whole draws): 4K soup 5212 -> 4217 us, 60k-triangle list 283 -> 207,
+// 256 meshes 3202 -> 3172, 16 differentiable views 637 -> 596, dense 1080p mesh 117 -> 113.
 // DIRECT: the raster of a small draw, which has no bins (RasterArgs.boxes).
 // A heavy tile of a depth-min shader (RasterArgs.dslice) is run by up to SWR_DSLICES CTAs,
 // each over its own run of whole chunks from the draw's starting State; the last run to
 // finish merges the runs' States in bin order (swr_depth_merge) and stores.
 template <class PS, int TILE, int CH, bool SPAN, bool DIRECT = false>
-__global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRasterOccupancy<PS>::value)
+__global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
+                                       : SPAN            ? SwrRasterOccupancy<PS>::value
+                                                         : SwrRasterOccupancy<PS>::block)
     k_raster(RasterArgs g) {
   swr_pdl_entry();
   typedef Rec<PS> RL;
-  typedef typename PS::Color Color;
   constexpr int PPT = TILE * TILE / 256;  // pixels per thread
   constexpr int NBX = TILE / SWR_BLOCK;   // blocks per tile row
   constexpr int NB = NBX * NBX;
-  constexpr bool kCompact = !SwrNoCompact<PS>::value;
-  constexpr int FB = !kCompact ? 32 : (sizeof(Color) > 4 ? 512 : 1024);  // compacted fragments per chunk
-  constexpr int SMALL = 64;
-  __shared__ float4 srec4[CH * RL::R / 4];
+  constexpr bool kCull = SWR_DEPTH_CULL && SwrDepthCull<PS>::value;
+  // Shaders without side effects are shaded once per pixel, after the tile's depth tests: a
+  // fragment that passes only records its primitive, and the last one that did is shaded from
+  // its record.
+  constexpr bool kDefer = !SwrNoCompact<PS>::value;
+  static_assert(!kDefer || (PS::HasDepth && RL::IZ), "a deferred fragment is one that passes the depth test");
+  // Staged records: words 0-23 where only coverage and z are read (header, edges or span
+  // halves, the z equation), 28 words apart so that the lanes' different records spread over
+  // the banks; else whole.
+  constexpr int RW4 = kDefer ? 6 : RL::R / 4, SR4 = kDefer ? 7 : RL::R / 4, SR = SR4 * 4;
+  static_assert(RL::EQ0 + 3 * RL::EQ_Z + 3 <= 24, "the z equation lies in the first 24 words");
+  __shared__ float4 srec4[CH * SR4];
   float* srec = (float*)srec4;
   __shared__ uint64_t smask[CH * NB];
   __shared__ int2 sspan[SPAN ? CH * TILE : 1];  // Span mode: each tile row's [xl, xr)
   __shared__ uint32_t sids[CH];
-  __shared__ uint32_t sex[CH];   // compacted-fragment base (monotone over the chunk)
-  __shared__ uint8_t scomp[CH];  // 1: compacted
-  __shared__ float sfz[FB];
-  __shared__ Color sfc[FB];
   __shared__ uint32_t sfr[32];
-  __shared__ uint32_t snc;
-  __shared__ uint32_t suncomp;  // some primitive of the chunk covers pixels and was not compacted
+  __shared__ uint32_t slast;  // sliced heavy tile: this run is the last to finish
   __shared__ uint16_t spart[CH * NB];  // partially covered (primitive, block) pairs
   __shared__ uint32_t snpart;
   __shared__ uint32_t ssorted[SWR_RASTER_SORT];  // the tile's ordered bin (self-sorted tiles)
   __shared__ uint32_t scs[SWR_SEGS + 1];          // its cell starts relative to the bin start
   static_assert(sizeof(srec4) >= SWR_RASTER_SORT * 4, "raw bin staging fits the record area");
-  constexpr bool kCull = SWR_DEPTH_CULL && SwrDepthCull<PS>::value;
   // Depth cull regions: the 8 x 4 pixels of one warp in one sub-tile (region q * 8 + warp).
   constexpr int NREG = 8 * PPT;
   __shared__ uint32_t swd[NREG];  // per region: order key of the largest depth it holds
-  __shared__ uint32_t scull_on;   // some region holds no +inf depth (0: nothing can be culled)
+  // Depth cull: the next primitives to rasterize, in order (up to CH - 1 left over plus a batch
+  // of 256), and per pixel row the coverage of primitives that were only counted (+1 at a run's
+  // first pixel, -1 past its last; used where the target records counts)
+  __shared__ uint32_t ssurv[kCull ? CH + 256 : 1];
+  // a batch's primitives to count: Span ones from the front, Block ones from the back; their
+  // partially covered blocks (entry * NB + block)
+  __shared__ uint32_t scul[kCull ? 256 : 1];
+  constexpr int SCP = 1024;
+  __shared__ uint16_t scp[kCull ? SCP : 1];
+  __shared__ int scnt[kCull ? TILE * (TILE + 1) : 1];
   constexpr int NW = CH / 32;      // 32-primitive words of a chunk
   static_assert(CH % 32 == 0 && CH <= 128, "chunks of 32, 64, 96 or 128 primitives");
   __shared__ uint32_t sculr[kCull ? NREG * NW : 1];  // per region: primitives only counted there
   __shared__ int sminx[kCull && SPAN ? CH : 1];  // Span mode: leftmost start of a span reaching the tile
-  // Per-pixel walk (shaders without the depth cull): each pixel keeps
-  // the set of compacted primitives covering it (set in C1), so in C2 every lane visits only
-  // its own pixel's primitives instead of all primitives touching its warp's half block.
   constexpr int HW = (CH + 63) / 64;  // 64-primitive words of a chunk
-  // (Not for the depth-culling shaders: measured on the 4K soup, whose chunks mix compacted
-  // small primitives with large ones, the per-lane loops cost 30 % more raster time.)
-  constexpr bool kPixWalk = SWR_PIX_WALK && kCompact && !kCull;
-  __shared__ uint64_t spm[kPixWalk ? TILE * TILE * HW : 1];
-  // per (primitive, block): the primitive's covered pixels in the tile's earlier blocks, so a
-  // compacted fragment's slot is sex + spre + its rank in the block's mask (a compacted
-  // primitive covers at most SMALL = 64 pixels of the tile: its prefixes fit a byte)
-  __shared__ uint8_t spre[kCompact ? CH * NB : 1];
-  __shared__ int32_t spid[CH];  // the primitives' ids as drawPixel sees them
   if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint32_t frags = 0, passes = 0;
@@ -1669,30 +1781,119 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
       ssorted[pos < ntot ? pos : 0] = v;
     }
   }
-  while (true) {  // once; small draws: per gathered run of the tile's primitives
-  for (uint32_t c0 = cb; c0 < ce; c0 += CH) {
-    const int n = (int)min((uint32_t)CH, ce - c0);
-    __syncthreads();  // the previous chunk's shared state is no longer read; ssorted is complete
-    if (threadIdx.x < n) sids[threadIdx.x] = self_sort ? ssorted[c0 - b + threadIdx.x] : g.bin[c0 + threadIdx.x];
-    if (threadIdx.x == 0) snpart = 0;
-    if constexpr (kPixWalk) {
+  // the CTA's pixels: the tile or its quadrant, inside the target
+  const int rx0 = ox + (quad < 0 ? 0 : (quad % NBX) * SWR_BLOCK), ry0 = oy + (quad < 0 ? 0 : (quad / NBX) * SWR_BLOCK);
+  const int rx1 = min(rx0 + (quad < 0 ? TILE : SWR_BLOCK), T.width), ry1 = min(ry0 + (quad < 0 ? TILE : SWR_BLOCK), T.height);
+  const bool counts = U.frag_count != nullptr;  // per-pixel drawPixel counts are recorded
+  bool cull_on = false;  // some region holds no +inf depth (else nothing can be culled)
+  uint32_t stands[PPT];  // kDefer: the last primitive to pass the pixel's depth test (none: ~0)
 #pragma unroll
-      for (int q = 0; q < PPT; ++q)
-#pragma unroll
-        for (int w = 0; w < HW; ++w) spm[((py[q] - oy) * TILE + (px[q] - ox)) * HW + w] = 0ull;
+  for (int q = 0; q < PPT; ++q) stands[q] = 0xffffffffu;
+  auto bin_id = [&](uint32_t i) { return self_sort ? ssorted[i - b] : __ldg(g.bin + i); };
+  // Whether a primitive's fragments here all fail their depth tests for certain -- its z is
+  // provably not below the largest depth of any region its box meets (z_not_below, as C0, over
+  // the box instead of the covered pixels): 1 a Span, 2 a Block primitive that need only be
+  // counted, 0 one to rasterize, 3 one that covers nothing here.
+  auto verdict = [&](uint32_t p) -> int {
+    const float4* rc = (const float4*)(g.recs + (size_t)p * RL::R);
+    const float4 q0 = __ldg(rc), q1 = __ldg(rc + 1), q4 = __ldg(rc + 4);
+    const float zc = __ldg(&rc[5].x);
+    const int flags = __float_as_int(q0.x);
+    const int x0 = max(__float_as_int(q0.z), rx0), x1 = min(__float_as_int(q1.x), rx1 - 1);
+    const int y0 = max(__float_as_int(q0.w), ry0), y1 = min(__float_as_int(q1.y), ry1 - 1);
+    if (!(flags & 1) || x0 > x1 || y0 > y1) return 3;
+    // Span pixels are stepped from their row's start.  Within a half a row's start is a
+    // monotone function of the row (every operation of span_row is, for finite slopes), so none
+    // lies left of the box, which spans the end rows' -- or of the scissor, where the box is
+    // cut off at 0.
+    int smin = 0;
+    if (SPAN && !(flags & 2)) {
+      const float4 q2 = __ldg(rc + 2);
+      if (!(fabsf(q2.z) < 0x1p100f && fabsf(q4.x) < 0x1p100f)) return 0;
+      smin = __float_as_int(q0.z);
+      if (smin <= 0) smin = min(0, g.draws[__float_as_int(q0.y)].sc_minx);
     }
-    if (kCull && SPAN && threadIdx.x < CH) sminx[threadIdx.x] = 0x7fffffff;
-    // Region depth bounds at the chunk's start (depth-tested shaders, tiles of more than one
-    // chunk): per region an order-preserving key of the largest depth its pixels hold (NaN
-    // depths, which every fragment fails, and pixels outside the target are ignored; key 0:
-    // none usable).  A region holding +inf can cull nothing (z is finite); the barrier's OR
-    // tells whether any region can.
-    int any_ok = 0;
-    bool cull_tile = false;
-    bool my_ok = false;
+    for (int cy = (y0 - oy) >> 2; cy <= (y1 - oy) >> 2; ++cy)
+      for (int cx = (x0 - ox) >> 3; cx <= (x1 - ox) >> 3; ++cx) {
+        // region of the 8 x 4 cell (cx, cy): sub-tile, then the warp that owns it
+        const int reg = ((cy >> 2) * (TILE / 16) + (cx >> 1)) * 8 + ((cx & 1) + ((cy >> 1) & 1) * 2) * 2 + (cy & 1);
+        const uint32_t key = swd[reg];
+        if (key == 0u || key >= 0xff800000u) return 0;
+        const float dmax = __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
+        const int xa = max(x0, ox + cx * 8), xb = min(x1, ox + cx * 8 + 7);
+        const int ya = max(y0, oy + cy * 4), yb = min(y1, oy + cy * 4 + 3);
+        int steps = 2 * (SWR_BLOCK - 1);
+        float X = (float)xb + 0.5f;
+        if (SPAN && !(flags & 2)) {
+          steps = max(0, xb - smin);
+          if (smin < 0) X = fmaxf(X, (float)(-smin) + 0.5f);
+        }
+        const float fyb = (float)yb + 0.5f;
+        if (!z_not_below(q4.z, q4.w, zc, (float)xa + 0.5f, (float)xb + 0.5f, (float)ya + 0.5f, fyb, X, fyb, steps, dmax))
+          return 0;
+      }
+    return SPAN && !(flags & 2) ? 1 : 2;
+  };
+  auto add_run = [&](int y, int xa, int xb) {  // pixels [xa, xb) of row y: covered once more, failing
+    frags += (uint32_t)(xb - xa);
+    if (counts) {
+      atomicAdd(&scnt[(y - oy) * (TILE + 1) + xa - ox], 1);
+      atomicAdd(&scnt[(y - oy) * (TILE + 1) + xb - ox], -1);
+    }
+  };
+  // Counts the listed primitives: ns Span ones a thread each, nb Block ones a thread per 8 x 8
+  // block, then a thread per partially covered block.
+  auto count_listed = [&](int ns, int nb) {
+    if constexpr (SPAN) {
+      for (int i = threadIdx.x; i < ns; i += 256) {
+        const float4* rc = (const float4*)(g.recs + (size_t)scul[i] * RL::R);
+        const float4 q0 = __ldg(rc);
+        const SwrDrawDesc& D = g.draws[__float_as_int(q0.y)];
+        span_runs(q0, __ldg(rc + 1), __ldg(rc + 2), __ldg(rc + 3), __ldg(rc + 4), D.sc_minx, D.sc_maxx, rx0, rx1, ry0,
+                  ry1, [&](int y, int xa, int xb, int) { add_run(y, xa, xb); });
+      }
+    }
+    auto count_block = [&](int i, bool classify) -> int {
+      const int j = i % NB;
+      const int bx = ox + (j % NBX) * SWR_BLOCK, by = oy + (j / NBX) * SWR_BLOCK;
+      const float4* rc = (const float4*)(g.recs + (size_t)scul[255 - i / NB] * RL::R);
+      const float4 q0 = __ldg(rc), q1 = __ldg(rc + 1), q2 = __ldg(rc + 2), q3 = __ldg(rc + 3);
+      const float r[15] = {0, 0, 0, 0, 0, 0, q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, q3.x, q3.y, q3.z};
+      int cls = 2;
+      if (classify) {
+        if (bx < rx0 || bx >= rx1 || by < ry0 || by >= ry1 || bx > __float_as_int(q1.x) || by > __float_as_int(q1.y) ||
+            bx + SWR_BLOCK - 1 < __float_as_int(q0.z) || by + SWR_BLOCK - 1 < __float_as_int(q0.w))
+          return 0;
+        cls = block_class(r, __float_as_int(q0.x), bx, by);
+        if (cls == 0 || cls == 2) return cls;
+      }
+      block_runs(r, __float_as_int(q0.x), cls, bx, by, min(SWR_BLOCK, rx1 - bx), by, min(by + SWR_BLOCK, ry1), add_run);
+      return 1;
+    };
+    for (int i = threadIdx.x; i < nb * NB; i += 256)
+      if (count_block(i, true) == 2) {
+        const uint32_t at = atomicAdd(&snpart, 1u);
+        if (at < SCP) scp[at] = (uint16_t)i; else count_block(i, false);
+      }
+    __syncthreads();
+    const int m = min((int)snpart, SCP);
+    for (int t = threadIdx.x; t < m; t += 256) count_block(scp[t], false);
+  };
+  if (kCull && counts)
+    for (int i = threadIdx.x; i < TILE * (TILE + 1); i += 256) scnt[i] = 0;  // (first used past the next barrier)
+  while (true) {  // once; small draws: per gathered run of the tile's primitives
+  uint32_t c0 = cb;        // next bin entry
+  uint32_t nsurv = 0;      // depth cull: primitives waiting in ssurv
+  while (c0 < ce || nsurv) {
+    __syncthreads();  // the previous chunk's shared state is no longer read; ssorted is complete
+    int n;
     if constexpr (kCull) {
-      cull_tile = ce - cb > (uint32_t)CH;
-      if (cull_tile) {
+      // Region depth bounds (tiles of more than one chunk): per region an order-preserving key
+      // of the largest depth its pixels hold (NaN depths, which every fragment fails, and
+      // pixels outside the target are ignored; key 0: none usable).  A region holding +inf can
+      // cull nothing (z is finite); the barrier's OR tells whether any region can.
+      if (ce - cb > (uint32_t)CH) {
+        bool my_ok = false;
 #pragma unroll
         for (int q = 0; q < PPT; ++q) {
           const float dq = swr_state_depth(st[q]);
@@ -1702,30 +1903,86 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
           if (lane == 0) swd[q * 8 + warp] = key;
           my_ok |= key != 0u && key < 0xff800000u;  // uniform per warp
         }
+        cull_on = __syncthreads_or(my_ok);
       }
+      // The next chunk's primitives.  Behind depths already written, one thread per entry
+      // counts the primitives that cannot show, and only the others are kept (in order).
+      while (nsurv < (uint32_t)CH && c0 < ce) {
+        if (!cull_on) {
+          const uint32_t take = min((uint32_t)CH - nsurv, ce - c0);
+          if (threadIdx.x < take) ssurv[nsurv + threadIdx.x] = bin_id(c0 + threadIdx.x);
+          nsurv += take;
+          c0 += take;
+          continue;
+        }
+        const uint32_t take = min(256u, ce - c0);
+        uint32_t p = 0;
+        int v = 3;
+        if (threadIdx.x < take) {
+          p = bin_id(c0 + threadIdx.x);
+          v = verdict(p);
+        }
+        const uint32_t lt_mask = (1u << lane) - 1u;
+        const uint32_t bk = __ballot_sync(0xffffffffu, v == 0), bs = __ballot_sync(0xffffffffu, v == 1);
+        const uint32_t bb = __ballot_sync(0xffffffffu, v == 2);
+        __syncthreads();  // the previous batch's lists are no longer read
+        if (lane == 0) scs[warp] = (uint32_t)(__popc(bk) | __popc(bs) << 8 | __popc(bb) << 16);
+        if (threadIdx.x == 0) snpart = 0;
+        __syncthreads();
+        uint32_t at_k = nsurv;
+        int ns = 0, nb = 0, at_s = 0, at_b = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+          const uint32_t c = scs[w];
+          if (w < warp) {
+            at_k += c & 255u;
+            at_s += (int)((c >> 8) & 255u);
+            at_b += (int)(c >> 16);
+          }
+          nsurv += c & 255u;
+          ns += (int)((c >> 8) & 255u);
+          nb += (int)(c >> 16);
+        }
+        if (v == 0) ssurv[at_k + (uint32_t)__popc(bk & lt_mask)] = p;
+        if (v == 1) scul[at_s + __popc(bs & lt_mask)] = p;
+        if (v == 2) scul[255 - at_b - __popc(bb & lt_mask)] = p;
+        __syncthreads();
+        count_listed(ns, nb);
+        c0 += take;
+      }
+      __syncthreads();
+      if (nsurv == 0) break;
+      n = (int)min((uint32_t)CH, nsurv);
+      if (threadIdx.x < n) sids[threadIdx.x] = ssurv[threadIdx.x];
+    } else {
+      n = (int)min((uint32_t)CH, ce - c0);
+      if (threadIdx.x < n) sids[threadIdx.x] = bin_id(c0 + threadIdx.x);
     }
-    // A: the chunk's setup records (ids read from the bin directly: sids is published by
-    // the barrier below)
+    if (threadIdx.x == 0) snpart = 0;
+    if (kCull && SPAN && threadIdx.x < CH) sminx[threadIdx.x] = 0x7fffffff;
+    // A: the chunk's setup records (ids read from their source: sids is published by the
+    // barrier below)
     {
-      constexpr int R4 = RL::R / 4;
       const float4* recs4 = (const float4*)g.recs;
 #pragma unroll 4
-      for (int i = threadIdx.x; i < n * R4; i += 256) {
-        const int k = i / R4, w = i - k * R4;
-        const uint32_t id = self_sort ? ssorted[c0 - b + k] : __ldg(g.bin + c0 + k);
-        srec4[i] = recs4[(size_t)id * R4 + w];
+      for (int i = threadIdx.x; i < n * RW4; i += 256) {
+        const int k = i / RW4, w = i - k * RW4;
+        const uint32_t id = kCull ? ssurv[k] : bin_id(c0 + k);
+        srec4[k * SR4 + w] = recs4[(size_t)id * (RL::R / 4) + w];
       }
     }
-    if (cull_tile)
-      any_ok = __syncthreads_or(my_ok);
-    else
-      __syncthreads();
+    __syncthreads();
+    uint32_t left = 0;  // depth cull: this thread's share of the primitives waiting after this chunk
+    if constexpr (kCull) {
+      if (threadIdx.x + n < nsurv) left = ssurv[threadIdx.x + n];
+    } else {
+      c0 += n;
+    }
     // B1: coverage per (primitive, block).  Fully covered / skipped blocks and Span rows are
     // finished here; partially covered Block-mode blocks are queued for B2.
-    if (kCull && threadIdx.x == 0) scull_on = any_ok;
     for (int i = threadIdx.x; i < n * NB; i += 256) {
       const int k = i / NB, j = i - k * NB;
-      const float* r = srec + k * RL::R;
+      const float* r = srec + k * SR;
       const int flags = __float_as_int(r[0]);
       if (SPAN && (flags & 3) == 1) continue;  // Span mode: rows below, masks after the barrier
       if (quad >= 0 && j != quad) {  // another CTA's quadrant
@@ -1744,78 +2001,69 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
       smask[i] = m;
     }
     if constexpr (SPAN) {
-      // B1 (Span mode): each tile row's span [xl, xr) of every primitive, once per row (kept
-      // as the row's interpolation start); the rows of one primitive are consecutive lanes,
-      // and whole warps iterate (the row reduction below shuffles across the warp)
-      for (int i = threadIdx.x; i < (n * TILE + 31) / 32 * 32; i += 256) {
-        const int k = i / TILE, row = i - k * TILE;
-        const float* r = srec + k * RL::R;
-        const int flags = k < n ? __float_as_int(r[0]) : 0;
-        int2 sp = make_int2(1, 0);
-        const int y = oy + row;
-        if ((flags & 3) == 1 && y >= __float_as_int(r[3]) && y <= __float_as_int(r[5])) {
-          SpanHalf h;
-          bool any = true;
-          if ((flags & 32) && y >= __float_as_int(r[6]) && y < __float_as_int(r[7])) {
-            h.ox = r[8]; h.oy = r[9]; h.is1 = r[10]; h.is2 = r[11];
-          } else if ((flags & 64) && y > __float_as_int(r[13]) && y <= __float_as_int(r[12])) {
-            h.ox = r[14]; h.oy = r[15]; h.is1 = r[16]; h.is2 = r[17];
-          } else {
-            any = false;
-          }
-          if (any) {
-            const SwrDrawDesc& D = g.draws[__float_as_int(r[1])];
-            span_row(h, y, D.sc_minx, D.sc_maxx, sp.x, sp.y);
-          }
-        }
-        if ((flags & 3) == 1) sspan[k * TILE + row] = sp;
-        if (kCull) {
-          // leftmost start of a span reaching the tile, over the primitive's TILE rows
-          int lmin = (sp.x < sp.y && sp.y > ox) ? sp.x : 0x7fffffff;
-#pragma unroll
-          for (int o = TILE / 2; o; o >>= 1) lmin = min(lmin, __shfl_xor_sync(0xffffffffu, lmin, o));
-          if (row == 0 && lmin != 0x7fffffff) atomicMin(&sminx[k], lmin);
-        }
-      }
-      __syncthreads();
-      // B1 (Span mode) masks from the spans: each row's [xl, xr) clipped to the block
-      for (int i = threadIdx.x; i < n * NB; i += 256) {
-        const int k = i / NB, j = i - k * NB;
-        const float* r = srec + k * RL::R;
+      // B1 (Span mode): four rows of a primitive per thread: each row's span [xl, xr), kept as the
+      // row's interpolation start, and its half of the masks of the blocks it crosses
+      constexpr int NR = TILE / 4;
+      for (int i = threadIdx.x; i < n * NR; i += 256) {
+        const int k = i / NR, br = i - k * NR;
+        const float* r = srec + k * SR;
         const int flags = __float_as_int(r[0]);
         if ((flags & 3) != 1) continue;
-        if (quad >= 0 && j != quad) {
-          smask[i] = 0;
-          continue;
-        }
-        const int bx = ox + (j % NBX) * SWR_BLOCK, by = oy + (j / NBX) * SWR_BLOCK;
-        const bool hit = bx <= __float_as_int(r[4]) && bx + SWR_BLOCK - 1 >= __float_as_int(r[2]) &&
-                         by <= __float_as_int(r[5]) && by + SWR_BLOCK - 1 >= __float_as_int(r[3]);
-        uint64_t m = 0;
-        if (hit) {
+        const int rows0 = __float_as_int(r[3]), rows1 = __float_as_int(r[5]);
+        const SwrDrawDesc& D = g.draws[__float_as_int(r[1])];
+        const int minx = D.sc_minx, maxx = D.sc_maxx;
+        const int ya = oy + br * 4;
+        uint32_t m[NBX];
 #pragma unroll
-          for (int rr = 0; rr < SWR_BLOCK; ++rr) {
-            const int2 sp = sspan[k * TILE + (by - oy) + rr];
-            const int c0b = max(sp.x, bx) - bx, c1b = min(sp.y, bx + SWR_BLOCK) - bx;
-            if (c1b > c0b) m |= (((1ull << (c1b - c0b)) - 1ull) << c0b) << (rr * 8);
+        for (int j = 0; j < NBX; ++j) m[j] = 0u;
+        int lmin = 0x7fffffff;  // leftmost start of a span reaching the tile
+#pragma unroll
+        for (int rr = 0; rr < 4; ++rr) {
+          const int y = ya + rr;
+          int2 sp = make_int2(1, 0);
+          if (y >= rows0 && y <= rows1) {
+            const bool in_bot = (flags & 32) && y >= __float_as_int(r[6]) && y < __float_as_int(r[7]);
+            const bool in_top = (flags & 64) && y > __float_as_int(r[13]) && y <= __float_as_int(r[12]);
+            if (in_bot || in_top) {
+              SpanHalf h;
+              h.ox = in_bot ? r[8] : r[14]; h.oy = in_bot ? r[9] : r[15];
+              h.is1 = in_bot ? r[10] : r[16]; h.is2 = in_bot ? r[11] : r[17];
+              span_row(h, y, minx, maxx, sp.x, sp.y);
+            }
+          }
+          sspan[k * TILE + br * 4 + rr] = sp;
+          if (sp.x < sp.y && sp.y > ox) lmin = min(lmin, sp.x);
+#pragma unroll
+          for (int j = 0; j < NBX; ++j) {
+            const int bx = ox + j * SWR_BLOCK;
+            const int c0b = min(max(sp.x, bx), bx + SWR_BLOCK) - bx, c1b = min(max(sp.y, bx), bx + SWR_BLOCK) - bx;
+            // columns [c0b, c1b): none where c1b <= c0b
+            m[j] |= ((0xffu << c0b) & ~(0xffffffffu << c1b) & 0xffu) << (rr * 8);
           }
         }
-        smask[i] = m;
+#pragma unroll
+        for (int j = 0; j < NBX; ++j) {
+          const int bx = ox + j * SWR_BLOCK, jj = (br >> 1) * NBX + j;
+          const bool hit = bx <= __float_as_int(r[4]) && bx + SWR_BLOCK - 1 >= __float_as_int(r[2]) && (quad < 0 || jj == quad);
+          ((uint32_t*)&smask[k * NB + jj])[br & 1] = hit ? m[j] : 0u;
+        }
+        if (kCull && lmin != 0x7fffffff) atomicMin(&sminx[k], lmin);
       }
-    } else {
-      __syncthreads();
     }
-    // B2: partially covered blocks, one row per lane (8 lanes per block); each lane stores
-    // its row's byte of the block's mask (bit row * 8 + col of the little-endian word)
+    __syncthreads();
+    if constexpr (kCull) {  // the waiting primitives move up
+      if (threadIdx.x + n < nsurv) ssurv[threadIdx.x] = left;
+      nsurv -= n;
+    }
+    // B2: partially covered blocks, four rows per lane: one half of the block's mask
     {
-      const int np8 = (int)snpart * SWR_BLOCK;
-      for (int t = threadIdx.x; t < np8; t += 256) {
-        const int i = spart[t >> 3];
-        const int row = t & 7;
+      const int np2 = (int)snpart * 2;
+      for (int t = threadIdx.x; t < np2; t += 256) {
+        const int i = spart[t >> 1];
         const int k = i / NB, j = i - k * NB;
-        const float* r = srec + k * RL::R;
-        ((uint8_t*)&smask[i])[row] = (uint8_t)block_row_bits(r, __float_as_int(r[0]), ox + (j % NBX) * SWR_BLOCK,
-                                                             oy + (j / NBX) * SWR_BLOCK, row);
+        const float* r = srec + k * SR;
+        ((uint32_t*)&smask[i])[t & 1] = block_rows_bits(r, __float_as_int(r[0]), ox + (j % NBX) * SWR_BLOCK,
+                                                        oy + (j / NBX) * SWR_BLOCK, t & 1);
       }
     }
     __syncthreads();
@@ -1823,11 +2071,11 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
     // provably not below the region's largest depth at the chunk's start (z_not_below over
     // the covered pixels' box in the region).  Depths only decrease, so such fragments fail
     // their depth tests: the primitive is only counted there.
-    if (kCull && scull_on) {
+    if (kCull && cull_on) {
       for (int t = threadIdx.x; t < NREG * CH; t += 256) {
         const int reg = t / CH, k = t - reg * CH;  // reg uniform per warp (CH is a multiple of 32)
         bool culled = false;
-        if (k < n && (__float_as_int(srec[k * RL::R]) & 1)) {
+        if (k < n && (__float_as_int(srec[k * SR]) & 1)) {
           const int q = reg >> 3, w = reg & 7, hb = w >> 1;
           const int lx0 = (q % (TILE / 16)) * 16 + (hb & 1) * 8;
           const int ly0 = (q / (TILE / 16)) * 16 + (hb >> 1) * 8 + (w & 1) * 4;
@@ -1840,7 +2088,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
             c &= 0xffu;
             const int x0 = ox + lx0 + __ffs(c) - 1, x1 = ox + lx0 + 31 - __clz(c);
             const int y0 = oy + ly0 + ((__ffs(mh) - 1) >> 3), y1 = oy + ly0 + ((31 - __clz(mh)) >> 3);
-            const float* r = srec + k * RL::R;
+            const float* r = srec + k * SR;
             // walk bounds: Block mode steps <= 7 rows then <= 7 columns inside the block;
             // Span mode steps from the row's span start (every covered pixel lies in a row
             // whose span reaches the tile) to the pixel
@@ -1862,241 +2110,41 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
       }
       __syncthreads();
     }
-    // C1 set-up (one thread per primitive in warps 0..NW-1, warp 0 scans): compact the small
-    // primitives' fragments (a prefix of the chunk's small primitives whose fragments fit in
-    // FB), leaving out primitives culled in every region they cover.
-    if (warp < NW) {
-      const bool try_cull = kCull && scull_on;
-      // cnt: the primitive's covered pixels in the tile; culled: culled in every region it
-      // covers (its fragments are then left out of the compaction)
-      auto prim_info = [&](int k, uint32_t& cnt, bool& culled) {
-        cnt = 0;
-        culled = false;
-        if (k >= n) return;
-        const float* r = srec + k * RL::R;
-        spid[k] = prim_id(g, r, sids[k]);
-        if (!(__float_as_int(r[0]) & 1)) return;
-        for (int j = 0; j < NB; ++j) {
-          const uint64_t m = smask[k * NB + j];
-          if (kCompact) spre[k * NB + j] = (uint8_t)min(cnt, 255u);
-          cnt += __popc((uint32_t)m) + __popc((uint32_t)(m >> 32));
-        }
-        if (kCull && try_cull && cnt) {
-          bool all = true;
-          for (int reg = 0; reg < NREG; ++reg) {
-            const int q = reg >> 3, w = reg & 7, hb = w >> 1;
-            const int lx0 = (q % (TILE / 16)) * 16 + (hb & 1) * 8;
-            const int ly0 = (q / (TILE / 16)) * 16 + (hb >> 1) * 8 + (w & 1) * 4;
-            const uint32_t mh = (uint32_t)(smask[k * NB + (ly0 >> 3) * NBX + (lx0 >> 3)] >> ((w & 1) * 32));
-            if (mh && !((sculr[reg * NW + (k >> 5)] >> (k & 31)) & 1u)) all = false;
-          }
-          culled = all;
-        }
-      };
-      // warps 0..NW-1 measure primitives warp * 32 + lane; warp 0 scans all of them
-      uint32_t cnt0;
-      bool cul0;
-      prim_info(threadIdx.x, cnt0, cul0);
-      if (warp > 0) {  // hand the primitive to warp 0 through sex / scomp
-        sex[threadIdx.x] = cnt0;
-        scomp[threadIdx.x] = cul0;
-      }
-      if (NW > 1) asm volatile("bar.sync 1, %0;" ::"r"(CH) : "memory");  // warps 0..NW-1 only
-      if (warp == 0) {
-        // Behind depths already written (a cull tile past its first chunk) most fragments fail
-        // their depth test: shading them ahead of the test (compaction) would be wasted, the
-        // in-place path tests z first.
-        const bool deep = kCull && scull_on;
-        uint32_t cnt[NW], cand[NW], inc[NW];
-        bool cul[NW];
-#pragma unroll
-        for (int w = 0; w < NW; ++w) {
-          cnt[w] = w ? sex[w * 32 + lane] : cnt0;
-          cul[w] = w ? scomp[w * 32 + lane] != 0 : cul0;
-          cand[w] = kCompact && cnt[w] <= SMALL && !cul[w] && !deep ? cnt[w] : 0u;
-          inc[w] = cand[w];
-        }
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {  // inclusive scans over lanes
-#pragma unroll
-          for (int w = 0; w < NW; ++w) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, inc[w], o);
-            if (lane >= o) inc[w] += y;
-          }
-        }
-        uint32_t carry = 0, hi = 0;
-        bool unc = false;
-#pragma unroll
-        for (int w = 0; w < NW; ++w) {
-          const uint32_t ex = carry + inc[w] - cand[w];
-          carry += __shfl_sync(0xffffffffu, inc[w], 31);
-          const bool comp = kCompact && !cul[w] && !deep && cnt[w] <= SMALL && ex + cnt[w] <= FB;
-          if (w * 32 + lane < n) {
-            sex[w * 32 + lane] = ex;
-            scomp[w * 32 + lane] = comp ? 1 : 0;
-          }
-          if (comp && cnt[w]) hi = max(hi, ex + cnt[w]);
-          unc |= !comp && cnt[w] != 0u;
-        }
-        const uint32_t nc_max = __reduce_max_sync(0xffffffffu, hi);
-        const bool any_unc = __any_sync(0xffffffffu, unc);
-        if (lane == 0) {
-          snc = nc_max;
-          suncomp = any_unc ? 1u : 0u;
-        }
-      }
-    }
-    __syncthreads();
-    // C1: interpolate and shade the compacted fragments
-    const int nc = (int)snc;
-    for (int f = threadIdx.x; f < nc; f += 256) {
-      int lo = 0, hi = n - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if ((int)sex[mid] <= f) lo = mid; else hi = mid - 1;
-      }
-      const int k = lo;
-      int jj = f - (int)sex[k];
-      const uint64_t* mk = smask + k * NB;
-      int blkj = 0;
-      for (; blkj < NB - 1; ++blkj) {
-        const int c = __popcll(mk[blkj]);
-        if (jj < c) break;
-        jj -= c;
-      }
-      const int bit = nth_bit64(mk[blkj], jj);
-      const int x = ox + (blkj % NBX) * SWR_BLOCK + (bit & 7);
-      const int y = oy + (blkj / NBX) * SWR_BLOCK + (bit >> 3);
-      const float* r = srec + k * RL::R;
-      const bool blockmode = !SPAN || (__float_as_int(r[0]) & 2);
-      float fx, fy;
-      int ka, kb;
-      if (blockmode) {
-        fx = swr_add((float)(x & ~7), 0.5f);
-        fy = swr_add((float)(y & ~7), 0.5f);
-        ka = x & 7;
-        kb = y & 7;
-      } else {
-        const int2 sp = sspan[k * TILE + (y - oy)];
-        fx = swr_add((float)sp.x, 0.5f);
-        fy = swr_add((float)y, 0.5f);
-        ka = x - sp.x;
-        kb = 0;
-      }
-      const float* eq = r + RL::EQ0;
-      GpuPixel<PS> pd;
-      pd.x = x;
-      pd.y = y;
-      pd.eq = eq;
-      pd.z = build_z<PS>(eq, blockmode, fx, fy, ka, kb);
-      build_pixel<PS>(eq, blockmode, fx, fy, ka, kb, pd);
-      sfz[f] = pd.z;
-      sfc[f] = PS::shade(pd, g.draws[__float_as_int(r[1])].u);
-      if constexpr (kPixWalk)
-        atomicOr((unsigned long long*)&spm[((y - oy) * TILE + (x - ox)) * HW + (k >> 6)], 1ull << (k & 63));
-    }
-    __syncthreads();
-    // C2: fragments in primitive order.  Each warp owns one 8 x 4 half block per sub-tile
-    // q; a ballot over the chunk gives the primitives whose masks touch it, visited in
-    // increasing order (per-pixel order = primitive order).
+    // C2: fragments in primitive order.  Each warp owns one 8 x 4 half block per sub-tile q;
+    // the chunk's masks of that half block, one primitive per lane, are turned across the warp
+    // into each pixel's set of covering primitives, which its lane visits in increasing order.
 #pragma unroll
     for (int q = 0; q < PPT; ++q) {
       const int half = (py[q] >> 2) & 1;
-      if constexpr (kPixWalk) {
-        // the warp's primitives that were not compacted and touch its half block (ballot),
-        // plus this pixel's compacted primitives; visited per lane in increasing order
-        uint64_t todo[HW];
+      uint64_t mine[HW];
 #pragma unroll
-        for (int w = 0; w < HW; ++w) todo[w] = 0;
-        if (suncomp) {  // (uniform; a chunk of compacted primitives only has nothing to ballot)
-#pragma unroll
-          for (int w = 0; w < NW; ++w) {
-            const int k = w * 32 + lane;
-            const bool h = k < n && !scomp[k] && ((uint32_t)(smask[k * NB + blk[q]] >> (half * 32)) != 0u);
-            todo[w >> 1] |= (uint64_t)__ballot_sync(0xffffffffu, h) << ((w & 1) * 32);
-          }
-        }
-        const int bit = (py[q] & 7) * 8 + (px[q] & 7);
-        if (!in[q]) continue;
-        const int pix = (py[q] - oy) * TILE + (px[q] - ox);
-#pragma unroll
-        for (int w = 0; w < HW; ++w) {
-          uint64_t t = todo[w] | spm[pix * HW + w];
-          while (t) {
-            const int k = w * 64 + __ffsll((long long)t) - 1;
-            t &= t - 1ull;
-            const uint64_t* mk = smask + k * NB;
-            const uint64_t m = mk[blk[q]];
-            if (!((m >> bit) & 1ull)) continue;
-            const float* r = srec + k * RL::R;
-            frags++;
-            if (scomp[k]) {
-              const int f = (int)sex[k] + (int)spre[k * NB + blk[q]] + __popcll(m & ((1ull << bit) - 1ull));
-              PS::apply(st[q], sfz[f], sfc[f], spid[k]);
-              continue;
-            }
-            const bool blockmode = !SPAN || (__float_as_int(r[0]) & 2);
-            float fx, fy;
-            int ka, kb;
-            if (blockmode) {
-              fx = swr_add((float)(px[q] & ~7), 0.5f);
-              fy = swr_add((float)(py[q] & ~7), 0.5f);
-              ka = px[q] & 7;
-              kb = py[q] & 7;
-            } else {
-              const int2 sp = sspan[k * TILE + (py[q] - oy)];
-              fx = swr_add((float)sp.x, 0.5f);
-              fy = swr_add((float)py[q], 0.5f);
-              ka = px[q] - sp.x;
-              kb = 0;
-            }
-            const float* eq = r + RL::EQ0;
-            GpuPixel<PS> pd;
-            pd.x = px[q];
-            pd.y = py[q];
-            pd.eq = eq;
-            pd.z = build_z<PS>(eq, blockmode, fx, fy, ka, kb);
-            if (RL::IZ && PS::earlyReject(pd.z, st[q])) continue;
-            build_pixel<PS>(eq, blockmode, fx, fy, ka, kb, pd);
-            PS::drawPixel(pd, spid[k], st[q], g.draws[__float_as_int(r[1])].u);
-          }
-        }
-        continue;
-      }
-      uint64_t hw[HW];
-#pragma unroll
-      for (int w = 0; w < HW; ++w) hw[w] = 0;
+      for (int w = 0; w < HW; ++w) mine[w] = 0;
 #pragma unroll
       for (int w = 0; w < NW; ++w) {
+        if (w && w * 32 >= n) break;  // (uniform)
         const int k = w * 32 + lane;
-        const bool h = k < n && ((uint32_t)(smask[k * NB + blk[q]] >> (half * 32)) != 0u);
-        hw[w >> 1] |= (uint64_t)__ballot_sync(0xffffffffu, h) << ((w & 1) * 32);
+        const uint32_t cov = warp_transpose(k < n ? (uint32_t)(smask[k * NB + blk[q]] >> (half * 32)) : 0u, lane);
+        mine[w >> 1] |= (uint64_t)(in[q] ? cov : 0u) << ((w & 1) * 32);
       }
-      const int bit = (py[q] & 7) * 8 + (px[q] & 7);
-      if (kCull && scull_on) {
-        // primitives culled in this warp's region: their fragments fail the depth test and
-        // are only counted, in any order (counters commute), outside the primitive-order walk
+      if constexpr (kDefer) {  // (other shaders count a fragment when they draw it)
+        uint32_t cnt = 0;
+#pragma unroll
+        for (int w = 0; w < HW; ++w) cnt += (uint32_t)__popcll(mine[w]);
+        frags += cnt;
+        st[q].frags += cnt;
+      }
+      if (kCull && cull_on) {
+        // primitives culled in this warp's region fail the depth test: counted only
         const uint32_t* cr = sculr + (q * 8 + warp) * NW;
 #pragma unroll
-        for (int w = 0; w < HW; ++w) {
-          const uint64_t cm = (uint64_t)cr[2 * w] | (2 * w + 1 < NW ? (uint64_t)cr[2 * w + 1] << 32 : 0ull);
-          uint64_t ch = hw[w] & cm;
-          hw[w] &= ~ch;
-          while (ch) {
-            const int k = w * 64 + __ffsll((long long)ch) - 1;
-            ch &= ch - 1ull;
-            if (in[q] && ((smask[k * NB + blk[q]] >> bit) & 1ull)) {
-              frags++;
-              PS::earlyReject(__int_as_float(0x7f800000), st[q]);  // counts the rejected fragment
-            }
-          }
-        }
+        for (int w = 0; w < HW; ++w)
+          mine[w] &= ~((uint64_t)cr[2 * w] | (2 * w + 1 < NW ? (uint64_t)cr[2 * w + 1] << 32 : 0ull));
       }
-      // primitive-order walk over the words (one copy of the loop body)
-      uint64_t hits = hw[0];
-      uint64_t later = HW > 1 ? hw[HW - 1] : 0ull;
+      int won = -1;  // kDefer: the chunk's last primitive to pass the pixel's depth test
+      uint64_t hits = mine[0];
+      uint64_t later = HW > 1 ? mine[HW - 1] : 0ull;
       int kbase = 0;
-      while (true) {
+      while (true) {  // (one copy of the loop body for both words)
         if (!hits) {
           if (HW == 1 || !later) break;
           hits = later;
@@ -2105,16 +2153,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
         }
         const int k = kbase + __ffsll((long long)hits) - 1;
         hits &= hits - 1ull;
-        const uint64_t* mk = smask + k * NB;
-        const uint64_t m = mk[blk[q]];
-        if (!in[q] || !((m >> bit) & 1ull)) continue;
-        const float* r = srec + k * RL::R;
-        frags++;
-        if (scomp[k]) {
-          const int f = (int)sex[k] + (int)spre[k * NB + blk[q]] + __popcll(m & ((1ull << bit) - 1ull));
-          PS::apply(st[q], sfz[f], sfc[f], spid[k]);
-          continue;
-        }
+        const float* r = srec + k * SR;
         const bool blockmode = !SPAN || (__float_as_int(r[0]) & 2);
         float fx, fy;
         int ka, kb;
@@ -2124,28 +2163,62 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
           ka = px[q] & 7;
           kb = py[q] & 7;
         } else {
-          const int2 sp = sspan[k * TILE + (py[q] - oy)];
-          fx = swr_add((float)sp.x, 0.5f);
+          const int xs = sspan[k * TILE + (py[q] - oy)].x;
+          fx = swr_add((float)xs, 0.5f);
           fy = swr_add((float)py[q], 0.5f);
-          ka = px[q] - sp.x;
+          ka = px[q] - xs;
           kb = 0;
         }
         const float* eq = r + RL::EQ0;
-        GpuPixel<PS> pd;
-        pd.x = px[q];
-        pd.y = py[q];
-        pd.eq = eq;
-        pd.z = build_z<PS>(eq, blockmode, fx, fy, ka, kb);
-        if (RL::IZ && PS::earlyReject(pd.z, st[q])) continue;
-        build_pixel<PS>(eq, blockmode, fx, fy, ka, kb, pd);
-        PS::drawPixel(pd, spid[k], st[q], g.draws[__float_as_int(r[1])].u);
+        const float z = build_z<PS>(eq, blockmode, fx, fy, ka, kb);
+        if constexpr (kDefer) {
+          if (z < st[q].depth) {
+            st[q].depth = z;
+            st[q].writes++;
+            won = k;
+          }
+        } else {
+          frags++;
+          GpuPixel<PS> pd;
+          pd.x = px[q];
+          pd.y = py[q];
+          pd.eq = eq;
+          pd.z = z;
+          build_pixel<PS>(eq, blockmode, fx, fy, ka, kb, pd);
+          PS::drawPixel(pd, prim_id(g, r, sids[k]), st[q], g.draws[__float_as_int(r[1])].u);
+        }
       }
+      if (kDefer && won >= 0) stands[q] = sids[won];
     }
   }
   if constexpr (!DIRECT) break;
   gather();
   if (e == 0) break;
   ce = e;
+  }
+  if constexpr (kDefer) {  // shade the fragments that stand
+#pragma unroll
+    for (int q = 0; q < PPT; ++q) {
+      if (stands[q] == 0xffffffffu) continue;
+      const float* r = g.recs + (size_t)stands[q] * RL::R;
+      GpuPixel<PS> pd;
+      pd.z = st[q].depth;
+      pixel_of_record<PS, SPAN>(r, g.draws, px[q], py[q], pd);
+      // its write, against a depth that lets it pass; its test was counted in the walk
+      st[q].depth = __int_as_float(0x7f800000);
+      PS::apply(st[q], pd.z, PS::shade(pd, g.draws[__float_as_int(r[1])].u), prim_id(g, r, stands[q]));
+      st[q].frags--;
+      st[q].writes--;
+    }
+  }
+  if (kCull && counts) {
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < PPT; ++q) {
+      int c = 0;
+      for (int k = 0; k <= px[q] - ox; ++k) c += scnt[(py[q] - oy) * (TILE + 1) + k];
+      if (in[q]) st[q].frags += (uint32_t)c;
+    }
   }
   if constexpr (SwrDepthMin<PS>::value && !DIRECT) {
     if (dslot >= 0) {
@@ -2160,9 +2233,9 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB : SwrRa
         }
       __threadfence();
       __syncthreads();
-      if (threadIdx.x == 0) snc = atomicAdd(&g.dslice_done[dslot], 1u) == (uint32_t)(nsl - 1);
+      if (threadIdx.x == 0) slast = atomicAdd(&g.dslice_done[dslot], 1u) == (uint32_t)(nsl - 1);
       __syncthreads();
-      if (snc) {
+      if (slast) {
         __threadfence();
 #pragma unroll
         for (int q = 0; q < PPT; ++q)
@@ -2274,82 +2347,38 @@ __global__ void __launch_bounds__(256) k_overwrite(RasterArgs g) {
   __syncthreads();
   uint32_t smin = 0;  // no pixel's winner is below it
   uint32_t frags = 0;
-  // pixels [x0, x1) of tile row `row` are covered by the primitive with id key - 1
-  auto run = [&](int row, int x0, int x1, uint32_t key) {
-    if (x1 <= x0) return;
-    frags += (uint32_t)(x1 - x0);
-    if (key > smin)
-      for (int x = x0; x < x1; ++x)
-        if (*(volatile uint32_t*)&sbest[row * TILE + x] < key) atomicMax(&sbest[row * TILE + x], key);
-    if (counts) {
-      atomicAdd(&scnt[row * (TILE + 1) + x0], 1);
-      atomicAdd(&scnt[row * (TILE + 1) + x1], -1);
-    }
-  };
   // rows [r0, r1) of the tile, primitive p
   auto cover = [&](uint32_t p, int r0, int r1) {
     const float4* rc = (const float4*)(g.recs + (size_t)p * RL::R);
-    const float4 q0 = __ldg(rc), q1 = __ldg(rc + 1), q2 = __ldg(rc + 2), q3 = __ldg(rc + 3);
+    const float4 q0 = __ldg(rc), q1 = __ldg(rc + 1), q2 = __ldg(rc + 2), q3 = __ldg(rc + 3), q4 = __ldg(rc + 4);
     const int flags = __float_as_int(q0.x);
     if (!(flags & 1)) return;
-    const int bx0 = __float_as_int(q0.z), by0 = __float_as_int(q0.w);
-    const int bx1 = __float_as_int(q1.x), by1 = __float_as_int(q1.y);
-    const int ylo = max(by0, oy + r0), yhi = min(min(by1 + 1, oy + r1), yend);
     const uint32_t key = p + 1u;
-    if (!(flags & 2)) {  // Span: a run per row of either half, inside the box's 8-px blocks
-      const float4 q4 = __ldg(rc + 4);
-      const SwrDrawDesc& D = g.draws[__float_as_int(q0.y)];
-      const int minx = D.sc_minx, maxx = D.sc_maxx;
-      const int cx0 = max(bx0 & ~(SWR_BLOCK - 1), ox), cx1 = min((bx1 | (SWR_BLOCK - 1)) + 1, xend);
-      SpanHalf bot, top;
-      bot.y0 = __float_as_int(q1.z); bot.y1 = __float_as_int(q1.w);
-      bot.ox = q2.x; bot.oy = q2.y; bot.is1 = q2.z; bot.is2 = q2.w;
-      top.y0 = __float_as_int(q3.x); top.y1 = __float_as_int(q3.y);
-      top.ox = q3.z; top.oy = q3.w; top.is1 = q4.x; top.is2 = q4.y;
-      for (int y = ylo; y < yhi; ++y) {
-        const bool inb = (flags & 32) && y >= bot.y0 && y < bot.y1;
-        const bool int_ = (flags & 64) && y > top.y1 && y <= top.y0;
-        if (!inb && !int_) continue;
-        int xl, xr;
-        span_row(inb ? bot : top, y, minx, maxx, xl, xr);
-        run(y - oy, max(xl, cx0) - ox, min(xr, cx1) - ox, key);
+    auto run = [&](int y, int xa, int xb) {
+      const int row = y - oy;
+      frags += (uint32_t)(xb - xa);
+      if (key > smin)
+        for (int i = row * TILE + xa - ox; i < row * TILE + xb - ox; ++i)
+          if (*(volatile uint32_t*)&sbest[i] < key) atomicMax(&sbest[i], key);
+      if (counts) {
+        atomicAdd(&scnt[row * (TILE + 1) + xa - ox], 1);
+        atomicAdd(&scnt[row * (TILE + 1) + xb - ox], -1);
       }
+    };
+    const int y0 = oy + r0, y1 = min(oy + r1, yend);
+    if (!(flags & 2)) {
+      const SwrDrawDesc& D = g.draws[__float_as_int(q0.y)];
+      span_runs(q0, q1, q2, q3, q4, D.sc_minx, D.sc_maxx, ox, xend, y0, y1,
+                [&](int y, int xa, int xb, int) { run(y, xa, xb); });
       return;
     }
-    // Block: whole blocks, or the rows of the reference's stepped edge tests
     const float r[15] = {0, 0, 0, 0, 0, 0, q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, q3.x, q3.y, q3.z};
-    const float t0 = (flags & 4) ? 0.0f : 0x1p-149f, t1 = (flags & 8) ? 0.0f : 0x1p-149f;
-    const float t2 = (flags & 16) ? 0.0f : 0x1p-149f;  // thresholds of edge_test
+    const int bx0 = __float_as_int(q0.z), bx1 = __float_as_int(q1.x);
+    const int ylo = max(__float_as_int(q0.w), y0), yhi = min(__float_as_int(q1.y) + 1, y1);
     for (int by = ylo & ~(SWR_BLOCK - 1); by < yhi; by += SWR_BLOCK)
       for (int bx = max(bx0 & ~(SWR_BLOCK - 1), ox); bx <= bx1 && bx < xend; bx += SWR_BLOCK) {
         const int cls = block_class(r, flags, bx, by);
-        if (cls == 0) continue;
-        const int wx = min(SWR_BLOCK, xend - bx);
-        const float fx = swr_add((float)bx, 0.5f), fy = swr_add((float)by, 0.5f);
-        float i0 = swr_eval(r[6], r[7], r[8], fx, fy), i1 = swr_eval(r[9], r[10], r[11], fx, fy);
-        float i2 = swr_eval(r[12], r[13], r[14], fx, fy);
-        for (int y = by; y < min(by + SWR_BLOCK, yhi); ++y) {
-          uint32_t m = (1u << wx) - 1u;
-          if (cls == 2) {  // block_row_bits, the row starts stepped from row to row
-            float c0 = i0, c1 = i1, c2 = i2;
-#pragma unroll
-            for (int col = 0; col < SWR_BLOCK; ++col) {
-              if (!(c0 >= t0 && c1 >= t1 && c2 >= t2)) m &= ~(1u << col);
-              c0 = swr_add(c0, r[6]);
-              c1 = swr_add(c1, r[9]);
-              c2 = swr_add(c2, r[12]);
-            }
-            i0 = swr_add(i0, r[7]);
-            i1 = swr_add(i1, r[10]);
-            i2 = swr_add(i2, r[13]);
-          }
-          if (y < ylo) continue;
-          while (m) {  // the row's runs of covered pixels (one, up to rounding)
-            const int x0 = __ffs(m) - 1, x1 = x0 + __ffs(~(m >> x0)) - 1;
-            m &= ~0u << x1;
-            run(y - oy, bx - ox + x0, bx - ox + x1, key);
-          }
-        }
+        if (cls) block_runs(r, flags, cls, bx, by, min(SWR_BLOCK, xend - bx), ylo, min(by + SWR_BLOCK, yhi), run);
       }
   };
   // rows per item: see above (n * groups items in all)
@@ -2431,37 +2460,12 @@ __global__ void __launch_bounds__(256) k_overwrite(RasterArgs g) {
     if (!best[q] || x >= xend || y >= yend) continue;
     const uint32_t p = best[q] - 1u;
     const float* r = g.recs + (size_t)p * RL::R;
-    const int flags = __float_as_int(r[0]);
-    const SwrDrawDesc& D = g.draws[__float_as_int(r[1])];
-    float fx, fy;
-    int ka, kb;
-    if (flags & 2) {
-      fx = swr_add((float)(x & ~7), 0.5f);
-      fy = swr_add((float)(y & ~7), 0.5f);
-      ka = x & 7;
-      kb = y & 7;
-    } else {  // from its row's span start
-      const bool inb = (flags & 32) && y >= __float_as_int(r[6]) && y < __float_as_int(r[7]);
-      SpanHalf h;
-      h.ox = inb ? r[8] : r[14]; h.oy = inb ? r[9] : r[15];
-      h.is1 = inb ? r[10] : r[16]; h.is2 = inb ? r[11] : r[17];
-      int xl, xr;
-      span_row(h, y, D.sc_minx, D.sc_maxx, xl, xr);
-      fx = swr_add((float)xl, 0.5f);
-      fy = swr_add((float)y, 0.5f);
-      ka = x - xl;
-      kb = 0;
-    }
-    const float* eq = r + RL::EQ0;
     GpuPixel<PS> pd;
-    pd.x = x;
-    pd.y = y;
-    pd.eq = eq;
-    pd.z = build_z<PS>(eq, flags & 2, fx, fy, ka, kb);
-    build_pixel<PS>(eq, flags & 2, fx, fy, ka, kb, pd);
+    pd.z = 0.0f;  // (no depth: SwrOverwrite)
+    pixel_of_record<PS, true>(r, g.draws, x, y, pd);
     typename PS::State st;
     PS::load(st, x, y, U);
-    PS::apply(st, pd.z, PS::shade(pd, D.u), prim_id(g, r, p));
+    PS::apply(st, pd.z, PS::shade(pd, g.draws[__float_as_int(r[1])].u), prim_id(g, r, p));
     st.frags = 0;  // counted above
     PS::store(st, x, y, U);
   }
