@@ -21,12 +21,12 @@ constexpr int kStatusWords = 16;
 constexpr int kSingleSlots = 8;            // pinned descriptor slots of single draws
 constexpr int kBatchSlots = 2;             // pinned descriptor slots (and cached graphs) of batches
 constexpr size_t kSingleSlotBytes = 1024;  // >= sizeof(SwrDrawDesc) + sizeof(SwrTargetDesc)
-constexpr size_t kBigSortSmem = 128 * 1024;  // shared memory of a k_sort_big CTA (bounds one warp's bitmap)
-constexpr int kBigSortWarps = 1216;          // warps of k_sort_big (8 per SM)
+constexpr size_t kSortSmem = 128 * 1024;  // bitmaps of a k_sort_tiles CTA (bounds its warps)
+constexpr int kSortWarps = 2432;          // warps of k_sort_tiles
 constexpr int kStickyBase = SWR_ST_STICKY;
 constexpr uint32_t kQuadMin = 3 * SWR_CHUNK;  // bin entries above which a 16-px tile is split into quadrant CTAs
 
-// Tiles k_sort_cells may list for quadrant CTAs: enough to cover the slow tail of a frame
+// Tiles k_cells may list for quadrant CTAs: enough to cover the slow tail of a frame
 // whose heavy tiles are few; every listed tile adds three CTAs.
 uint32_t quad_cap(uint32_t ntiles) {
   uint32_t cap = ntiles / 8;
@@ -34,7 +34,7 @@ uint32_t quad_cap(uint32_t ntiles) {
   return cap < ntiles ? cap : ntiles;
 }
 
-// Tiles k_sort_cells may list for heavy-tile runs (depth-min shaders): every slot adds
+// Tiles k_cells may list for heavy-tile runs (depth-min shaders): every slot adds
 // SWR_DSLICES CTAs at the front of the raster grid, used or not.  On the dense 1080p mesh
 // (about 350 tiles of more than one chunk) 512 slots measured 0.9 % faster than 1020 and
 // 304 slots 7 % slower (heavy tiles left whole).
@@ -82,11 +82,6 @@ __global__ void k_stage_copy(const StageCopy sc) {
     uint32_t* d = (uint32_t*)sc.dst[k];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < sc.words[k]; i += gridDim.x * blockDim.x) d[i] = s[i];
   }
-}
-
-__global__ void k_close_draw(uint32_t* st) {
-  swr_pdl_entry();
-  swr_close_status(st);
 }
 
 // swr_finish: the status words to pinned host memory, and zero again for the next draws, in
@@ -166,10 +161,9 @@ struct swr_context {
   // device buffers
   swr::Buffer draws, targets, draw_vbase, draw_bbase, target_tile_base;
   swr::Buffer ptv, clipv, clip_table, clip_slot, tri_flags, batch_counts, batch_base;
-  swr::Buffer tris, recs, tile_count, pair_off, keys0, vals0, keys1, vals1, tile_start;
+  swr::Buffer tris, recs, tile_count, pair_off, keys0, vals0, keys1, vals1;
   swr::Buffer scratch, status, direct_keep, direct_pos, lp_refs, cell_count, cell_start, cell_fill, draw_pbase;
-  swr::Buffer big_cells;  // k_sort_cells -> k_sort_big: [count, cell ids...]
-  swr::Buffer quad_flag, quad_tiles, quad_count;  // heavy 16-px tiles rasterized as four quadrant CTAs
+  swr::Buffer tile_list, heavy_tiles, sort_tiles, tile_counts;  // SwrTiles
   int quad_mode = 0;  // 0: off, 1: heavy tiles (more than kQuadMin entries), 2: every tile (8-px raster tiles)
   bool persistent_geometry = false;  // swr_set_persistent_geometry
   bool geo_stall = false;             // swr_test_stall_geometry_barrier
@@ -219,9 +213,9 @@ struct swr_context {
   void attach_budget() {
     swr::Buffer* all[] = {&draws, &targets, &draw_vbase, &draw_bbase, &target_tile_base, &ptv, &clipv,
                           &clip_table, &clip_slot, &tri_flags, &batch_counts, &batch_base, &tris, &recs,
-                          &tile_count, &pair_off, &keys0, &vals0, &keys1, &vals1, &tile_start, &scratch,
+                          &tile_count, &pair_off, &keys0, &vals0, &keys1, &vals1, &scratch,
                           &status, &direct_keep, &direct_pos, &lp_refs, &cell_count, &cell_start, &cell_fill, &draw_pbase,
-                          &big_cells, &over_best, &over_done, &quad_flag, &quad_tiles, &quad_count, &geo_bar,
+                          &tile_list, &heavy_tiles, &sort_tiles, &tile_counts, &over_best, &over_done, &geo_bar,
                           &dslice_state, &dslice_done};
     for (swr::Buffer* b : all) b->budget = &budget;
   }
@@ -289,17 +283,15 @@ int ensure_capacity(swr_context* c, uint32_t nverts_ptv, int S, uint32_t nsub, u
   ok &= c->vals0.ensure((size_t)c->cap_pairs * 4 + 16);
   ok &= c->keys1.ensure((size_t)c->cap_pairs * 4 + 16);
   ok &= c->vals1.ensure((size_t)c->cap_pairs * 4 + 16);
-  ok &= c->tile_start.ensure((size_t)(ntiles + 1) * 4 + 16);
   // the per-cell counters start at zero and every draw leaves them at zero (k_fill_bins)
   ok &= zeroed(c->cell_count, (size_t)ntiles * SWR_SEGS * 4 + 16, s);
   ok &= c->cell_start.ensure(((size_t)ntiles * SWR_SEGS + 1) * 4 + 16);
   if (ndraws == 1) ok &= c->cell_fill.ensure((size_t)ntiles * SWR_SEGS * 4 + 16);
-  ok &= c->quad_flag.ensure((size_t)ntiles + 16);
-  ok &= c->quad_tiles.ensure((size_t)quad_cap(ntiles) * 4 + 16);
-  ok &= c->quad_count.ensure(16);
+  ok &= c->tile_list.ensure((size_t)ntiles * 16);
+  ok &= c->sort_tiles.ensure((size_t)ntiles * 16);
+  ok &= c->heavy_tiles.ensure((size_t)quad_cap(ntiles) * 16);
+  ok &= c->tile_counts.ensure(16);
   ok &= c->geo_bar.ensure(16);
-  // (the list length and completion counter start at zero; k_sort_big resets them)
-  ok &= zeroed(c->big_cells, ((size_t)ntiles * SWR_SEGS + 2) * 4 + 16, s);
   // Overwrite shaders: a sliced tile's winners and finished slices (optional; both start at
   // zero, and the last slice of a tile leaves them at zero)
   c->slices = 1;
@@ -315,7 +307,7 @@ int ensure_capacity(swr_context* c, uint32_t nverts_ptv, int S, uint32_t nsub, u
     c->dslice_ok = c->dslice_state.ensure(slots * SWR_DSLICES * c->tile * c->tile * (size_t)ps->state_bytes + 16) &&
                    zeroed(c->dslice_done, slots * 4 + 16, s);
   }
-  const size_t sw = scan_scratch_words(c->cap_prims) + 64 + 2 * scan_scratch_words(ntiles * SWR_SEGS);
+  const size_t sw = scan_scratch_words(c->cap_prims) + 64;
   ok &= c->scratch.ensure(sw * 4);
   ok &= c->draws.ensure(sizeof(SwrDrawDesc));
   ok &= c->targets.ensure(sizeof(SwrTargetDesc));
@@ -392,22 +384,25 @@ bool geometry_front(swr_context* c, const VsOps* vs, const SwrDrawDesc* draws, i
   return true;
 }
 
-// Launches k_sort_big over the listed cells (ids in `in`, ordered into `out`), one warp per
-// cell with a bitmap of the segment's id range in shared memory, where that range fits in
-// kBigSortSmem (big_list); its last block also closes the draw.  The list buffer is [list
-// length, blocks done, cell ids...]; both words are zeroed when it is allocated and reset by
-// that last block.
-uint32_t* big_list(swr_context* c, uint32_t ncells, int seg_shift) {
-  const bool fits = ((size_t)1 << seg_shift) / 8 <= kBigSortSmem && c->big_cells.bytes >= (size_t)(ncells + 2) * 4;
-  return fits ? c->big_cells.as<uint32_t>() : nullptr;
+SwrTiles tiles_of(const swr_context* c, uint32_t ntiles, uint32_t heavy_cap) {
+  SwrTiles t;
+  t.start = c->cell_start.as<uint32_t>();
+  t.list = c->tile_list.as<uint4>();
+  t.heavy = c->heavy_tiles.as<uint4>();
+  t.sort = c->sort_tiles.as<uint4>();
+  t.counts = c->tile_counts.as<uint32_t>();  // (zeroed by the draw's k_stage_copy)
+  t.ntiles = ntiles;
+  t.heavy_cap = heavy_cap;
+  return t;
 }
 
-void sort_big(swr_context* c, const uint32_t* cstart, uint32_t ncells, int seg_shift, const uint32_t* in,
-              uint32_t* out, uint32_t* big, cudaStream_t s) {
-  const size_t bm_bytes = ((size_t)1 << seg_shift) / 8;  // one warp's bitmap
-  const int warps = (int)std::min<size_t>(8, std::max<size_t>(1, kBigSortSmem / std::max<size_t>(bm_bytes, 1)));
-  swr::launch(k_sort_big, kBigSortWarps / warps, 32 * warps, bm_bytes * warps, s, c->status.as<uint32_t>(), cstart,
-              ncells, c->cap_pairs, seg_shift, in, out, big + 2, big);
+void sort_tiles(swr_context* c, const SwrTiles& t, int seg_shift, uint32_t cell_min, const uint32_t* in, uint32_t* out,
+                cudaStream_t s) {
+  const size_t bm = ((size_t)1 << seg_shift) / 8;  // bytes of one warp's bitmap
+  const bool fits = bm >= 4 && bm <= kSortSmem;
+  const int warps = fits ? (int)std::min<size_t>(8, kSortSmem / bm) : 8;
+  swr::launch(k_sort_tiles, kSortWarps / warps, 32 * warps, fits ? warps * bm : 0, s, c->status.as<uint32_t>(), t,
+              seg_shift, fits ? (uint32_t)(bm / 4) : 0u, cell_min, in, out);
   c->launches += 1;
 }
 
@@ -419,9 +414,10 @@ int segment_shift(uint32_t cap) {
 }
 
 // Setup, binning and tile raster for the primitives in c->tris (count on the device).
-// Binning: setup counts (tile, primitive segment) cells, a scan turns the counts into
-// offsets, k_fill_bins scatters primitive ids into their cells, k_sort_cells restores the
-// primitive order inside each cell; a tile's bin is then its cells' contiguous range.
+// Binning: setup counts (tile, primitive segment) cells, k_cells turns the counts into
+// offsets and lists the tiles that have any, k_fill_bins scatters primitive ids into their
+// cells; a tile's bin is its cells' contiguous range.  Tiles of more than SWR_RASTER_SORT
+// entries are put in primitive order by k_sort_tiles, the others by their raster CTA.
 int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, int vs_a, int vs_p,
                  uint32_t ntiles, cudaStream_t s, int ndraws, int ntargets, bool has_span) {
   uint32_t* st = c->status.as<uint32_t>();
@@ -450,55 +446,43 @@ int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, i
   sa.seg_shift = seg_shift;
   ps->setup(sa, s);
   mark(c, 3, s);
-  uint32_t* scr = c->scratch.as<uint32_t>();
-  uint32_t* cstart = c->cell_start.as<uint32_t>();
-  const uint32_t* fill = cstart;
-  if (cells.tile_stride == 1) {
-    fill = c->cell_fill.as<uint32_t>();
-    scan_cells(c->cell_count.as<uint32_t>(), ntiles, cstart, c->cell_fill.as<uint32_t>(), scr, s);
-  } else {
-    scan_exclusive(c->cell_count.as<uint32_t>(), cstart, nullptr, ncells, cstart + ncells, scr, s);
-  }
-  ps->fill_bins(st, c->cap_prims, c->recs.as<float>(), c->cell_count.as<uint32_t>(),
-                fill, cstart + ncells, ncells, cells, seg_shift, c->cap_pairs,
-                c->draws.as<SwrDrawDesc>(), c->targets.as<SwrTargetDesc>(),
-                c->tile, c->keys0.as<uint32_t>(), st, s);
-  // heavy tiles listed by k_sort_cells: rasterized in runs of chunks (depth-min shaders,
-  // tiles of more than slice_chunks raster chunks), or else as quadrant CTAs (16-px tiles,
-  // shaders other than the overwrite ones; 8-px raster tiles split every tile)
+  // heavy tiles: rasterized in runs of chunks (depth-min shaders, tiles of more than
+  // slice_chunks raster chunks), or else as quadrant CTAs (16-px tiles, shaders other than the
+  // overwrite ones; 8-px raster tiles split every tile)
   const int slice_chunks = c->dslice_chunks < 0 ? ps->slice_chunks : c->dslice_chunks;
   const bool dsl = ps->depth_min && slice_chunks > 0 && c->dslice_ok && c->quad_mode != 2;
   const bool quads = !dsl && c->tile == 16 && !ps->overwrite && c->quad_mode != 0;
   const bool quad_list = quads && c->quad_mode == 1;
-  const bool listed = dsl || quad_list;
-  const uint32_t qcap = dsl ? slice_cap(ntiles) : quad_cap(ntiles);
-  // (quad_count was zeroed by the draw's k_stage_copy)
-  bool closed = ps->overwrite != 0;  // (k_overwrite takes the bins as they are, and closes the draw)
-  if (!ps->overwrite) {
-    uint32_t* big = big_list(c, ncells, seg_shift);
-    swr::launch(k_sort_cells, (ntiles + 7) / 8, 256, 0, s, st, cstart, ntiles, c->cap_pairs, c->keys0.as<uint32_t>(),
-                c->vals0.as<uint32_t>(), big ? big + 2 : nullptr, big, (uint32_t)SWR_RASTER_SORT,
-                listed ? c->quad_flag.as<uint8_t>() : nullptr, c->quad_tiles.as<uint32_t>(),
-                c->quad_count.as<uint32_t>(), qcap, dsl ? (uint32_t)(slice_chunks * ps->chunk) : kQuadMin);
-    c->launches += 1;
-    if (big) {
-      sort_big(c, cstart, ncells, seg_shift, c->keys0.as<uint32_t>(), c->vals0.as<uint32_t>(), big, s);
-      closed = true;
-    }
-  }
+  CellsArgs ca;
+  ca.status = st;
+  ca.count = c->cell_count.as<uint32_t>();
+  ca.cells = cells;
+  ca.fill_start = cells.tile_stride == 1 ? c->cell_fill.as<uint32_t>() : c->cell_start.as<uint32_t>();
+  ca.total = st + SWR_ST_PAIRS;
+  ca.t = tiles_of(c, ntiles, dsl ? slice_cap(ntiles) : quad_list ? quad_cap(ntiles) : 0u);
+  ca.heavy_min = dsl ? (uint32_t)(slice_chunks * ps->chunk) : kQuadMin;
+  ca.sort_min = ps->overwrite ? 0xffffffffu : (uint32_t)SWR_RASTER_SORT;
+  // Tiles of several chunks first, so that the longest do not finish last; a batch, many times
+  // the GPU's CTAs, stays in tile order.
+  ca.front_min = ndraws == 1 ? (uint32_t)ps->chunk : 0u;
+  ca.target_tile_base = c->target_tile_base.as<uint32_t>();
+  ca.ntargets = ntargets;
+  place_cells(ca, s);
+  ps->fill_bins(st, c->cap_prims, c->recs.as<float>(), c->cell_count.as<uint32_t>(), ca.fill_start, ca.total, ncells,
+                cells, seg_shift, c->cap_pairs, c->draws.as<SwrDrawDesc>(), c->targets.as<SwrTargetDesc>(), c->tile,
+                c->keys0.as<uint32_t>(), st, s);
+  if (!ps->overwrite)  // (k_overwrite takes the bins as they are)
+    sort_tiles(c, ca.t, seg_shift, 0, c->keys0.as<uint32_t>(), c->vals0.as<uint32_t>(), s);
   mark(c, 4, s);
   RasterArgs ra;
   memset(&ra, 0, sizeof(ra));
   ra.status = st;
-  ra.tile_start = cstart;
-  ra.tile_stride = SWR_SEGS;
+  ra.tiles = ca.t;
   ra.bin = c->vals0.as<uint32_t>();
   ra.bin_raw = c->keys0.as<uint32_t>();  // tiles of <= SWR_RASTER_SORT entries are ordered in k_raster
   ra.recs = c->recs.as<float>();
   ra.draws = c->draws.as<SwrDrawDesc>();
   ra.targets = c->targets.as<SwrTargetDesc>();
-  ra.target_tile_base = c->target_tile_base.as<uint32_t>();
-  ra.ntargets = ntargets;
   ra.draw_prim_base = c->use_draw_pbase ? c->draw_pbase.as<uint32_t>() : nullptr;
   ra.status_w = st;
   ra.ntiles = ntiles;
@@ -506,21 +490,14 @@ int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, i
   ra.slices = ps->overwrite ? c->slices : 1;
   ra.best = c->over_best.as<uint32_t>();
   ra.best_done = c->over_done.as<uint32_t>();
-  ra.quad_flag = listed ? c->quad_flag.as<uint8_t>() : nullptr;
-  ra.quad_tiles = c->quad_tiles.as<uint32_t>();
-  ra.quad_count = c->quad_count.as<uint32_t>();
-  ra.quad_cap = qcap;
+  ra.quad = quad_list ? 1 : 0;
   ra.quad_all = quads && c->quad_mode == 2;
   ra.dslice = dsl ? 1 : 0;
   ra.dslice_state = c->dslice_state.p;
   ra.dslice_done = c->dslice_done.as<uint32_t>();
   ps->raster(ra, ntiles, c->tile, s);
   mark(c, 5, s);
-  if (!closed) {
-    swr::launch(k_close_draw, 1, 1, 0, s, st);
-    c->launches += 1;
-  }
-  c->launches += 1 + 2 + 1 + (ntiles ? 1 : 0);
+  c->launches += 1 + 1 + 1 + (ntiles ? 1 : 0);
   return cuda_err(cudaGetLastError());
 }
 
@@ -573,7 +550,6 @@ int small_raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int of
   ra.recs = c->recs.as<float>();
   ra.draws = c->draws.as<SwrDrawDesc>();
   ra.targets = c->targets.as<SwrTargetDesc>();
-  ra.ntargets = 1;
   ra.draw_prim_base = c->use_draw_pbase ? c->draw_pbase.as<uint32_t>() : nullptr;
   ra.status_w = st;
   ra.ntiles = ntiles;
@@ -618,7 +594,6 @@ int lp_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, int v
   // segments over the fragments there can be: a point has one (its cells would be several times
   // larger than needed over the whole queue), a line any number
   const int seg_shift = segment_shift(mode == SWR_DRAW_POINT ? std::min(nsub, c->cap_pairs) : c->cap_pairs);
-  const uint32_t ncells = ntiles * SWR_SEGS;
   const SwrCells cells = {1u, ntiles};
   LpFragArgs fa;
   fa.status = st;
@@ -637,21 +612,24 @@ int lp_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, int v
   fa.seg_shift = seg_shift;
   fa.status_w = st;
   ps->lp_frags(fa, s);
-  uint32_t* cstart = c->cell_start.as<uint32_t>();
-  scan_cells(c->cell_count.as<uint32_t>(), ntiles, cstart, c->cell_fill.as<uint32_t>(), scr, s);
-  uint32_t* big = big_list(c, ncells, seg_shift);
+  CellsArgs ca;
+  ca.status = st;
+  ca.count = c->cell_count.as<uint32_t>();
+  ca.cells = cells;
+  ca.fill_start = c->cell_fill.as<uint32_t>();
+  ca.total = st + SWR_ST_FRAGS;  // fragments in the target
+  ca.t = tiles_of(c, ntiles, 0);
+  ca.heavy_min = 0xffffffffu;
+  ca.sort_min = SWR_LP_CHUNK;
+  ca.front_min = 2 * SWR_LP_CHUNK;
+  ca.target_tile_base = nullptr;
+  ca.ntargets = 1;
+  place_cells(ca, s);
   const uint32_t want = (c->cap_pairs + 255) / 256;
   swr::launch(k_lp_fill, want < 1216u ? (want ? want : 1u) : 1216u, 256, 0, s, st, st + SWR_ST_PAIRS, c->cap_pairs,
-              c->keys0.as<uint32_t>(), c->cell_count.as<uint32_t>(), c->cell_fill.as<uint32_t>(), cstart, ncells, cells, seg_shift,
-              c->keys1.as<uint32_t>(),
-              big ? big + 2 : nullptr, big);
-  if (big) {
-    sort_big(c, cstart, ncells, seg_shift, c->keys1.as<uint32_t>(), c->vals1.as<uint32_t>(), big, s);
-  } else {  // a segment beyond the bitmaps: every cell ordered by its tile's warp
-    swr::launch(k_sort_cells, (ntiles + 7) / 8, 256, 0, s, st, cstart, ntiles, c->cap_pairs, c->keys1.as<uint32_t>(),
-                c->vals1.as<uint32_t>(), nullptr, nullptr, 0u, nullptr, nullptr, nullptr, 0u, 0u);
-    c->launches += 1;
-  }
+              c->keys0.as<uint32_t>(), c->cell_count.as<uint32_t>(), ca.fill_start, cells, seg_shift,
+              c->keys1.as<uint32_t>());
+  sort_tiles(c, ca.t, seg_shift, SWR_LP_CHUNK, c->keys1.as<uint32_t>(), c->vals1.as<uint32_t>(), s);
   mark(c, 4, s);
   LpRasterArgs ra;
   ra.status = st;
@@ -659,20 +637,15 @@ int lp_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, int v
   ra.frag_off = c->pair_off.as<uint32_t>();
   ra.keys = c->keys0.as<uint32_t>();
   ra.prims = c->vals0.as<uint32_t>();
-  ra.cell_start = cstart;
+  ra.tiles = ca.t;
   ra.bin_raw = c->keys1.as<uint32_t>();
   ra.bin = c->vals1.as<uint32_t>();
   ra.draws = c->draws.as<SwrDrawDesc>();
   ra.targets = c->targets.as<SwrTargetDesc>();
-  ra.ntiles = ntiles;
   ra.status_w = st;
   ps->lp_raster(ra, s);
   mark(c, 5, s);
-  if (!big) {
-    swr::launch(k_close_draw, 1, 1, 0, s, st);
-    c->launches += 1;
-  }
-  c->launches += 1 + 2 + 1 + 2 + 1 + (ntiles ? 1 : 0);
+  c->launches += 1 + 2 + 1 + 1 + 1 + (ntiles ? 1 : 0);
   return cuda_err(cudaGetLastError());
 }
 
@@ -705,7 +678,7 @@ int upload_single(swr_context* c, const SwrDrawDesc& D, const SwrTargetDesc& T, 
   sc.clear(c->draw_bbase.p, 4);
   sc.clear(c->target_tile_base.p, 4);
   sc.clear(c->status.as<uint32_t>() + SWR_ST_CLIP_SLOTS, 5 * 4);
-  sc.clear(c->quad_count.p, 4);
+  sc.clear(c->tile_counts.p, 16);
   swr::launch(k_stage_copy, 1, 256, 0, s, sc);
   c->launches += 1;
   c->single_cur = slot;
@@ -752,8 +725,8 @@ int swr_create(swr_context** out) {
   swr_context* c = new swr_context();
   memset(&c->u, 0, sizeof(c->u));
   c->attach_budget();
-  // the segment bitmaps of k_sort_big may exceed the default 48 KB of dynamic shared memory
-  cudaFuncSetAttribute(k_sort_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBigSortSmem);
+  // the segment bitmaps of k_sort_tiles may exceed the default 48 KB of dynamic shared memory
+  cudaFuncSetAttribute(k_sort_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortSmem);
   cudaGetLastError();
   if (!c->status.ensure(kStatusWords * 4)) {
     delete c;
@@ -1248,9 +1221,9 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
   const void* bufs[] = {c->ptv.p, c->clipv.p, c->clip_table.p, c->clip_slot.p, c->tri_flags.p, c->batch_counts.p,
                         c->tris.p, c->recs.p, c->tile_count.p, c->keys0.p, c->vals0.p, c->cell_count.p,
                         c->cell_start.p, c->cell_fill.p, c->scratch.p, c->draws.p, c->targets.p, c->draw_vbase.p,
-                        c->draw_bbase.p, c->target_tile_base.p, c->draw_pbase.p, c->big_cells.p, h,
-                        c->over_best.p, c->over_done.p, (const void*)(uintptr_t)c->slices, c->quad_flag.p, c->quad_tiles.p,
-                        c->quad_count.p, c->geo_bar.p, c->dslice_state.p, c->dslice_done.p,
+                        c->draw_bbase.p, c->target_tile_base.p, c->draw_pbase.p, h,
+                        c->over_best.p, c->over_done.p, (const void*)(uintptr_t)c->slices, c->tile_list.p,
+                        c->heavy_tiles.p, c->sort_tiles.p, c->tile_counts.p, c->geo_bar.p, c->dslice_state.p, c->dslice_done.p,
                         (const void*)(uintptr_t)c->dslice_ok, (const void*)(intptr_t)c->dslice_chunks};
   for (const void* b : bufs) mix((uint64_t)(uintptr_t)b);
   if (c->graph_mode && c->gexec[slot] && sig == c->gsig[slot]) {
@@ -1280,7 +1253,7 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
     // the per-draw working counters and the heavy-tile list restart (flags and fragment
     // totals are sticky)
     sc.clear(c->status.as<uint32_t>() + SWR_ST_CLIP_SLOTS, 5 * 4);
-    sc.clear(c->quad_count.p, 4);
+    sc.clear(c->tile_counts.p, 16);
     swr::launch(k_stage_copy, kStageCopyBlocks, 256, 0, s, sc);
     c->launches += 1;
     q = cuda_err(cudaGetLastError());

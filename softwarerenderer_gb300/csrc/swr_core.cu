@@ -88,86 +88,89 @@ __global__ void __launch_bounds__(kThreads) k_scan_down(const uint32_t* in, uint
 }
 
 // --- (tile, segment) cells ------------------------------------------------------------
-// Blocks own contiguous ranges of whole 32-tile groups; a group's 32 x 32 counts are read a
-// segment row at a time and turned in shared memory.
+// One block per 32 tiles: their 32 x 32 counts, read a segment row at a time and turned in
+// shared memory (segment-major) or tile by tile.  Bound by its chain: counts, one atomic, the
+// lists' atomics.
 constexpr int kGroup = 32;
-static_assert(SWR_SEGS == 32, "a group of 32 tiles is a 32 x 32 square of cells");
+static_assert(SWR_SEGS == 32 && kThreads == 256, "a group of 32 tiles is a 32 x 32 square of cells, four a thread");
 
-__global__ void __launch_bounds__(kThreads) k_cells_reduce(const uint32_t* count, uint32_t ntiles, uint32_t chunk,
-                                                           uint32_t* partials) {
-  swr_pdl_entry();
-  __shared__ uint32_t tmp[32];
-  uint32_t b, e;
-  chunk_range(ntiles, chunk, b, e);
-  uint32_t s = 0;
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (uint32_t seg = warp; seg < SWR_SEGS; seg += kThreads / 32) {
-    const uint32_t* row = count + (size_t)seg * ntiles;
-#pragma unroll 4
-    for (uint32_t t = b + lane; t < e; t += 32) s += row[t];
-  }
-  uint32_t tot;
-  swr_block_exscan(s, tmp, &tot);
-  if (threadIdx.x == 0) partials[blockIdx.x] = tot;
-}
-
-__global__ void __launch_bounds__(kThreads) k_cells_down(const uint32_t* count, uint32_t ntiles, uint32_t chunk,
-                                                         const uint32_t* partials, uint32_t* start,
-                                                         uint32_t* fill_start) {
+__global__ void __launch_bounds__(kThreads) k_cells(const CellsArgs a) {
   swr_pdl_entry();
   __shared__ uint32_t tmp[32];
   __shared__ uint32_t sq[kGroup][SWR_SEGS + 1];
-  __shared__ uint32_t pref[2];
-  uint32_t b, e;
-  chunk_range(ntiles, chunk, b, e);
-  {
-    uint32_t mine = 0, all = 0;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += kThreads) {
-      const uint32_t v = partials[i];
-      all += v;
-      if (i < (int)blockIdx.x) mine += v;
-    }
-    uint32_t t0, t1;
-    swr_block_exscan(mine, tmp, &t0);
-    swr_block_exscan(all, tmp, &t1);
-    if (threadIdx.x == 0) { pref[0] = t0; pref[1] = t1; }
-    __syncthreads();
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) start[(size_t)ntiles * SWR_SEGS] = pref[1];
-  uint32_t run = pref[0];
+  __shared__ uint32_t stot[kGroup], sfirst[kGroup];
+  __shared__ uint32_t sbase;
+  if (a.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
+  const uint32_t nt = a.t.ntiles, t0 = blockIdx.x * kGroup;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t tl = threadIdx.x >> 3, sg = (threadIdx.x & 7) * 4;  // this thread's four cells of a group
-  for (uint32_t t0 = b; t0 < e; t0 += kGroup) {
-    const bool on = t0 + lane < e;
+  const uint32_t tl = threadIdx.x >> 3, sg = (threadIdx.x & 7) * 4;  // this thread's four cells
+  const bool seg_major = a.cells.tile_stride == 1;
+  uint32_t v[4] = {0, 0, 0, 0};
+  if (seg_major) {
 #pragma unroll
     for (int k = 0; k < SWR_SEGS / (kThreads / 32); ++k) {
       const uint32_t seg = warp + k * (kThreads / 32);
-      sq[lane][seg] = on ? count[(size_t)seg * ntiles + t0 + lane] : 0u;
+      sq[lane][seg] = t0 + lane < nt ? a.count[(size_t)seg * nt + t0 + lane] : 0u;
     }
     __syncthreads();
-    uint32_t v[4], s = 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      v[j] = sq[tl][sg + j];
-      s += v[j];
+    for (int j = 0; j < 4; ++j) v[j] = sq[tl][sg + j];
+  } else if (t0 + tl < nt) {
+    const uint4 c = *(const uint4*)(a.count + (size_t)(t0 + tl) * SWR_SEGS + sg);
+    v[0] = c.x; v[1] = c.y; v[2] = c.z; v[3] = c.w;
+  }
+  const uint32_t s = v[0] + v[1] + v[2] + v[3];
+  uint32_t tile_tot = s;  // the tile's entries: over its eight lanes
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) tile_tot += __shfl_xor_sync(0xffffffffu, tile_tot, o);
+  uint32_t tot;
+  uint32_t ex = swr_block_exscan(s, tmp, &tot);  // (its barriers order the reads of sq above)
+  if (tot == 0) return;  // uniform
+  if (threadIdx.x == 0) sbase = atomicAdd(a.total, tot);
+  if (sg == 0) {
+    stot[tl] = tile_tot;
+    sfirst[tl] = ex;
+  }
+  __syncthreads();
+  ex += sbase;
+  uint4 o;
+  o.x = ex;
+  o.y = o.x + v[0];
+  o.z = o.y + v[1];
+  o.w = o.z + v[2];
+  if (tile_tot) *(uint4*)(a.t.start + (size_t)(t0 + tl) * SWR_SEGS + sg) = o;
+  if (warp == 0) {  // one tile per lane
+    const uint32_t n = stot[lane], t = t0 + lane, below = (1u << lane) - 1u, b = sfirst[lane] + sbase;
+    uint4 entry = make_uint4(t, b, b + n, 0u);
+    if (n && a.ntargets > 1) entry.w = (uint32_t)swr_find_le(a.target_tile_base, a.ntargets, t);
+    auto append = [&](bool on, uint32_t* counter) -> uint32_t {
+      const uint32_t ons = __ballot_sync(0xffffffffu, on);
+      uint32_t at = 0;
+      if (lane == 0 && ons) at = atomicAdd(counter, (uint32_t)__popc(ons));
+      return __shfl_sync(0xffffffffu, at, 0) + (uint32_t)__popc(ons & below);
+    };
+    bool heavy = a.t.heavy_cap && n > a.heavy_min;
+    if (a.t.heavy_cap) {
+      const uint32_t at = append(heavy, a.t.counts);
+      heavy = heavy && at < a.t.heavy_cap;
+      if (heavy) a.t.heavy[at] = entry;
     }
-    uint32_t tot;
-    uint32_t ex = swr_block_exscan(s, tmp, &tot) + run;  // (its barriers order the reads above)
-    uint4 o;
-    o.x = ex;
-    o.y = o.x + v[0];
-    o.z = o.y + v[1];
-    o.w = o.z + v[2];
-    if (t0 + tl < e) *(uint4*)(start + (size_t)(t0 + tl) * SWR_SEGS + sg) = o;
-    sq[tl][sg] = o.x; sq[tl][sg + 1] = o.y; sq[tl][sg + 2] = o.z; sq[tl][sg + 3] = o.w;
-    __syncthreads();
+    const bool front = n > a.front_min && !heavy, back = n && !front && !heavy;
+    const uint32_t af = append(front, a.t.counts + 1), ab = append(back, a.t.counts + 2);
+    if (front) a.t.list[af] = entry;
+    if (back) a.t.list[nt - 1u - ab] = entry;
+    const uint32_t as = append(n > a.sort_min, a.t.counts + 3);
+    if (n > a.sort_min) a.t.sort[as] = entry;
+  }
+  if (!seg_major) return;
+  sq[tl][sg] = o.x; sq[tl][sg + 1] = o.y; sq[tl][sg + 2] = o.z; sq[tl][sg + 3] = o.w;
+  __syncthreads();
+  if (t0 + lane < nt && stot[lane]) {
 #pragma unroll
     for (int k = 0; k < SWR_SEGS / (kThreads / 32); ++k) {
       const uint32_t seg = warp + k * (kThreads / 32);
-      if (on) fill_start[(size_t)seg * ntiles + t0 + lane] = sq[lane][seg];
+      a.fill_start[(size_t)seg * nt + t0 + lane] = sq[lane][seg];
     }
-    __syncthreads();
-    run += tot;
   }
 }
 
@@ -309,12 +312,8 @@ void scan_exclusive(const uint32_t* in, uint32_t* out, const uint32_t* n_dev, ui
   swr::launch(k_scan_down, kScanBlocks, kThreads, 0, s, in, out, n_dev, n_max, chunk, scratch, total);
 }
 
-void scan_cells(const uint32_t* count, uint32_t ntiles, uint32_t* start, uint32_t* fill_start, uint32_t* scratch,
-                cudaStream_t s) {
-  const uint32_t groups = (ntiles + kGroup - 1) / kGroup;
-  const uint32_t chunk = (groups + kScanBlocks - 1) / kScanBlocks * kGroup;
-  swr::launch(k_cells_reduce, kScanBlocks, kThreads, 0, s, count, ntiles, chunk, scratch);
-  swr::launch(k_cells_down, kScanBlocks, kThreads, 0, s, count, ntiles, chunk, scratch, start, fill_start);
+void place_cells(const CellsArgs& a, cudaStream_t s) {
+  swr::launch(k_cells, (a.t.ntiles + kGroup - 1) / kGroup, kThreads, 0, s, a);
 }
 
 size_t sort_scratch_words(uint32_t) { return 2 * 256 * kSortBlocks + 256; }

@@ -18,11 +18,29 @@ size_t scan_scratch_words(uint32_t n_max);
 void scan_exclusive(const uint32_t* in, uint32_t* out, const uint32_t* n_dev, uint32_t n_max,
                     uint32_t* total, uint32_t* scratch, cudaStream_t s);
 
-// Exclusive scan of the binning's (tile, segment) counts, in tile-major order (a tile's cells
-// are consecutive).  `count` and `fill_start` are segment-major (SwrCells), `start` is
-// tile-major with the total at start[ntiles * SWR_SEGS].  scratch: kScanBlocks words.
-void scan_cells(const uint32_t* count, uint32_t ntiles, uint32_t* start, uint32_t* fill_start, uint32_t* scratch,
-                cudaStream_t s);
+// Places the (tile, segment) cells of a binned draw: every non-empty tile gets a range of
+// *total (advanced by the entries), its cells in segment order.  Ranges are handed out as
+// blocks of 32 tiles come, not in tile order: nothing needs one tile's range to follow
+// another's, and the exclusive scan that put them in order was two launches (10 us of a small
+// draw's chain; on 256 meshes' 491,520 mostly empty tiles 79 us).  The same kernel makes the
+// lists of t, so that empty tiles cost the later kernels nothing.
+//   count       per cell (layout `cells`)
+//   fill_start  the starts in that layout (segment-major only; tile-major it is t.start itself)
+//   heavy_min   tiles of more entries go to t.heavy, up to t.heavy_cap, and not to t.list
+//   sort_min    tiles of more entries go to t.sort
+//   front_min   tiles of more entries go to t.list's front (rasterized first), others to its back
+struct CellsArgs {
+  const uint32_t* status;
+  const uint32_t* count;
+  SwrCells cells;
+  uint32_t* fill_start;
+  uint32_t* total;
+  SwrTiles t;
+  uint32_t heavy_min, sort_min, front_min;
+  const uint32_t* target_tile_base;  // per target, for the tile -> target lookup
+  int ntargets;
+};
+void place_cells(const CellsArgs& a, cudaStream_t s);
 
 // Stable LSD radix sort of (key, value) pairs by the low `bits` bits of key; three kernels
 // per 8-bit pass (block histograms, per-digit offsets, stable scatter).

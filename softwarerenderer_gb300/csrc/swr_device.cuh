@@ -152,11 +152,35 @@ struct SwrClipEntry {
 //   tile-major (SWR_SEGS, 1), batches of several items: the items being processed at one time
 //     lie in one or two segments, whose counters would share few 32-byte sectors: on 256
 //     meshes k_setup took 265 us segment-major, 194 us tile-major.
-// The raster's starts are always tile-major: a tile's bin is one range.
+// The cells' starts are always tile-major.
 struct SwrCells {
   uint32_t tile_stride, seg_stride;
   __device__ __forceinline__ uint32_t at(uint32_t tile, uint32_t seg) const { return tile * tile_stride + seg * seg_stride; }
 };
+
+// Tiles of a binned draw, as k_cells leaves them.  Empty tiles are in no list and their starts
+// are not written.  A list entry is (tile, its bin [y, z), its target): one load tells a CTA
+// all of it (separate loads of the tile, its range and a search for its target cost 256
+// meshes' raster 100 us of 1,920).
+struct SwrTiles {
+  uint32_t* start;    // per tile: its cells' starts, SWR_SEGS each (the last cell ends with the bin)
+  uint4* list;        // tiles to rasterize whole: from the front, and the others from the back
+  uint4* heavy;       // tiles to rasterize in runs or quadrants (at most heavy_cap)
+  uint4* sort;        // tiles whose cells have to be ordered ahead of the raster
+  uint32_t* counts;   // list lengths (zero at the draw's start): heavy (may exceed heavy_cap),
+                      // list front, list back, sort
+  uint32_t ntiles, heavy_cap;
+};
+
+// Entry i (< ntiles) of the list of tiles; false past its end.
+__device__ __forceinline__ bool swr_listed_tile(const SwrTiles& t, uint32_t i, uint4& entry) {
+  const uint4 n = __ldg((const uint4*)t.counts);
+  entry = __ldg(t.list + i);  // (with the counts: most lists have no back)
+  if (i < n.y) return true;
+  if (i - n.y >= n.z) return false;
+  entry = __ldg(t.list + (t.ntiles - 1u - (i - n.y)));
+  return true;
+}
 
 // Index of the last element of sorted `base[0..n)` that is <= key.
 __device__ __forceinline__ int swr_find_le(const uint32_t* base, int n, uint32_t key) {

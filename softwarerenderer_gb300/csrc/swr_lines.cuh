@@ -10,9 +10,9 @@
 //                                step order: the stepped position by exact fold, the
 //                                per-step scissor test, the pixel; counts (tile, segment) cells
 //   k_lp_fill                    fragment numbers into their tile's bin (the triangles' cells:
-//                                a tile's fragments in SWR_SEGS runs of fragment numbers) and
-//                                a list of the cells above SWR_LP_CHUNK entries, which
-//                                k_sort_big orders; the tile's CTA orders the others
+//                                a tile's fragments in SWR_SEGS runs of fragment numbers);
+//                                k_sort_tiles orders cells above SWR_LP_CHUNK entries, the
+//                                tile's CTA the others
 //   k_lp_raster                  one CTA per 16 x 16 tile: each thread owns a pixel and applies
 //                                its fragments in order (a line may hit a pixel twice)
 //
@@ -339,14 +339,11 @@ __global__ void __launch_bounds__(256) k_lp_frags(LpFragArgs g) {
 }
 
 // Fragment numbers into their cells (arbitrary order inside a cell); takes every count of
-// k_lp_frags back, so the counters are zero again after the draw.  Lists the cells that do
-// not fit a raster chunk for k_sort_big (big_list holds every cell; null: none are listed).
+// k_lp_frags back, so the counters are zero again after the draw.
 static __global__ void __launch_bounds__(256) k_lp_fill(const uint32_t* status, const uint32_t* nfrags,
                                                         uint32_t cap_frags, const uint32_t* keys,
                                                         uint32_t* cell_count, const uint32_t* fill_start,
-                                                        const uint32_t* cell_start, uint32_t ncells,
-                                                        SwrCells cells, int seg_shift, uint32_t* bin,
-                                                        uint32_t* big_list, uint32_t* big_count) {
+                                                        SwrCells cells, int seg_shift, uint32_t* bin) {
   swr_pdl_entry();
   if (status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;  // (k_lp_frags counted nothing then)
   const uint32_t nf = min(*nfrags, cap_frags);
@@ -366,9 +363,6 @@ static __global__ void __launch_bounds__(256) k_lp_fill(const uint32_t* status, 
     pos = __shfl_sync(0xffffffffu, pos, leader);
     if (cell != SWR_LP_INVALID) bin[pos + (uint32_t)__popc(peers & ((1u << lane) - 1u))] = f;
   }
-  if (!big_list) return;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ncells; i += stride)
-    if (cell_start[i + 1] - cell_start[i] > SWR_LP_CHUNK) big_list[atomicAdd(big_count, 1u)] = i;
 }
 
 struct LpRasterArgs {
@@ -377,17 +371,16 @@ struct LpRasterArgs {
   const uint32_t* frag_off;
   const uint32_t* keys;        // per fragment (LpFragArgs)
   const uint32_t* prims;
-  const uint32_t* cell_start;  // per (tile, segment) cell, plus the end
+  SwrTiles tiles;              // the tiles with fragments, their bins and cells
   const uint32_t* bin_raw;     // fragment numbers, unordered inside a cell
-  const uint32_t* bin;         // ordered by k_sort_big, for cells of more than SWR_LP_CHUNK entries
+  const uint32_t* bin;         // ordered by k_sort_tiles, for cells of more than SWR_LP_CHUNK entries
   const SwrDrawDesc* draws;
   const SwrTargetDesc* targets;
-  uint32_t ntiles;
   uint32_t* status_w;
 };
 
 // One CTA per 16 x 16 tile, one pixel per thread.  A chunk is as many whole cells of the
-// tile's bin as hold at most 256 fragments (a larger cell, ordered by k_sort_big, is a run of
+// tile's bin as hold at most 256 fragments (a larger cell, ordered by k_sort_tiles, is a run of
 // chunks by itself): one fragment per thread is ranked inside its cell, interpolated, shaded
 // and marked under its rank in its pixel's set; then each thread applies its pixel's
 // fragments in increasing order (shaders with side effects of their own are evaluated there
@@ -411,12 +404,12 @@ __global__ void __launch_bounds__(256) k_lp_raster(LpRasterArgs g) {
   __shared__ float sz[kCompact ? CH : 1];
   __shared__ Color sc[kCompact ? CH : 1];
   __shared__ uint32_t sfr[32];
+  if (blockIdx.x == 0 && threadIdx.x == 0) swr_close_status(g.status_w);
   if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
-  const uint32_t tile = blockIdx.x;
-  if (tile >= g.ntiles) return;
-  const uint32_t* cells = g.cell_start + (size_t)tile * SWR_SEGS;
-  const uint32_t b = cells[0], e = cells[SWR_SEGS];
-  if (b == e) return;  // uniform per CTA
+  uint4 entry;
+  if (!swr_listed_tile(g.tiles, blockIdx.x, entry)) return;
+  const uint32_t tile = entry.x, b = entry.y, e = entry.z;
+  const uint32_t* cells = g.tiles.start + (size_t)tile * SWR_SEGS;
   const SwrDrawDesc& D = g.draws[0];
   const SwrTargetDesc& T = g.targets[D.target];
   const SwrUniforms& U = D.u;
@@ -428,7 +421,7 @@ __global__ void __launch_bounds__(256) k_lp_raster(LpRasterArgs g) {
   const bool in = x < T.width && y < T.height;
   typename PS::State st;
   if (in) PS::load(st, x, y, U);
-  if (tid <= SWR_SEGS) scs[tid] = cells[tid] - b;
+  if (tid <= SWR_SEGS) scs[tid] = (tid < SWR_SEGS ? cells[tid] : e) - b;
   // Rasterizer::pixelDataFromVertex (Rasterizer.h:161-173) of step j of primitive `prim`
   auto pixel = [&](uint32_t prim, int j, int fx, int fy, GpuPixel<PS>& pd) {
     const float* rec = g.recs + (size_t)prim * W;

@@ -51,7 +51,7 @@ constexpr size_t kBytes = 8u << 20;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kBytes];
 
 struct Layout {
-  size_t status, draw, target, zeros, ptv, keep, pos, tris, recs, tile_count, pair_off;
+  size_t status, draw, target, ptv, keep, pos, tris, recs, tile_count, pair_off;
   size_t keys0, vals0, keys1, vals1, tile_start, scan_scr, sort_scr, end;
 };
 
@@ -64,7 +64,6 @@ Layout make_layout() {
   L.status = take(16 * 4);
   L.draw = take(sizeof(SwrDrawDesc));
   L.target = take(sizeof(SwrTargetDesc));
-  L.zeros = take(64);
   L.ptv = take((size_t)kMaxVerts * kMaxS * 4);
   L.keep = take((size_t)kMaxTris * 4);
   L.pos = take((size_t)kMaxTris * 4);
@@ -200,7 +199,6 @@ extern "C" int swr_draw_triangle_list_noalloc(const struct SwrUniforms* u, int p
   uint32_t* st = (uint32_t*)(base + L.status);
   SwrDrawDesc* dd = (SwrDrawDesc*)(base + L.draw);
   SwrTargetDesc* dt = (SwrTargetDesc*)(base + L.target);
-  uint32_t* zeros = (uint32_t*)(base + L.zeros);
   float* ptv = (float*)(base + L.ptv);
   uint32_t* keep = (uint32_t*)(base + L.keep);
   uint32_t* pos = (uint32_t*)(base + L.pos);
@@ -216,10 +214,9 @@ extern "C" int swr_draw_triangle_list_noalloc(const struct SwrUniforms* u, int p
   uint32_t* scan_scr = (uint32_t*)(base + L.scan_scr);
   uint32_t* sort_scr = (uint32_t*)(base + L.sort_scr);
 
-  // The previous call's contents stay in the array: reset the status words, the primitive
-  // count and the per-target lookup words before any kernel reads them.
+  // The previous call's contents stay in the array: reset the status words and the primitive
+  // count before any kernel reads them.
   cudaMemsetAsync(st, 0, 16 * 4, s);
-  cudaMemsetAsync(zeros, 0, 64, s);
   cudaMemcpyAsync(dd, &D, sizeof(D), cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(dt, &T, sizeof(T), cudaMemcpyHostToDevice, s);
   if ((rc = (cudaGetLastError() == cudaSuccess ? SWR_OK : SWR_ECUDA))) return rc;
@@ -259,32 +256,17 @@ extern "C" int swr_draw_triangle_list_noalloc(const struct SwrUniforms* u, int p
   uint32_t* vals = which ? v1 : v0;
   segment_starts(keys, st + SWR_ST_PAIRS, kMaxPairs, ntiles, tile_start, s);
   RasterArgs ra;
+  memset(&ra, 0, sizeof(ra));  // no cells (every tile's range is ordered), no buffers of sliced tiles
   ra.status = st;
   ra.tile_start = tile_start;
-  ra.tile_stride = 1;
   ra.bin = vals;
-  ra.bin_raw = nullptr;  // the radix sort already ordered every tile
   ra.recs = recs;
   ra.draws = dd;
   ra.targets = dt;
-  ra.target_tile_base = zeros;
-  ra.ntargets = 1;
-  ra.draw_prim_base = nullptr;
   ra.status_w = st;
   ra.ntiles = ntiles;
   ra.has_span = raster_mode != SWR_RASTER_BLOCK;
-  ra.slices = 1;  // no buffer for sliced tiles' winners without allocation
-  ra.best = nullptr;
-  ra.best_done = nullptr;
-  ra.quad_flag = nullptr;  // no heavy-tile quadrant CTAs: every tile is one CTA
-  ra.quad_tiles = nullptr;
-  ra.quad_count = nullptr;
-  ra.quad_cap = 0;
-  ra.quad_all = 0;
-  ra.dslice = 0;  // no heavy-tile runs: they need the runs' State buffer
-  ra.dslice_state = nullptr;
-  ra.dslice_done = nullptr;
-  ra.boxes = nullptr;
+  ra.slices = 1;
   ra.cap_prims = kMaxTris;
   ps->raster(ra, ntiles, kTile, s);
   if (cudaGetLastError() != cudaSuccess) return SWR_ECUDA;  // a launch failed: the status words are stale

@@ -61,12 +61,8 @@ void run_raster(const RasterArgs& a, uint32_t ntiles, int tile, cudaStream_t s) 
     }
     // one CTA per tile; Block-only submissions run the instantiation without the Span-mode passes
     uint32_t grid = ntiles;
-    if (SwrDepthMin<PS>::value && a.dslice) {  // the listed tiles' runs, then the other tiles
-      grid = SWR_DSLICES * a.quad_cap + ntiles;
-    } else if (tile == 16) {  // quadrant CTAs (RasterArgs)
-      if (a.quad_all) grid = 4 * ntiles;
-      else if (a.quad_flag) grid = 4 * a.quad_cap + ntiles;
-    }
+    if (a.quad_all) grid = 4 * ntiles;
+    else if (a.dslice || a.quad) grid = 4 * a.tiles.heavy_cap + ntiles;  // the heavy tiles' runs or quadrants first
     if (tile == 32) {
       if (a.has_span) swr::launch(k_raster<PS, 32, kChunk, true>, grid, 256, 0, s, a);
       else swr::launch(k_raster<PS, 32, kChunk, false>, grid, 256, 0, s, a);
@@ -89,7 +85,7 @@ void run_lp_frags(const LpFragArgs& a, cudaStream_t s) {
 
 template <class PS>
 void run_lp_raster(const LpRasterArgs& a, cudaStream_t s) {
-  if (a.ntiles) swr::launch(k_lp_raster<PS>, a.ntiles, 256, 0, s, a);
+  if (a.tiles.ntiles) swr::launch(k_lp_raster<PS>, a.tiles.ntiles, 256, 0, s, a);
 }
 
 template <class PS>

@@ -1014,7 +1014,8 @@ __global__ void __launch_bounds__(256) k_emit_pairs(const uint32_t* status, uint
 // Segmented binning.  The primitive list is cut into SWR_SEGS contiguous segments; a
 // (tile, segment) cell holds the segment's primitives that touch the tile.  Cells are laid
 // out tile-major, so a tile's bin is one contiguous range ordered by segment; inside a cell
-// the fill order is arbitrary and k_sort_cells restores increasing primitive order.
+// the fill order is arbitrary; k_raster (or k_sort_tiles ahead of it, for tiles it cannot
+// order itself) restores increasing primitive order.
 template <class PS>
 __global__ void __launch_bounds__(256) k_fill_bins(const uint32_t* status, uint32_t cap_prims, const float* recs,
                                                    uint32_t* cell_count, const uint32_t* fill_start,
@@ -1029,14 +1030,10 @@ __global__ void __launch_bounds__(256) k_fill_bins(const uint32_t* status, uint3
   const uint32_t total = *pairs;
   const bool overflow = status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW;
   if (overflow || total > cap_pairs) {
-    if (!overflow && blockIdx.x == 0 && threadIdx.x == 0) {
-      atomicOr(&status_w[SWR_ST_FLAGS], SWR_F_PAIR_OVERFLOW);
-      status_w[SWR_ST_PAIRS] = total;
-    }
+    if (!overflow && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&status_w[SWR_ST_FLAGS], SWR_F_PAIR_OVERFLOW);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ncells; i += gridDim.x * blockDim.x) cell_count[i] = 0u;
     return;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) status_w[SWR_ST_PAIRS] = total;
   uint32_t np = status[SWR_ST_PRIMS];
   if (np > cap_prims) np = cap_prims;
   // draw 0's target, read up front: every primitive of a single-draw submission uses it
@@ -1095,156 +1092,84 @@ __global__ void __launch_bounds__(256) k_fill_bins(const uint32_t* status, uint3
   }
 }
 
-// One warp per tile: every cell of the tile is copied to `out` in increasing primitive
-// order.  Lane c owns cell c: cells of up to 16 entries are sorted in registers by the
-// lane; cells of up to 64 are ranked by the whole warp (primitive ids are unique); larger
-// cells go to `big_list` for k_sort_big when it is given (its capacity is the cell count,
-// so it cannot overflow), else the warp ranks them too.
-static __global__ void __launch_bounds__(256) k_sort_cells(const uint32_t* status, const uint32_t* cell_start,
-                                                          uint32_t ntiles, uint32_t cap_pairs, const uint32_t* in,
-                                                          uint32_t* out, uint32_t* big_list, uint32_t* big_count,
-                                                          uint32_t self_sorted, uint8_t* quad_flag,
-                                                          uint32_t* quad_tiles, uint32_t* quad_count,
-                                                          uint32_t quad_cap, uint32_t quad_min) {
-  swr_pdl_entry();
-  if (status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
-  if (cell_start[(size_t)ntiles * SWR_SEGS] > cap_pairs) return;
-  const int lane = threadIdx.x & 31;
-  const uint32_t t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (t >= ntiles) return;
-  const uint32_t last = cell_start[(size_t)t * SWR_SEGS + SWR_SEGS];
-  // heavy tiles: listed for k_raster's quadrant CTAs (quad_count is zeroed before this kernel)
-  if (quad_flag && lane == 0) {
-    uint8_t f = 0;
-    if (last - cell_start[(size_t)t * SWR_SEGS] > quad_min) {
-      const uint32_t slot = atomicAdd(quad_count, 1u);
-      if (slot < quad_cap) {
-        quad_tiles[slot] = t;
-        f = 1;
-      }
-    }
-    quad_flag[t] = f;
-  }
-  // tiles of at most `self_sorted` entries are ordered by the raster kernel itself
-  if (last - cell_start[(size_t)t * SWR_SEGS] <= self_sorted) return;  // uniform per warp
-  const uint32_t s = cell_start[(size_t)t * SWR_SEGS + lane];
-  // every lane takes part in the shuffle; lane 31 then uses the next tile's first start
-  const uint32_t nxt = __shfl_down_sync(0xffffffffu, s, 1);
-  const uint32_t e = lane < SWR_SEGS - 1 ? nxt : last;
-  // starts are an exclusive scan (monotone, bounded by the total <= cap_pairs); anything
-  // else leaves the cell empty instead of walking a wrapped length
-  const uint32_t m = (e >= s && e <= cap_pairs) ? e - s : 0u;
-  constexpr int kSmall = 16;
-  if (m <= kSmall) {
-    uint32_t v[kSmall];
-#pragma unroll
-    for (int i = 0; i < kSmall; ++i) v[i] = (uint32_t)i < m ? in[s + i] : 0xffffffffu;
-    // odd-even transposition network on 16 registers
-#pragma unroll
-    for (int r = 0; r < kSmall; ++r)
-#pragma unroll
-      for (int i = r & 1; i + 1 < kSmall; i += 2)
-        if (v[i] > v[i + 1]) { const uint32_t x = v[i]; v[i] = v[i + 1]; v[i + 1] = x; }
-#pragma unroll
-    for (int i = 0; i < kSmall; ++i)
-      if ((uint32_t)i < m) out[s + i] = v[i];
-  }
-  constexpr uint32_t kListed = 64;  // above this the warp rank sort below costs more than a bitmap
-  const bool listed = big_list && m > kListed;
-  if (listed) big_list[atomicAdd(big_count, 1u)] = t * SWR_SEGS + (uint32_t)lane;
-  uint32_t big = __ballot_sync(0xffffffffu, m > kSmall && !listed);
-  while (big) {
-    const int c = __ffs(big) - 1;
-    big &= big - 1u;
-    const uint32_t cs = __shfl_sync(0xffffffffu, s, c), cm = __shfl_sync(0xffffffffu, m, c);
-    for (uint32_t i0 = 0; i0 < cm; i0 += 32) {
-      const uint32_t i = i0 + lane;
-      const uint32_t val = i < cm ? in[cs + i] : 0xffffffffu;
-      uint32_t rank = 0;
-      for (uint32_t j0 = 0; j0 < cm; j0 += 32) {
-        const uint32_t w = j0 + lane < cm ? in[cs + j0 + lane] : 0xffffffffu;
-#pragma unroll 8
-        for (int l = 0; l < 32; ++l) rank += __shfl_sync(0xffffffffu, w, l) < val;
-      }
-      if (i < cm) out[cs + rank] = val;
-    }
-  }
-}
-
-// The cells listed by k_sort_cells, one warp per cell (grid-stride over the list): the ids
-// of cell (tile, seg) all lie in segment seg's range [seg << shift, (seg + 1) << shift), so
-// a bitmap of that range in the warp's slice of shared memory sorts them: set one bit per
-// id (only the words between the cell's smallest and largest id are touched), prefix-count
-// the words across the lanes, write the set bits out in order.  Dynamic shared memory:
-// (1 << shift) / 8 bytes per warp.  big_count[0] is the list length (reset after the draw).
-static __global__ void k_sort_big(uint32_t* status, const uint32_t* cell_start, uint32_t ncells,
-                                  uint32_t cap_pairs, int seg_shift, const uint32_t* in, uint32_t* out,
-                                  const uint32_t* big_list, uint32_t* big_count) {
+// Orders the cells of the listed tiles (ids in `in`, increasing within a cell in `out`): one
+// CTA per tile, its cells dealt to the CTA's warps.  Cells of up to 32 ids are ranked by
+// shuffles; larger ones through a bitmap of the segment's id range [seg << shift, (seg + 1) <<
+// shift) in the warp's slice of shared memory (bm_words words; only those between the cell's
+// smallest and largest id are touched): set one bit per id, prefix-count the words across the
+// lanes, write the set bits out in order.  Without a bitmap (bm_words 0: the range does not
+// fit) larger cells are ranked 32 ids at a time.  Cells of at most cell_min ids are left alone.
+static __global__ void __launch_bounds__(256) k_sort_tiles(const uint32_t* status, const SwrTiles tiles, int seg_shift,
+                                                           uint32_t bm_words, uint32_t cell_min, const uint32_t* in,
+                                                           uint32_t* out) {
   swr_pdl_entry();
   extern __shared__ uint32_t smem_bm[];
-  const bool skip = (status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) || cell_start[ncells] > cap_pairs;
-  const uint32_t nbig = skip ? 0u : min(*(volatile uint32_t*)big_count, ncells);
+  if (status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  uint32_t* bm = smem_bm + (size_t)wib * bm_words;
   const uint32_t R = 1u << seg_shift;
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  uint32_t* bm = smem_bm + (size_t)wib * (R >> 5);
-  const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
-  for (uint32_t bi = blockIdx.x * (blockDim.x >> 5) + wib; bi < nbig; bi += nwarps) {
-    const uint32_t cell = big_list[bi];
-    if (cell >= ncells) continue;  // uniform per warp
-    const uint32_t s = cell_start[cell], e = cell_start[cell + 1];
-    const uint32_t m = (e >= s && e <= cap_pairs) ? e - s : 0u;
-    const uint32_t lo_id = (cell % SWR_SEGS) << seg_shift;
-    uint32_t lo = 0xffffffffu, hi = 0u;
-    for (uint32_t j = lane; j < m; j += 32) {
-      const uint32_t v = in[s + j] - lo_id;
-      if (v < R) {
-        lo = min(lo, v);
-        hi = max(hi, v);
+  const uint32_t nsort = min(tiles.counts[3], tiles.ntiles);
+  for (uint32_t i = blockIdx.x; i < nsort; i += gridDim.x) {
+    const uint4 entry = tiles.sort[i];
+    const uint32_t* cells = tiles.start + (size_t)entry.x * SWR_SEGS;
+    for (uint32_t c = wib; c < SWR_SEGS; c += nwarps) {  // (uniform per warp, like all below)
+      const uint32_t s = cells[c], e = c + 1 < SWR_SEGS ? cells[c + 1] : entry.z;
+      const uint32_t m = e > s ? e - s : 0u;
+      if (m == 0 || m <= cell_min) continue;
+      if (m <= 32 || !bm_words) {
+        for (uint32_t i0 = 0; i0 < m; i0 += 32) {
+          const uint32_t val = i0 + lane < m ? in[s + i0 + lane] : 0xffffffffu;
+          uint32_t rank = 0;
+          for (uint32_t j0 = 0; j0 < m; j0 += 32) {
+            const uint32_t w = j0 + lane < m ? in[s + j0 + lane] : 0xffffffffu;
+#pragma unroll 8
+            for (int l = 0; l < 32; ++l) rank += __shfl_sync(0xffffffffu, w, l) < val;
+          }
+          if (i0 + lane < m) out[s + rank] = val;
+        }
+        continue;
       }
-    }
-    lo = __reduce_min_sync(0xffffffffu, lo);
-    hi = __reduce_max_sync(0xffffffffu, hi);
-    if (lo > hi) continue;  // uniform: no valid id
-    const uint32_t w0 = lo >> 5, nw = (hi >> 5) - w0 + 1;
-    for (uint32_t w = lane; w < nw; w += 32) bm[w0 + w] = 0u;
-    __syncwarp();
-    for (uint32_t j = lane; j < m; j += 32) {
-      const uint32_t v = in[s + j] - lo_id;
-      if (v < R) atomicOr(&bm[v >> 5], 1u << (v & 31));
-    }
-    __syncwarp();
-    // lane l owns words [l * per, (l + 1) * per) of the range
-    const uint32_t per = (nw + 31) / 32;
-    const uint32_t a = min(nw, (uint32_t)lane * per), b = min(nw, a + per);
-    uint32_t cnt = 0;
-    for (uint32_t w = a; w < b; ++w) cnt += __popc(bm[w0 + w]);
-    uint32_t inc = cnt;
+      const uint32_t lo_id = c << seg_shift;
+      uint32_t lo = 0xffffffffu, hi = 0u;
+      for (uint32_t j = lane; j < m; j += 32) {
+        const uint32_t v = in[s + j] - lo_id;
+        if (v < R) {
+          lo = min(lo, v);
+          hi = max(hi, v);
+        }
+      }
+      lo = __reduce_min_sync(0xffffffffu, lo);
+      hi = __reduce_max_sync(0xffffffffu, hi);
+      if (lo > hi) continue;
+      const uint32_t w0 = lo >> 5, nw = (hi >> 5) - w0 + 1;
+      for (uint32_t w = lane; w < nw; w += 32) bm[w0 + w] = 0u;
+      __syncwarp();
+      for (uint32_t j = lane; j < m; j += 32) {
+        const uint32_t v = in[s + j] - lo_id;
+        if (v < R) atomicOr(&bm[v >> 5], 1u << (v & 31));
+      }
+      __syncwarp();
+      const uint32_t per = (nw + 31) / 32;  // lane l owns words [l * per, (l + 1) * per) of the range
+      const uint32_t a = min(nw, (uint32_t)lane * per), b = min(nw, a + per);
+      uint32_t cnt = 0;
+      for (uint32_t w = a; w < b; ++w) cnt += __popc(bm[w0 + w]);
+      uint32_t inc = cnt;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += y;
-    }
-    uint32_t pos = inc - cnt;
-    for (uint32_t w = a; w < b; ++w) {
-      uint32_t bits = bm[w0 + w];
-      while (bits) {
-        const int bit = __ffs(bits) - 1;
-        bits &= bits - 1u;
-        if (pos < m) out[s + pos] = lo_id + ((w0 + w) << 5) + (uint32_t)bit;
-        ++pos;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
       }
-    }
-    __syncwarp();
-  }
-  // The last block to finish closes the draw: the list ([length, blocks done]) is consumed,
-  // and every counting stage has run (the tile raster counts only fragments).
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    if (atomicAdd(&big_count[1], 1u) == gridDim.x - 1) {
-      swr_close_status(status);
-      big_count[0] = 0u;
-      big_count[1] = 0u;
+      uint32_t pos = inc - cnt;
+      for (uint32_t w = a; w < b; ++w) {
+        uint32_t bits = bm[w0 + w];
+        while (bits) {
+          const int bit = __ffs(bits) - 1;
+          bits &= bits - 1u;
+          if (pos < m) out[s + pos] = lo_id + ((w0 + w) << 5) + (uint32_t)bit;
+          ++pos;
+        }
+      }
+      __syncwarp();
     }
   }
 }
@@ -1275,17 +1200,15 @@ __device__ __forceinline__ void swr_persp_deriv(const GpuPixel<PS>& p, int i, fl
 
 struct RasterArgs {
   const uint32_t* status;
-  const uint32_t* tile_start;  // bin start of tile t at tile_start[t * tile_stride] (plus the end)
-  uint32_t tile_stride;        // 1 for per-tile starts, SWR_SEGS for per-(tile, segment) cells
+  SwrTiles tiles;              // the tiles to rasterize, their bins and cells (k_cells); or, with
+                               // tiles.list null, all of them:
+  const uint32_t* tile_start;  // bin start of tile t at tile_start[t] (plus the end)
   const uint32_t* bin;         // primitive ids, each tile's range in increasing order
-  const uint32_t* bin_raw;     // optional: the unsorted ids (cell layout, tile_stride SWR_SEGS);
-                               // tiles of <= SWR_RASTER_SORT entries order them in the kernel
-                               // (k_sort_cells skips them)
+  const uint32_t* bin_raw;     // optional: the unsorted ids (cells); tiles of <= SWR_RASTER_SORT
+                               // entries order them in the kernel, and have no range in `bin`
   const float* recs;
   const SwrDrawDesc* draws;
   const SwrTargetDesc* targets;
-  const uint32_t* target_tile_base;  // per target, for the tile -> target lookup
-  int ntargets;
   const uint32_t* draw_prim_base;    // per draw first primitive (null: a single draw from 0)
   uint32_t* status_w;
   uint32_t ntiles;
@@ -1294,24 +1217,20 @@ struct RasterArgs {
   uint32_t* best;                    // their pixels' winners, primitive id + 1, [tile][TILE * TILE]
   uint32_t* best_done;               // per tile: the slices finished (both zero between draws)
   int has_span;                      // some draw rasterizes in Span or Adaptive mode (selects k_raster<..., true>)
-  // Quadrant CTAs (16-px tiles): a heavy tile -- more
-  // than quad_min bin entries; k_sort_cells lists up to quad_cap of them -- is rasterized by
-  // four CTAs, one per 8 x 8 quadrant, each walking the whole bin for its own pixels, so the
-  // slowest tiles no longer set the kernel's length.  CTAs [0, 4 quad_cap) take the listed
-  // tiles' quadrants first; CTA 4 quad_cap + t takes tile t unless it is listed.  With
-  // quad_all every tile is split (CTA 4 t + q: quadrant q of tile t): an 8-px raster tile
-  // over 16-px bins.
-  const uint8_t* quad_flag;          // per tile: 1 = listed (null: no heavy-tile split)
-  const uint32_t* quad_tiles;        // listed tiles
-  const uint32_t* quad_count;        // tiles k_sort_cells listed (may exceed quad_cap)
-  uint32_t quad_cap;
+  // Quadrant CTAs (quad; 16-px tiles): a heavy tile -- more than three chunks of bin entries;
+  // k_cells lists up to tiles.heavy_cap of them -- is rasterized by four CTAs, one per 8 x 8
+  // quadrant, each walking the whole bin for its own pixels, so the slowest tiles no longer
+  // set the kernel's length.  CTAs [0, 4 heavy_cap) take the listed tiles' quadrants; CTA
+  // 4 heavy_cap + i takes entry i of the list of the others.  With quad_all every tile is split
+  // (CTA 4 i + q: quadrant q of entry i): an 8-px raster tile over 16-px bins.
+  int quad;
   int quad_all;
-  // Sliced heavy tiles (depth-min shaders, SwrDepthMin): with dslice set, each tile of the
-  // same list is rasterized by SWR_DSLICES CTAs instead, each over a run of whole chunks of
+  // Sliced heavy tiles (depth-min shaders, SwrDepthMin): with dslice set, each tile of
+  // tiles.heavy is rasterized by SWR_DSLICES CTAs instead, each over a run of whole chunks of
   // its ordered bin and from the draw's starting State; each writes its States to
   // dslice_state, and the last of the tile's CTAs to finish merges them in bin order
-  // (swr_depth_merge) and stores.  CTAs [0, SWR_DSLICES quad_cap) take the listed tiles'
-  // slices; CTA SWR_DSLICES quad_cap + t takes tile t unless it is listed.
+  // (swr_depth_merge) and stores.  CTAs [0, SWR_DSLICES heavy_cap) take the listed tiles'
+  // slices; CTA SWR_DSLICES heavy_cap + i takes entry i of the list of the others.
   int dslice;
   // Small draws (k_raster<..., true>): no bins; every CTA picks its tile's primitives, in order,
   // from the packed tile boxes of all `status[SWR_ST_PRIMS]` primitives.
@@ -1651,6 +1570,8 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
   __shared__ uint32_t sculr[kCull ? NREG * NW : 1];  // per region: primitives only counted there
   __shared__ int sminx[kCull && SPAN ? CH : 1];  // Span mode: leftmost start of a span reaching the tile
   constexpr int HW = (CH + 63) / 64;  // 64-primitive words of a chunk
+  // the draw's queue requests are final (nothing after this stage counts)
+  if (!DIRECT && blockIdx.x == 0 && threadIdx.x == 0) swr_close_status(g.status_w);
   if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint32_t frags = 0, passes = 0;
@@ -1659,44 +1580,44 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
   uint32_t tile = blockIdx.x, slice = 0;
   int quad = -1;  // the 8 x 8 quadrant (block) this CTA rasterizes alone, -1: the whole tile
   int dslot = -1;  // sliced heavy tile: its list slot (slice = its run)
-  if constexpr (SwrDepthMin<PS>::value && !DIRECT) {
-    if (g.dslice) {
-      const uint32_t nq = SWR_DSLICES * g.quad_cap;
-      if (blockIdx.x < nq) {
-        const uint32_t slot = blockIdx.x / SWR_DSLICES;
-        if (slot >= min(*g.quad_count, g.quad_cap)) return;
-        tile = g.quad_tiles[slot];
-        slice = blockIdx.x - slot * SWR_DSLICES;
-        dslot = (int)slot;
-      } else {
-        tile = blockIdx.x - nq;
-        if (tile < g.ntiles && g.quad_flag[tile]) return;  // rasterized in slices
-      }
-    }
-  }
-  if constexpr (TILE == 16 && !DIRECT) {
-    if (g.dslice) {
-    } else if (g.quad_all) {
-      tile = blockIdx.x >> 2;
-      quad = (int)(blockIdx.x & 3u);
-    } else if (g.quad_flag) {
-      const uint32_t nq = 4u * g.quad_cap;
+  uint32_t b = 0, e = 0;
+  int ti = 0;  // its target
+  if constexpr (!DIRECT) {
+    if (g.tiles.list) {
+      uint4 entry;
+      constexpr uint32_t kRuns = SWR_DSLICES > 4 ? SWR_DSLICES : 4;
+      static_assert(kRuns == 4 && SWR_DSLICES == 4, "four CTAs per heavy tile, as runs or as quadrants");
+      const bool heavy = (SwrDepthMin<PS>::value && g.dslice) || (TILE == 16 && g.quad);
+      const uint32_t nq = heavy ? 4u * g.tiles.heavy_cap : 0u;
       if (blockIdx.x < nq) {
         const uint32_t slot = blockIdx.x >> 2;
-        if (slot >= min(*g.quad_count, g.quad_cap)) return;
-        tile = g.quad_tiles[slot];
-        quad = (int)(blockIdx.x & 3u);
+        if (slot >= min(g.tiles.counts[0], g.tiles.heavy_cap)) return;
+        entry = __ldg(g.tiles.heavy + slot);
+        if (SwrDepthMin<PS>::value && g.dslice) {
+          slice = blockIdx.x & 3u;
+          dslot = (int)slot;
+        } else {
+          quad = (int)(blockIdx.x & 3u);
+        }
       } else {
-        tile = blockIdx.x - nq;
-        if (tile < g.ntiles && g.quad_flag[tile]) return;  // rasterized by its quadrant CTAs
+        uint32_t i = blockIdx.x - nq;
+        if (TILE == 16 && g.quad_all) {
+          quad = (int)(i & 3u);
+          i >>= 2;
+        }
+        if (!swr_listed_tile(g.tiles, i, entry)) return;
       }
+      tile = entry.x;
+      b = entry.y;
+      e = entry.z;
+      ti = (int)entry.w;
+    } else {
+      if (tile >= g.ntiles) return;
+      b = g.tile_start[tile];
+      e = g.tile_start[tile + 1];
     }
-  }
-  if (tile >= g.ntiles) return;
-  uint32_t b = 0, e = 0;
-  if constexpr (!DIRECT) {
-    b = g.tile_start[(size_t)tile * g.tile_stride];
-    e = g.tile_start[(size_t)(tile + 1) * g.tile_stride];
+  } else {
+    if (tile >= g.ntiles) return;
   }
   // Small draws: the tile's primitives out of the next windows of 256 boxes, in order, until
   // more than 256 are found (e = their count; ssorted holds SWR_RASTER_SORT) or none is left.
@@ -1738,7 +1659,6 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
     cb = b + (uint32_t)((uint64_t)nch * slice / (uint32_t)nsl) * CH;
     ce = min(e, b + (uint32_t)((uint64_t)nch * (slice + 1) / (uint32_t)nsl) * CH);
   }
-  const int ti = !DIRECT && g.ntargets > 1 ? swr_find_le(g.target_tile_base, g.ntargets, tile) : 0;
   const SwrTargetDesc& T = g.targets[ti];
   const SwrUniforms& U = g.draws[T.first_draw].u;
   const uint32_t lt = tile - T.tile_base;
@@ -1766,7 +1686,8 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
   if (!DIRECT && self_sort) {
     uint32_t* sraw = (uint32_t*)srec4;
     const uint32_t ntot = e - b;
-    if (threadIdx.x <= SWR_SEGS) scs[threadIdx.x] = g.tile_start[(size_t)tile * SWR_SEGS + threadIdx.x] - b;
+    if (threadIdx.x <= SWR_SEGS)
+      scs[threadIdx.x] = (threadIdx.x < SWR_SEGS ? g.tiles.start[(size_t)tile * SWR_SEGS + threadIdx.x] : e) - b;
     for (uint32_t j = threadIdx.x; j < ntot; j += 256) sraw[j] = g.bin_raw[b + j];
     __syncthreads();
     for (uint32_t j = threadIdx.x; j < ntot; j += 256) {
@@ -2311,7 +2232,7 @@ __global__ void __launch_bounds__(256) k_overwrite(RasterArgs g) {
   if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
   const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint32_t tile = blockIdx.x, slice = 0, n = 0, hi = 0;
-  int nsl = 1;
+  int nsl = 1, ti = 0;
   if constexpr (DIRECT) {
     n = min(g.status[SWR_ST_PRIMS], g.cap_prims);
   } else {
@@ -2319,8 +2240,19 @@ __global__ void __launch_bounds__(256) k_overwrite(RasterArgs g) {
       tile = blockIdx.x / (uint32_t)g.slices;
       slice = blockIdx.x - tile * (uint32_t)g.slices;
     }
-    if (tile >= g.ntiles) return;
-    const uint32_t b = g.tile_start[(size_t)tile * g.tile_stride], e = g.tile_start[(size_t)(tile + 1) * g.tile_stride];
+    uint32_t b, e;
+    if (g.tiles.list) {
+      uint4 entry;
+      if (!swr_listed_tile(g.tiles, tile, entry)) return;
+      tile = entry.x;
+      b = entry.y;
+      e = entry.z;
+      ti = (int)entry.w;
+    } else {
+      if (tile >= g.ntiles) return;
+      b = g.tile_start[tile];
+      e = g.tile_start[tile + 1];
+    }
     hi = e;
     n = e - b;
     if (n > (uint32_t)SWR_RASTER_SORT && g.slices > 1) {
@@ -2333,7 +2265,6 @@ __global__ void __launch_bounds__(256) k_overwrite(RasterArgs g) {
     }
   }
   if (tile >= g.ntiles || n == 0) return;  // (a slice of more than SWR_RASTER_SORT entries is never empty)
-  const int ti = !DIRECT && g.ntargets > 1 ? swr_find_le(g.target_tile_base, g.ntargets, tile) : 0;
   const SwrTargetDesc& T = g.targets[ti];
   const SwrUniforms& U = g.draws[T.first_draw].u;
   const uint32_t lt = tile - T.tile_base;
