@@ -162,7 +162,7 @@ struct swr_context {
   swr::Buffer draws, targets, draw_vbase, draw_bbase, target_tile_base;
   swr::Buffer ptv, clipv, clip_table, clip_slot, tri_flags, batch_counts, batch_base;
   swr::Buffer tris, recs, tile_count, pair_off, keys0, vals0, keys1, vals1;
-  swr::Buffer scratch, status, direct_keep, direct_pos, lp_refs, cell_count, cell_start, cell_fill, draw_pbase;
+  swr::Buffer scratch, status, lp_refs, cell_count, cell_start, cell_fill, draw_pbase;
   swr::Buffer tile_list, heavy_tiles, sort_tiles, tile_counts;  // SwrTiles
   int quad_mode = 0;  // 0: off, 1: heavy tiles (more than kQuadMin entries), 2: every tile (8-px raster tiles)
   bool persistent_geometry = false;  // swr_set_persistent_geometry
@@ -214,7 +214,7 @@ struct swr_context {
     swr::Buffer* all[] = {&draws, &targets, &draw_vbase, &draw_bbase, &target_tile_base, &ptv, &clipv,
                           &clip_table, &clip_slot, &tri_flags, &batch_counts, &batch_base, &tris, &recs,
                           &tile_count, &pair_off, &keys0, &vals0, &keys1, &vals1, &scratch,
-                          &status, &direct_keep, &direct_pos, &lp_refs, &cell_count, &cell_start, &cell_fill, &draw_pbase,
+                          &status, &lp_refs, &cell_count, &cell_start, &cell_fill, &draw_pbase,
                           &tile_list, &heavy_tiles, &sort_tiles, &tile_counts, &over_best, &over_done, &geo_bar,
                           &dslice_state, &dslice_done};
     for (swr::Buffer* b : all) b->budget = &budget;
@@ -290,7 +290,7 @@ int ensure_capacity(swr_context* c, uint32_t nverts_ptv, int S, uint32_t nsub, u
   ok &= c->tile_list.ensure((size_t)ntiles * 16);
   ok &= c->sort_tiles.ensure((size_t)ntiles * 16);
   ok &= c->heavy_tiles.ensure((size_t)quad_cap(ntiles) * 16);
-  ok &= c->tile_counts.ensure(16);
+  ok &= c->tile_counts.ensure(32);
   ok &= c->geo_bar.ensure(16);
   // Overwrite shaders: a sliced tile's winners and finished slices (optional; both start at
   // zero, and the last slice of a tile leaves them at zero)
@@ -343,6 +343,9 @@ void fill_draw(const swr_context* c, SwrDrawDesc& D, int mode) {
   D.u = c->u;
 }
 
+// Zeroed word for the last-block scan of a draw's counting kernel.
+uint32_t* block_counter(const swr_context* c) { return c->tile_counts.as<uint32_t>() + 4; }
+
 AssembleArgs assemble_args(swr_context* c, int ndraws, uint32_t* draw_prim_base) {
   AssembleArgs aa;
   memset(&aa, 0, sizeof(aa));
@@ -358,6 +361,7 @@ AssembleArgs assemble_args(swr_context* c, int ndraws, uint32_t* draw_prim_base)
   aa.batch_base = c->batch_base.as<uint32_t>();
   aa.tris = c->tris.as<uint4>();
   aa.lp_refs = c->lp_refs.as<uint2>();
+  aa.done = block_counter(c);
   aa.draw_prim_base = draw_prim_base;
   aa.status = c->status.as<uint32_t>();
   aa.cap_clip_slots = c->cap_clip_slots;
@@ -390,7 +394,7 @@ SwrTiles tiles_of(const swr_context* c, uint32_t ntiles, uint32_t heavy_cap) {
   t.list = c->tile_list.as<uint4>();
   t.heavy = c->heavy_tiles.as<uint4>();
   t.sort = c->sort_tiles.as<uint4>();
-  t.counts = c->tile_counts.as<uint32_t>();  // (zeroed by the draw's k_stage_copy)
+  t.counts = c->tile_counts.as<uint32_t>();  // (zeroed by the draw's k_stage_copy; word 4: block_counter)
   t.ntiles = ntiles;
   t.heavy_cap = heavy_cap;
   return t;
@@ -678,7 +682,7 @@ int upload_single(swr_context* c, const SwrDrawDesc& D, const SwrTargetDesc& T, 
   sc.clear(c->draw_bbase.p, 4);
   sc.clear(c->target_tile_base.p, 4);
   sc.clear(c->status.as<uint32_t>() + SWR_ST_CLIP_SLOTS, 5 * 4);
-  sc.clear(c->tile_counts.p, 16);
+  sc.clear(c->tile_counts.p, 32);
   swr::launch(k_stage_copy, 1, 256, 0, s, sc);
   c->launches += 1;
   c->single_cur = slot;
@@ -996,7 +1000,7 @@ int swr_draw_elements(swr_context* c, int mode, uint64_t count, const uint32_t* 
   const bool geo = mode == SWR_DRAW_TRIANGLE && c->persistent_geometry && nbatches;
   if (!geo) vs->vertex(c->draws.as<SwrDrawDesc>(), 1, c->draw_vbase.as<uint32_t>(), (uint32_t)nverts, c->ptv.as<float>(), s);
   mark(c, 1, s);
-  c->launches += (nverts ? 1 : 0) + (nbatches ? 2 : 0) + (mode == SWR_DRAW_TRIANGLE ? 0 : 1);
+  c->launches += (nverts ? 1 : 0) + (nbatches ? 2 : 0);
   const AssembleArgs aa = assemble_args(c, 1, nullptr);  // a single draw numbers its primitives from 0
   c->use_draw_pbase = false;
   if (mode == SWR_DRAW_TRIANGLE) {
@@ -1009,8 +1013,6 @@ int swr_draw_elements(swr_context* c, int mode, uint64_t count, const uint32_t* 
     }
   } else {
     vs->assemble_lp_count(aa, nbatches, s);
-    swr::launch(k_batch_scan, 1, 1024, 0, s, c->batch_counts.as<uint2>(), nbatches, c->batch_base.as<uint32_t>(), st,
-                                    c->cap_prims);
     vs->assemble_lp_emit(aa, nbatches, s);
   }
   mark(c, 2, s);
@@ -1034,10 +1036,9 @@ int swr_draw_list(swr_context* c, int mode, const float* vertices, uint64_t nver
   const uint32_t nsub = (uint32_t)(count / per);
   const SwrTargetDesc T = make_target(c, mode);
   const uint32_t ntiles = (uint32_t)T.tiles_x * (uint32_t)T.tiles_y;
-  int rc = ensure_capacity(c, (uint32_t)nverts, ps->S, nsub, 1, ntiles, ps->R > ps->lp_R ? ps->R : ps->lp_R, ps, 1, s);
+  const uint32_t nbatches = (nsub + SWR_BATCH_PRIMS - 1) / SWR_BATCH_PRIMS;
+  int rc = ensure_capacity(c, (uint32_t)nverts, ps->S, nsub, nbatches, ntiles, ps->R > ps->lp_R ? ps->R : ps->lp_R, ps, 1, s);
   if (rc) return rc;
-  if (!c->direct_keep.ensure((size_t)nsub * 4 + 16) || !c->direct_pos.ensure((size_t)nsub * 4 + 16))
-    return SWR_ENOMEM;
   SwrDrawDesc D;
   fill_draw(c, D, mode);
   D.direct = 1;
@@ -1046,17 +1047,21 @@ int swr_draw_list(swr_context* c, int mode, const float* vertices, uint64_t nver
   if ((rc = upload_single(c, D, T, s))) return rc;
   uint32_t* st = c->status.as<uint32_t>();
   mark(c, 0, s);
-  ps->direct_vertices(vertices, (uint32_t)nverts, c->ptv.as<float>(), s);
+  DirectArgs da;
+  da.rv = vertices;
+  da.nverts = (uint32_t)nverts;
+  da.ptv = c->ptv.as<float>();
+  da.idx = indices;
+  da.nprims = nsub;
+  da.per = per;
+  da.base = c->batch_base.as<uint32_t>();
+  da.done = block_counter(c);
+  da.status = st;
+  da.cap_prims = c->cap_prims;
+  ps->direct_vertices(da, s);
   mark(c, 1, s);
-  c->launches += (nverts ? 1 : 0) + (nsub ? 4 : 0);
-  if (nsub) {
-    const int grid = (int)((nsub + 255) / 256 < 1216 ? (nsub + 255) / 256 : 1216);
-    swr::launch(k_direct_flags, grid, 256, 0, s, indices, nsub, per, c->direct_keep.as<uint32_t>());
-    scan_exclusive(c->direct_keep.as<uint32_t>(), c->direct_pos.as<uint32_t>(), nullptr, nsub,
-                   st + SWR_ST_PRIMS, c->scratch.as<uint32_t>(), s);
-    swr::launch(k_direct_emit, grid, 256, 0, s, indices, nsub, per, (uint32_t)nverts, c->direct_keep.as<uint32_t>(),
-                                       c->direct_pos.as<uint32_t>(), c->tris.as<uint4>(), st);
-  }
+  if (nsub) swr::launch(k_direct_emit, nbatches, 256, 0, s, da, c->tris.as<uint4>());
+  c->launches += (nverts || nsub ? 1 : 0) + (nsub ? 1 : 0);
   mark(c, 2, s);
   c->last_ntiles = ntiles;
   if (mode == SWR_DRAW_TRIANGLE && small_draw(c, nsub, T)) {
@@ -1253,7 +1258,7 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
     // the per-draw working counters and the heavy-tile list restart (flags and fragment
     // totals are sticky)
     sc.clear(c->status.as<uint32_t>() + SWR_ST_CLIP_SLOTS, 5 * 4);
-    sc.clear(c->tile_counts.p, 16);
+    sc.clear(c->tile_counts.p, 32);
     swr::launch(k_stage_copy, kStageCopyBlocks, 256, 0, s, sc);
     c->launches += 1;
     q = cuda_err(cudaGetLastError());

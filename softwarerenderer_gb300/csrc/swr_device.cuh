@@ -237,3 +237,30 @@ __device__ __forceinline__ uint32_t swr_block_exscan(uint32_t v, uint32_t* tmp, 
   __syncthreads();
   return warp_off + x - v;
 }
+
+// End of a counting kernel: the last block to finish turns the blocks' counts into exclusive
+// bases (in place) and returns true in every thread, with their sum; the others return false.
+// Each thread of it takes a contiguous run of counts, so the tail is two short passes.  `done`
+// is zero before the kernel and after it.  Every block calls this once, whatever it counted.
+__device__ __forceinline__ bool swr_last_block_scan(uint32_t* counts, uint32_t n, uint32_t* done, uint32_t* total) {
+  __shared__ uint32_t tmp[32];
+  __shared__ uint32_t last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  const uint32_t per = (n + blockDim.x - 1) / blockDim.x;
+  const uint32_t b = min(n, threadIdx.x * per), e = min(n, b + per);
+  uint32_t s = 0;
+  for (uint32_t i = b; i < e; ++i) s += __ldcg(counts + i);
+  uint32_t run = swr_block_exscan(s, tmp, total);
+  for (uint32_t i = b; i < e; ++i) {
+    const uint32_t c = __ldcg(counts + i);
+    counts[i] = run;
+    run += c;
+  }
+  if (threadIdx.x == 0) *done = 0u;
+  return true;
+}

@@ -125,7 +125,12 @@ __global__ void __launch_bounds__(256) k_assemble_lp_count(AssembleArgs g) {
   }
   uint32_t tot;
   swr_block_exscan(sum, tmp, &tot);
-  if (threadIdx.x == 0) g.batch_counts[b] = make_uint2(tot, 0u);
+  if (threadIdx.x == 0) g.batch_base[b] = tot;
+  uint32_t total;
+  if (swr_last_block_scan(g.batch_base, gridDim.x, g.done, &total) && threadIdx.x == 0) {
+    g.status[SWR_ST_PRIMS] = total;
+    if (total > g.cap_prims) atomicOr(&g.status[SWR_ST_FLAGS], SWR_F_PRIM_OVERFLOW);
+  }
 }
 
 static __global__ void __launch_bounds__(256) k_assemble_lp_emit(AssembleArgs g) {
@@ -403,7 +408,7 @@ __global__ void __launch_bounds__(256) k_lp_raster(LpRasterArgs g) {
   __shared__ int sstep[kCompact ? 1 : CH];
   __shared__ float sz[kCompact ? CH : 1];
   __shared__ Color sc[kCompact ? CH : 1];
-  __shared__ uint32_t sfr[32];
+  __shared__ uint32_t sfr[64];
   if (blockIdx.x == 0 && threadIdx.x == 0) swr_close_status(g.status_w);
   if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
   uint4 entry;
@@ -509,8 +514,7 @@ __global__ void __launch_bounds__(256) k_lp_raster(LpRasterArgs g) {
     passes = st.writes;
   }
   uint32_t tot, ptot;
-  swr_block_exscan(frags, sfr, &tot);
-  swr_block_exscan(passes, sfr, &ptot);
+  swr_block_sum2(frags, passes, sfr, tot, ptot);
   if (tid == 0 && tot) {
     atomicAdd((unsigned long long*)&g.status_w[SWR_ST_SHADED_LO], (unsigned long long)tot);
     atomicAdd((unsigned long long*)&g.status_w[SWR_ST_PASSES_LO], (unsigned long long)ptot);

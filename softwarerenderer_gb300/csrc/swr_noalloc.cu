@@ -51,7 +51,7 @@ constexpr size_t kBytes = 8u << 20;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kBytes];
 
 struct Layout {
-  size_t status, draw, target, ptv, keep, pos, tris, recs, tile_count, pair_off;
+  size_t status, draw, target, ptv, base, tris, recs, tile_count, pair_off;
   size_t keys0, vals0, keys1, vals1, tile_start, scan_scr, sort_scr, end;
 };
 
@@ -61,12 +61,11 @@ Layout make_layout() {
   Layout L;
   size_t o = 0;
   auto take = [&](size_t bytes) { const size_t at = o; o = align256(o + bytes); return at; };
-  L.status = take(16 * 4);
+  L.status = take(32 * 4);
   L.draw = take(sizeof(SwrDrawDesc));
   L.target = take(sizeof(SwrTargetDesc));
   L.ptv = take((size_t)kMaxVerts * kMaxS * 4);
-  L.keep = take((size_t)kMaxTris * 4);
-  L.pos = take((size_t)kMaxTris * 4);
+  L.base = take((size_t)(kMaxTris / SWR_BATCH_PRIMS) * 4);
   L.tris = take((size_t)kMaxTris * 16);
   L.recs = take((size_t)kMaxTris * kMaxR * 4);
   L.tile_count = take((size_t)kMaxTris * 4);
@@ -200,8 +199,6 @@ extern "C" int swr_draw_triangle_list_noalloc(const struct SwrUniforms* u, int p
   SwrDrawDesc* dd = (SwrDrawDesc*)(base + L.draw);
   SwrTargetDesc* dt = (SwrTargetDesc*)(base + L.target);
   float* ptv = (float*)(base + L.ptv);
-  uint32_t* keep = (uint32_t*)(base + L.keep);
-  uint32_t* pos = (uint32_t*)(base + L.pos);
   uint4* tris = (uint4*)(base + L.tris);
   float* recs = (float*)(base + L.recs);
   uint32_t* tile_count = (uint32_t*)(base + L.tile_count);
@@ -216,18 +213,24 @@ extern "C" int swr_draw_triangle_list_noalloc(const struct SwrUniforms* u, int p
 
   // The previous call's contents stay in the array: reset the status words and the primitive
   // count before any kernel reads them.
-  cudaMemsetAsync(st, 0, 16 * 4, s);
+  cudaMemsetAsync(st, 0, 32 * 4, s);
   cudaMemcpyAsync(dd, &D, sizeof(D), cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(dt, &T, sizeof(T), cudaMemcpyHostToDevice, s);
   if ((rc = (cudaGetLastError() == cudaSuccess ? SWR_OK : SWR_ECUDA))) return rc;
 
-  ps->direct_vertices(vertices, (uint32_t)nverts, ptv, s);
-  if (nsub) {
-    const int grid = (int)((nsub + 255) / 256);
-    k_direct_flags<<<grid, 256, 0, s>>>(indices, nsub, 3, keep);
-    scan_exclusive(keep, pos, nullptr, nsub, st + SWR_ST_PRIMS, scan_scr, s);
-    k_direct_emit<<<grid, 256, 0, s>>>(indices, nsub, 3, (uint32_t)nverts, keep, pos, tris, st);
-  }
+  DirectArgs da;
+  da.rv = vertices;
+  da.nverts = (uint32_t)nverts;
+  da.ptv = ptv;
+  da.idx = indices;
+  da.nprims = nsub;
+  da.per = 3;
+  da.base = (uint32_t*)(base + L.base);
+  da.done = st + 16;
+  da.status = st;
+  da.cap_prims = kMaxTris;
+  ps->direct_vertices(da, s);
+  if (nsub) k_direct_emit<<<(nsub + SWR_BATCH_PRIMS - 1) / SWR_BATCH_PRIMS, 256, 0, s>>>(da, tris);
   SetupArgs sa;
   memset(&sa, 0, sizeof(sa));  // no cell counting: this path bins with the radix sort
   sa.tris = tris;

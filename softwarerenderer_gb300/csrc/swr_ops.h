@@ -25,7 +25,7 @@ struct VsOps {
 
 struct PsOps {
   int A, P, R, S;  // AVarCount, PVarCount, setup record words, direct-path vertex stride
-  void (*direct_vertices)(const float* rv, uint32_t n, float* ptv, cudaStream_t s);
+  void (*direct_vertices)(const DirectArgs& a, cudaStream_t s);
   void (*setup)(const SetupArgs& a, cudaStream_t s);
   void (*emit_pairs)(const uint32_t* status, uint32_t cap_prims, const float* recs,
                      const uint32_t* tile_count, const uint32_t* pair_off, const uint32_t* npairs,

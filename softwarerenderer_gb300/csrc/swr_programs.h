@@ -269,7 +269,7 @@ struct PsLambert {
 // Lambert-lit and textured (nearest RGBA8), depth-tested (config: batched meshes).
 struct PsLambertTex {
   enum { AVarCount = 3, PVarCount = 2, InterpolateZ = 1, InterpolateW = 1, HasDepth = 1, RasterOccupancy = 6,
-         RasterOccupancyBlock = 7, DepthCull = 0, DepthMin = 1 };
+         RasterOccupancyBlock = 6, RasterThreadsBlock = 128, DepthCull = 0, DepthMin = 1 };
   typedef SwrStateRGBA8 State;
   SWR_HD static void load(State& s, int x, int y, const SwrUniforms& u) { swr_load_rgba8<true>(s, x, y, u); }
   SWR_HD static void store(const State& s, int x, int y, const SwrUniforms& u) { swr_store_rgba8(s, x, y, u, true); }
@@ -717,7 +717,7 @@ SWR_HD void swr_depth_merge(SwrStateRGBA8& acc, const SwrStateRGBA8& later) {
 // 6 / 7 CTAs per SM: vertex colour (4K soup) 4401 / 4217 / 4339 / 4569 us; Lambert (dense
 // 1080p mesh) 119.7 / 115.6 / 112.7 / 120.2; Lambert-textured in Block mode (256 meshes) 3914 /
 // 3524 / 3292 / 3172, in Span mode (20k triangles) 81 / 80 / 79 / 88; differentiable (16
-// views) 619 / 592 / 577 / 602.
+// views) 619 / 592 / 577 / 602.  In units of 256 threads: CTAs of 128 threads count half.
 template <class PS, class = void>
 struct SwrRasterOccupancySpan {
   enum { value = 4 };
@@ -733,6 +733,22 @@ struct SwrRasterOccupancy {
 template <class PS>
 struct SwrRasterOccupancy<PS, decltype((void)PS::RasterOccupancyBlock)> {
   enum { value = SwrRasterOccupancySpan<PS>::value, block = PS::RasterOccupancyBlock };
+};
+
+// Threads per tile-raster CTA for submissions of Block-mode draws on 16-px tiles
+// (RasterThreadsBlock in the shader: 128 or 256, the default).  Tiles of few primitives do not
+// fill 256 threads in the stages between a CTA's barriers, and more, smaller CTAs hide more of
+// their latency: 256 meshes (30 entries in a tile that has any) 3025 us a draw with 256
+// threads, 2956 / 2925 / 2874 / 2932 with 8 / 10 / 12 / 14 CTAs of 128 per SM.  The others lose
+// by it (4K soup 4180 -> 6058, 60k-triangle list 200 -> 239, 20k-triangle Span mesh 73 -> 77,
+// dense 1080p mesh 96 -> 98).
+template <class PS, class = void>
+struct SwrRasterThreadsBlock {
+  enum { value = 256 };
+};
+template <class PS>
+struct SwrRasterThreadsBlock<PS, decltype((void)PS::RasterThreadsBlock)> {
+  enum { value = PS::RasterThreadsBlock };
 };
 
 // Pixel shaders whose drawPixel has side effects beyond its State (user shaders that write

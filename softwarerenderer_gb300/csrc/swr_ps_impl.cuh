@@ -10,11 +10,11 @@ namespace {
 constexpr int kGrid = 152 * 8;
 
 template <class PS>
-void run_direct(const float* rv, uint32_t n, float* ptv, cudaStream_t s) {
-  if (!n) return;
-  const uint32_t want = (n + 255) / 256;
-  const int grid = (int)(want < (uint32_t)kGrid ? want : (uint32_t)kGrid);
-  swr::launch(k_direct_vertices<PS::AVarCount, PS::PVarCount>, grid, 256, 0, s, rv, n, ptv);
+void run_direct(const DirectArgs& a, cudaStream_t s) {
+  const uint32_t nb = (a.nprims + SWR_BATCH_PRIMS - 1) / SWR_BATCH_PRIMS, nv = (a.nverts + 255) / 256;
+  const uint32_t want = nb > nv ? nb : nv;
+  const uint32_t grid = want < (uint32_t)kGrid ? want : (uint32_t)kGrid;
+  if (grid) swr::launch(k_direct_vertices<PS::AVarCount, PS::PVarCount>, grid, 256, 0, s, a);
 }
 
 template <class PS>
@@ -67,8 +67,9 @@ void run_raster(const RasterArgs& a, uint32_t ntiles, int tile, cudaStream_t s) 
       if (a.has_span) swr::launch(k_raster<PS, 32, kChunk, true>, grid, 256, 0, s, a);
       else swr::launch(k_raster<PS, 32, kChunk, false>, grid, 256, 0, s, a);
     } else {
+      constexpr int kBlockThreads = SwrRasterThreadsBlock<PS>::value;
       if (a.has_span) swr::launch(k_raster<PS, 16, kChunk, true>, grid, 256, 0, s, a);
-      else swr::launch(k_raster<PS, 16, kChunk, false>, grid, 256, 0, s, a);
+      else swr::launch(k_raster<PS, 16, kChunk, false, false, kBlockThreads>, grid, kBlockThreads, 0, s, a);
     }
   }
 }

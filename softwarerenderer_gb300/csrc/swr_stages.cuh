@@ -103,17 +103,77 @@ __global__ void __launch_bounds__(256) k_vertex(const SwrDrawDesc* __restrict__ 
 
 // Direct Rasterizer path: RasterizerVertex (x, y, z, w, avar[16], pvar[16]) records are
 // already in screen space; convert them to the post-transform layout of the pixel shader.
+// Primitives whose first index is -1 are skipped (Rasterizer::drawTriangleList,
+// Rasterizer.h:134-141); others keep their order: the same launch counts the kept ones of
+// every SWR_BATCH_PRIMS submitted, and its last block turns the counts into bases (a flag
+// per primitive and a scan of them were three more launches, 10 us of a list draw's chain).
+struct DirectArgs {
+  const float* rv;
+  uint32_t nverts;
+  float* ptv;
+  const int32_t* idx;
+  uint32_t nprims;
+  int per;             // indices per primitive
+  uint32_t* base;      // per SWR_BATCH_PRIMS primitives: kept ones before them
+  uint32_t* done;      // zero between draws
+  uint32_t* status;
+  uint32_t cap_prims;
+};
+
 template <int A, int P>
-__global__ void k_direct_vertices(const float* __restrict__ rv, uint32_t nverts, float* __restrict__ ptv) {
+__global__ void __launch_bounds__(256) k_direct_vertices(DirectArgs g) {
   swr_pdl_entry();
+  __shared__ uint32_t tmp[32];
   typedef VLayout<A, P> L;
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nverts; v += gridDim.x * blockDim.x) {
-    const float* s = rv + (size_t)v * 36;
-    float* o = ptv + (size_t)v * L::S;
+  const uint32_t nb = (g.nprims + SWR_BATCH_PRIMS - 1) / SWR_BATCH_PRIMS;
+  for (uint32_t b = blockIdx.x; b < nb; b += gridDim.x) {
+    uint32_t c = 0, tot;
+    for (uint32_t p = b * SWR_BATCH_PRIMS + threadIdx.x; p < min(g.nprims, (b + 1) * SWR_BATCH_PRIMS); p += 256)
+      c += g.idx[(size_t)g.per * p] != -1;
+    swr_block_exscan(c, tmp, &tot);
+    if (threadIdx.x == 0) g.base[b] = tot;
+  }
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < g.nverts; v += gridDim.x * blockDim.x) {
+    const float* s = g.rv + (size_t)v * 36;
+    float* o = g.ptv + (size_t)v * L::S;
     o[0] = s[0]; o[1] = s[1]; o[2] = s[2]; o[3] = s[3];
     o[4] = s[0]; o[5] = s[1]; o[6] = s[2]; o[7] = __int_as_float(0);
     for (int i = 0; i < A; ++i) o[L::OFF_A + i] = s[4 + i];
     for (int i = 0; i < P; ++i) o[L::OFF_P + i] = s[20 + i];
+  }
+  uint32_t total;
+  if (swr_last_block_scan(g.base, nb, g.done, &total) && threadIdx.x == 0) {
+    g.status[SWR_ST_PRIMS] = total;
+    if (total > g.cap_prims) atomicOr(&g.status[SWR_ST_FLAGS], SWR_F_PRIM_OVERFLOW);
+  }
+}
+
+// One block per SWR_BATCH_PRIMS primitives, four consecutive ones per thread.
+static __global__ void __launch_bounds__(256) k_direct_emit(DirectArgs g, uint4* __restrict__ tris) {
+  swr_pdl_entry();
+  __shared__ uint32_t tmp[32];
+  if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
+  const uint32_t p0 = blockIdx.x * SWR_BATCH_PRIMS + threadIdx.x * 4;
+  int32_t first[4];
+  uint32_t c = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    first[k] = p0 + k < g.nprims ? g.idx[(size_t)g.per * (p0 + k)] : -1;
+    c += first[k] != -1;
+  }
+  uint32_t at = g.base[blockIdx.x] + swr_block_exscan(c, tmp, nullptr);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (first[k] == -1) continue;
+    uint32_t r[3] = {0, 0, 0};
+    for (int j = 0; j < g.per; ++j) {
+      const int32_t i = j ? g.idx[(size_t)g.per * (p0 + k) + j] : first[k];
+      if (i < 0 || (uint32_t)i >= g.nverts)
+        atomicOr(&g.status[SWR_ST_FLAGS], SWR_F_BAD_INDEX);
+      else
+        r[j] = (uint32_t)i;
+    }
+    tris[at++] = make_uint4(r[0], r[1], r[2], 0u);
   }
 }
 
@@ -197,9 +257,10 @@ struct AssembleArgs {
   uint32_t* clip_slot;      // per submitted primitive (valid when clipped)
   uint8_t* tri_flags;       // per submitted primitive: bit0 keep, bit1 swap, bit2 clipped
   uint2* batch_counts;      // per batch: (kept input slots, kept extra fan triangles)
-  const uint32_t* batch_base;
+  uint32_t* batch_base;     // points, lines: per batch, survivors before it
   uint4* tris;              // output primitives: v0, v1, v2 references + draw id
   uint2* lp_refs;           // per submitted point / line: endpoint references after clipping
+  uint32_t* done;           // points, lines: blocks finished (zero between draws)
   uint32_t* draw_prim_base; // per draw: index of its first emitted primitive (optional)
   uint32_t* status;
   uint32_t cap_clip_slots, cap_clip_verts, cap_prims;
@@ -338,26 +399,6 @@ template <int A, int P>
 __global__ void __launch_bounds__(SWR_HALF) k_assemble_count(AssembleArgs g) {
   swr_pdl_entry();
   assemble_count_block<A, P, false>(g, blockIdx.x);
-}
-
-// Exclusive scan of per-batch totals -> batch bases; primitive total into the status word.
-static __global__ void __launch_bounds__(1024) k_batch_scan(const uint2* counts, uint32_t nbatches, uint32_t* base,
-                                                     uint32_t* status, uint32_t cap_prims) {
-  swr_pdl_entry();
-  __shared__ uint32_t tmp[32];
-  uint32_t run = 0;
-  for (uint32_t b0 = 0; b0 < nbatches; b0 += 1024) {
-    const uint32_t b = b0 + threadIdx.x;
-    const uint32_t v = b < nbatches ? counts[b].x + counts[b].y : 0u;
-    uint32_t tot;
-    const uint32_t ex = swr_block_exscan(v, tmp, &tot);
-    if (b < nbatches) base[b] = run + ex;
-    run += tot;
-  }
-  if (threadIdx.x == 0) {
-    status[SWR_ST_PRIMS] = run;
-    if (run > cap_prims) atomicOr(&status[SWR_ST_FLAGS], SWR_F_PRIM_OVERFLOW);
-  }
 }
 
 // Writes the surviving triangles of one batch at their effective-order positions.  The
@@ -551,35 +592,6 @@ __global__ void __launch_bounds__(SWR_HALF) k_front(const __grid_constant__ Fron
   for (uint32_t hb = 0; hb < a.nhb; ++hb) {
     assemble_emit_block<VS::AVarCount, VS::PVarCount>(g, hb, a.nhb);
     __syncthreads();
-  }
-}
-
-// Direct Rasterizer path: triangles whose first index is -1 are skipped
-// (Rasterizer::drawTriangleList, Rasterizer.h:134-141); others keep their order.
-static __global__ void k_direct_flags(const int32_t* __restrict__ idx, uint32_t nprims, int per,
-                               uint32_t* __restrict__ keep) {
-  swr_pdl_entry();
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < nprims; p += gridDim.x * blockDim.x)
-    keep[p] = idx[(size_t)per * p] != -1 ? 1u : 0u;
-}
-
-static __global__ void k_direct_emit(const int32_t* __restrict__ idx, uint32_t nprims, int per, uint32_t nverts,
-                              const uint32_t* __restrict__ keep, const uint32_t* __restrict__ pos,
-                              uint4* __restrict__ tris, uint32_t* status) {
-  swr_pdl_entry();
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < nprims; p += gridDim.x * blockDim.x) {
-    if (!keep[p]) continue;
-    uint32_t r[3] = {0, 0, 0};
-    for (int k = 0; k < per; ++k) {
-      const int32_t i = idx[(size_t)per * p + k];
-      if (i < 0 || (uint32_t)i >= nverts) {
-        atomicOr(&status[SWR_ST_FLAGS], SWR_F_BAD_INDEX);
-        r[k] = 0;
-      } else {
-        r[k] = (uint32_t)i;
-      }
-    }
-    tris[pos[p]] = make_uint4(r[0], r[1], r[2], 0u);
   }
 }
 
@@ -1519,14 +1531,15 @@ __device__ __forceinline__ void pixel_of_record(const float* r, const SwrDrawDes
 // A heavy tile of a depth-min shader (RasterArgs.dslice) is run by up to SWR_DSLICES CTAs,
 // each over its own run of whole chunks from the draw's starting State; the last run to
 // finish merges the runs' States in bin order (swr_depth_merge) and stores.
-template <class PS, int TILE, int CH, bool SPAN, bool DIRECT = false>
-__global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
+template <class PS, int TILE, int CH, bool SPAN, bool DIRECT = false, int NT = 256>
+__global__ void __launch_bounds__(NT, SWR_RASTER_MINB ? SWR_RASTER_MINB
                                        : SPAN            ? SwrRasterOccupancy<PS>::value
-                                                         : SwrRasterOccupancy<PS>::block)
+                                                         : SwrRasterOccupancy<PS>::block * (256 / NT))
     k_raster(RasterArgs g) {
   swr_pdl_entry();
   typedef Rec<PS> RL;
-  constexpr int PPT = TILE * TILE / 256;  // pixels per thread
+  constexpr int PPT = TILE * TILE / NT;  // pixels per thread
+  constexpr int NWARP = NT / 32;
   constexpr int NBX = TILE / SWR_BLOCK;   // blocks per tile row
   constexpr int NB = NBX * NBX;
   constexpr bool kCull = SWR_DEPTH_CULL && SwrDepthCull<PS>::value;
@@ -1545,28 +1558,29 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
   __shared__ uint64_t smask[CH * NB];
   __shared__ int2 sspan[SPAN ? CH * TILE : 1];  // Span mode: each tile row's [xl, xr)
   __shared__ uint32_t sids[CH];
-  __shared__ uint32_t sfr[32];
+  __shared__ uint32_t sfr[64];
   __shared__ uint32_t slast;  // sliced heavy tile: this run is the last to finish
   __shared__ uint16_t spart[CH * NB];  // partially covered (primitive, block) pairs
   __shared__ uint32_t snpart;
   __shared__ uint32_t ssorted[SWR_RASTER_SORT];  // the tile's ordered bin (self-sorted tiles)
   __shared__ uint32_t scs[SWR_SEGS + 1];          // its cell starts relative to the bin start
   static_assert(sizeof(srec4) >= SWR_RASTER_SORT * 4, "raw bin staging fits the record area");
-  // Depth cull regions: the 8 x 4 pixels of one warp in one sub-tile (region q * 8 + warp).
-  constexpr int NREG = 8 * PPT;
+  // Regions of 8 x 4 pixels (half blocks), eight to a 16 x 16 sub-tile: a warp's q-th is region
+  // q * NWARP + warp.
+  constexpr int NREG = TILE * TILE / 32;
   __shared__ uint32_t swd[NREG];  // per region: order key of the largest depth it holds
   // Depth cull: the next primitives to rasterize, in order (up to CH - 1 left over plus a batch
-  // of 256), and per pixel row the coverage of primitives that were only counted (+1 at a run's
+  // of NT), and per pixel row the coverage of primitives that were only counted (+1 at a run's
   // first pixel, -1 past its last; used where the target records counts)
-  __shared__ uint32_t ssurv[kCull ? CH + 256 : 1];
+  __shared__ uint32_t ssurv[kCull ? CH + NT : 1];
   // a batch's primitives to count: Span ones from the front, Block ones from the back; their
   // partially covered blocks (entry * NB + block)
-  __shared__ uint32_t scul[kCull ? 256 : 1];
+  __shared__ uint32_t scul[kCull ? NT : 1];
   constexpr int SCP = 1024;
   __shared__ uint16_t scp[kCull ? SCP : 1];
   __shared__ int scnt[kCull ? TILE * (TILE + 1) : 1];
   constexpr int NW = CH / 32;      // 32-primitive words of a chunk
-  static_assert(CH % 32 == 0 && CH <= 128, "chunks of 32, 64, 96 or 128 primitives");
+  static_assert(CH % 32 == 0 && CH <= 128 && CH <= NT, "chunks of 32, 64, 96 or 128 primitives");
   __shared__ uint32_t sculr[kCull ? NREG * NW : 1];  // per region: primitives only counted there
   __shared__ int sminx[kCull && SPAN ? CH : 1];  // Span mode: leftmost start of a span reaching the tile
   constexpr int HW = (CH + 63) / 64;  // 64-primitive words of a chunk
@@ -1619,13 +1633,13 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
   } else {
     if (tile >= g.ntiles) return;
   }
-  // Small draws: the tile's primitives out of the next windows of 256 boxes, in order, until
-  // more than 256 are found (e = their count; ssorted holds SWR_RASTER_SORT) or none is left.
+  // Small draws: the tile's primitives out of the next windows of NT boxes, in order, until
+  // ssorted (SWR_RASTER_SORT) may not hold another window's, or none is left (e: their count).
   uint32_t scan_pos = 0, scan_np = 0;
   auto gather = [&]() {
     const uint32_t tx = tile % (uint32_t)g.targets[0].tiles_x, ty = tile / (uint32_t)g.targets[0].tiles_x;
     e = 0;
-    while (scan_pos < scan_np && e <= SWR_RASTER_SORT - 256) {
+    while (scan_pos < scan_np && e <= SWR_RASTER_SORT - NT) {
       const uint32_t i = scan_pos + threadIdx.x;
       const bool hit = i < scan_np && swr_box_hit(g.boxes[i], tx, ty);
       const uint32_t bal = __ballot_sync(0xffffffffu, hit);
@@ -1634,14 +1648,14 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
       __syncthreads();
       uint32_t at = e, all = 0;
 #pragma unroll
-      for (int w = 0; w < 8; ++w) {
+      for (int w = 0; w < NWARP; ++w) {
         const uint32_t c = scs[w];
         if (w < warp) at += c;
         all += c;
       }
       if (hit) ssorted[at + (uint32_t)__popc(bal & ((1u << lane) - 1u))] = i;
       e += all;
-      scan_pos += 256;
+      scan_pos += NT;
     }
   };
   if constexpr (DIRECT) {
@@ -1663,16 +1677,15 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
   const SwrUniforms& U = g.draws[T.first_draw].u;
   const uint32_t lt = tile - T.tile_base;
   const int ox = (int)(lt % (uint32_t)T.tiles_x) * TILE, oy = (int)(lt / (uint32_t)T.tiles_x) * TILE;
-  // Thread -> pixels: each warp covers an 8 x 4 half block; 16 x 16 sub-tiles repeat.
+  // Thread -> pixels: each warp covers 8 x 4 half blocks.
   int px[PPT], py[PPT], blk[PPT];
   bool in[PPT];
   typename PS::State st[PPT];
 #pragma unroll
   for (int q = 0; q < PPT; ++q) {
-    const int sxo = (q % (TILE / 16)) * 16, syo = (q / (TILE / 16)) * 16;
-    const int hb = warp >> 1;
-    const int lx = sxo + (hb & 1) * 8 + (lane & 7);
-    const int ly = syo + (hb >> 1) * 8 + (warp & 1) * 4 + (lane >> 3);
+    const int reg = q * NWARP + warp, sub = reg >> 3, hb = (reg & 7) >> 1;
+    const int lx = (sub % (TILE / 16)) * 16 + (hb & 1) * 8 + (lane & 7);
+    const int ly = (sub / (TILE / 16)) * 16 + (hb >> 1) * 8 + (reg & 1) * 4 + (lane >> 3);
     px[q] = ox + lx;
     py[q] = oy + ly;
     blk[q] = (ly >> 3) * NBX + (lx >> 3);
@@ -1688,9 +1701,9 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
     const uint32_t ntot = e - b;
     if (threadIdx.x <= SWR_SEGS)
       scs[threadIdx.x] = (threadIdx.x < SWR_SEGS ? g.tiles.start[(size_t)tile * SWR_SEGS + threadIdx.x] : e) - b;
-    for (uint32_t j = threadIdx.x; j < ntot; j += 256) sraw[j] = g.bin_raw[b + j];
+    for (uint32_t j = threadIdx.x; j < ntot; j += NT) sraw[j] = g.bin_raw[b + j];
     __syncthreads();
-    for (uint32_t j = threadIdx.x; j < ntot; j += 256) {
+    for (uint32_t j = threadIdx.x; j < ntot; j += NT) {
       int lo = 0, hi = SWR_SEGS - 1;  // the cell holding j: last c with scs[c] <= j
       while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
@@ -1766,7 +1779,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
   // block, then a thread per partially covered block.
   auto count_listed = [&](int ns, int nb) {
     if constexpr (SPAN) {
-      for (int i = threadIdx.x; i < ns; i += 256) {
+      for (int i = threadIdx.x; i < ns; i += NT) {
         const float4* rc = (const float4*)(g.recs + (size_t)scul[i] * RL::R);
         const float4 q0 = __ldg(rc);
         const SwrDrawDesc& D = g.draws[__float_as_int(q0.y)];
@@ -1777,7 +1790,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
     auto count_block = [&](int i, bool classify) -> int {
       const int j = i % NB;
       const int bx = ox + (j % NBX) * SWR_BLOCK, by = oy + (j / NBX) * SWR_BLOCK;
-      const float4* rc = (const float4*)(g.recs + (size_t)scul[255 - i / NB] * RL::R);
+      const float4* rc = (const float4*)(g.recs + (size_t)scul[NT - 1 - i / NB] * RL::R);
       const float4 q0 = __ldg(rc), q1 = __ldg(rc + 1), q2 = __ldg(rc + 2), q3 = __ldg(rc + 3);
       const float r[15] = {0, 0, 0, 0, 0, 0, q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, q3.x, q3.y, q3.z};
       int cls = 2;
@@ -1791,17 +1804,17 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
       block_runs(r, __float_as_int(q0.x), cls, bx, by, min(SWR_BLOCK, rx1 - bx), by, min(by + SWR_BLOCK, ry1), add_run);
       return 1;
     };
-    for (int i = threadIdx.x; i < nb * NB; i += 256)
+    for (int i = threadIdx.x; i < nb * NB; i += NT)
       if (count_block(i, true) == 2) {
         const uint32_t at = atomicAdd(&snpart, 1u);
         if (at < SCP) scp[at] = (uint16_t)i; else count_block(i, false);
       }
     __syncthreads();
     const int m = min((int)snpart, SCP);
-    for (int t = threadIdx.x; t < m; t += 256) count_block(scp[t], false);
+    for (int t = threadIdx.x; t < m; t += NT) count_block(scp[t], false);
   };
   if (kCull && counts)
-    for (int i = threadIdx.x; i < TILE * (TILE + 1); i += 256) scnt[i] = 0;  // (first used past the next barrier)
+    for (int i = threadIdx.x; i < TILE * (TILE + 1); i += NT) scnt[i] = 0;  // (first used past the next barrier)
   while (true) {  // once; small draws: per gathered run of the tile's primitives
   uint32_t c0 = cb;        // next bin entry
   uint32_t nsurv = 0;      // depth cull: primitives waiting in ssurv
@@ -1821,7 +1834,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
           const uint32_t u = __float_as_uint(dq);
           const uint32_t kq = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
           const uint32_t key = __reduce_max_sync(0xffffffffu, in[q] && !swr_isnan(dq) ? kq : 0u);
-          if (lane == 0) swd[q * 8 + warp] = key;
+          if (lane == 0) swd[q * NWARP + warp] = key;
           my_ok |= key != 0u && key < 0xff800000u;  // uniform per warp
         }
         cull_on = __syncthreads_or(my_ok);
@@ -1836,7 +1849,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
           c0 += take;
           continue;
         }
-        const uint32_t take = min(256u, ce - c0);
+        const uint32_t take = min((uint32_t)NT, ce - c0);
         uint32_t p = 0;
         int v = 3;
         if (threadIdx.x < take) {
@@ -1853,7 +1866,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
         uint32_t at_k = nsurv;
         int ns = 0, nb = 0, at_s = 0, at_b = 0;
 #pragma unroll
-        for (int w = 0; w < 8; ++w) {
+        for (int w = 0; w < NWARP; ++w) {
           const uint32_t c = scs[w];
           if (w < warp) {
             at_k += c & 255u;
@@ -1866,7 +1879,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
         }
         if (v == 0) ssurv[at_k + (uint32_t)__popc(bk & lt_mask)] = p;
         if (v == 1) scul[at_s + __popc(bs & lt_mask)] = p;
-        if (v == 2) scul[255 - at_b - __popc(bb & lt_mask)] = p;
+        if (v == 2) scul[NT - 1 - at_b - __popc(bb & lt_mask)] = p;
         __syncthreads();
         count_listed(ns, nb);
         c0 += take;
@@ -1886,7 +1899,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
     {
       const float4* recs4 = (const float4*)g.recs;
 #pragma unroll 4
-      for (int i = threadIdx.x; i < n * RW4; i += 256) {
+      for (int i = threadIdx.x; i < n * RW4; i += NT) {
         const int k = i / RW4, w = i - k * RW4;
         const uint32_t id = kCull ? ssurv[k] : bin_id(c0 + k);
         srec4[k * SR4 + w] = recs4[(size_t)id * (RL::R / 4) + w];
@@ -1901,7 +1914,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
     }
     // B1: coverage per (primitive, block).  Fully covered / skipped blocks and Span rows are
     // finished here; partially covered Block-mode blocks are queued for B2.
-    for (int i = threadIdx.x; i < n * NB; i += 256) {
+    for (int i = threadIdx.x; i < n * NB; i += NT) {
       const int k = i / NB, j = i - k * NB;
       const float* r = srec + k * SR;
       const int flags = __float_as_int(r[0]);
@@ -1925,7 +1938,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
       // B1 (Span mode): four rows of a primitive per thread: each row's span [xl, xr), kept as the
       // row's interpolation start, and its half of the masks of the blocks it crosses
       constexpr int NR = TILE / 4;
-      for (int i = threadIdx.x; i < n * NR; i += 256) {
+      for (int i = threadIdx.x; i < n * NR; i += NT) {
         const int k = i / NR, br = i - k * NR;
         const float* r = srec + k * SR;
         const int flags = __float_as_int(r[0]);
@@ -1979,7 +1992,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
     // B2: partially covered blocks, four rows per lane: one half of the block's mask
     {
       const int np2 = (int)snpart * 2;
-      for (int t = threadIdx.x; t < np2; t += 256) {
+      for (int t = threadIdx.x; t < np2; t += NT) {
         const int i = spart[t >> 1];
         const int k = i / NB, j = i - k * NB;
         const float* r = srec + k * SR;
@@ -1993,7 +2006,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
     // the covered pixels' box in the region).  Depths only decrease, so such fragments fail
     // their depth tests: the primitive is only counted there.
     if (kCull && cull_on) {
-      for (int t = threadIdx.x; t < NREG * CH; t += 256) {
+      for (int t = threadIdx.x; t < NREG * CH; t += NT) {
         const int reg = t / CH, k = t - reg * CH;  // reg uniform per warp (CH is a multiple of 32)
         bool culled = false;
         if (k < n && (__float_as_int(srec[k * SR]) & 1)) {
@@ -2056,7 +2069,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
       }
       if (kCull && cull_on) {
         // primitives culled in this warp's region fail the depth test: counted only
-        const uint32_t* cr = sculr + (q * 8 + warp) * NW;
+        const uint32_t* cr = sculr + (q * NWARP + warp) * NW;
 #pragma unroll
         for (int w = 0; w < HW; ++w)
           mine[w] &= ~((uint64_t)cr[2 * w] | (2 * w + 1 < NW ? (uint64_t)cr[2 * w + 1] << 32 : 0ull));
@@ -2174,8 +2187,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
         if (threadIdx.x == 0) g.dslice_done[dslot] = 0u;  // ready for the next draw
       }
       uint32_t tot, ptot;
-      swr_block_exscan(frags, sfr, &tot);
-      swr_block_exscan(passes, sfr, &ptot);
+      swr_block_sum2(frags, passes, sfr, tot, ptot);
       if (threadIdx.x == 0 && tot) {
         atomicAdd((unsigned long long*)&g.status_w[SWR_ST_SHADED_LO], (unsigned long long)tot);
         atomicAdd((unsigned long long*)&g.status_w[SWR_ST_PASSES_LO], (unsigned long long)ptot);
@@ -2191,8 +2203,7 @@ __global__ void __launch_bounds__(256, SWR_RASTER_MINB ? SWR_RASTER_MINB
     }
   // fragment statistics: drawPixel calls and colour writes
   uint32_t tot, ptot;
-  swr_block_exscan(frags, sfr, &tot);
-  swr_block_exscan(passes, sfr, &ptot);
+  swr_block_sum2(frags, passes, sfr, tot, ptot);
   if (threadIdx.x == 0 && tot) {
     atomicAdd((unsigned long long*)&g.status_w[SWR_ST_SHADED_LO], (unsigned long long)tot);
     atomicAdd((unsigned long long*)&g.status_w[SWR_ST_PASSES_LO], (unsigned long long)ptot);
