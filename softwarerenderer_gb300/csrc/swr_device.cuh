@@ -238,29 +238,47 @@ __device__ __forceinline__ uint32_t swr_block_exscan(uint32_t v, uint32_t* tmp, 
   return warp_off + x - v;
 }
 
-// End of a counting kernel: the last block to finish turns the blocks' counts into exclusive
-// bases (in place) and returns true in every thread, with their sum; the others return false.
+// End of a counting kernel: the last block to finish turns n counts, count(i), into exclusive
+// bases and returns true in every thread, with their sum; the others return false.
 // Each thread of it takes a contiguous run of counts, so the tail is two short passes.  `done`
-// is zero before the kernel and after it.  Every block calls this once, whatever it counted.
-__device__ __forceinline__ bool swr_last_block_scan(uint32_t* counts, uint32_t n, uint32_t* done, uint32_t* total) {
+// is zero before the kernel and after it.  Every block calls this once, whatever it counted;
+// its counts were written by its thread 0.
+// bases may be where the counts are: each is read by the thread that overwrites it.
+template <class F>
+__device__ __forceinline__ bool swr_last_block_scan(F count, uint32_t* bases, uint32_t n, uint32_t* done,
+                                                    uint32_t* total) {
   __shared__ uint32_t tmp[32];
   __shared__ uint32_t last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(done, 1u) == gridDim.x - 1;
+  }
   __syncthreads();
   if (!last) return false;
   __threadfence();
   const uint32_t per = (n + blockDim.x - 1) / blockDim.x;
   const uint32_t b = min(n, threadIdx.x * per), e = min(n, b + per);
+  constexpr int U = 8;  // counts in flight per thread
   uint32_t s = 0;
-  for (uint32_t i = b; i < e; ++i) s += __ldcg(counts + i);
+  for (uint32_t i = b; i < e; i += U) {
+#pragma unroll
+    for (int k = 0; k < U; ++k) s += i + k < e ? count(i + k) : 0u;
+  }
   uint32_t run = swr_block_exscan(s, tmp, total);
-  for (uint32_t i = b; i < e; ++i) {
-    const uint32_t c = __ldcg(counts + i);
-    counts[i] = run;
-    run += c;
+  for (uint32_t i = b; i < e; i += U) {
+    uint32_t c[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) c[k] = i + k < e ? count(i + k) : 0u;
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      if (i + k < e) bases[i + k] = run;
+      run += c[k];
+    }
   }
   if (threadIdx.x == 0) *done = 0u;
   return true;
+}
+
+__device__ __forceinline__ bool swr_last_block_scan(uint32_t* counts, uint32_t n, uint32_t* done, uint32_t* total) {
+  return swr_last_block_scan([&](uint32_t i) { return __ldcg(counts + i); }, counts, n, done, total);
 }
