@@ -68,7 +68,11 @@ void run_raster(const RasterArgs& a, uint32_t ntiles, int tile, cudaStream_t s) 
       else swr::launch(k_raster<PS, 32, kChunk, false>, grid, 256, 0, s, a);
     } else {
       constexpr int kBlockThreads = SwrRasterThreadsBlock<PS>::value;
-      if (a.has_span) swr::launch(k_raster<PS, 16, kChunk, true>, grid, 256, 0, s, a);
+      if (grid == ntiles && ntiles > SWR_RASTER_LOOP) {
+        const uint32_t half = (ntiles + 1) / 2;
+        if (a.has_span) swr::launch(k_raster_two<PS, kChunk, true, 256>, half, 256, 0, s, a);
+        else swr::launch(k_raster_two<PS, kChunk, false, kBlockThreads>, half, kBlockThreads, 0, s, a);
+      } else if (a.has_span) swr::launch(k_raster<PS, 16, kChunk, true>, grid, 256, 0, s, a);
       else swr::launch(k_raster<PS, 16, kChunk, false, false, kBlockThreads>, grid, kBlockThreads, 0, s, a);
     }
   }

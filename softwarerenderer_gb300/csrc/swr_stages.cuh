@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(SWR_HALF) k_assemble_count(AssembleArgs g) {
 // every emitting block sums the counts before it: those sums grow with the square of the
 // batches, the scan costs every counting block an atomic and the launch a serial tail.  256
 // meshes, 6,810 batches: emit 115 us summed, 71 scanned, for 30 us more in the counting launch
-// (2861 -> 2838 us in all); 1,024 batches of a soup take the same time either way, and 48
+// (2861 -> 2838 us in all); 1,024 batches of a soup take the same time either way, and 320
 // batches of one mesh are slower scanned (95.7 -> 97.6 us in all).
 #ifndef SWR_SCAN_BATCHES
 #define SWR_SCAN_BATCHES 2048
@@ -1576,12 +1576,11 @@ __device__ __forceinline__ void pixel_of_record(const float* r, const SwrDrawDes
 // A heavy tile of a depth-min shader (RasterArgs.dslice) is run by up to SWR_DSLICES CTAs,
 // each over its own run of whole chunks from the draw's starting State; the last run to
 // finish merges the runs' States in bin order (swr_depth_merge) and stores.
-template <class PS, int TILE, int CH, bool SPAN, bool DIRECT = false, int NT = 256>
-__global__ void __launch_bounds__(NT, SWR_RASTER_MINB ? SWR_RASTER_MINB
-                                       : SPAN            ? SwrRasterOccupancy<PS>::value
-                                                         : SwrRasterOccupancy<PS>::block * (256 / NT))
-    k_raster(RasterArgs g) {
-  swr_pdl_entry();
+//
+// raster_tile: the work of CTA `bid` of a launch that gives every tile its own; false when it
+// has none.
+template <class PS, int TILE, int CH, bool SPAN, bool DIRECT, int NT>
+__device__ __forceinline__ bool raster_tile(const RasterArgs& g, uint32_t bid) {
   typedef Rec<PS> RL;
   constexpr int PPT = TILE * TILE / NT;  // pixels per thread
   constexpr int NWARP = NT / 32;
@@ -1630,13 +1629,13 @@ __global__ void __launch_bounds__(NT, SWR_RASTER_MINB ? SWR_RASTER_MINB
   __shared__ int sminx[kCull && SPAN ? CH : 1];  // Span mode: leftmost start of a span reaching the tile
   constexpr int HW = (CH + 63) / 64;  // 64-primitive words of a chunk
   // the draw's queue requests are final (nothing after this stage counts)
-  if (!DIRECT && blockIdx.x == 0 && threadIdx.x == 0) swr_close_status(g.status_w);
-  if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
+  if (!DIRECT && bid == 0 && threadIdx.x == 0) swr_close_status(g.status_w);
+  if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return false;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint32_t frags = 0, passes = 0;
   // One CTA per tile (a persistent grid pulling tiles from a counter measured no faster on
   // the dense mesh and slower where few tiles carry the work: they gather on fewer SMs).
-  uint32_t tile = blockIdx.x, slice = 0;
+  uint32_t tile = bid, slice = 0;
   int quad = -1;  // the 8 x 8 quadrant (block) this CTA rasterizes alone, -1: the whole tile
   int dslot = -1;  // sliced heavy tile: its list slot (slice = its run)
   uint32_t b = 0, e = 0;
@@ -1648,35 +1647,35 @@ __global__ void __launch_bounds__(NT, SWR_RASTER_MINB ? SWR_RASTER_MINB
       static_assert(kRuns == 4 && SWR_DSLICES == 4, "four CTAs per heavy tile, as runs or as quadrants");
       const bool heavy = (SwrDepthMin<PS>::value && g.dslice) || (TILE == 16 && g.quad);
       const uint32_t nq = heavy ? 4u * g.tiles.heavy_cap : 0u;
-      if (blockIdx.x < nq) {
-        const uint32_t slot = blockIdx.x >> 2;
-        if (slot >= min(g.tiles.counts[0], g.tiles.heavy_cap)) return;
+      if (bid < nq) {
+        const uint32_t slot = bid >> 2;
+        if (slot >= min(g.tiles.counts[0], g.tiles.heavy_cap)) return false;
         entry = __ldg(g.tiles.heavy + slot);
         if (SwrDepthMin<PS>::value && g.dslice) {
-          slice = blockIdx.x & 3u;
+          slice = bid & 3u;
           dslot = (int)slot;
         } else {
-          quad = (int)(blockIdx.x & 3u);
+          quad = (int)(bid & 3u);
         }
       } else {
-        uint32_t i = blockIdx.x - nq;
+        uint32_t i = bid - nq;
         if (TILE == 16 && g.quad_all) {
           quad = (int)(i & 3u);
           i >>= 2;
         }
-        if (!swr_listed_tile(g.tiles, i, entry)) return;
+        if (!swr_listed_tile(g.tiles, i, entry)) return false;
       }
       tile = entry.x;
       b = entry.y;
       e = entry.z;
       ti = (int)entry.w;
     } else {
-      if (tile >= g.ntiles) return;
+      if (tile >= g.ntiles) return false;
       b = g.tile_start[tile];
       e = g.tile_start[tile + 1];
     }
   } else {
-    if (tile >= g.ntiles) return;
+    if (tile >= g.ntiles) return false;
   }
   // Small draws: the tile's primitives out of the next windows of NT boxes, in order, until
   // ssorted (SWR_RASTER_SORT) may not hold another window's, or none is left (e: their count).
@@ -1707,14 +1706,14 @@ __global__ void __launch_bounds__(NT, SWR_RASTER_MINB ? SWR_RASTER_MINB
     scan_np = min(g.status[SWR_ST_PRIMS], g.cap_prims);
     gather();
   }
-  if (b == e) return;  // uniform per CTA
+  if (b == e) return true;  // uniform per CTA
   // the chunks this CTA rasterizes: the whole bin, or a sliced heavy tile's run
   uint32_t cb = b, ce = e;
   int nsl = 1;
   if (dslot >= 0) {
     const uint32_t nch = (e - b + CH - 1) / CH;
     nsl = (int)min(nch, (uint32_t)SWR_DSLICES);
-    if ((int)slice >= nsl) return;  // (uniform per tile: these CTAs take no part)
+    if ((int)slice >= nsl) return false;  // (uniform per tile: these CTAs take no part)
     cb = b + (uint32_t)((uint64_t)nch * slice / (uint32_t)nsl) * CH;
     ce = min(e, b + (uint32_t)((uint64_t)nch * (slice + 1) / (uint32_t)nsl) * CH);
   }
@@ -2237,7 +2236,7 @@ __global__ void __launch_bounds__(NT, SWR_RASTER_MINB ? SWR_RASTER_MINB
         atomicAdd((unsigned long long*)&g.status_w[SWR_ST_SHADED_LO], (unsigned long long)tot);
         atomicAdd((unsigned long long*)&g.status_w[SWR_ST_PASSES_LO], (unsigned long long)ptot);
       }
-      return;
+      return true;
     }
   }
 #pragma unroll
@@ -2253,6 +2252,35 @@ __global__ void __launch_bounds__(NT, SWR_RASTER_MINB ? SWR_RASTER_MINB
     atomicAdd((unsigned long long*)&g.status_w[SWR_ST_SHADED_LO], (unsigned long long)tot);
     atomicAdd((unsigned long long*)&g.status_w[SWR_ST_PASSES_LO], (unsigned long long)ptot);
   }
+  return true;
+}
+
+template <class PS, int TILE, int CH, bool SPAN, bool DIRECT = false, int NT = 256>
+__global__ void __launch_bounds__(NT, SWR_RASTER_MINB ? SWR_RASTER_MINB
+                                       : SPAN            ? SwrRasterOccupancy<PS>::value
+                                                         : SwrRasterOccupancy<PS>::block * (256 / NT))
+    k_raster(RasterArgs g) {
+  swr_pdl_entry();
+  raster_tile<PS, TILE, CH, SPAN, DIRECT, NT>(g, blockIdx.x);
+}
+
+// Draws of more than SWR_RASTER_LOOP tiles: a CTA for every two, which rasterizes its entry of
+// the list and the one a grid further on.  Meshes leave most of a batch's tiles empty, and a CTA
+// that finds none costs 1 ns of launching: 256 meshes of 491,520 tiles took 2741 us, this way
+// 2540 (one for every four tiles or eight: 1 % slower).  Where no tile is empty the second
+// tile's state costs registers (32,400 tiles of a soup 4134 -> 4185 us), so one target's tiles
+// keep k_raster.
+#ifndef SWR_RASTER_LOOP
+#define SWR_RASTER_LOOP 65536
+#endif
+template <class PS, int CH, bool SPAN, int NT>
+__global__ void __launch_bounds__(NT, SWR_RASTER_MINB ? SWR_RASTER_MINB
+                                       : SPAN            ? SwrRasterOccupancy<PS>::value
+                                                         : SwrRasterOccupancy<PS>::block * (256 / NT))
+    k_raster_two(RasterArgs g) {
+  swr_pdl_entry();
+  for (uint32_t bid = blockIdx.x; bid < g.ntiles && raster_tile<PS, 16, CH, SPAN, false, NT>(g, bid); bid += gridDim.x)
+    __syncthreads();  // the tile's shared state is no longer read
 }
 
 // ---------------------------------------------------------------------------------
