@@ -2311,6 +2311,8 @@ __global__ void __launch_bounds__(256) k_overwrite(RasterArgs g) {
   __shared__ uint32_t sred[8];
   __shared__ uint32_t sfr[32];
   __shared__ uint32_t slast;
+  constexpr uint32_t OVB = 1024;  // entries classified at a time
+  __shared__ uint32_t swalk[DIRECT ? 1 : OVB], snwalk;
   // the draw's queue requests are final (nothing after this stage counts)
   if (blockIdx.x == 0 && threadIdx.x == 0 && !DIRECT) swr_close_status(g.status_w);
   if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
@@ -2396,12 +2398,105 @@ __global__ void __launch_bounds__(256) k_overwrite(RasterArgs g) {
         if (cls) block_runs(r, flags, cls, bx, by, min(SWR_BLOCK, xend - bx), ylo, min(by + SWR_BLOCK, yhi), run);
       }
   };
+  int round = 0;
+  auto raise_smin = [&]() {  // (uniform)
+    __syncthreads();
+    uint32_t m = 0xffffffffu;
+#pragma unroll
+    for (int q = 0; q < PPT; ++q) {
+      const int i = q * 256 + tid;
+      if (ox + i % TILE < xend && oy + i / TILE < yend) m = min(m, sbest[i]);
+    }
+    m = __reduce_min_sync(0xffffffffu, m);
+    if (lane == 0) sred[warp] = m;
+    __syncthreads();
+    smin = sred[0];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) smin = min(smin, sred[w]);
+  };
+  // Whether primitive p has to be walked row by row.  A Span primitive whose halves each miss
+  // the tile's columns or cover all of theirs, in all the rows they have here, only adds its
+  // fragments: an extent's ends are monotone functions of the row within a half (every
+  // operation of span_row is, for finite slopes), so the end rows tell.
+  auto classify = [&](uint32_t p) -> bool {
+    const float4* rc = (const float4*)(g.recs + (size_t)p * RL::R);
+    const float4 q0 = __ldg(rc), q1 = __ldg(rc + 1), q2 = __ldg(rc + 2), q3 = __ldg(rc + 3), q4 = __ldg(rc + 4);
+    const int flags = __float_as_int(q0.x);
+    if (!(flags & 1)) return false;
+    if (flags & 2) return true;
+    const SwrDrawDesc& D = g.draws[__float_as_int(q0.y)];
+    const int ylo = max(__float_as_int(q0.w), oy), yhi = min(__float_as_int(q1.y) + 1, yend);
+    const int cx0 = max(__float_as_int(q0.z) & ~(SWR_BLOCK - 1), ox);
+    const int cx1 = min((__float_as_int(q1.x) | (SWR_BLOCK - 1)) + 1, xend);
+    if (cx0 >= cx1) return false;
+    bool walk = false;
+    int area = 0, fy0[2], fy1[2];  // covered rows of each half
+    int pb1 = INT_MIN, pb0 = INT_MAX;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      SpanHalf hf;
+      hf.ox = t ? q3.z : q2.x; hf.oy = t ? q3.w : q2.y; hf.is1 = t ? q4.x : q2.z; hf.is2 = t ? q4.y : q2.w;
+      int y0 = t ? __float_as_int(q3.y) : __float_as_int(q1.z), y1 = t ? __float_as_int(q3.x) : __float_as_int(q1.w);
+      if (t) { y0 = y0 < INT_MAX ? y0 + 1 : y0; y1 = y1 < INT_MAX ? y1 + 1 : y1; }  // (y1, y0] as [y1 + 1, y0 + 1)
+      y0 = max(y0, ylo);
+      y1 = min(y1, yhi);
+      fy0[t] = fy1[t] = 0;
+      if (!(flags & (t ? 64 : 32)) || y0 >= y1) continue;
+      if (t && y0 < pb1 && y1 > pb0) walk = true;  // rows of both halves
+      pb0 = y0;
+      pb1 = y1;
+      int a0, b0, a1, b1;
+      span_row(hf, y0, D.sc_minx, D.sc_maxx, a0, b0);
+      span_row(hf, y1 - 1, D.sc_minx, D.sc_maxx, a1, b1);
+      if (!(fabsf(hf.is1) < 0x1p100f && fabsf(hf.is2) < 0x1p100f)) {
+        walk = true;
+      } else if (max(a0, a1) <= cx0 && min(b0, b1) >= cx1) {
+        area += (y1 - y0) * (cx1 - cx0);
+        fy0[t] = y0;
+        fy1[t] = y1;
+      } else if (!(max(b0, b1) <= cx0 || min(a0, a1) >= cx1)) {
+        walk = true;
+      }
+    }
+    if (walk || (area && p + 1u > smin)) return true;
+    frags += (uint32_t)area;
+    if (counts && area)
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+        for (int y = fy0[t]; y < fy1[t]; ++y) {
+          atomicAdd(&scnt[(y - oy) * (TILE + 1) + cx0 - ox], 1);
+          atomicAdd(&scnt[(y - oy) * (TILE + 1) + cx1 - ox], -1);
+        }
+    return false;
+  };
   // rows per item: see above (n * groups items in all)
   const int shift = n >= 128u ? 0 : (n >= 32u ? 2 : (TILE == 16 ? 4 : 5));
   const int rows = TILE >> shift;
   const uint32_t* bin = g.bin_raw ? g.bin_raw : g.bin;
   const uint64_t items = (uint64_t)n << shift;
-  int round = 0;
+  if (!DIRECT && shift == 0) {
+    constexpr uint32_t G = TILE / 4;
+    for (uint32_t base = 0; base < n; ++round) {
+      const uint32_t m = min(n - base, round < 3 ? 256u : OVB);
+      __syncthreads();  // the previous list is no longer read
+      if (tid == 0) snwalk = 0u;
+      __syncthreads();
+      for (uint32_t k0 = 0; k0 < m; k0 += 256) {
+        const uint32_t k = k0 + (uint32_t)tid, p = k < m ? bin[hi - 1u - (base + k)] : 0u;
+        const bool walk = k < m && classify(p);
+        const uint32_t bal = __ballot_sync(0xffffffffu, walk);
+        uint32_t at = 0;
+        if (lane == 0 && bal) at = atomicAdd(&snwalk, (uint32_t)__popc(bal));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (walk) swalk[at + (uint32_t)__popc(bal & ((1u << lane) - 1u))] = p;
+      }
+      __syncthreads();
+      const uint32_t work = snwalk * G;
+      for (uint32_t t = (uint32_t)tid; t < work; t += 256) cover(swalk[t / G], (int)(t % G) * 4, (int)(t % G) * 4 + 4);
+      base += m;
+      if (round < 3 && base < n) raise_smin();  // a later, larger bound would save little
+    }
+  } else
   for (uint64_t base = 0; base < items; base += 256, ++round) {
     const uint64_t it = base + (uint64_t)tid;
     if (it < items) {
@@ -2414,21 +2509,7 @@ __global__ void __launch_bounds__(256) k_overwrite(RasterArgs g) {
         cover(bin[hi - 1u - k], r0, r0 + rows);
       }
     }
-    if (round < 3 && base + 256 < items) {  // (uniform) a later, larger bound would save little
-      __syncthreads();
-      uint32_t m = 0xffffffffu;
-#pragma unroll
-      for (int q = 0; q < PPT; ++q) {
-        const int i = q * 256 + tid;
-        if (ox + i % TILE < xend && oy + i / TILE < yend) m = min(m, sbest[i]);
-      }
-      m = __reduce_min_sync(0xffffffffu, m);
-      if (lane == 0) sred[warp] = m;
-      __syncthreads();
-      smin = sred[0];
-#pragma unroll
-      for (int w = 1; w < 8; ++w) smin = min(smin, sred[w]);
-    }
+    if (round < 3 && base + 256 < items) raise_smin();
   }
   __syncthreads();
   uint32_t tot;

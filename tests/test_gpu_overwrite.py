@@ -68,3 +68,22 @@ def test_two_draws_into_one_target(gpu_lib, port):
         port.draw(sc, t)
     want, got = t.arrays(), tg.to_host()
     assert not diff(want, got), [describe(want, got, k) for k in diff(want, got)]
+
+
+@pytest.mark.parametrize("raster", [RasterMode.Span, RasterMode.Block, RasterMode.Adaptive])
+@pytest.mark.parametrize("tile", [16, 32])
+@pytest.mark.parametrize("scissor", [None, (5, 3, 171, 120), (-40, -3, 190, 140)])
+def test_halves_told_by_their_end_rows(gpu_lib, port, raster, tile, scissor):
+    """Bins of 128 entries and more (several classified batches): triangles that miss a tile's
+    columns, cover all of them or cut them, thin slanted ones, scissors cutting both sides."""
+    for sc in (scenes.benchmark_scene(6000), scenes.soup_scene(1 << 13, seed=23), scenes.soup_scene(3000, seed=24)):
+        sc.width, sc.height, sc.raster = 203, 151, raster
+        sc.viewport = (0, 0, 203, 151)
+        sc.scissor = scissor or sc.viewport
+        sc.vs, sc.ps = VS.POS_RGB_AFFINE, PS.VCOLOR_AFFINE
+        ref, rst = oracle_render(port, sc)
+        for aux in (True, False):
+            got, st = _draw(sc, tile, aux)
+            want = ref if aux else {k: ref[k] for k in got}
+            assert not diff(want, got), (aux, [describe(want, got, k) for k in diff(want, got)])
+            assert st["fragments"] == st["passes"] == rst["fragments"]
