@@ -14,7 +14,7 @@
 #define SWR_RASTER_MINB 0         // k_raster CTAs per SM to plan registers for (0: per shader)
 #endif
 #define SWR_RASTER_SORT 512       // tiles with at most this many bin entries are ordered by k_raster
-#define SWR_SLICES_MAX 8          // overwrite shaders: CTAs per tile of more than SWR_RASTER_SORT entries
+#define SWR_SLICES_MAX 32         // overwrite shaders: most CTAs per tile of more than SWR_RASTER_SORT entries
 #define SWR_DSLICES 4             // depth-min shaders: CTAs (runs of whole chunks) per listed heavy tile
 #ifndef SWR_DEPTH_CULL
 #define SWR_DEPTH_CULL 1          // k_raster's per-chunk tile depth cull (depth-tested shaders)

@@ -1073,6 +1073,9 @@ __global__ void __launch_bounds__(256) k_emit_pairs(const uint32_t* status, uint
 // out tile-major, so a tile's bin is one contiguous range ordered by segment; inside a cell
 // the fill order is arbitrary; k_raster (or k_sort_tiles ahead of it, for tiles it cannot
 // order itself) restores increasing primitive order.
+#ifndef SWR_FILL_TILES
+#define SWR_FILL_TILES 512
+#endif
 template <class PS>
 __global__ void __launch_bounds__(256) k_fill_bins(const uint32_t* status, uint32_t cap_prims, const float* recs,
                                                    uint32_t* cell_count, const uint32_t* fill_start,
@@ -1099,10 +1102,16 @@ __global__ void __launch_bounds__(256) k_fill_bins(const uint32_t* status, uint3
   const int tw0 = T0.tiles_x;
   const int tshift = __ffs(tile) - 1;  // tiles are 16 or 32 pixels; pixel boxes are >= 0
   const int lane = threadIdx.x & 31;
-  // one warp per 32 consecutive primitives (the loop is uniform per warp)
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t p0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; p0 < np; p0 += stride) {
-    const uint32_t p = p0 + (uint32_t)lane;
+  // One warp per `per` consecutive primitives (the loop is uniform per warp): 32, or as many as
+  // SWR_FILL_TILES entries belong to.  A warp works through its entries 128 at a time, each a
+  // chain of an atomic and a store, so few primitives of many tiles have to spread over warps:
+  // 40,960 triangles of 94 tiles took 87 us as 1,280 warps of 32, and take 45 as 10,240 of 4
+  // (256 or 1,024 entries a warp: 1 % of the draw slower).
+  uint32_t per = 32;
+  while (per > 1 && (uint64_t)total * per > (uint64_t)np * SWR_FILL_TILES) per >>= 1;
+  const uint32_t stride = gridDim.x * (blockDim.x >> 5) * per;
+  for (uint32_t p0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per; p0 < np; p0 += stride) {
+    const uint32_t p = (uint32_t)lane < per ? p0 + (uint32_t)lane : 0xffffffffu;
     // record words 0-5: flags (0: no tile, as tile_count), draw, pixel box (two float4
     // reads of the 16-byte aligned record)
     int tx0 = 0, ty0 = 0, nx = 1, cnt = 0;
@@ -2289,19 +2298,25 @@ __global__ void __launch_bounds__(NT, SWR_RASTER_MINB ? SWR_RASTER_MINB
 // Neither needs the bin in order, and only one fragment per pixel needs shading.
 //
 // One CTA per tile, or g.slices CTAs over parts of a tile's bin of more than SWR_RASTER_SORT
-// entries.  A work item is an entry and a group of its rows: the whole tile's rows, one
-// thread per entry, where entries are many (the record is read once, straight from global
-// memory; no staging, no barriers), single rows where they are few (a small draw's large
-// triangles would leave one thread walking 256 pixels).  An item adds up the lengths of its
-// rows' runs, and writes its id over smaller ones in the tile's winners; entries are taken
-// from the bin's end (the largest ids up to the order inside a cell), and once every pixel
-// has a winner, entries below all of them only count.  The last CTA of a tile shades its
-// winners.  Bound by the issue of the row loop.  Against ordering every bin and walking
-// 64-primitive chunks pixel by pixel (sorts 91 us, raster 1463 us), the 40,960 large
-// triangles of the reference's Benchmark program (640x480, 240M fragments) went
-// from 1888 to 585 us a draw.
+// entries.  Entries are taken from the bin's end (the largest ids up to the order inside a
+// cell); an entry adds up the lengths of its rows' runs here and writes its id over smaller
+// ones in the tile's winners, and once every pixel has a winner, entries below all of them only
+// count.  The last CTA of a tile shades its winners.
+//
+// Of 128 entries and more, a thread first classifies one each: a Span primitive whose two end
+// rows per half show that it misses the tile's columns or covers all of them, and that can win
+// no pixel, is counted there.  The others are listed and walked four rows a work item; walked
+// by one thread each, a warp waited for the tallest of its 32 (17 lanes active; the 40,960
+// large triangles below: 257 us, 210 this way).  Fewer entries are split into rows at once, down
+// to single ones (a small draw's large triangles would leave one thread walking 256 pixels).
+// Nothing is staged: a record is read from the cache by the threads that need it.
+//
+// Bound by latency: the record reads and the barriers around the lists, at five CTAs per SM
+// (four, with all the registers wanted: 354 us a draw, five 333).  The 40,960 triangles of the
+// reference's Benchmark program (640x480, 240M fragments): bins ordered and walked in
+// 64-primitive chunks pixel by pixel, 1888 us a draw; this way 333.
 template <class PS, int TILE, bool DIRECT>
-__global__ void __launch_bounds__(256) k_overwrite(RasterArgs g) {
+__global__ void __launch_bounds__(256, 5) k_overwrite(RasterArgs g) {
   swr_pdl_entry();
   typedef Rec<PS> RL;
   constexpr int PPT = TILE * TILE / 256;
