@@ -10,12 +10,16 @@
 //                     in parent order (VertexProcessor.cpp:254-260)
 //   k_setup           TriangleEquations (TriangleEquations.h:47-71) and the raster-mode
 //                     decision, bounding boxes and tile counts per primitive
-//   k_emit_pairs      (tile, primitive) pairs in primitive order -> stable radix sort
-//   k_raster          one CTA per screen tile; each thread owns pixels and walks the
-//                     tile's bin in primitive order, reproducing Span (Rasterizer.h:309-411)
-//                     and Block (Rasterizer.h:225-306, PixelShaderBase.h:55-112) coverage
-//                     and incrementally stepped interpolants exactly, then calls the pixel
-//                     shader in the same per-pixel order as the reference.
+//   k_front           small draws: the stages up to k_assemble_emit in one launch
+//   k_fill_bins       primitive ids into (tile, primitive segment) cells; k_emit_pairs:
+//                     (tile, primitive) pairs in primitive order for a stable radix sort
+//   k_raster          one CTA per listed screen tile (k_raster_two: per two); each thread owns
+//                     pixels and walks the tile's bin in primitive order, reproducing Span
+//                     (Rasterizer.h:309-411) and Block (Rasterizer.h:225-306,
+//                     PixelShaderBase.h:55-112) coverage and incrementally stepped
+//                     interpolants exactly, with the effects of calling the pixel shader in
+//                     the same per-pixel order as the reference
+//   k_overwrite       the same for shaders without depth test that only overwrite
 //
 // All arithmetic on the parity path uses the _rn intrinsics (no FMA contraction).
 #pragma once
@@ -728,9 +732,9 @@ __device__ __forceinline__ bool swr_box_hit(uint32_t box, uint32_t tx, uint32_t 
 // serialise the warp and the pairs' memory operations are in flight together.  Every lane
 // brings the tile box of its primitive: `cnt` tiles (0: none), nx a row, from (tx0, ty0), in
 // a target of tiles_x tiles a row starting at tile tbase.  `put` returns nothing; it is called
-// by whole warps with on = false for lanes without a pair.  Serial walks per lane made the
-// counting make k_setup 104 us on the Benchmark program and 192 us on the 1M-triangle soup;
-// with this 85 and 98 us.
+// by whole warps with on = false for lanes without a pair.  Counting by serial walks
+// per lane, k_setup took 104 us on the Benchmark program and 192 us on the 1M-triangle soup;
+// this way 85 and 98, and with the counters segment-major (SwrCells) 37 and 81.
 template <class F>
 __device__ __forceinline__ void warp_tiles(int cnt, int nx, int tx0, int ty0, uint32_t tbase, int tiles_x, F put) {
   constexpr int G = 4;
