@@ -26,19 +26,24 @@ __device__ __forceinline__ void chunk_range(uint32_t n, uint32_t chunk, uint32_t
   if (e > n) e = n;
 }
 
+// A count too large for 32 bits is the largest 32-bit value: sums of saturated counts are exact
+// below it and never wrap to a small one.
+__device__ __forceinline__ uint32_t saturated(unsigned long long v) {
+  return v < SWR_COUNT_MAX ? (uint32_t)v : SWR_COUNT_MAX;
+}
+
 __global__ void __launch_bounds__(kThreads) k_scan_reduce(const uint32_t* in, const uint32_t* n_dev,
                                                           uint32_t n_max, uint32_t chunk,
                                                           uint32_t* partials) {
   swr_pdl_entry();
-  __shared__ uint32_t tmp[32];
+  __shared__ unsigned long long tmp[32];
   const uint32_t n = load_n(n_dev, n_max);
   uint32_t b, e;
   chunk_range(n, chunk, b, e);
-  uint32_t s = 0;
+  unsigned long long s = 0, tot;
   for (uint32_t i = b + threadIdx.x; i < e; i += kThreads) s += in[i];
-  uint32_t tot;
   swr_block_exscan(s, tmp, &tot);
-  if (threadIdx.x == 0) partials[blockIdx.x] = tot;
+  if (threadIdx.x == 0) partials[blockIdx.x] = saturated(tot);
 }
 
 __global__ void __launch_bounds__(kThreads) k_scan_down(const uint32_t* in, uint32_t* out,
@@ -53,16 +58,19 @@ __global__ void __launch_bounds__(kThreads) k_scan_down(const uint32_t* in, uint
   // prefix of the partial sums of the blocks before this one (and the grand total)
   __shared__ uint32_t pref[2];
   {
-    uint32_t mine = 0, all = 0;
+    __shared__ unsigned long long tmp64[32];
+    uint32_t mine = 0;
+    unsigned long long all = 0;
     for (int i = threadIdx.x; i < (int)gridDim.x; i += kThreads) {
       const uint32_t v = partials[i];
       all += v;
       if (i < (int)blockIdx.x) mine += v;
     }
-    uint32_t t0, t1;
+    uint32_t t0;
+    unsigned long long t1;
     swr_block_exscan(mine, tmp, &t0);
-    swr_block_exscan(all, tmp, &t1);
-    if (threadIdx.x == 0) { pref[0] = t0; pref[1] = t1; }
+    swr_block_exscan(all, tmp64, &t1);
+    if (threadIdx.x == 0) { pref[0] = t0; pref[1] = saturated(t1); }
     __syncthreads();
   }
   if (blockIdx.x == 0 && threadIdx.x == 0 && total) *total = pref[1];
@@ -238,7 +246,7 @@ __global__ void __launch_bounds__(kThreads) k_radix_scatter(const uint32_t* kin,
   for (int w = 0; w < kWarps; ++w) wcnt[w][threadIdx.x] = 0;
   {
     // digit d starts at (keys with a smaller digit) + (digit-d keys in earlier blocks)
-    const uint32_t dbase = swr_block_exscan(tot[threadIdx.x], tmp, nullptr);
+    const uint32_t dbase = swr_block_exscan(tot[threadIdx.x], tmp);
     base[threadIdx.x] = dbase + off[blockIdx.x * 256 + threadIdx.x];
   }
   __syncthreads();

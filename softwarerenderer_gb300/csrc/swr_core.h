@@ -11,7 +11,8 @@ namespace swr {
 constexpr int kScanBlocks = 304;  // 2 x 152 SMs
 
 // Exclusive prefix sum of in[0..n) into out, where n = min(*n_dev, n_max) when n_dev is
-// given (device-resident length) else n_max.  total (device) receives the sum.
+// given (device-resident length) else n_max.  total (device) receives the sum, or
+// SWR_COUNT_MAX when it is that or more: the prefixes are then of no use.
 // scratch needs scan_scratch_words(n_max) words.  Two kernels: block partial sums, then
 // each block prefixes the partials before it and scans its chunk.
 size_t scan_scratch_words(uint32_t n_max);

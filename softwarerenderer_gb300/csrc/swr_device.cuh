@@ -47,6 +47,7 @@ enum SwrStatusFlags {
   SWR_F_BARRIER_TIMEOUT = 256,  // a grid barrier of a persistent launch gave up waiting
 };
 #define SWR_F_ANY_OVERFLOW (SWR_F_CLIP_OVERFLOW | SWR_F_PRIM_OVERFLOW | SWR_F_PAIR_OVERFLOW | SWR_F_FRAG_OVERFLOW)
+#define SWR_COUNT_MAX 0xffffffffu  // a queue request of this many entries or more: no queue holds it
 #define SWR_ST_STICKY 8  // words SWR_ST_STICKY + i keep the largest value word i reached (i = CLIP_SLOTS..FRAGS)
 
 // Programmatic dependent launch.  Kernels of a draw are launched so that the next one may
@@ -210,29 +211,31 @@ __device__ __forceinline__ void swr_block_sum2(uint32_t a, uint32_t b, uint32_t*
 }
 
 // Block-wide exclusive scan of one value per thread (blockDim.x multiple of 32, <= 1024).
-// `tmp` needs 32 words.  Returns the exclusive prefix; *total receives the block sum.
-__device__ __forceinline__ uint32_t swr_block_exscan(uint32_t v, uint32_t* tmp, uint32_t* total) {
+// `tmp` needs 32 elements.  Returns the exclusive prefix; *total receives the block sum.
+// T: uint32_t, or unsigned long long where the sum may exceed 32 bits.
+template <class T>
+__device__ __forceinline__ T swr_block_exscan(T v, T* tmp, T* total = nullptr) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nwarps = blockDim.x >> 5;
-  uint32_t x = v;
+  T x = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    const T y = __shfl_up_sync(0xffffffffu, x, o);
     if (lane >= o) x += y;
   }
   if (lane == 31) tmp[warp] = x;
   __syncthreads();
   if (warp == 0) {
-    uint32_t s = lane < nwarps ? tmp[lane] : 0u;
+    T s = lane < nwarps ? tmp[lane] : T(0);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
+      const T y = __shfl_up_sync(0xffffffffu, s, o);
       if (lane >= o) s += y;
     }
     tmp[lane] = s;  // inclusive warp totals
   }
   __syncthreads();
-  const uint32_t warp_off = warp ? tmp[warp - 1] : 0u;
+  const T warp_off = warp ? tmp[warp - 1] : T(0);
   if (total) *total = tmp[nwarps - 1];
   __syncthreads();
   return warp_off + x - v;

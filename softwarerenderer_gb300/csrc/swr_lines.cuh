@@ -242,7 +242,7 @@ struct LpFragArgs {
   const float* recs;
   const uint32_t* steps;      // per primitive: its fragments
   const uint32_t* frag_off;   // their exclusive scan
-  const uint32_t* nfrags;     // device total
+  const uint32_t* nfrags;     // device total (SWR_COUNT_MAX: that or more)
   uint32_t cap_frags;
   const SwrDrawDesc* draws;
   const SwrTargetDesc* targets;
@@ -262,8 +262,10 @@ __global__ void __launch_bounds__(256) k_lp_frags(LpFragArgs g) {
   swr_pdl_entry();
   typedef LpRec<PS> RL;
   if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
+  // The sum of the steps, never wrapped: screen-space lines are not clipped, and one may take
+  // 2^31 - 1 steps.  Past the queue nothing is written; past SWR_COUNT_MAX no queue would do.
   const uint32_t nf = *g.nfrags;
-  if (nf > g.cap_frags) {
+  if (nf > g.cap_frags || nf == SWR_COUNT_MAX) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       atomicOr(&g.status_w[SWR_ST_FLAGS], SWR_F_PAIR_OVERFLOW);
       g.status_w[SWR_ST_PAIRS] = nf;
@@ -281,7 +283,7 @@ __global__ void __launch_bounds__(256) k_lp_frags(LpFragArgs g) {
   // one fragment per lane (every lane of the warp calls it)
   auto put = [&](bool on, uint32_t f, uint32_t prim, float x, float y) {
     uint32_t key = SWR_LP_INVALID;
-    if (on) {
+    if (on && f < g.cap_frags) {
       // Rasterizer::scissorTest on the stepped float position (Rasterizer.h:144-147)
       if (x >= sx0 && x < sx1 && y >= sy0 && y < sy1) {
         const int ix = swr_trunc_int(x), iy = swr_trunc_int(y);

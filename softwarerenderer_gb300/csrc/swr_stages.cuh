@@ -165,7 +165,7 @@ static __global__ void __launch_bounds__(256) k_direct_emit(DirectArgs g, uint4*
     first[k] = p0 + k < g.nprims ? g.idx[(size_t)g.per * (p0 + k)] : -1;
     c += first[k] != -1;
   }
-  uint32_t at = g.base[blockIdx.x] + swr_block_exscan(c, tmp, nullptr);
+  uint32_t at = g.base[blockIdx.x] + swr_block_exscan(c, tmp);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     if (first[k] == -1) continue;
