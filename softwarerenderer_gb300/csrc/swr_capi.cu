@@ -100,6 +100,7 @@ __global__ void k_report_status(uint32_t* st, uint32_t* host) {
 struct MemBudget {
   size_t used = 0;
   size_t limit = 0;
+  uint64_t moves = 0;  // allocations so far: while it stays, every buffer is where it was
 };
 
 struct Buffer {
@@ -115,7 +116,10 @@ struct Buffer {
     // over the context's budget: fail like an allocation failure, keeping the old buffer
     if (budget && budget->limit && budget->used - bytes + want > budget->limit) return false;
     if (p) cudaFree(p);
-    if (budget) budget->used -= bytes;
+    if (budget) {
+      budget->used -= bytes;
+      budget->moves++;
+    }
     p = nullptr;
     bytes = 0;
     if (cudaMalloc(&p, want) != cudaSuccess) {
@@ -1232,14 +1236,11 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
   mix((uint64_t)small);
   mix((uint64_t)vs->S); mix((uint64_t)ps->R); mix((uint64_t)c->tile); mix((uint64_t)n);
   mix(c->cap_prims); mix(c->cap_pairs); mix(c->cap_clip_slots); mix(c->cap_clip_verts);
-  const void* bufs[] = {c->ptv.p, c->clipv.p, c->clip_table.p, c->clip_slot.p, c->tri_flags.p, c->batch_counts.p,
-                        c->tris.p, c->recs.p, c->tile_count.p, c->keys0.p, c->vals0.p, c->cell_count.p,
-                        c->cell_start.p, c->cell_fill.p, c->scratch.p, c->draws.p, c->targets.p, c->draw_vbase.p,
-                        c->draw_bbase.p, c->target_tile_base.p, c->draw_pbase.p, h,
-                        c->over_best.p, c->over_done.p, (const void*)(uintptr_t)c->slices, c->tile_list.p,
-                        c->heavy_tiles.p, c->sort_tiles.p, c->tile_counts.p, c->geo_bar.p, c->dslice_state.p, c->dslice_done.p,
-                        (const void*)(uintptr_t)c->dslice_ok, (const void*)(intptr_t)c->dslice_chunks};
-  for (const void* b : bufs) mix((uint64_t)(uintptr_t)b);
+  // A captured graph holds the addresses of the context's buffers: it is good until one of them
+  // is allocated anew, whichever it is.
+  mix(c->budget.moves);
+  mix((uint64_t)(uintptr_t)h);
+  mix((uint64_t)c->slices); mix((uint64_t)c->dslice_ok); mix((uint64_t)(uint32_t)c->dslice_chunks);
   if (c->graph_mode && c->gexec[slot] && sig == c->gsig[slot]) {
     if ((rc = cuda_err(cudaGraphLaunch(c->gexec[slot], s)))) return rc;
     c->launches += c->glaunches[slot];
