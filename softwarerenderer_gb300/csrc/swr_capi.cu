@@ -1338,7 +1338,7 @@ int swr_finish(swr_context* c, void* stream, swr_stats* stats) {
   if (stats) {
     stats->fragments = (uint64_t)h[SWR_ST_SHADED_LO] | ((uint64_t)h[SWR_ST_SHADED_HI] << 32);
     stats->primitives = h[SWR_ST_PRIMS];
-    stats->bin_pairs = h[SWR_ST_PAIRS];
+    stats->bin_pairs = h[kStickyBase + SWR_ST_PAIRS] == SWR_COUNT_MAX ? SWR_COUNT_MAX : h[SWR_ST_PAIRS];
     stats->clip_polygons = h[SWR_ST_CLIP_SLOTS];
     stats->flags = h[SWR_ST_FLAGS];
     stats->launches = c->launches;

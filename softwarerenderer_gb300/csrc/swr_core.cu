@@ -104,11 +104,13 @@ static_assert(SWR_SEGS == 32 && kThreads == 256, "a group of 32 tiles is a 32 x 
 
 __global__ void __launch_bounds__(kThreads) k_cells(const CellsArgs a) {
   swr_pdl_entry();
-  __shared__ uint32_t tmp[32];
+  __shared__ unsigned long long tmp[32];
   __shared__ uint32_t sq[kGroup][SWR_SEGS + 1];
   __shared__ uint32_t stot[kGroup], sfirst[kGroup];
   __shared__ uint32_t sbase;
-  if (a.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
+  // (A pair overflow of a kernel before left no counts; one that another block finds here must
+  // not part this block's threads.)
+  if (a.status[SWR_ST_FLAGS] & (SWR_F_ANY_OVERFLOW & ~SWR_F_PAIR_OVERFLOW)) return;
   const uint32_t nt = a.t.ntiles, t0 = blockIdx.x * kGroup;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t tl = threadIdx.x >> 3, sg = (threadIdx.x & 7) * 4;  // this thread's four cells
@@ -131,10 +133,19 @@ __global__ void __launch_bounds__(kThreads) k_cells(const CellsArgs a) {
   uint32_t tile_tot = s;  // the tile's entries: over its eight lanes
 #pragma unroll
   for (int o = 1; o < 8; o <<= 1) tile_tot += __shfl_xor_sync(0xffffffffu, tile_tot, o);
-  uint32_t tot;
-  uint32_t ex = swr_block_exscan(s, tmp, &tot);  // (its barriers order the reads of sq above)
+  unsigned long long tot;
+  // (its barriers order the reads of sq above)
+  uint32_t ex = (uint32_t)swr_block_exscan((unsigned long long)s, tmp, &tot);
   if (tot == 0) return;  // uniform
-  if (threadIdx.x == 0) sbase = atomicAdd(a.total, tot);
+  if (threadIdx.x == 0) {
+    sbase = atomicAdd(a.total, (uint32_t)tot);
+    // A total past 32 bits wraps and would read as one that fits: the draw is refused here, and
+    // its request recorded as one that no queue holds.
+    if (tot >= SWR_COUNT_MAX - sbase) {
+      atomicOr(&a.status[SWR_ST_FLAGS], SWR_F_PAIR_OVERFLOW);
+      a.status[SWR_ST_STICKY + SWR_ST_PAIRS] = SWR_COUNT_MAX;
+    }
+  }
   if (sg == 0) {
     stot[tl] = tile_tot;
     sfirst[tl] = ex;

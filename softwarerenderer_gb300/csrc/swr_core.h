@@ -24,14 +24,15 @@ void scan_exclusive(const uint32_t* in, uint32_t* out, const uint32_t* n_dev, ui
 // blocks of 32 tiles come, not in tile order: nothing needs one tile's range to follow
 // another's, and the exclusive scan that put them in order was two launches (10 us of a small
 // draw's chain; on 256 meshes' 491,520 mostly empty tiles 79 us).  The same kernel makes the
-// lists of t, so that empty tiles cost the later kernels nothing.
+// lists of t, so that empty tiles cost the later kernels nothing.  SWR_COUNT_MAX entries or more
+// set SWR_F_PAIR_OVERFLOW (*total is then of no use).
 //   count       per cell (layout `cells`)
 //   fill_start  the starts in that layout (segment-major only; tile-major it is t.start itself)
 //   heavy_min   tiles of more entries go to t.heavy, up to t.heavy_cap, and not to t.list
 //   sort_min    tiles of more entries go to t.sort
 //   front_min   tiles of more entries go to t.list's front (rasterized first), others to its back
 struct CellsArgs {
-  const uint32_t* status;
+  uint32_t* status;
   const uint32_t* count;
   SwrCells cells;
   uint32_t* fill_start;
