@@ -415,11 +415,13 @@ SwrTiles tiles_of(const swr_context* c, uint32_t ntiles, uint32_t heavy_cap) {
 
 void sort_tiles(swr_context* c, const SwrTiles& t, int seg_shift, uint32_t cell_min, const uint32_t* in, uint32_t* out,
                 cudaStream_t s) {
-  const size_t bm = ((size_t)1 << seg_shift) / 8;  // bytes of one warp's bitmap
-  const bool fits = bm >= 4 && bm <= kSortSmem;
-  const int warps = fits ? (int)std::min<size_t>(8, kSortSmem / bm) : 8;
-  swr::launch(k_sort_tiles, kSortWarps / warps, 32 * warps, fits ? warps * bm : 0, s, c->status.as<uint32_t>(), t,
-              seg_shift, fits ? (uint32_t)(bm / 4) : 0u, cell_min, in, out);
+  // bytes of one warp's bitmap: the segment's range, where one fits; else an eighth for each of
+  // eight warps (a window of a segment costs a warp the same per id as a range that fits)
+  const size_t range = std::max<size_t>(((size_t)1 << seg_shift) / 8, 4);
+  const size_t bm = range <= kSortSmem ? range : kSortSmem / 8;
+  const int warps = (int)std::min<size_t>(8, kSortSmem / bm);
+  swr::launch(k_sort_tiles, kSortWarps / warps, 32 * warps, warps * bm, s, c->status.as<uint32_t>(), t, seg_shift,
+              (uint32_t)(bm / 4), cell_min, in, out);
   c->launches += 1;
 }
 
