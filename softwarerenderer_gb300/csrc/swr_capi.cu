@@ -804,9 +804,9 @@ int swr_set_vertex_shader(swr_context* c, int id) {
 
 static bool program_ok(const swr_program* p, uint32_t kind) {
   if (!p || p->magic != SWR_PROGRAM_MAGIC || p->abi != SWR_PROGRAM_ABI || p->kind != kind) return false;
-  uint32_t mine[10];
+  uint32_t mine[SWR_PROGRAM_SIZES];
   swr_program_layout(mine);
-  for (int i = 0; i < 10; ++i)
+  for (int i = 0; i < SWR_PROGRAM_SIZES; ++i)
     if (p->sizes[i] != mine[i]) return false;
   return kind == SWR_PROGRAM_VERTEX ? p->vs != nullptr : p->ps != nullptr;
 }

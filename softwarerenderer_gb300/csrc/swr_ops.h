@@ -59,15 +59,16 @@ const PsOps* ps_ops(int id);
 // these headers in the caller's unit, so the library checks that both sides agree on the
 // layout of every structure that crosses between them.
 #define SWR_PROGRAM_MAGIC 0x50525753u  // "SWRP"
-#define SWR_PROGRAM_ABI 4u             // bumped with any change to VsOps, PsOps or their argument structs
+#define SWR_PROGRAM_ABI 5u             // bumped with any change to VsOps, PsOps or their argument structs
 #define SWR_PROGRAM_VERTEX 1u
 #define SWR_PROGRAM_PIXEL 2u
+#define SWR_PROGRAM_SIZES 13           // entries of swr_program_layout()
 
 struct swr_program {
   uint32_t magic;     // SWR_PROGRAM_MAGIC
   uint32_t abi;       // SWR_PROGRAM_ABI
   uint32_t kind;      // SWR_PROGRAM_VERTEX or SWR_PROGRAM_PIXEL
-  uint32_t sizes[10]; // swr_program_layout()
+  uint32_t sizes[SWR_PROGRAM_SIZES];  // swr_program_layout()
   const swr::VsOps* vs;
   const swr::PsOps* ps;
 };
@@ -83,5 +84,8 @@ inline void swr_program_layout(uint32_t* s) {
   s[6] = (uint32_t)sizeof(swr::RasterArgs);
   s[7] = (uint32_t)sizeof(swr::LpFragArgs);
   s[8] = (uint32_t)sizeof(swr::LpRasterArgs);
-  s[9] = (uint32_t)sizeof(SwrUniforms) + ((uint32_t)sizeof(swr::FrontArgs) << 16);
+  s[9] = (uint32_t)sizeof(SwrUniforms);
+  s[10] = (uint32_t)sizeof(swr::FrontArgs);
+  s[11] = (uint32_t)sizeof(swr::DirectArgs);
+  s[12] = (uint32_t)sizeof(SwrCells);
 }
