@@ -1479,6 +1479,12 @@ __device__ __forceinline__ uint32_t warp_transpose(uint32_t x, int lane) {
   return x;
 }
 
+// A 64-bit word or'ed over the warp.
+__device__ __forceinline__ uint64_t warp_or(uint64_t x) {
+  const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)x), hi = __reduce_or_sync(0xffffffffu, (uint32_t)(x >> 32));
+  return lo | (uint64_t)hi << 32;
+}
+
 // Rebuilds the reference's incrementally stepped PixelData for pixel (x, y): the value
 // at the evaluation point (block corner or span start) stepped kb times along y and ka
 // times along x (PixelData::init/stepY/stepX, PixelData.h:61-125).
@@ -1620,6 +1626,15 @@ __device__ __forceinline__ bool raster_tile(const RasterArgs& g, uint32_t bid) {
   // fragment that passes only records its primitive, and the last one that did is shaded from
   // its record.
   constexpr bool kDefer = !SwrNoCompact<PS>::value;
+  // Shaders with side effects interpolate every fragment in the walk.  In Span mode its steps
+  // from the row's span start are a loop whose course depends on the primitive (swr_fold), and
+  // lanes that visit different ones wait for each other: the warp's lanes then visit the same
+  // primitives, unless that is many more steps than the pixel with most of them takes.  A
+  // depth-tested user shader at 1920x1080, us a draw with every pixel on its own / together /
+  // by that rule: 20,000 triangles of 300 px 27700 / 21800 / 21700, 200,000 of 40 px
+  // 8560 / 6790 / 6890, 200,000 of 6 px 396 / 544 / 422.  Block mode's are at most 14 predicated
+  // steps, the same for every primitive: there each pixel goes on its own.
+  constexpr bool kTogether = !kDefer && SPAN;
   static_assert(!kDefer || (PS::HasDepth && RL::IZ), "a deferred fragment is one that passes the depth test");
   // Staged records: words 0-23 where only coverage and z are read (header, edges or span
   // halves, the z equation), 28 words apart so that the lanes' different records spread over
@@ -2148,8 +2163,15 @@ __device__ __forceinline__ bool raster_tile(const RasterArgs& g, uint32_t bid) {
           mine[w] &= ~((uint64_t)cr[2 * w] | (2 * w + 1 < NW ? (uint64_t)cr[2 * w + 1] << 32 : 0ull));
       }
       int won = -1;  // kDefer: the chunk's last primitive to pass the pixel's depth test
-      uint64_t hits = mine[0];
-      uint64_t later = HW > 1 ? mine[HW - 1] : 0ull;
+      // kTogether: the primitives of any of the warp's pixels where they are not many more than
+      // one pixel's, else the pixel's own
+      auto visits = [&](uint64_t own) -> uint64_t {
+        if (!kTogether) return own;
+        const uint64_t any = warp_or(own);
+        return 4 * __popcll(any) <= 7 * (int)__reduce_max_sync(0xffffffffu, (uint32_t)__popcll(own)) ? any : own;
+      };
+      uint64_t hits = visits(mine[0]);
+      uint64_t later = HW > 1 ? visits(mine[HW - 1]) : 0ull;
       int kbase = 0;
       while (true) {  // (one copy of the loop body for both words)
         if (!hits) {
@@ -2160,6 +2182,7 @@ __device__ __forceinline__ bool raster_tile(const RasterArgs& g, uint32_t bid) {
         }
         const int k = kbase + __ffsll((long long)hits) - 1;
         hits &= hits - 1ull;
+        if (kTogether && !((mine[HW > 1 ? k >> 6 : 0] >> (k & 63)) & 1ull)) continue;
         const float* r = srec + k * SR;
         const bool blockmode = !SPAN || (__float_as_int(r[0]) & 2);
         float fx, fy;
