@@ -256,7 +256,12 @@ struct LpFragArgs {
 
 // Fragments of the primitives, one warp per 32 consecutive primitives whose fragments are
 // spread over its lanes 32 at a time, so a long line does not hold up the warp and no
-// fragment has to search for its primitive.
+// fragment has to search for its primitive.  Fewer primitives a warp where they have many
+// fragments each, about SWR_LP_FRAGS in all: 2,500 lines of 20 steps are 78 warps of 32, too few
+// to hide each step's latency (the binning stage 57 us, 27 this way).
+#ifndef SWR_LP_FRAGS
+#define SWR_LP_FRAGS 128
+#endif
 template <class PS>
 __global__ void __launch_bounds__(256) k_lp_frags(LpFragArgs g) {
   swr_pdl_entry();
@@ -298,12 +303,14 @@ __global__ void __launch_bounds__(256) k_lp_frags(LpFragArgs g) {
     const uint32_t peers = __match_any_sync(0xffffffffu, cell);  // neighbours share cells
     if (cell != SWR_LP_INVALID && lane == __ffs(peers) - 1) atomicAdd(&g.cell_count[cell], (uint32_t)__popc(peers));
   };
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t p0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; p0 < np; p0 += stride) {
+  uint32_t per = 32;  // primitives a warp: 32, or as many as SWR_LP_FRAGS fragments belong to
+  while (per > 1 && (uint64_t)nf * per > (uint64_t)np * SWR_LP_FRAGS) per >>= 1;
+  const uint32_t stride = gridDim.x * (blockDim.x >> 5) * per;
+  for (uint32_t p0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per; p0 < np; p0 += stride) {
     const uint32_t p = p0 + (uint32_t)lane;
     uint32_t cnt = 0, off = 0;
     float x = 0.0f, y = 0.0f, dx = 0.0f, dy = 0.0f;
-    if (p < np) {
+    if ((uint32_t)lane < per && p < np) {
       cnt = g.steps[p];
       off = g.frag_off[p];
       const float* rec = g.recs + (size_t)p * W;
@@ -386,12 +393,33 @@ struct LpRasterArgs {
   uint32_t* status_w;
 };
 
+// The words of an interpolated fragment: f(i, word) for each.
+template <class PS>
+struct LpPixelWords {
+  enum { W = PS::InterpolateW ? 2 : 0, value = 1 + W + PS::AVarCount + PS::PVarCount };
+};
+template <class PS, class F>
+__device__ __forceinline__ void lp_words(GpuPixel<PS>& pd, F f) {
+  typedef LpPixelWords<PS> PW;
+  f(0, pd.z);
+  if (PS::InterpolateW) {
+    f(1, pd.w);
+    f(2, pd.invw);
+  }
+#pragma unroll
+  for (int a = 0; a < PS::AVarCount; ++a) f(1 + PW::W + a, pd.avar[a]);
+#pragma unroll
+  for (int a = 0; a < PS::PVarCount; ++a) f(1 + PW::W + PS::AVarCount + a, pd.pvar[a]);
+}
+
 // One CTA per 16 x 16 tile, one pixel per thread.  A chunk is as many whole cells of the
 // tile's bin as hold at most 256 fragments (a larger cell, ordered by k_sort_tiles, is a run of
 // chunks by itself): one fragment per thread is ranked inside its cell, interpolated, shaded
 // and marked under its rank in its pixel's set; then each thread applies its pixel's
-// fragments in increasing order (shaders with side effects of their own are evaluated there
-// instead, one drawPixel at a time).  Bound by the latency of the dependent gathers bin ->
+// fragments in increasing order (shaders with side effects of their own are not shaded ahead:
+// each gets its interpolated fragments' words there, one drawPixel at a time.  Interpolated
+// there as well, in lanes that few of a tile's pixels keep busy, 200,000 lines of 40 steps of a
+// user shader took 3435 us a draw; this way 1394).  Bound by the latency of the dependent gathers bin ->
 // primitive -> record.  Ordering the cells here instead of ahead (a warp ranking each cell of
 // 17 to 64 entries, a bitmap above) took the two sorts from 184 to 4 us on the points and
 // from 64 to 4 us on the lines.
@@ -407,9 +435,9 @@ __global__ void __launch_bounds__(256) k_lp_raster(LpRasterArgs g) {
   __shared__ uint32_t scs[SWR_SEGS + 1];
   __shared__ uint32_t smask[CW][256];  // per pixel: the chunk's fragments that hit it
   __shared__ uint32_t sprim[CH];
-  __shared__ int sstep[kCompact ? 1 : CH];
   __shared__ float sz[kCompact ? CH : 1];
   __shared__ Color sc[kCompact ? CH : 1];
+  __shared__ float spd[kCompact ? 1 : LpPixelWords<PS>::value * CH];  // others: interpolated, not shaded
   __shared__ uint32_t sfr[64];
   if (blockIdx.x == 0 && threadIdx.x == 0) swr_close_status(g.status_w);
   if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
@@ -445,8 +473,8 @@ __global__ void __launch_bounds__(256) k_lp_raster(LpRasterArgs g) {
     for (int a = 0; a < RL::NP; ++a) pd.pvar[a] = lp_value<PS>(rec, 4 + RL::NA + a, j);
   };
   uint32_t frags = 0, passes = 0;
-  __syncthreads();
   const uint32_t total = e - b;
+  __syncthreads();
   uint32_t c0 = 0;  // first entry of the chunk, relative to b
   int cell = 0;     // the cell it lies in
   while (c0 < total) {
@@ -487,7 +515,9 @@ __global__ void __launch_bounds__(256) k_lp_raster(LpRasterArgs g) {
         sz[k] = pd.z;
         sc[k] = PS::shade(pd, U);
       } else {
-        sstep[k] = j;
+        GpuPixel<PS> pd;
+        pixel(prim, j, 0, 0, pd);
+        lp_words<PS>(pd, [&](int i, float& v) { spd[i * CH + k] = v; });
       }
       atomicOr(&smask[k >> 5][pix], 1u << (k & 31));
     }
@@ -505,7 +535,10 @@ __global__ void __launch_bounds__(256) k_lp_raster(LpRasterArgs g) {
           PS::apply(st, sz[k], sc[k], (int)sprim[k]);
         } else {
           GpuPixel<PS> pd;
-          pixel(sprim[k], sstep[k], x, y, pd);
+          pd.x = x;
+          pd.y = y;
+          pd.eq = nullptr;  // points and lines carry no triangle equations
+          lp_words<PS>(pd, [&](int i, float& v) { v = spd[i * CH + k]; });
           PS::drawPixel(pd, (int)sprim[k], st, U);
         }
       }
