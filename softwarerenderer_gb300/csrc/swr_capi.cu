@@ -525,6 +525,15 @@ int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, i
 // and sort kernels (5 launches of about 4 us each) and, for large triangles, the setup's and
 // the fill's walks over every tile of a primitive (14 us each for the textured cube) cost more
 // than reading 1,024 boxes per tile does.  Options that act on bins keep the general path.
+//   The line is drawn by triangles alone: past it lie draws that either route may win, by a
+// little or by much, and the host does not know the triangles' sizes.  us a draw, this route /
+// general route, vertex colour in Block mode, triangles of 8 px, 64 px and the whole target:
+//              640x480                        1920x1080                      3840x2160
+//     200      27/34    28/49    49/234       32/37    48/69    197/1361     58/61    82/100   710/5289
+//     500      28/35    32/54    80/281       37/41    72/89    347/1591     60/67    124/137  1286/6164
+//   1,024      31/39    37/57    132/362      48/48    96/101   669/2033     79/74    201/177
+// A pile of 1,024 on 64 x 64 pixels loses the heavy tiles' runs that the Lambert shader has on
+// the general route: 85/67 (175 before either had its present form).
 constexpr uint32_t kSmallTris = 1024;   // submitted triangles (one batch)
 constexpr uint32_t kSmallVerts = 4096;  // vertices one CTA shades (k_front)
 
