@@ -542,9 +542,18 @@ bool small_draw(const swr_context* c, uint64_t nsub, const SwrTargetDesc& T) {
          !c->fixed_pairs && T.tiles_x <= 255 && T.tiles_y <= 255;
 }
 
-// ... and their vertex shading and assembly run as one CTA (k_front) in one launch.
-bool small_front(const swr_context* c, uint64_t nsub, uint64_t nverts, const SwrTargetDesc& T) {
+// The same with a vertex stage ...
+bool small_elements(const swr_context* c, uint64_t nsub, uint64_t nverts, const SwrTargetDesc& T) {
   return small_draw(c, nsub, T) && nverts <= kSmallVerts && !c->persistent_geometry;
+}
+
+// ... which runs with the assembly as one CTA in one launch (k_front) for one half batch of
+// triangles.  A second one in that CTA would be clipped after the first: 1,024 triangles at
+// 640x480, 46 of them clipped, took 74 us a draw so and take 38 with the three kernels; none
+// clipped, 28 and 26.  512 with 24 clipped take 45 in one CTA, 46 on the general route; none
+// clipped, 23 and 35.
+bool small_front(const swr_context* c, uint64_t nsub, uint64_t nverts, const SwrTargetDesc& T) {
+  return small_elements(c, nsub, nverts, T) && nsub <= SWR_HALF;
 }
 
 int small_raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, int vs_a, int vs_p, uint32_t nsub,
@@ -1041,6 +1050,9 @@ int swr_draw_elements(swr_context* c, int mode, uint64_t count, const uint32_t* 
   }
   mark(c, 2, s);
   c->last_ntiles = ntiles;
+  if (mode == SWR_DRAW_TRIANGLE && small_elements(c, nsub, nverts, T))
+    return end_single(c, s, small_raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, nsub, ntiles, s,
+                                               c->raster_mode != SWR_RASTER_BLOCK));
   if (mode != SWR_DRAW_TRIANGLE) return end_single(c, s, lp_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, ntiles, mode, nsub, s));
   return end_single(c, s, raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, ntiles, s, 1, 1,
                                        c->raster_mode != SWR_RASTER_BLOCK));
@@ -1243,8 +1255,8 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
   mix((uint64_t)(uintptr_t)vs); mix((uint64_t)(uintptr_t)ps);  // the programs (their kernels)
   mix((uint64_t)c->quad_mode);
   mix((uint64_t)c->persistent_geometry);
-  const bool small = n == 1 && small_front(c, P, V, T[0]);
-  mix((uint64_t)small);
+  const bool small = n == 1 && small_elements(c, P, V, T[0]), small_geo = n == 1 && small_front(c, P, V, T[0]);
+  mix((uint64_t)small); mix((uint64_t)small_geo);
   mix((uint64_t)vs->S); mix((uint64_t)ps->R); mix((uint64_t)c->tile); mix((uint64_t)n);
   mix(c->cap_prims); mix(c->cap_pairs); mix(c->cap_clip_slots); mix(c->cap_clip_verts);
   // A captured graph holds the addresses of the context's buffers: it is good until one of them
@@ -1289,7 +1301,7 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
   mark(c, 0, s);
   const AssembleArgs aa = assemble_args(c, n, c->draw_pbase.as<uint32_t>());
   c->use_draw_pbase = true;
-  if (small) {
+  if (small_geo) {
     FrontArgs fa;
     memset(&fa, 0, sizeof(fa));
     fa.staged = 1;
@@ -1301,7 +1313,6 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
     c->launches += 1;
     mark(c, 1, s);
     mark(c, 2, s);
-    rc = small_raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, (uint32_t)P, (uint32_t)NT, s, any_span);
   } else {
     const bool geo = c->persistent_geometry && B;
     if (!geo) vs->vertex(c->draws.as<SwrDrawDesc>(), n, c->draw_vbase.as<uint32_t>(), (uint32_t)V, c->ptv.as<float>(), s);
@@ -1314,9 +1325,10 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
     }
     mark(c, 2, s);
     c->launches += (V ? 1 : 0) + (B ? 2 : 0);
-    if (!q) q = cuda_err(cudaGetLastError());
-    rc = raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, (uint32_t)NT, s, n, ntg, any_span);
   }
+  if (!q) q = cuda_err(cudaGetLastError());
+  rc = small ? small_raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, (uint32_t)P, (uint32_t)NT, s, any_span)
+             : raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, (uint32_t)NT, s, n, ntg, any_span);
   if (q) rc = q;
   c->use_draw_pbase = false;
   if (c->graph_mode) {

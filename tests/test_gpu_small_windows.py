@@ -13,7 +13,7 @@ from .parity import describe, diff, oracle_render
 pytestmark = pytest.mark.gpu
 
 
-def _check(port, sc):
+def _check(port, sc, graph=False):
     from softwarerenderer_gb300.device import DeviceScene, DeviceTarget
     ref, rst = oracle_render(port, sc)
     stats = []
@@ -22,6 +22,7 @@ def _check(port, sc):
         if general:
             ds.rast.ctx.set_queue_capacity(0, 1 << 22)
             ds.rast.ctx.set_tile_slicing(0)
+        ds.rast.ctx.set_graph_mode(graph)
         st = ds.draw(tg)
         got = tg.to_host()
         assert not diff(ref, got), [describe(ref, got, k) for k in diff(ref, got)]
@@ -51,3 +52,10 @@ def test_one_tile_of_many(gpu_lib, port, ps, first):
     sc = dataclasses.replace(sc, width=1000, height=600, viewport=(0, 0, 1000, 600), scissor=(0, 0, 1000, 600),
                              vs=VS.POS_RGB_AFFINE if ps == PS.VCOLOR_AFFINE else sc.vs)
     _check(port, sc)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("n", [511, 512, 513, 1024])  # one and two half batches of geometry
+def test_clipped_half_batches(gpu_lib, port, graph, n):
+    sc = scenes.soup_scene(n, width=300, height=200, seed=n)
+    _check(port, sc, graph)
