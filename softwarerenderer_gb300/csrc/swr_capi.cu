@@ -300,17 +300,20 @@ int ensure_capacity(swr_context* c, uint32_t nverts_ptv, int S, uint32_t nsub, u
   // zero, and the last slice of a tile leaves them at zero)
   c->slices = 1;
   if (ps && ps->overwrite) {
-    const size_t px = (size_t)ntiles * c->tile * c->tile * 4;
-    if (zeroed(c->over_best, px, s) && zeroed(c->over_done, (size_t)ntiles * 4 + 16, s)) {
-      // As many as leave the grid at eight CTAs for each of four slots of the SMs, above eight
-      // slices at four: with more the slices of a tile walk what one winner of it would let them
-      // count, with fewer SMs idle.  40,960 large triangles, us in 2 / 4 / 8 / 16 / 32 slices:
-      // 16 tiles 1131 / 712 / 415 / 264 / 190, 300 tiles 450 / 300 / 226 / 214 / 225, 600 tiles
-      // 422 / 295 / 268 / 272 / 313, 1,200 tiles 413 / 353 / 357 / 397 / 494, 4,800 tiles
-      // 717 / 749 / 852 / 1114 / 1592.
-      c->slices = SWR_SLICES_MAX;
-      while (c->slices > 2 && (uint64_t)c->slices * ntiles > 152 * 4 * (c->slices > 8 ? 4 : 8)) c->slices >>= 1;
-    }
+    // As many as leave the grid at eight CTAs for each of four slots of the SMs, above eight
+    // slices at four: with more the slices of a tile walk what one winner of it would let them
+    // count, with fewer SMs idle.  40,960 large triangles, us in 2 / 4 / 8 / 16 / 32 slices:
+    // 16 tiles 1131 / 712 / 415 / 264 / 190, 300 tiles 450 / 300 / 226 / 214 / 225, 600 tiles
+    // 422 / 295 / 268 / 272 / 313, 1,200 tiles 413 / 353 / 357 / 397 / 494, 4,800 tiles
+    // 717 / 749 / 852 / 1114 / 1592.  Whole tiles against two slices, 40,960 triangles of 300 px:
+    // 2,432 tiles and fewer have slices; 2,508 tiles 555 / 626 us, 8,160 792 / 1072, 32,400
+    // 1630 / 1796.  Every slice of an empty tile is a CTA (1,500 triangles of 8 px on 65,025
+    // tiles: 108 / 173).
+    int k = SWR_SLICES_MAX;
+    while (k > 1 && (uint64_t)k * ntiles > 152 * 4 * (k > 8 ? 4 : 8)) k >>= 1;
+    if (k > 1 && zeroed(c->over_best, (size_t)ntiles * c->tile * c->tile * 4, s) &&
+        zeroed(c->over_done, (size_t)ntiles * 4 + 16, s))
+      c->slices = k;
   }
   // Depth-min shaders: the listed heavy tiles' runs (optional, like the slices above; the
   // per-slot completion counters start at zero and every merge leaves its own at zero)
