@@ -441,7 +441,7 @@ int segment_shift(uint32_t cap) {
 // cells; a tile's bin is its cells' contiguous range.  Tiles of more than SWR_RASTER_SORT
 // entries are put in primitive order by k_sort_tiles, the others by their raster CTA.
 int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, int vs_a, int vs_p,
-                 uint32_t ntiles, cudaStream_t s, int ndraws, int ntargets, bool has_span) {
+                 uint32_t ntiles, cudaStream_t s, int ndraws, int ntargets, bool has_span, bool has_block) {
   uint32_t* st = c->status.as<uint32_t>();
   const uint32_t ncells = ntiles * SWR_SEGS;
   const int seg_shift = segment_shift(c->cap_prims);
@@ -509,6 +509,7 @@ int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, i
   ra.status_w = st;
   ra.ntiles = ntiles;
   ra.has_span = has_span ? 1 : 0;
+  ra.has_block = has_block ? 1 : 0;
   ra.slices = ps->overwrite ? c->slices : 1;
   ra.best = c->over_best.as<uint32_t>();
   ra.best_done = c->over_done.as<uint32_t>();
@@ -1058,7 +1059,7 @@ int swr_draw_elements(swr_context* c, int mode, uint64_t count, const uint32_t* 
                                                c->raster_mode != SWR_RASTER_BLOCK));
   if (mode != SWR_DRAW_TRIANGLE) return end_single(c, s, lp_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, ntiles, mode, nsub, s));
   return end_single(c, s, raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, ntiles, s, 1, 1,
-                                       c->raster_mode != SWR_RASTER_BLOCK));
+                                       c->raster_mode != SWR_RASTER_BLOCK, c->raster_mode != SWR_RASTER_SPAN));
 }
 
 int swr_draw_list(swr_context* c, int mode, const float* vertices, uint64_t nverts, const int32_t* indices,
@@ -1110,7 +1111,7 @@ int swr_draw_list(swr_context* c, int mode, const float* vertices, uint64_t nver
   }
   if (mode != SWR_DRAW_TRIANGLE) return end_single(c, s, lp_stage(c, ps, ps->S, 8, 8 + ps->A, ps->A, ps->P, ntiles, mode, nsub, s));
   return end_single(c, s, raster_stage(c, ps, ps->S, 8, 8 + ps->A, ps->A, ps->P, ntiles, s, 1, 1,
-                                       c->raster_mode != SWR_RASTER_BLOCK));
+                                       c->raster_mode != SWR_RASTER_BLOCK, c->raster_mode != SWR_RASTER_SPAN));
 }
 
 int swr_set_graph_mode(swr_context* c, int on) {
@@ -1127,7 +1128,7 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
   if (!vs || !ps) return SWR_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
   std::vector<SwrDrawDesc> D(n);
-  bool any_span = false;  // some item rasterizes in Span or Adaptive mode
+  bool any_span = false, any_block = false;  // some item rasterizes in Span (Block) or Adaptive mode
   std::vector<SwrTargetDesc> T;
   std::vector<const void*> tcolor;
   std::vector<uint32_t> vbase(n), bbase(n), tbase;
@@ -1189,6 +1190,7 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
     d.cull = it.cull_mode;
     d.raster_mode = it.raster_mode;
     any_span |= it.raster_mode != SWR_RASTER_BLOCK;
+    any_block |= it.raster_mode != SWR_RASTER_SPAN;
     d.vp_px = (float)it.viewport[2] / 2.0f;
     d.vp_py = (float)it.viewport[3] / 2.0f;
     d.vp_ox = (float)it.viewport[0] + d.vp_px;
@@ -1331,7 +1333,7 @@ int swr_draw_batch(swr_context* c, const swr_draw_item* items, int n, void* stre
   }
   if (!q) q = cuda_err(cudaGetLastError());
   rc = small ? small_raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, (uint32_t)P, (uint32_t)NT, s, any_span)
-             : raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, (uint32_t)NT, s, n, ntg, any_span);
+             : raster_stage(c, ps, vs->S, 8, 8 + vs->A, vs->A, vs->P, (uint32_t)NT, s, n, ntg, any_span, any_block);
   if (q) rc = q;
   c->use_draw_pbase = false;
   if (c->graph_mode) {

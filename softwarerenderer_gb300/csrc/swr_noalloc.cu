@@ -269,6 +269,7 @@ extern "C" int swr_draw_triangle_list_noalloc(const struct SwrUniforms* u, int p
   ra.status_w = st;
   ra.ntiles = ntiles;
   ra.has_span = raster_mode != SWR_RASTER_BLOCK;
+  ra.has_block = raster_mode != SWR_RASTER_SPAN;
   ra.slices = 1;
   ra.cap_prims = kMaxTris;
   ps->raster(ra, ntiles, kTile, s);

@@ -47,11 +47,13 @@ void run_raster(const RasterArgs& a, uint32_t ntiles, int tile, cudaStream_t s) 
   if (!ntiles) return;
   if constexpr (SwrOverwrite<PS>::value) {
     if (a.boxes) {
-      swr::launch(k_overwrite<PS, 16, true>, ntiles, 256, 0, s, a);
+      swr::launch(k_overwrite<PS, 16, true, false>, ntiles, 256, 0, s, a);
     } else {
       const uint32_t grid = a.slices > 1 ? ntiles * (uint32_t)a.slices : ntiles;
-      if (tile == 32) swr::launch(k_overwrite<PS, 32, false>, grid, 256, 0, s, a);
-      else swr::launch(k_overwrite<PS, 16, false>, grid, 256, 0, s, a);
+      if (tile == 32 && a.has_block) swr::launch(k_overwrite<PS, 32, false, true>, grid, 256, 0, s, a);
+      else if (tile == 32) swr::launch(k_overwrite<PS, 32, false, false>, grid, 256, 0, s, a);
+      else if (a.has_block) swr::launch(k_overwrite<PS, 16, false, true>, grid, 256, 0, s, a);
+      else swr::launch(k_overwrite<PS, 16, false, false>, grid, 256, 0, s, a);
     }
   } else {
     if (a.boxes) {  // a small draw: 16-px tiles, one CTA each

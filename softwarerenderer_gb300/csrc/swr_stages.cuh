@@ -1316,6 +1316,7 @@ struct RasterArgs {
   uint32_t* best;                    // their pixels' winners, primitive id + 1, [tile][TILE * TILE]
   uint32_t* best_done;               // per tile: the slices finished (both zero between draws)
   int has_span;                      // some draw rasterizes in Span or Adaptive mode (selects k_raster<..., true>)
+  int has_block;                     // some draw rasterizes in Block or Adaptive mode
   // Quadrant CTAs (quad; 16-px tiles): a heavy tile -- more than three chunks of bin entries;
   // k_cells lists up to tiles.heavy_cap of them -- is rasterized by four CTAs, one per 8 x 8
   // quadrant, each walking the whole bin for its own pixels, so the slowest tiles no longer
@@ -1454,13 +1455,15 @@ __device__ __forceinline__ void block_runs(const float* r, int flags, int cls, i
   for (int y = by; y < yhi; ++y) {
     uint32_t m = (1u << wx) - 1u;
     if (cls == 2) {
-      float c0 = i0, c1 = i1, c2 = i2;
+      if (y >= ylo) {
+        float c0 = i0, c1 = i1, c2 = i2;
 #pragma unroll
-      for (int col = 0; col < SWR_BLOCK; ++col) {
-        if (!(c0 >= t0 && c1 >= t1 && c2 >= t2)) m &= ~(1u << col);
-        c0 = swr_add(c0, r[6]);
-        c1 = swr_add(c1, r[9]);
-        c2 = swr_add(c2, r[12]);
+        for (int col = 0; col < SWR_BLOCK; ++col) {
+          if (!(c0 >= t0 && c1 >= t1 && c2 >= t2)) m &= ~(1u << col);
+          c0 = swr_add(c0, r[6]);
+          c1 = swr_add(c1, r[9]);
+          c2 = swr_add(c2, r[12]);
+        }
       }
       i0 = swr_add(i0, r[7]);
       i1 = swr_add(i1, r[10]);
@@ -2372,7 +2375,7 @@ __global__ void __launch_bounds__(NT, SWR_RASTER_MINB ? SWR_RASTER_MINB
 // (four, with all the registers wanted: 354 us a draw, five 333).  The 40,960 triangles of the
 // reference's Benchmark program (640x480, 240M fragments): bins ordered and walked in
 // 64-primitive chunks pixel by pixel, 1888 us a draw; this way 333.
-template <class PS, int TILE, bool DIRECT>
+template <class PS, int TILE, bool DIRECT, bool MASKS>
 __global__ void __launch_bounds__(256, 5) k_overwrite(RasterArgs g) {
   swr_pdl_entry();
   typedef Rec<PS> RL;
@@ -2385,6 +2388,10 @@ __global__ void __launch_bounds__(256, 5) k_overwrite(RasterArgs g) {
   __shared__ uint32_t slast;
   constexpr uint32_t OVB = 1024;  // entries classified at a time
   __shared__ uint32_t swalk[OVB], snwalk;
+  // light tiles with Block primitives: their coverage masks, as k_raster's
+  constexpr int NBX = TILE / SWR_BLOCK, NB = NBX * NBX;
+  constexpr uint32_t LIGHT = 32;
+  __shared__ uint64_t smask[MASKS ? LIGHT * NB : 1];
   // the draw's queue requests are final (nothing after this stage counts)
   if (blockIdx.x == 0 && threadIdx.x == 0 && !DIRECT) swr_close_status(g.status_w);
   if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
@@ -2437,8 +2444,9 @@ __global__ void __launch_bounds__(256, 5) k_overwrite(RasterArgs g) {
   __syncthreads();
   uint32_t smin = 0;  // no pixel's winner is below it
   uint32_t frags = 0;
-  // rows [r0, r1) of the tile, primitive p
-  auto cover = [&](uint32_t p, int r0, int r1) {
+  // Part `part` of 2^lp of primitive p in the tile: a share of the rows, in Block mode block after
+  // block.
+  auto cover = [&](uint32_t p, int part, int lp, bool span_only = false) {
     const float4* rc = (const float4*)(g.recs + (size_t)p * RL::R);
     const float4 q0 = __ldg(rc), q1 = __ldg(rc + 1), q2 = __ldg(rc + 2), q3 = __ldg(rc + 3), q4 = __ldg(rc + 4);
     const int flags = __float_as_int(q0.x);
@@ -2455,21 +2463,25 @@ __global__ void __launch_bounds__(256, 5) k_overwrite(RasterArgs g) {
         atomicAdd(&scnt[row * (TILE + 1) + xb - ox], -1);
       }
     };
-    const int y0 = oy + r0, y1 = min(oy + r1, yend);
     if (!(flags & 2)) {
+      const int rows = TILE >> lp, y0 = oy + part * rows, y1 = min(y0 + rows, yend);
       const SwrDrawDesc& D = g.draws[__float_as_int(q0.y)];
       span_runs(q0, q1, q2, q3, q4, D.sc_minx, D.sc_maxx, ox, xend, y0, y1,
                 [&](int y, int xa, int xb, int) { run(y, xa, xb); });
       return;
     }
+    if (span_only) return;
     const float r[15] = {0, 0, 0, 0, 0, 0, q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, q3.x, q3.y, q3.z};
-    const int bx0 = __float_as_int(q0.z), bx1 = __float_as_int(q1.x);
-    const int ylo = max(__float_as_int(q0.w), y0), yhi = min(__float_as_int(q1.y) + 1, y1);
-    for (int by = ylo & ~(SWR_BLOCK - 1); by < yhi; by += SWR_BLOCK)
-      for (int bx = max(bx0 & ~(SWR_BLOCK - 1), ox); bx <= bx1 && bx < xend; bx += SWR_BLOCK) {
-        const int cls = block_class(r, flags, bx, by);
-        if (cls) block_runs(r, flags, cls, bx, by, min(SWR_BLOCK, xend - bx), ylo, min(by + SWR_BLOCK, yhi), run);
-      }
+    constexpr int ROWS = SWR_BLOCK * NB;  // the blocks' rows, block by block
+    for (int h = part * (ROWS >> lp), he = h + (ROWS >> lp); h < he;) {
+      const int j = h / SWR_BLOCK, r0 = h % SWR_BLOCK, r1 = min(r0 + he - h, SWR_BLOCK);
+      h += r1 - r0;
+      const int bx = ox + (j % NBX) * SWR_BLOCK, by = oy + (j / NBX) * SWR_BLOCK;
+      const int ylo = max(by + r0, __float_as_int(q0.w)), yhi = min(min(by + r1, __float_as_int(q1.y) + 1), yend);
+      if (ylo >= yhi || bx >= xend || bx > __float_as_int(q1.x) || bx + SWR_BLOCK - 1 < __float_as_int(q0.z)) continue;
+      const int cls = block_class(r, flags, bx, by);
+      if (cls) block_runs(r, flags, cls, bx, by, min(SWR_BLOCK, xend - bx), ylo, yhi, run);
+    }
   };
   int round = 0;
   auto raise_smin = [&]() {  // (uniform)
@@ -2542,12 +2554,75 @@ __global__ void __launch_bounds__(256, 5) k_overwrite(RasterArgs g) {
         }
     return false;
   };
-  // rows per item: see above (n * groups items in all)
-  const int shift = n >= 128u ? 0 : (n >= 32u ? 2 : (TILE == 16 ? 4 : 5));
-  const int rows = TILE >> shift;
+  // parts of a primitive: see above (n << shift items in all)
+  const int shift = n >= 128u ? 0 : (n >= 32u ? 2 : n >= 16u ? (TILE == 16 ? 3 : 4) : (TILE == 16 ? 4 : 5));
   const uint32_t* bin = g.bin_raw ? g.bin_raw : g.bin;
   const uint64_t items = (uint64_t)n << shift;
-  if (shift == 0) {
+  if (MASKS && (!g.has_span || n < 400u)) {
+    // Block primitives by masks, LIGHT at a time: one thread per (primitive, block) classifies it,
+    // one per half of a partially covered block steps its rows, and each pixel takes the largest of
+    // the ids covering it.  Scattered by their rows like Span primitives, lanes at skipped, whole
+    // and partial blocks waited for each other: 40,960 triangles of 60 px, us a draw so / this
+    // way: 640x480 510 / 225, 1920x1080 468 / 229, 3840x2160 1222 / 343, 4080x4080 1756 / 516.
+    // Tiles of more entries in a draw that has Span primitives too scatter both, since those only
+    // count once every pixel's winner is known (40,960 triangles of 300 px in Adaptive mode at
+    // 640x480: 1760, all by masks 2490).
+    if (g.has_span)
+      for (uint32_t t = (uint32_t)tid; t < n << shift; t += 256)
+        cover(bin[hi - 1u - (t >> shift)], (int)(t & ((1u << shift) - 1u)), shift, true);
+    for (uint32_t base = 0; base < n; base += LIGHT) {
+      const uint32_t m = min(LIGHT, n - base);
+      __syncthreads();  // the previous masks and ids are no longer read; Span's winners are written
+      if (tid == 0) snwalk = 0u;
+      if ((uint32_t)tid < m) swalk[tid] = bin[hi - 1u - (base + (uint32_t)tid)];
+      __syncthreads();
+      auto block_of = [&](uint32_t t, int& bx, int& by) -> const float* {
+        const int j = (int)(t % NB);
+        bx = ox + (j % NBX) * SWR_BLOCK;
+        by = oy + (j / NBX) * SWR_BLOCK;
+        return g.recs + (size_t)swalk[t / NB] * RL::R;
+      };
+      for (uint32_t t = (uint32_t)tid; t < m * NB; t += 256) {
+        int bx, by;
+        const float* r = block_of(t, bx, by);
+        const float4 q0 = __ldg((const float4*)r), q1 = __ldg((const float4*)r + 1);
+        const int flags = __float_as_int(q0.x);
+        int cls = 0;
+        if ((flags & 3) == 3 && bx <= __float_as_int(q1.x) && bx + SWR_BLOCK - 1 >= __float_as_int(q0.z) &&
+            by <= __float_as_int(q1.y) && by + SWR_BLOCK - 1 >= __float_as_int(q0.w))
+          cls = block_class(r, flags, bx, by);
+        smask[t] = cls == 1 ? ~0ull : 0ull;
+        if (cls == 2) swalk[LIGHT + atomicAdd(&snwalk, 1u)] = t;
+      }
+      __syncthreads();
+      const uint32_t halves = 2u * snwalk;
+      for (uint32_t h = (uint32_t)tid; h < halves; h += 256) {
+        int bx, by;
+        const uint32_t t = swalk[LIGHT + (h >> 1)];
+        const float* r = block_of(t, bx, by);
+        ((uint32_t*)&smask[t])[h & 1u] = block_rows_bits(r, __float_as_int(r[0]), bx, by, (int)(h & 1u));
+      }
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < PPT; ++q) {
+        const int reg = q * 8 + warp, sub = reg >> 3, hb = (reg & 7) >> 1;  // the warp's half block (raster_tile)
+        const int lx = (sub % (TILE / 16)) * 16 + (hb & 1) * 8 + (lane & 7);
+        const int ly = (sub / (TILE / 16)) * 16 + (hb >> 1) * 8 + (reg & 1) * 4 + (lane >> 3);
+        const int blk = (ly >> 3) * NBX + (lx >> 3);
+        uint32_t cov = warp_transpose((uint32_t)lane < m ? (uint32_t)(smask[lane * NB + blk] >> ((reg & 1) * 32)) : 0u, lane);
+        if (ox + lx >= xend || oy + ly >= yend || !cov) continue;
+        const uint32_t c = (uint32_t)__popc(cov);
+        frags += c;
+        uint32_t b = sbest[ly * TILE + lx];
+        for (; cov; cov &= cov - 1u) b = max(b, swalk[__ffs(cov) - 1] + 1u);
+        sbest[ly * TILE + lx] = b;
+        if (counts) {
+          uint32_t* fc = U.frag_count + (size_t)(oy + ly) * (size_t)U.width + (size_t)(ox + lx);
+          if (nsl > 1) atomicAdd(fc, c); else *fc += c;
+        }
+      }
+    }
+  } else if (shift == 0) {
     for (uint32_t base = 0; base < n; ++round) {
       const uint32_t m = min(n - base, round < 3 ? 256u : OVB);
       __syncthreads();  // the previous list is no longer read
@@ -2565,9 +2640,10 @@ __global__ void __launch_bounds__(256, 5) k_overwrite(RasterArgs g) {
       }
       __syncthreads();
       // four rows an item; few primitives of a small draw's window: one
-      const uint32_t per = DIRECT && snwalk < 32u ? 1u : 4u, G = TILE / per, work = snwalk * G;
-      for (uint32_t t = (uint32_t)tid; t < work; t += 256)
-        cover(swalk[t / G], (int)(t % G * per), (int)(t % G * per + per));
+      constexpr int LT = TILE == 16 ? 4 : 5;
+      const int lp = DIRECT && snwalk < 32u ? LT : LT - 2;
+      const uint32_t work = snwalk << lp;
+      for (uint32_t t = (uint32_t)tid; t < work; t += 256) cover(swalk[t >> lp], (int)(t & ((1u << lp) - 1u)), lp);
       base += m;
       // (a later, larger bound would save little; nothing was walked: there is no larger one)
       if (round < 3 && base < n && snwalk) raise_smin();
@@ -2577,12 +2653,12 @@ __global__ void __launch_bounds__(256, 5) k_overwrite(RasterArgs g) {
     const uint64_t it = base + (uint64_t)tid;
     if (it < items) {
       const uint32_t k = (uint32_t)(it >> shift);
-      const int r0 = (int)((uint32_t)it & ((1u << shift) - 1u)) * rows;
+      const int part = (int)((uint32_t)it & ((1u << shift) - 1u));
       if constexpr (DIRECT) {
         const uint32_t p = n - 1u - k;
-        if (swr_box_hit(g.boxes[p], tx, ty)) cover(p, r0, r0 + rows);
+        if (swr_box_hit(g.boxes[p], tx, ty)) cover(p, part, shift);
       } else {
-        cover(bin[hi - 1u - k], r0, r0 + rows);
+        cover(bin[hi - 1u - k], part, shift);
       }
     }
     if (round < 3 && base + 256 < items) raise_smin();
