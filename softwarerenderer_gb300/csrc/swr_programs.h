@@ -712,7 +712,7 @@ SWR_HD void swr_depth_merge(SwrStateRGBA8& acc, const SwrStateRGBA8& later) {
 }
 
 // Resident tile-raster CTAs per SM the register allocation of a shader's k_raster must
-// allow: RasterOccupancy in the shader (default 4), and RasterOccupancyBlock for submissions
+// allow on 16-px tiles: RasterOccupancy in the shader (default 4), and RasterOccupancyBlock for submissions
 // of Block-mode draws alone where that differs.  Measured per workload, whole draws at 4 / 5 /
 // 6 / 7 CTAs per SM: vertex colour (4K soup) 4401 / 4217 / 4339 / 4569 us; Lambert (dense
 // 1080p mesh) 119.7 / 115.6 / 112.7 / 120.2; Lambert-textured in Block mode (256 meshes) 3914 /

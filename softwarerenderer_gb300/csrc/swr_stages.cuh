@@ -2324,8 +2324,13 @@ __device__ __forceinline__ bool raster_tile(const RasterArgs& g, uint32_t bid) {
   return true;
 }
 
+// (32-px tiles: four pixels a thread want the registers of four CTAs per SM, whatever the shader.
+// Planned for as many as 16-px tiles, the Lambert, Lambert-textured and differentiable shaders
+// spilled: 2,000 triangles of 300 px at 640x480 in Adaptive mode, Lambert-textured, 1042 us a draw
+// with six CTAs, 773 with four.)
 template <class PS, int TILE, int CH, bool SPAN, bool DIRECT = false, int NT = 256>
 __global__ void __launch_bounds__(NT, SWR_RASTER_MINB ? SWR_RASTER_MINB
+                                       : TILE == 32      ? 4
                                        : SPAN            ? SwrRasterOccupancy<PS>::value
                                                          : SwrRasterOccupancy<PS>::block * (256 / NT))
     k_raster(RasterArgs g) {
@@ -2381,6 +2386,7 @@ __global__ void __launch_bounds__(256, 5) k_overwrite(RasterArgs g) {
   typedef Rec<PS> RL;
   constexpr int PPT = TILE * TILE / 256;
   static_assert(RL::R >= 20, "words 0-19 of a record are read as five float4s");
+  static_assert(PPT == 1 || TILE * TILE <= 1024, "a tile's pixels are listed in swalk");
   __shared__ uint32_t sbest[TILE * TILE];      // per pixel: winner's id + 1
   __shared__ int scnt[TILE * (TILE + 1)];      // per row: +1 at a run's first pixel, -1 past its last
   __shared__ uint32_t sred[8];
@@ -2388,7 +2394,7 @@ __global__ void __launch_bounds__(256, 5) k_overwrite(RasterArgs g) {
   __shared__ uint32_t slast;
   constexpr uint32_t OVB = 1024;  // entries classified at a time
   __shared__ uint32_t swalk[OVB], snwalk;
-  // light tiles with Block primitives: their coverage masks, as k_raster's
+  // Block primitives' coverage masks, as k_raster's, LIGHT primitives at a time
   constexpr int NBX = TILE / SWR_BLOCK, NB = NBX * NBX;
   constexpr uint32_t LIGHT = 32;
   __shared__ uint64_t smask[MASKS ? LIGHT * NB : 1];
@@ -2701,12 +2707,39 @@ __global__ void __launch_bounds__(256, 5) k_overwrite(RasterArgs g) {
     }
     if (tid == 0) g.best_done[tile] = 0u;
   }
+  // A thread's pixels are shaded one after the other: where it has several, the tile's winners are
+  // first dealt out over the CTA (few of a tile's pixels may have one).
+  uint32_t shade = PPT;
+  if constexpr (PPT > 1) {
+    __syncthreads();  // swalk and sbest are no longer read
+    if (tid == 0) snwalk = 0u;
+    __syncthreads();
 #pragma unroll
-  for (int q = 0; q < PPT; ++q) {
-    const int i = q * 256 + tid;
+    for (int q = 0; q < PPT; ++q) {
+      const int i = q * 256 + tid;
+      const bool on = best[q] && ox + i % TILE < xend && oy + i / TILE < yend;
+      const uint32_t bal = __ballot_sync(0xffffffffu, on);
+      uint32_t at = 0;
+      if (lane == 0 && bal) at = atomicAdd(&snwalk, (uint32_t)__popc(bal));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (on) swalk[at + (uint32_t)__popc(bal & ((1u << lane) - 1u))] = (uint32_t)i;
+      sbest[i] = best[q];
+    }
+    __syncthreads();
+    shade = (snwalk + 255u) / 256u;
+  }
+  for (uint32_t q = 0; q < shade; ++q) {
+    int i = tid;
+    uint32_t b = best[0];
+    if constexpr (PPT > 1) {
+      const uint32_t t = q * 256u + (uint32_t)tid;
+      if (t >= snwalk) break;
+      i = (int)swalk[t];
+      b = sbest[i];
+    }
     const int x = ox + i % TILE, y = oy + i / TILE;
-    if (!best[q] || x >= xend || y >= yend) continue;
-    const uint32_t p = best[q] - 1u;
+    if (!b || x >= xend || y >= yend) continue;
+    const uint32_t p = b - 1u;
     const float* r = g.recs + (size_t)p * RL::R;
     GpuPixel<PS> pd;
     pd.z = 0.0f;  // (no depth: SwrOverwrite)
