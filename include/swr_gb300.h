@@ -37,7 +37,9 @@ extern "C" {
 /* Status codes. */
 #define SWR_OK 0
 #define SWR_EINVAL 1     /* invalid argument (the reference asserts or has undefined behaviour) */
-#define SWR_ENOMEM 2     /* device allocation failed */
+#define SWR_ENOMEM 2     /* device allocation failed, or (swr_finish) a draw asked for more bin entries
+                            or fragments than a queue can have (2^32 with the room for growth): it
+                            left its targets untouched, and would again */
 #define SWR_EOVERFLOW 3  /* a scratch queue was too small: the draw left its targets untouched,
                             the context has grown the queue; issue the draw again */
 #define SWR_ECUDA 4      /* CUDA runtime error */

@@ -1375,12 +1375,12 @@ int swr_finish(swr_context* c, void* stream, swr_stats* stats) {
   c->launches = 0;
   const uint32_t flags = h[SWR_ST_FLAGS];
   if (flags & SWR_F_ANY_OVERFLOW) {
-    grow_u32(c->cap_clip_slots, h[kStickyBase + SWR_ST_CLIP_SLOTS]);
-    grow_u32(c->cap_clip_verts, h[kStickyBase + SWR_ST_CLIP_VERTS]);
-    grow_u32(c->cap_prims, h[kStickyBase + SWR_ST_PRIMS]);
-    grow_u32(c->cap_pairs, h[kStickyBase + SWR_ST_PAIRS]);
+    bool can = grow_u32(c->cap_clip_slots, h[kStickyBase + SWR_ST_CLIP_SLOTS]);
+    can &= grow_u32(c->cap_clip_verts, h[kStickyBase + SWR_ST_CLIP_VERTS]);
+    can &= grow_u32(c->cap_prims, h[kStickyBase + SWR_ST_PRIMS]);
+    can &= grow_u32(c->cap_pairs, h[kStickyBase + SWR_ST_PAIRS]);
+    return can ? SWR_EOVERFLOW : SWR_ENOMEM;  // (ENOMEM: the draw would overflow again)
   }
-  if (flags & SWR_F_ANY_OVERFLOW) return SWR_EOVERFLOW;
   if (flags & SWR_F_BARRIER_TIMEOUT) return SWR_ECUDA;
   if (flags & (SWR_F_BAD_INDEX | SWR_F_BAD_GRAD_INPUT)) return SWR_EINDEX;
   if (flags & SWR_F_SRC_OVERFLOW) return SWR_EINVAL;
