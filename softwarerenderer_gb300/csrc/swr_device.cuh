@@ -27,7 +27,7 @@ enum SwrStatusWord {
   SWR_ST_CLIP_VERTS = 2,  // clip vertices requested
   SWR_ST_PRIMS = 3,       // primitives after clipping and culling
   SWR_ST_PAIRS = 4,       // (tile, primitive) pairs requested
-  SWR_ST_FRAGS = 5,       // line/point fragments requested
+  SWR_ST_FRAGS = 5,       // line/point fragments inside the target
   SWR_ST_SHADED_LO = 6,   // drawPixel calls (64-bit, low word)
   SWR_ST_SHADED_HI = 7,
   SWR_ST_WORDS = 8,

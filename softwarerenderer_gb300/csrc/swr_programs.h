@@ -655,8 +655,8 @@ struct SwrOverwrite<PS, decltype((void)PS::Overwrite)> {
 // may therefore count, without interpolating, every fragment of a primitive whose z is
 // provably not below the largest depth held by the pixels it covers.  A shader may opt out
 // with DepthCull = 0.  The Lambert and differentiable shaders do: their single-mesh workloads
-// have nothing to cull, and the cull's code takes registers from rasters that run at 6-7 CTAs
-// per SM.
+// have nothing to cull, and the cull's code takes registers from rasters planned for 6 CTAs of
+// 256 threads (or 12 of 128) per SM.
 template <class PS, class = void>
 struct SwrDepthCull {
   enum { value = PS::HasDepth && PS::InterpolateZ && !SwrOverwrite<PS>::value };
