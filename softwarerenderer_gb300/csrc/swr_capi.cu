@@ -416,15 +416,15 @@ SwrTiles tiles_of(const swr_context* c, uint32_t ntiles, uint32_t heavy_cap) {
   return t;
 }
 
-void sort_tiles(swr_context* c, const SwrTiles& t, int seg_shift, uint32_t cell_min, const uint32_t* in, uint32_t* out,
-                cudaStream_t s) {
+void sort_tiles(swr_context* c, const SwrTiles& t, int seg_shift, uint32_t cell_min, uint32_t all_min, const uint32_t* in,
+                uint32_t* out, cudaStream_t s) {
   // bytes of one warp's bitmap: the segment's range, where one fits; else an eighth for each of
   // eight warps (a window of a segment costs a warp the same per id as a range that fits)
   const size_t range = std::max<size_t>(((size_t)1 << seg_shift) / 8, 4);
   const size_t bm = range <= kSortSmem ? range : kSortSmem / 8;
   const int warps = (int)std::min<size_t>(8, kSortSmem / bm);
   swr::launch(k_sort_tiles, kSortWarps / warps, 32 * warps, warps * bm, s, c->status.as<uint32_t>(), t, seg_shift,
-              (uint32_t)(bm / 4), cell_min, in, out);
+              (uint32_t)(bm / 4), cell_min, all_min, in, out);
   c->launches += 1;
 }
 
@@ -494,7 +494,7 @@ int raster_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, i
                 cells, seg_shift, c->cap_pairs, c->draws.as<SwrDrawDesc>(), c->targets.as<SwrTargetDesc>(), c->tile,
                 c->keys0.as<uint32_t>(), st, s);
   if (!ps->overwrite)  // (k_overwrite takes the bins as they are)
-    sort_tiles(c, ca.t, seg_shift, 0, c->keys0.as<uint32_t>(), c->vals0.as<uint32_t>(), s);
+    sort_tiles(c, ca.t, seg_shift, 0, 0, c->keys0.as<uint32_t>(), c->vals0.as<uint32_t>(), s);
   mark(c, 4, s);
   RasterArgs ra;
   memset(&ra, 0, sizeof(ra));
@@ -659,8 +659,8 @@ int lp_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, int v
   ca.cells = cells;
   ca.fill_start = c->cell_fill.as<uint32_t>();
   ca.total = st + SWR_ST_FRAGS;  // fragments in the target
-  ca.t = tiles_of(c, ntiles, 0);
-  ca.heavy_min = 0xffffffffu;
+  ca.t = tiles_of(c, ntiles, std::min<uint32_t>(quad_cap(ntiles), SWR_LP_SLOTS));
+  ca.heavy_min = SWR_LP_HEAVY;
   ca.sort_min = SWR_LP_CHUNK;
   ca.front_min = 2 * SWR_LP_CHUNK;
   ca.target_tile_base = nullptr;
@@ -670,7 +670,7 @@ int lp_stage(swr_context* c, const PsOps* ps, int S, int off_a, int off_p, int v
   swr::launch(k_lp_fill, want < 1216u ? (want ? want : 1u) : 1216u, 256, 0, s, st, st + SWR_ST_PAIRS, c->cap_pairs,
               c->keys0.as<uint32_t>(), c->cell_count.as<uint32_t>(), ca.fill_start, cells, seg_shift,
               c->keys1.as<uint32_t>());
-  sort_tiles(c, ca.t, seg_shift, SWR_LP_CHUNK, c->keys1.as<uint32_t>(), c->vals1.as<uint32_t>(), s);
+  sort_tiles(c, ca.t, seg_shift, SWR_LP_CHUNK, SWR_LP_HEAVY, c->keys1.as<uint32_t>(), c->vals1.as<uint32_t>(), s);
   mark(c, 4, s);
   LpRasterArgs ra;
   ra.status = st;

@@ -235,6 +235,9 @@ __device__ __forceinline__ float lp_value(const float* rec, int i, int j) {
 #define SWR_LP_TILE 16                // tile edge of the point / line bins (one pixel per thread)
 #define SWR_LP_CHUNK 256              // fragments per raster chunk (one per thread)
 #define SWR_LP_INVALID 0xffffffffu    // key of a fragment that reaches no target pixel
+#define SWR_LP_HEAVY 4096             // tiles of more fragments are rasterized by SWR_LP_PARTS CTAs,
+#define SWR_LP_PARTS 4                // each for its quarter of the tile's rows,
+#define SWR_LP_SLOTS 64               // this many tiles at most
 
 struct LpFragArgs {
   const uint32_t* status;
@@ -412,6 +415,154 @@ __device__ __forceinline__ void lp_words(GpuPixel<PS>& pd, F f) {
   for (int a = 0; a < PS::PVarCount; ++a) f(1 + PW::W + PS::AVarCount + a, pd.pvar[a]);
 }
 
+// Rasterizer::pixelDataFromVertex (Rasterizer.h:161-173) of step j of a primitive's record.
+template <class PS>
+__device__ __forceinline__ void lp_pixel(const float* rec, int j, int fx, int fy, GpuPixel<PS>& pd) {
+  typedef LpRec<PS> RL;
+  pd.x = fx;
+  pd.y = fy;
+  pd.eq = nullptr;  // points and lines carry no triangle equations
+  pd.z = 0.0f;
+  if (PS::InterpolateZ) pd.z = lp_value<PS>(rec, 2, j);
+  if (PS::InterpolateW) {
+    pd.w = lp_value<PS>(rec, 3, j);
+    pd.invw = swr_div(1.0f, pd.w);
+  }
+  for (int a = 0; a < RL::NA; ++a) pd.avar[a] = lp_value<PS>(rec, 4 + a, j);
+  for (int a = 0; a < RL::NP; ++a) pd.pvar[a] = lp_value<PS>(rec, 4 + RL::NA + a, j);
+}
+
+// A quarter of the rows of a heavy tile, whose cells are all ordered: the CTA looks through the
+// tile's fragments 512 at a time, keeps those of its rows, in order, and rasterizes them in chunks
+// as k_lp_raster does, its first 64 threads owning the pixels.  A chunk is a chain of a few
+// microseconds however few pixels it is for, and one CTA had all of a tile's: 10,000 lines inside
+// one tile, 80,000 fragments, took 1811 us in the raster, four CTAs 870; 100,000 points 959 and 432.
+// Tiles of fewer fragments have most cells within a chunk, and ordering those ahead costs more
+// than this gains (1M points on a sphere 213 us a draw, 278 with the line at 2,048).
+// The lists lie where the other tiles' masks do: more shared memory is less cache for all.
+struct LpHeavy {
+  enum { FIND = 512, CH = SWR_LP_CHUNK, PART = 256 / SWR_LP_PARTS };
+  uint32_t mask[CH / 32][PART];  // per pixel: the chunk's fragments that hit it
+  uint32_t f[FIND];              // the finds: fragment number
+  uint8_t pix[FIND];             // and pixel, from the first row's first
+  uint32_t count[FIND / 32];
+};
+
+template <class PS, class Shared>
+__device__ __forceinline__ uint2 lp_heavy_rows(const LpRasterArgs& g, uint4 entry, int first, Shared& sh) {
+  typedef LpHeavy H;
+  static_assert(sizeof(H) <= sizeof(sh.mask), "the lists fit the masks' place");
+  H& h = *(H*)sh.mask;
+  const uint32_t tile = entry.x, b = entry.y, total = entry.z - entry.y;
+  const SwrDrawDesc& D = g.draws[0];
+  const SwrTargetDesc& T = g.targets[D.target];
+  const SwrUniforms& U = D.u;
+  const uint32_t W = (uint32_t)lp_stride<PS>(D.draw_mode);
+  const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ox = (int)(tile % (uint32_t)T.tiles_x) * SWR_LP_TILE;
+  const int oy = (int)(tile / (uint32_t)T.tiles_x) * SWR_LP_TILE + first / SWR_LP_TILE;
+  const int x = ox + tid % SWR_LP_TILE, y = oy + tid / SWR_LP_TILE;
+  const bool in = tid < H::PART && x < T.width && y < T.height;
+  uint32_t frags = 0;
+  typename PS::State st;
+  if (in) PS::load(st, x, y, U);
+  for (uint32_t base = 0; base < total; base += H::FIND) {
+    constexpr int R = H::FIND / H::CH;
+    uint32_t f[R], key[R], bal[R];
+    __syncthreads();  // the previous finds are no longer read
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const uint32_t i = base + (uint32_t)(r * H::CH + tid);
+      f[r] = i < total ? g.bin[b + i] : 0u;
+      key[r] = i < total ? (g.keys[f[r]] & 255u) - (uint32_t)first : 256u;
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      bal[r] = __ballot_sync(0xffffffffu, key[r] < (uint32_t)H::PART);
+      if (lane == 0) h.count[r * (H::CH / 32) + warp] = (uint32_t)__popc(bal[r]);
+    }
+    __syncthreads();
+    static_assert(R * (H::CH / 32) <= 32, "one count per lane");
+    const uint32_t cnt = lane < R * (H::CH / 32) ? h.count[lane] : 0u;
+    uint32_t inc = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    const int m = (int)__shfl_sync(0xffffffffu, inc, 31);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const uint32_t at = __shfl_sync(0xffffffffu, inc - cnt, r * (H::CH / 32) + warp) +
+                          (uint32_t)__popc(bal[r] & ((1u << lane) - 1u));
+      if (key[r] < (uint32_t)H::PART) {
+        h.f[at] = f[r];
+        h.pix[at] = (uint8_t)key[r];
+      }
+    }
+    for (int c0 = 0; c0 < m; c0 += H::CH) {
+      const int n = min((int)H::CH, m - c0), words = (n + 31) / 32;
+      if (tid < H::PART)
+        for (int w = 0; w < words; ++w) h.mask[w][tid] = 0u;
+      __syncthreads();
+      if (tid < n) {
+        const uint32_t fr = h.f[c0 + tid], prim = g.prims[fr];
+        const int pix = h.pix[c0 + tid], j = D.draw_mode == 0 ? 0 : (int)(fr - g.frag_off[prim]);
+        sh.put(tid, g.recs + (size_t)prim * W, prim, j, ox + pix % SWR_LP_TILE, oy + pix / SWR_LP_TILE, U);
+        atomicOr(&h.mask[tid >> 5][pix], 1u << (tid & 31));
+      }
+      __syncthreads();
+      if (in)
+        for (int w = 0; w < words; ++w)
+          for (uint32_t s = h.mask[w][tid]; s; s &= s - 1u) {
+            frags++;
+            sh.take(w * 32 + __ffs(s) - 1, x, y, st, U);
+          }
+      __syncthreads();  // the chunk is no longer read
+    }
+  }
+  if (!in || !frags) return make_uint2(0u, 0u);
+  PS::store(st, x, y, U);
+  return make_uint2(frags, st.writes);  // (fragments and writes)
+}
+
+// A chunk's fragments in shared memory.
+template <class PS>
+struct LpChunk {
+  enum { CH = SWR_LP_CHUNK, CW = CH / 32, COMPACT = !SwrNoCompact<PS>::value };
+  uint32_t mask[CW][256];  // per pixel: the chunk's fragments that hit it
+  uint32_t prim[CH];
+  float z[COMPACT ? CH : 1];
+  typename PS::Color color[COMPACT ? CH : 1];
+  float words[COMPACT ? 1 : LpPixelWords<PS>::value * CH];  // shaders with side effects: interpolated, not shaded
+  // Interpolates (and shades) step j of a primitive as the k-th fragment ...
+  __device__ __forceinline__ void put(int k, const float* rec, uint32_t p, int j, int fx, int fy, const SwrUniforms& U) {
+    prim[k] = p;
+    GpuPixel<PS> pd;
+    if constexpr (COMPACT) {
+      lp_pixel<PS>(rec, j, fx, fy, pd);
+      z[k] = pd.z;
+      color[k] = PS::shade(pd, U);
+    } else {
+      lp_pixel<PS>(rec, j, 0, 0, pd);
+      lp_words<PS>(pd, [&](int i, float& v) { words[i * CH + k] = v; });
+    }
+  }
+  // ... and applies it to the pixel (x, y) it hits.
+  __device__ __forceinline__ void take(int k, int x, int y, typename PS::State& st, const SwrUniforms& U) {
+    if constexpr (COMPACT) {
+      PS::apply(st, z[k], color[k], (int)prim[k]);
+    } else {
+      GpuPixel<PS> pd;
+      pd.x = x;
+      pd.y = y;
+      pd.eq = nullptr;  // points and lines carry no triangle equations
+      lp_words<PS>(pd, [&](int i, float& v) { v = words[i * CH + k]; });
+      PS::drawPixel(pd, (int)prim[k], st, U);
+    }
+  }
+};
+
 // One CTA per 16 x 16 tile, one pixel per thread.  A chunk is as many whole cells of the
 // tile's bin as hold at most 256 fragments (a larger cell, ordered by k_sort_tiles, is a run of
 // chunks by itself): one fragment per thread is ranked inside its cell, interpolated, shaded
@@ -424,25 +575,34 @@ __device__ __forceinline__ void lp_words(GpuPixel<PS>& pd, F f) {
 // 17 to 64 entries, a bitmap above) took the two sorts from 184 to 4 us on the points and
 // from 64 to 4 us on the lines.
 template <class PS>
-__global__ void __launch_bounds__(256) k_lp_raster(LpRasterArgs g) {
+__global__ void __launch_bounds__(256) k_lp_raster(const __grid_constant__ LpRasterArgs g) {
   swr_pdl_entry();
-  typedef LpRec<PS> RL;
-  typedef typename PS::Color Color;
-  constexpr bool kCompact = !SwrNoCompact<PS>::value;
-  constexpr int CH = SWR_LP_CHUNK, CW = CH / 32;
+  constexpr int CH = SWR_LP_CHUNK;
   static_assert(CH == 256 && SWR_SEGS == 32, "one fragment per thread, one cell per lane");
   __shared__ uint32_t sraw[CH];
   __shared__ uint32_t scs[SWR_SEGS + 1];
-  __shared__ uint32_t smask[CW][256];  // per pixel: the chunk's fragments that hit it
-  __shared__ uint32_t sprim[CH];
-  __shared__ float sz[kCompact ? CH : 1];
-  __shared__ Color sc[kCompact ? CH : 1];
-  __shared__ float spd[kCompact ? 1 : LpPixelWords<PS>::value * CH];  // others: interpolated, not shaded
+  __shared__ LpChunk<PS> sh;
   __shared__ uint32_t sfr[64];
   if (blockIdx.x == 0 && threadIdx.x == 0) swr_close_status(g.status_w);
   if (g.status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
   uint4 entry;
-  if (!swr_listed_tile(g.tiles, blockIdx.x, entry)) return;
+  auto report = [&](uint32_t frags, uint32_t passes) {
+    uint32_t tot, ptot;
+    swr_block_sum2(frags, passes, sfr, tot, ptot);
+    if (threadIdx.x == 0 && tot) {
+      atomicAdd((unsigned long long*)&g.status_w[SWR_ST_SHADED_LO], (unsigned long long)tot);
+      atomicAdd((unsigned long long*)&g.status_w[SWR_ST_PASSES_LO], (unsigned long long)ptot);
+    }
+  };
+  const uint32_t nheavy = SWR_LP_PARTS * g.tiles.heavy_cap;
+  if (blockIdx.x < nheavy) {
+    if (blockIdx.x / SWR_LP_PARTS >= min(g.tiles.counts[0], g.tiles.heavy_cap)) return;
+    const uint2 done = lp_heavy_rows<PS>(g, __ldg(g.tiles.heavy + blockIdx.x / SWR_LP_PARTS),
+                                         (int)(blockIdx.x % SWR_LP_PARTS) * LpHeavy::PART, sh);
+    report(done.x, done.y);
+    return;
+  }
+  if (!swr_listed_tile(g.tiles, blockIdx.x - nheavy, entry)) return;
   const uint32_t tile = entry.x, b = entry.y, e = entry.z;
   const uint32_t* cells = g.tiles.start + (size_t)tile * SWR_SEGS;
   const SwrDrawDesc& D = g.draws[0];
@@ -457,21 +617,6 @@ __global__ void __launch_bounds__(256) k_lp_raster(LpRasterArgs g) {
   typename PS::State st;
   if (in) PS::load(st, x, y, U);
   if (tid <= SWR_SEGS) scs[tid] = (tid < SWR_SEGS ? cells[tid] : e) - b;
-  // Rasterizer::pixelDataFromVertex (Rasterizer.h:161-173) of step j of primitive `prim`
-  auto pixel = [&](uint32_t prim, int j, int fx, int fy, GpuPixel<PS>& pd) {
-    const float* rec = g.recs + (size_t)prim * W;
-    pd.x = fx;
-    pd.y = fy;
-    pd.eq = nullptr;  // points and lines carry no triangle equations
-    pd.z = 0.0f;
-    if (PS::InterpolateZ) pd.z = lp_value<PS>(rec, 2, j);
-    if (PS::InterpolateW) {
-      pd.w = lp_value<PS>(rec, 3, j);
-      pd.invw = swr_div(1.0f, pd.w);
-    }
-    for (int a = 0; a < RL::NA; ++a) pd.avar[a] = lp_value<PS>(rec, 4 + a, j);
-    for (int a = 0; a < RL::NP; ++a) pd.pvar[a] = lp_value<PS>(rec, 4 + RL::NA + a, j);
-  };
   uint32_t frags = 0, passes = 0;
   const uint32_t total = e - b;
   __syncthreads();
@@ -490,7 +635,7 @@ __global__ void __launch_bounds__(256) k_lp_raster(LpRasterArgs g) {
       f = whole ? g.bin_raw[b + c0 + tid] : g.bin[b + c0 + tid];
       sraw[tid] = f;
     }
-    for (int w = 0; w < words; ++w) smask[w][tid] = 0u;
+    for (int w = 0; w < words; ++w) sh.mask[w][tid] = 0u;
     __syncthreads();
     if (tid < n) {
       const uint32_t prim = g.prims[f];
@@ -508,39 +653,21 @@ __global__ void __launch_bounds__(256) k_lp_raster(LpRasterArgs g) {
         k = r0;
         for (int i = r0; i < r1; ++i) k += sraw[i] < f;  // numbers are unique
       }
-      sprim[k] = prim;
-      if constexpr (kCompact) {
-        GpuPixel<PS> pd;
-        pixel(prim, j, x - tid % SWR_LP_TILE + pix % SWR_LP_TILE, y - tid / SWR_LP_TILE + pix / SWR_LP_TILE, pd);
-        sz[k] = pd.z;
-        sc[k] = PS::shade(pd, U);
-      } else {
-        GpuPixel<PS> pd;
-        pixel(prim, j, 0, 0, pd);
-        lp_words<PS>(pd, [&](int i, float& v) { spd[i * CH + k] = v; });
-      }
-      atomicOr(&smask[k >> 5][pix], 1u << (k & 31));
+      sh.put(k, g.recs + (size_t)prim * W, prim, j, x - tid % SWR_LP_TILE + pix % SWR_LP_TILE,
+             y - tid / SWR_LP_TILE + pix / SWR_LP_TILE, U);
+      atomicOr(&sh.mask[k >> 5][pix], 1u << (k & 31));
     }
     __syncthreads();
     c0 = c1;
     while (cell < SWR_SEGS && scs[cell + 1] <= c0) ++cell;
     if (!in) continue;
     for (int w = 0; w < words; ++w) {
-      uint32_t m = smask[w][tid];
+      uint32_t m = sh.mask[w][tid];
       while (m) {
         const int k = w * 32 + __ffs(m) - 1;
         m &= m - 1u;
         frags++;
-        if constexpr (kCompact) {
-          PS::apply(st, sz[k], sc[k], (int)sprim[k]);
-        } else {
-          GpuPixel<PS> pd;
-          pd.x = x;
-          pd.y = y;
-          pd.eq = nullptr;  // points and lines carry no triangle equations
-          lp_words<PS>(pd, [&](int i, float& v) { v = spd[i * CH + k]; });
-          PS::drawPixel(pd, (int)sprim[k], st, U);
-        }
+        sh.take(k, x, y, st, U);
       }
     }
   }
@@ -548,12 +675,7 @@ __global__ void __launch_bounds__(256) k_lp_raster(LpRasterArgs g) {
     PS::store(st, x, y, U);
     passes = st.writes;
   }
-  uint32_t tot, ptot;
-  swr_block_sum2(frags, passes, sfr, tot, ptot);
-  if (tid == 0 && tot) {
-    atomicAdd((unsigned long long*)&g.status_w[SWR_ST_SHADED_LO], (unsigned long long)tot);
-    atomicAdd((unsigned long long*)&g.status_w[SWR_ST_PASSES_LO], (unsigned long long)ptot);
-  }
+  report(frags, passes);
 }
 
 }  // namespace swr

@@ -59,7 +59,7 @@ const PsOps* ps_ops(int id);
 // these headers in the caller's unit, so the library checks that both sides agree on the
 // layout of every structure that crosses between them.
 #define SWR_PROGRAM_MAGIC 0x50525753u  // "SWRP"
-#define SWR_PROGRAM_ABI 6u             // bumped with any change to VsOps, PsOps or their argument structs
+#define SWR_PROGRAM_ABI 7u             // bumped with any change to VsOps, PsOps or their argument structs
 #define SWR_PROGRAM_VERTEX 1u
 #define SWR_PROGRAM_PIXEL 2u
 #define SWR_PROGRAM_SIZES 13           // entries of swr_program_layout()

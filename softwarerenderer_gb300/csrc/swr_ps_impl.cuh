@@ -92,7 +92,7 @@ void run_lp_frags(const LpFragArgs& a, cudaStream_t s) {
 
 template <class PS>
 void run_lp_raster(const LpRasterArgs& a, cudaStream_t s) {
-  if (a.tiles.ntiles) swr::launch(k_lp_raster<PS>, a.tiles.ntiles, 256, 0, s, a);
+  if (a.tiles.ntiles) swr::launch(k_lp_raster<PS>, SWR_LP_PARTS * a.tiles.heavy_cap + a.tiles.ntiles, 256, 0, s, a);
 }
 
 template <class PS>

@@ -1184,10 +1184,10 @@ __global__ void __launch_bounds__(256) k_fill_bins(const uint32_t* status, uint3
 // than 32M ids) is gone through in windows of what does, unless ranking 32 ids at a time takes
 // less (the windows' words cost their number, ranks the square of the ids): 100,000 lines of 300
 // steps over each other, 30M fragments, took 28 s a draw with every such cell ranked, 75 ms so.  Cells of
-// at most cell_min ids are left alone.
+// at most cell_min ids in tiles of at most all_min are left alone.
 static __global__ void __launch_bounds__(256) k_sort_tiles(const uint32_t* status, const SwrTiles tiles, int seg_shift,
-                                                           uint32_t bm_words, uint32_t cell_min, const uint32_t* in,
-                                                           uint32_t* out) {
+                                                           uint32_t bm_words, uint32_t cell_min, uint32_t all_min,
+                                                           const uint32_t* in, uint32_t* out) {
   swr_pdl_entry();
   extern __shared__ uint32_t smem_bm[];
   if (status[SWR_ST_FLAGS] & SWR_F_ANY_OVERFLOW) return;
@@ -1201,7 +1201,7 @@ static __global__ void __launch_bounds__(256) k_sort_tiles(const uint32_t* statu
     for (uint32_t c = wib; c < SWR_SEGS; c += nwarps) {  // (uniform per warp, like all below)
       const uint32_t s = cells[c], e = c + 1 < SWR_SEGS ? cells[c + 1] : entry.z;
       const uint32_t m = e > s ? e - s : 0u;
-      if (m == 0 || m <= cell_min) continue;
+      if (m == 0 || (m <= cell_min && entry.z - entry.y <= all_min)) continue;
       auto rank = [&]() {
         for (uint32_t i0 = 0; i0 < m; i0 += 32) {
           const uint32_t val = i0 + lane < m ? in[s + i0 + lane] : 0xffffffffu;

@@ -55,3 +55,19 @@ def test_lines_of_one_tile(gpu_lib, port, n):
 def test_lines_of_many_steps(gpu_lib, port, n):
     """Few lines of many fragments: fewer than 32 of them a warp, down to one."""
     _check(port, _scene(DrawMode.Line, n, -500, 3000, -400, 900, 1300, 500, n))
+
+
+@pytest.mark.parametrize("mode,n", [(DrawMode.Point, 4096), (DrawMode.Point, 4097), (DrawMode.Point, 9001),
+                                    (DrawMode.Line, 600), (DrawMode.Line, 4000)])
+def test_heavy_tiles(gpu_lib, port, mode, n):
+    """Tiles of around and above 4,096 fragments, rasterized by four CTAs of four rows each: one
+    whole tile, one at the target's right and lower edges, all fragments in one row and one pixel."""
+    _check(port, _scene(mode, n, 0, 16, 0, 16, 50, 37, n))
+    _check(port, _scene(mode, n, 46, 50, 33, 37, 50, 37, n))
+    _check(port, _scene(mode, n, 0, 16, 7.1, 7.9, 50, 37, n))
+    _check(port, _scene(mode, n, 5.1, 5.9, 9.1, 9.9, 50, 37, n))
+
+
+@pytest.mark.parametrize("mode,n", [(DrawMode.Point, 1000000), (DrawMode.Line, 20000)])
+def test_more_heavy_tiles_than_slots(gpu_lib, port, mode, n):
+    _check(port, _scene(mode, n, 0, 200, 0, 200, 200, 200, n))
