@@ -104,7 +104,7 @@ static_assert(SWR_SEGS == 32 && kThreads == 256, "a group of 32 tiles is a 32 x 
 
 __global__ void __launch_bounds__(kThreads) k_cells(const CellsArgs a) {
   swr_pdl_entry();
-  __shared__ unsigned long long tmp[32];
+  __shared__ uint32_t tmp[32];
   __shared__ uint32_t sq[kGroup][SWR_SEGS + 1];
   __shared__ uint32_t stot[kGroup], sfirst[kGroup];
   __shared__ uint32_t sbase;
@@ -133,9 +133,12 @@ __global__ void __launch_bounds__(kThreads) k_cells(const CellsArgs a) {
   uint32_t tile_tot = s;  // the tile's entries: over its eight lanes
 #pragma unroll
   for (int o = 1; o < 8; o <<= 1) tile_tot += __shfl_xor_sync(0xffffffffu, tile_tot, o);
-  unsigned long long tot;
-  // (its barriers order the reads of sq above)
-  uint32_t ex = (uint32_t)swr_block_exscan((unsigned long long)s, tmp, &tot);
+  if (sg == 0) stot[tl] = tile_tot;
+  uint32_t ex = swr_block_exscan(s, tmp);  // (its barriers order the reads of sq above and publish stot)
+  const uint32_t n = stot[lane];  // one tile per lane
+  // the block's entries, in 64 bits: a 64-bit scan was half a microsecond of a small draw's chain
+  const unsigned long long tot = ((unsigned long long)__reduce_add_sync(0xffffffffu, n >> 16) << 16) +
+                                 __reduce_add_sync(0xffffffffu, n & 0xffffu);
   if (tot == 0) return;  // uniform
   if (threadIdx.x == 0) {
     sbase = atomicAdd(a.total, (uint32_t)tot);
@@ -146,10 +149,7 @@ __global__ void __launch_bounds__(kThreads) k_cells(const CellsArgs a) {
       a.status[SWR_ST_STICKY + SWR_ST_PAIRS] = SWR_COUNT_MAX;
     }
   }
-  if (sg == 0) {
-    stot[tl] = tile_tot;
-    sfirst[tl] = ex;
-  }
+  if (sg == 0) sfirst[tl] = ex;
   __syncthreads();
   ex += sbase;
   uint4 o;
@@ -158,8 +158,8 @@ __global__ void __launch_bounds__(kThreads) k_cells(const CellsArgs a) {
   o.z = o.y + v[1];
   o.w = o.z + v[2];
   if (tile_tot) *(uint4*)(a.t.start + (size_t)(t0 + tl) * SWR_SEGS + sg) = o;
-  if (warp == 0) {  // one tile per lane
-    const uint32_t n = stot[lane], t = t0 + lane, below = (1u << lane) - 1u, b = sfirst[lane] + sbase;
+  if (warp == 0) {
+    const uint32_t t = t0 + lane, below = (1u << lane) - 1u, b = sfirst[lane] + sbase;
     uint4 entry = make_uint4(t, b, b + n, 0u);
     if (n && a.ntargets > 1) entry.w = (uint32_t)swr_find_le(a.target_tile_base, a.ntargets, t);
     auto append = [&](bool on, uint32_t* counter) -> uint32_t {
