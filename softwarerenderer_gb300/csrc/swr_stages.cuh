@@ -2383,6 +2383,8 @@ __global__ void __launch_bounds__(NT, SWR_RASTER_MINB ? SWR_RASTER_MINB
 // (four, with all the registers wanted: 354 us a draw, five 333).  The 40,960 triangles of the
 // reference's Benchmark program (640x480, 240M fragments): bins ordered and walked in
 // 64-primitive chunks pixel by pixel, 1888 us a draw; this way 333.
+//
+// MASKS: some draw is in Block or Adaptive mode.
 template <class PS, int TILE, bool DIRECT, bool MASKS>
 __global__ void __launch_bounds__(256, 5) k_overwrite(RasterArgs g) {
   swr_pdl_entry();
@@ -2479,7 +2481,7 @@ __global__ void __launch_bounds__(256, 5) k_overwrite(RasterArgs g) {
                 [&](int y, int xa, int xb, int) { run(y, xa, xb); });
       return;
     }
-    if (span_only) return;
+    if (span_only || (!MASKS && !DIRECT)) return;  // (without MASKS a binned draw has no Block primitives)
     const float r[15] = {0, 0, 0, 0, 0, 0, q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, q3.x, q3.y, q3.z};
     constexpr int ROWS = SWR_BLOCK * NB;  // the blocks' rows, block by block
     for (int h = part * (ROWS >> lp), he = h + (ROWS >> lp); h < he;) {
