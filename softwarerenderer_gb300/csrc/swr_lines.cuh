@@ -11,10 +11,11 @@
 //                                per-step scissor test, the pixel; counts (tile, segment) cells
 //   k_lp_fill                    fragment numbers into their tile's bin (the triangles' cells:
 //                                a tile's fragments in SWR_SEGS runs of fragment numbers);
-//                                k_sort_tiles orders cells above SWR_LP_CHUNK entries, the
-//                                tile's CTA the others
-//   k_lp_raster                  one CTA per 16 x 16 tile: each thread owns a pixel and applies
-//                                its fragments in order (a line may hit a pixel twice)
+//                                k_sort_tiles orders cells above SWR_LP_CHUNK entries and all
+//                                cells of heavy tiles, the tile's CTA the others
+//   k_lp_raster                  one CTA per 16 x 16 tile, four per heavy one: each thread owns a
+//                                pixel and applies its fragments in order (a line may hit a
+//                                pixel twice)
 //
 // Binning by tile took the place of a stable radix sort of all fragments by pixel (three
 // 8-bit passes of three kernels, then one thread per covered pixel searching each fragment's
@@ -391,6 +392,7 @@ struct LpRasterArgs {
   SwrTiles tiles;              // the tiles with fragments, their bins and cells
   const uint32_t* bin_raw;     // fragment numbers, unordered inside a cell
   const uint32_t* bin;         // ordered by k_sort_tiles, for cells of more than SWR_LP_CHUNK entries
+                               // and all cells of tiles of more than SWR_LP_HEAVY
   const SwrDrawDesc* draws;
   const SwrTargetDesc* targets;
   uint32_t* status_w;
@@ -563,7 +565,8 @@ struct LpChunk {
   }
 };
 
-// One CTA per 16 x 16 tile, one pixel per thread.  A chunk is as many whole cells of the
+// One CTA per listed 16 x 16 tile, one pixel per thread (the first SWR_LP_PARTS * heavy_cap CTAs take
+// the heavy tiles' rows: lp_heavy_rows).  A chunk is as many whole cells of the
 // tile's bin as hold at most 256 fragments (a larger cell, ordered by k_sort_tiles, is a run of
 // chunks by itself): one fragment per thread is ranked inside its cell, interpolated, shaded
 // and marked under its rank in its pixel's set; then each thread applies its pixel's
